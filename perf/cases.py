@@ -251,3 +251,97 @@ def tolerance(case):
     if case.get("dtype") == "fp16":
         return {"rel": 1e-3, "max": 4e-3}
     return {"rel": 1e-2, "max": 0.16} if case.get("backward") else {"rel": 8.5e-3, "max": 0.08}
+
+
+def exact(case, seed):
+    """What run() returns for these inputs, in 64 bits and plain torch."""
+    kind = case["kind"]
+    if kind == "cache_write":
+        return None                          # bytes, compared bit for bit
+    st = prepare(case, seed)
+    with torch.no_grad():
+        return dict(decode=_exact_decode, sparse_decode=_exact_sparse_decode, sparse_prefill=_exact_sparse_prefill,
+                    mha=_exact_mha)[kind](st)
+
+
+def _attend(q, k, v, scale, visible=None):
+    """softmax(scale q k^T) v over the visible keys, its natural log-sum-exp and its largest scaled logit."""
+    s = (q @ k.transpose(-1, -2)) * scale
+    if visible is not None:
+        s.masked_fill_(~visible, -math.inf)
+    lse = torch.logsumexp(s, dim=-1)
+    top = s.amax(dim=-1)
+    return torch.exp_(s.sub_(lse.unsqueeze(-1))) @ v, lse, top
+
+
+def _exact_decode(st):
+    case = st["case"]
+    b, s_q, h = case["b"], case["s_q"], case["h_q"]
+    out = torch.empty((b, s_q, h, DV), dtype=torch.float64, device=DEV)
+    lse = torch.empty((b, h, s_q), dtype=torch.float64, device=DEV)
+    for i, n in enumerate(st["lens"].tolist()):
+        k = st["cache"][st["table"][i, :(n + PAGE - 1) // PAGE].long()].reshape(-1, D)[:n].double()
+        for t in range(s_q):
+            seen = n - (s_q - 1 - t) if case["causal"] else n
+            out[i, t], lse[i, :, t], _ = _attend(st["q"][i, t].double(), k[:seen], k[:seen, :DV], D ** -0.5)
+    return out, lse
+
+
+def _exact_sparse_decode(st):
+    case = st["case"]
+    b, s_q, h = case["b"], case["s_q"], case["h_q"]
+    records = st["cache"].view(torch.uint8).view(-1, 656)
+    out = torch.empty((b, s_q, h, DV), dtype=torch.float64, device=DEV)
+    lse = torch.empty((b, h, s_q), dtype=torch.float64, device=DEV)
+    for i in range(b):
+        slots = st["indices"][i].long()
+        rec = records[slots.clamp(min=0)]                                          # [s_q, topk, 656]
+        nope = rec[..., :DV].contiguous().view(torch.float8_e4m3fn).float().unflatten(-1, (4, 128))
+        nope = (nope * rec[..., 512:528].contiguous().view(torch.float32).unsqueeze(-1)).to(torch.bfloat16).flatten(-2)
+        k = torch.cat([nope, rec[..., 528:].contiguous().view(torch.bfloat16)], dim=-1).double()
+        out[i], l, _ = _attend(st["q"][i].double(), k, k[..., :DV], D ** -0.5, (slots >= 0).unsqueeze(1))
+        lse[i] = l.transpose(0, 1)
+    return out, lse
+
+
+def _exact_sparse_prefill(st):
+    s_q, h = st["case"]["s_q"], st["case"]["h_q"]
+    out = torch.empty((s_q, h, DV), dtype=torch.float64, device=DEV)
+    top = torch.empty((s_q, h), dtype=torch.float64, device=DEV)
+    lse = torch.empty((s_q, h), dtype=torch.float64, device=DEV)
+    kv = st["kv"].view(-1, D)
+    for t0 in range(0, s_q, 128):
+        t = slice(t0, min(t0 + 128, s_q))
+        idx = st["indices"][t, 0].long()
+        k = kv[idx.clamp(min=0)].double()
+        out[t], l, m = _attend(st["q"][t].double(), k, k[..., :DV], D ** -0.5, (idx >= 0).unsqueeze(1))
+        top[t], lse[t] = m / math.log(2), l / math.log(2)                          # base 2
+    return out, top, lse
+
+
+def _exact_mha(st):
+    case = st["case"]
+    q, k, v, d_out = st["q"].detach(), st["k"].detach(), st["v"].detach(), st.get("d_out")
+    scale, group, lens = case["d_qk"] ** -0.5, case["h_q"] // case["h_k"], _lens(case)
+    out = torch.empty((*q.shape[:2], 128), dtype=torch.float64, device=DEV)
+    lse = torch.empty(q.shape[:2], dtype=torch.float64, device=DEV)
+    dq, dk, dv = (torch.empty(x.shape, dtype=torch.float64, device=DEV) for x in (q, k, v))
+    at = 0
+    for n in lens:
+        rows = slice(at, at + n)
+        at += n
+        visible = torch.ones((n, n), dtype=torch.bool, device=DEV).tril_() if case["causal"] else None
+        for h in range(case["h_q"]):
+            qh, kh, vh = q[rows, h].double(), k[rows, h // group].double(), v[rows, h // group].double()
+            out[rows, h], lse[rows, h], _ = _attend(qh, kh, vh, scale, visible)
+            if d_out is None:
+                continue
+            s = (qh @ kh.T).mul_(scale)
+            if visible is not None:
+                s.masked_fill_(~visible, -math.inf)
+            p = s.sub_(lse[rows, h].unsqueeze(1)).exp_()
+            g = d_out[rows, h].double()
+            dv[rows, h] = p.T @ g
+            ds = (g @ vh.T).sub_((g * out[rows, h]).sum(1, keepdim=True)).mul_(p)
+            dq[rows, h], dk[rows, h] = (ds @ kh) * scale, (ds.T @ qh) * scale
+    return (out, lse) if d_out is None else (out, lse, dq, dk, dv)
