@@ -6,6 +6,7 @@ package fails; there is no Python / torch fallback.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -115,7 +116,23 @@ def _load() -> C.CDLL:
     return lib
 
 
+def _load_native():
+    """The native marshalling module (csrc/torch_binding.cpp), which links against the library loaded above."""
+    path = os.path.join(os.path.dirname(LIB_PATH), "_fmla_torch.so")
+    if not os.path.exists(path):
+        raise ImportError(
+            f"{path} is missing: build it with `python flashmla_windows_linux_sm120_b200/build.py`. "
+            "There is no fallback path.")
+    import torch  # noqa: F401  its libraries have to be loaded first
+
+    spec = importlib.util.spec_from_file_location("_fmla_torch", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
 lib = _load()
+native = _load_native()
 
 
 def check(status: int) -> None:

@@ -1,23 +1,27 @@
 """In-tree build of the C-ABI library: nvcc, sm_100a only.
 
 ``python flashmla_windows_linux_sm120_b200/build.py`` (run as a script, so that a stale library cannot block its own rebuild) compiles
-``csrc/*.cu`` into ``flashmla_windows_linux_sm120_b200/lib/libflashmla_b200.so``.
+``csrc/*.cu`` into ``flashmla_windows_linux_sm120_b200/lib/libflashmla_b200.so`` and the torch marshalling module
+``csrc/torch_binding.cpp`` into ``lib/_fmla_torch.so``, which finds the library beside it.
 Objects are rebuilt only when a source or header is newer.
 """
 from __future__ import annotations
 
 import concurrent.futures
 import glob
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_DIR = os.path.join(PKG_DIR, "lib")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(LIB_DIR, "libflashmla_b200.so")
+BINDING_PATH = os.path.join(LIB_DIR, "_fmla_torch.so")
 INCLUDE_DIR = os.path.join(os.path.dirname(PKG_DIR), "include")
 
 NVCC_FLAGS = [
@@ -74,7 +78,27 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    _build_binding(force)
     return LIB_PATH
+
+
+def _build_binding(force: bool) -> None:
+    src = os.path.join(CSRC, "torch_binding.cpp")
+    header = os.path.join(INCLUDE_DIR, "flashmla_b200.h")
+    if not force and os.path.exists(BINDING_PATH) and os.path.getmtime(BINDING_PATH) >= _newest([src, header]):
+        return
+    # torch is located, not imported: importing it takes longer than this compilation
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    cuda_home = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", src, "-o", BINDING_PATH,
+           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(torch_dir, "include"),
+           "-I", os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+           "-I", os.path.join(cuda_home, "include"),
+           "-L", os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+           "-L", LIB_DIR, "-l:libflashmla_b200.so", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"building {BINDING_PATH} failed:\n{r.stdout}\n{r.stderr}")
 
 
 if __name__ == "__main__":

@@ -2,7 +2,8 @@
 positional signatures and return conventions as the module csrc/pybind.cpp
 builds in the reference (:870-911), implemented as a thin marshalling layer
 over the C ABI.  Tensors are allocated with torch (device memory, streams);
-everything else happens inside libflashmla_b200.so.
+everything else happens inside libflashmla_b200.so.  The calls of a decode step
+are marshalled natively (csrc/torch_binding.cpp), the dense ones here.
 """
 from __future__ import annotations
 
@@ -13,10 +14,9 @@ from typing import List, Optional
 import torch
 
 from . import _cabi
-from ._cabi import DecodeParams, DenseParams, SparsePrefillParams, check, lib
+from ._cabi import DenseParams, check, lib, native as _native
 
 __flash_mla_variant__ = lib.fmla_variant().decode()
-TILE_SCHEDULER_METADATA_SIZE = 8
 
 
 def _stream(t: torch.Tensor) -> int:
@@ -52,22 +52,9 @@ def get_mla_decoding_metadata(seqlens_k: torch.Tensor, num_q_tokens_per_head_k: 
                               h_q: Optional[int] = None, is_fp8_kvcache: bool = False,
                               topk: Optional[int] = None) -> List[torch.Tensor]:
     """csrc/pybind.cpp:383-428.  Returns [tile_scheduler_metadata int32[num_sm_parts, 8], num_splits int32[b+1]]."""
-    is_sparse = topk is not None
-    _cuda(seqlens_k, "seqlens_k")
-    _require(seqlens_k.is_contiguous(), "seqlens_k must be contiguous")
-    _require(seqlens_k.dtype == torch.int32, "seqlens_k must have dtype int32")
-    if is_sparse:
-        _require(h_q is not None, "num_heads_q must be provided when topk is provided")
-    n = C.c_int(0)
-    check(lib.fmla_get_num_sm_parts(seqlens_k.device.index or 0, int(num_q_tokens_per_head_k), int(h_k),
-                                    int(h_q) if h_q is not None else 0, int(bool(is_fp8_kvcache)), int(is_sparse),
-                                    C.byref(n)))
-    b = seqlens_k.shape[0]
-    with torch.cuda.device(seqlens_k.device):
-        md = torch.empty((n.value, TILE_SCHEDULER_METADATA_SIZE), dtype=torch.int32, device=seqlens_k.device)
-        ns = torch.empty((b + 1,), dtype=torch.int32, device=seqlens_k.device)
-        check(lib.fmla_get_mla_metadata(seqlens_k.data_ptr(), b, n.value, int(topk) if is_sparse else -1,
-                                        md.data_ptr(), ns.data_ptr(), _stream(seqlens_k)))
+    md, ns, whole = _native.metadata(seqlens_k, num_q_tokens_per_head_k, h_k, h_q, is_fp8_kvcache, topk)
+    if whole is not None and not ns.is_inference():
+        ns._fmla_no_split, ns._fmla_no_split_version = whole, ns._version
     return [md, ns]
 
 
@@ -83,129 +70,33 @@ def fwd_kvcache_mla(q: torch.Tensor, kcache: torch.Tensor, head_size_v: int, seq
     partial of a split request merges it (one kernel per step) instead of a second, dependent-launched merge kernel.
     Default: the environment variable FMLA_MERGE_IN_KERNEL=1, else off (the inline merge stalls the pipeline of the
     merging CTA for longer than the separate kernel takes)."""
-    sparse = indices is not None
-    _require(q.dtype in (torch.bfloat16, torch.float16), "q must be bfloat16 or float16")
-    if not is_fp8:
-        _require(kcache.dtype == q.dtype, "query and key must have the same dtype")
-    else:
-        _require(kcache.dtype in (torch.float8_e4m3fn, torch.int8, torch.uint8),
-                 "key must have dtype fp8_e4m3fn or int8 or uint8")
-    _require(seqlens_k.dtype == torch.int32, "seqlens_k must have dtype int32")
-    _require(block_table.dtype == torch.int32, "block_table must have dtype torch.int32")
-    _require(tile_scheduler_metadata.dtype == torch.int32, "tile_scheduler_metadata must have dtype int32")
-    _require(num_splits.dtype == torch.int32, "num_splits must have dtype int32")
-    _require(not sparse or indices.dtype == torch.int32, "indices must have dtype int32")
-    for t, n in ((q, "q"), (kcache, "kcache"), (seqlens_k, "seqlens_k"), (block_table, "block_table"),
-                 (tile_scheduler_metadata, "tile_scheduler_metadata"), (num_splits, "num_splits")):
-        _cuda(t, n)
-    if sparse:
-        _cuda(indices, "indices")
-    _require(q.dim() == 4 and kcache.dim() == 4, "q and kcache must be 4-D")
-    _require(q.stride(-1) == 1, "q must have contiguous last dimension")
-    _require(kcache.stride(-1) == 1, "kcache must have contiguous last dimension")
-    _require(seqlens_k.is_contiguous(), "seqlens_k must be contiguous")
-    _require(block_table.stride(-1) == 1, "block_table must have contiguous last dimension")
-    _require(tile_scheduler_metadata.is_contiguous() and num_splits.is_contiguous(),
-             "tile_scheduler_metadata and num_splits must be contiguous")
-    _require(not sparse or indices.stride(-1) == 1, "indices must have contiguous last dimension")
-
-    b, s_q, h_q, d = q.shape
-    num_blocks, page, h_k, last = kcache.shape
-    _require(tile_scheduler_metadata.dim() == 2 and tile_scheduler_metadata.shape[1] == TILE_SCHEDULER_METADATA_SIZE,
-             "tile_scheduler_metadata must be [num_sm_parts, 8]")
-    _require(tuple(seqlens_k.shape) == (b,), "seqlens_k must be [batch]")
-    _require(tuple(num_splits.shape) == (b + 1,), "num_splits must be [batch + 1]")
-    _require(block_table.dim() == 2 and block_table.shape[0] == b, "block_table must be [batch, max_blocks]")
-    if is_fp8:
-        _require(last == 656, "FP8 kcache must have 656 bytes per token")
-    else:
-        _require(last == d, "kcache head dim must equal q head dim")
-    topk = -1
-    if sparse:
-        _require(indices.dim() == 3 and indices.shape[0] == b and indices.shape[1] == s_q, "indices must be [b, s_q, topk]")
-        topk = indices.shape[2]
-    if q.dtype == torch.float16 and (sparse or is_fp8):
-        raise RuntimeError("flashmla_b200: unsupported configuration: float16 queries are supported for the dense "
-                           "(float16 cache) decode only")
-
-    num_sm_parts = tile_scheduler_metadata.shape[0]
-    with torch.cuda.device(q.device):
-        out = torch.empty((b, s_q, h_q, head_size_v), dtype=q.dtype, device=q.device)
-        lse = torch.empty((b, h_q, s_q), dtype=torch.float32, device=q.device)
-        slots = b + num_sm_parts
-        lse_accum = torch.empty((slots, s_q * h_q), dtype=torch.float32, device=q.device)
-        o_accum = torch.empty((slots, s_q * h_q, head_size_v), dtype=torch.float32, device=q.device)
-        p = DecodeParams()
-        p.b, p.s_q, p.h_q, p.h_k, p.d, p.d_v = b, s_q, h_q, h_k, d, int(head_size_v)
-        p.num_blocks, p.page_block_size = num_blocks, page
-        p.is_causal, p.is_fp8, p.topk = int(bool(is_causal)), int(bool(is_fp8)), topk
-        p.q_dtype = 1 if q.dtype == torch.float16 else 0
-        p.softmax_scale = float(softmax_scale)
-        p.q, p.q_stride_b, p.q_stride_s, p.q_stride_h = q.data_ptr(), q.stride(0), q.stride(1), q.stride(2)
-        p.kcache = kcache.data_ptr()
-        p.k_stride_block, p.k_stride_row, p.k_stride_head = kcache.stride(0), kcache.stride(1), kcache.stride(2)
-        p.block_table, p.block_table_stride_b = block_table.data_ptr(), block_table.stride(0)
-        p.seqlens_k = seqlens_k.data_ptr()
-        if sparse:
-            p.indices, p.indices_stride_b, p.indices_stride_s = indices.data_ptr(), indices.stride(0), indices.stride(1)
-            p.indices_logical = int(bool(indices_logical))
-        p.tile_scheduler_metadata, p.num_sm_parts = tile_scheduler_metadata.data_ptr(), num_sm_parts
-        p.num_splits = num_splits.data_ptr()
-        p.out, p.o_stride_b, p.o_stride_s, p.o_stride_h = out.data_ptr(), out.stride(0), out.stride(1), out.stride(2)
-        p.softmax_lse, p.lse_accum, p.o_accum = lse.data_ptr(), lse_accum.data_ptr(), o_accum.data_ptr()
-        if merge_in_kernel is None:
-            merge_in_kernel = _MERGE_IN_KERNEL_DEFAULT
-        if merge_in_kernel and not sparse and (h_q // h_k) % 128 == 0:
-            p.arrival_counters = _counters_for(q, b * s_q * (h_q // 64)).data_ptr()
-        p.no_split_hint = int(_no_request_is_split(num_splits, b))
-        if profile_events is not None:
-            p.profile_event_begin = profile_events[0].cuda_event
-            p.profile_event_end = profile_events[1].cuda_event
-        check(lib.fmla_fwd_kvcache_mla(C.byref(p), _stream(q)))
-    return [out, lse]
+    counters = 0
+    if merge_in_kernel is None:
+        merge_in_kernel = _MERGE_IN_KERNEL_DEFAULT
+    if merge_in_kernel and indices is None and q.dim() == 4 and kcache.dim() == 4:
+        b, s_q, h_q, _ = q.shape
+        if q.is_cuda and (h_q // kcache.shape[2]) % 128 == 0:
+            counters = _counters_for(q, b * s_q * (h_q // 64)).data_ptr()
+    begin, end = (e.cuda_event for e in profile_events) if profile_events is not None else (0, 0)
+    return _native.decode(q, kcache, head_size_v, seqlens_k, block_table, softmax_scale, is_causal,
+                          tile_scheduler_metadata, num_splits, is_fp8, indices, begin, end, indices_logical, counters,
+                          _no_request_is_split(num_splits))
 
 
-def _no_request_is_split(num_splits: torch.Tensor, b: int) -> bool:
-    """True when the schedule gives every request to one partition (num_splits[b] == b): the merge kernel is then
-    not launched.  Read back from the device once per metadata tensor (one synchronisation, remembered on the
-    tensor object; a decode step reuses its metadata for every layer); unknown -- and therefore False -- while the
-    stream is being captured into a CUDA graph before that first read."""
-    known = getattr(num_splits, "_fmla_no_split", None)
-    if known is None:
-        if torch.cuda.is_current_stream_capturing():
-            return False
-        known = bool(int(num_splits[b].item()) == b)
-        num_splits._fmla_no_split = known
-    return known
+def _no_request_is_split(num_splits: torch.Tensor) -> bool:
+    """True when the schedule is known to give every request to one partition: the merge kernel is then not launched.
+    A sparse schedule is a function of numbers the host has (batch, topk, partitions), so get_mla_decoding_metadata
+    says so on the tensor it returns; an in-place write to that tensor withdraws it.  The lengths of a dense batch are
+    on the device, and reading the outcome back costs a synchronisation per plan (40 us against the 2 us of a merge
+    kernel that finds nothing to do): it counts as not known."""
+    known = getattr(num_splits, "_fmla_no_split", False)
+    return known and getattr(num_splits, "_fmla_no_split_version", None) in (None, num_splits._version)
 
 
 def sparse_prefill_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor, sm_scale: float,
                        d_v: int = 512) -> List[torch.Tensor]:
     """csrc/pybind.cpp:730-814.  Returns [out bf16 [s_q,h_q,d_v], max_logits fp32 [s_q,h_q], lse fp32 [s_q,h_q]]."""
-    for t, n in ((q, "q"), (kv, "kv"), (indices, "indices")):
-        _cuda(t, n)
-    _require(q.dtype == torch.bfloat16 and kv.dtype == torch.bfloat16, "q and kv must be bfloat16")
-    _require(indices.dtype == torch.int32, "indices must be int32")
-    _require(q.dim() == 3 and kv.dim() == 3 and indices.dim() == 3, "q, kv, indices must be 3-D")
-    _require(q.stride(-1) == 1 and kv.stride(-1) == 1 and indices.stride(-1) == 1, "last dimensions must be contiguous")
-    s_q, h_q, d_qk = q.shape
-    s_kv, h_kv, _ = kv.shape
-    topk = indices.shape[2]
-    _require(kv.shape[2] == d_qk, "q and kv head dims differ")
-    _require(tuple(indices.shape[:2]) == (s_q, h_kv), "indices must be [s_q, h_kv, topk]")
-    with torch.cuda.device(q.device):
-        out = torch.empty((s_q, h_q, d_v), dtype=torch.bfloat16, device=q.device)
-        mx = torch.empty((s_q, h_q), dtype=torch.float32, device=q.device)
-        lse = torch.empty((s_q, h_q), dtype=torch.float32, device=q.device)
-        p = SparsePrefillParams()
-        p.s_q, p.s_kv, p.h_q, p.h_kv, p.d_qk, p.d_v, p.topk = s_q, s_kv, h_q, h_kv, d_qk, int(d_v), topk
-        p.sm_scale = float(sm_scale)
-        p.q, p.q_stride_s, p.q_stride_h = q.data_ptr(), q.stride(0), q.stride(1)
-        p.kv, p.kv_stride_s, p.kv_stride_h = kv.data_ptr(), kv.stride(0), kv.stride(1)
-        p.indices, p.indices_stride_s, p.indices_stride_h = indices.data_ptr(), indices.stride(0), indices.stride(1)
-        p.out, p.max_logits, p.lse = out.data_ptr(), mx.data_ptr(), lse.data_ptr()
-        check(lib.fmla_sparse_prefill_fwd(C.byref(p), _stream(q)))
-    return [out, mx, lse]
+    return _native.sparse_prefill(q, kv, indices, sm_scale, d_v)
 
 
 def _dense_params(q, k, v, cu_q, cu_k, o, lse, mask_mode_code, softmax_scale, max_q, max_k) -> DenseParams:
@@ -294,19 +185,4 @@ def quantize_kv_fp8(kv: torch.Tensor, cache: Optional[torch.Tensor] = None,
                     dst_slots: Optional[torch.Tensor] = None) -> torch.Tensor:
     """bf16 [n, 576] (or [num_blocks, 64, 1, 576]) -> FP8 records.  Without `cache` a fresh
     [*, 656] float8_e4m3fn tensor of the same leading shape is returned."""
-    _require(kv.is_cuda and kv.dtype == torch.bfloat16 and kv.shape[-1] == 576, "kv must be CUDA bf16 [..., 576]")
-    lead = kv.shape[:-1]
-    flat = kv.reshape(-1, 576)
-    _require(flat.stride(-1) == 1, "kv rows must be contiguous")
-    with torch.cuda.device(kv.device):
-        if cache is None:
-            cache = torch.empty((*lead, 656), dtype=torch.float8_e4m3fn, device=kv.device)
-        cflat = cache.view(torch.uint8).reshape(-1, 656)
-        slots_ptr = None
-        if dst_slots is not None:
-            _require(dst_slots.is_cuda and dst_slots.dtype == torch.int32 and dst_slots.is_contiguous(),
-                     "dst_slots must be a contiguous CUDA int32 tensor")
-            slots_ptr = dst_slots.data_ptr()
-        check(lib.fmla_quantize_kv_fp8(flat.data_ptr(), flat.stride(0), flat.shape[0], slots_ptr, cflat.data_ptr(),
-                                       cflat.stride(0), _stream(kv)))
-    return cache
+    return _native.quantize(kv, cache, dst_slots)
