@@ -88,7 +88,8 @@ void ensure_status_mirror(int dev) {
     return;
   }
   int* w = static_cast<int*>(dptr);
-  if (fmla::set_status_mirror_mla(w) != cudaSuccess || fmla::set_status_mirror_pair(w) != cudaSuccess ||
+  if (fmla::set_status_mirror_prefill64(w) != cudaSuccess || fmla::set_status_mirror_pair(w) != cudaSuccess ||
+      fmla::set_status_mirror_few_rows(w) != cudaSuccess ||
       fmla::set_status_mirror_merge(w) != cudaSuccess ||
       fmla::set_status_mirror_dense_fwd(w) != cudaSuccess || fmla::set_status_mirror_dense_bwd(w) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -404,12 +405,16 @@ int fmla_dense_prefill_bwd(const fmla_dense_params* P, void* stream) {
 
 int fmla_device_status(int* status_host, int reset) {
   FMLA_REQUIRE(status_host != nullptr, "status_host is null");
-  cudaError_t e = fmla::read_decode_tc_status(status_host, reset != 0);
+  cudaError_t e = fmla::read_decode_pair_status(status_host, reset != 0);
   if (e != cudaSuccess) return cuda_fail(e, "reading the device status word");
-  int pair_status = 0;
-  e = fmla::read_decode_pair_status(&pair_status, reset != 0);
+  int other_status = 0;
+  e = fmla::read_prefill64_status(&other_status, reset != 0);
   if (e != cudaSuccess) return cuda_fail(e, "reading the device status word");
-  if (*status_host == 0) *status_host = pair_status;
+  if (*status_host == 0) *status_host = other_status;
+  int few_status = 0;
+  e = fmla::read_decode_few_rows_status(&few_status, reset != 0);
+  if (e != cudaSuccess) return cuda_fail(e, "reading the device status word");
+  if (*status_host == 0) *status_host = few_status;
   int merge_status = 0;
   e = fmla::read_merge_status(&merge_status, reset != 0);
   if (e != cudaSuccess) return cuda_fail(e, "reading the device status word");

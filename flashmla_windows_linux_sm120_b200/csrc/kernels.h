@@ -65,6 +65,7 @@ struct SparsePrefillKernelParams {
 struct DenseKernelParams {
   int batch, h_q, h_k, d_qk, d_v, max_seqlen_q, max_seqlen_k, is_causal;
   int total_q, total_k;
+  int tiles_outer;             // forward: order of the CTAs (launch_fwd_tc)
   float scale, scale_log2;
   const void* q; int64_t q_stride_t, q_stride_h;
   const void* k; int64_t k_stride_t, k_stride_h;
@@ -86,7 +87,6 @@ int set_error(int code, const char* message);
 
 // Each kernel translation unit keeps a pointer to a host-mapped status word beside its device status word
 // (tc_common.cuh); these set it for the current device.
-cudaError_t set_status_mirror_mla(int* mapped_host_word);
 cudaError_t set_status_mirror_pair(int* mapped_host_word);
 cudaError_t set_status_mirror_merge(int* mapped_host_word);
 cudaError_t set_status_mirror_dense_fwd(int* mapped_host_word);
@@ -94,12 +94,11 @@ cudaError_t set_status_mirror_dense_bwd(int* mapped_host_word);
 
 cudaError_t launch_get_mla_metadata(const int* seqlens_k, int batch, int num_sm_parts, int topk, int* md,
                                     int* num_splits, cudaStream_t stream);
-// tcgen05 / TMA / TMEM kernels (mla_tc.cu): dense decode, sparse FP8 decode, sparse prefill
+// dense decode, sparse FP8 decode, sparse prefill: the kernel is chosen in mla_dispatch.cu
 cudaError_t launch_decode_dense_tc(const DecodeKernelParams& p, cudaStream_t stream);
 cudaError_t launch_decode_sparse_tc(const DecodeKernelParams& p, cudaStream_t stream);
 cudaError_t launch_sparse_prefill_tc(const SparsePrefillKernelParams& p, cudaStream_t stream);
-// reads (and optionally clears) the status word the tcgen05 kernels set when a bounded wait expires
-cudaError_t read_decode_tc_status(int* host_status, bool reset);
+// read_*_status: reads (and optionally clears) the status word a kernel sets when a bounded wait expires
 // dense decode as a CTA pair (mla_pair.cu): 128 heads per pair, tcgen05 cta_group::2; used by
 // launch_decode_dense_tc whenever the heads per kv head are a multiple of 128
 bool decode_dense_pair_applies(const DecodeKernelParams& p);
@@ -107,9 +106,18 @@ bool decode_dense_pair_applies(const DecodeKernelParams& p);
 bool decode_dense_merges_in_kernel(const DecodeKernelParams& p);
 cudaError_t launch_decode_dense_pair(const DecodeKernelParams& p, cudaStream_t stream);
 cudaError_t read_decode_pair_status(int* host_status, bool reset);
-// sparse prefill forward as CTA pairs with TMA row gathers (mla_pair.cu); used by launch_sparse_prefill_tc for 128 heads
+// at most 64 query rows per CTA (mla_few_rows.cu): every head count the pair kernel does not take
+cudaError_t launch_decode_few_rows(const DecodeKernelParams& p, cudaStream_t stream);
+cudaError_t launch_decode_sparse_few_rows(const DecodeKernelParams& p, cudaStream_t stream);
+cudaError_t read_decode_few_rows_status(int* host_status, bool reset);
+cudaError_t set_status_mirror_few_rows(int* mapped_host_word);
+// sparse decode and sparse prefill as CTA pairs (mla_pair.cu): 128 heads
 bool decode_sparse_pair_applies(const DecodeKernelParams& p);
 cudaError_t launch_decode_sparse_pair(const DecodeKernelParams& p, cudaStream_t stream);
+// sparse prefill, one CTA per 64 heads (mla_prefill64.cu)
+cudaError_t launch_sparse_prefill_64(const SparsePrefillKernelParams& sp, cudaStream_t stream);
+cudaError_t read_prefill64_status(int* host_status, bool reset);
+cudaError_t set_status_mirror_prefill64(int* mapped_host_word);
 bool sparse_prefill_pair_applies(const SparsePrefillKernelParams& sp);
 cudaError_t launch_sparse_prefill_pair(const SparsePrefillKernelParams& sp, cudaStream_t stream);
 // Merge of split partials for a decode call (reads num_splits; skips unsplit requests).

@@ -20,8 +20,8 @@
 // The six chunks pass through the V ring on their way (free between the last P V of a request and the first of
 // the next); the K loads depend on nothing but the K ring and run ahead into the next request.
 //
-//   warps 0-3 softmax : as in mla_tc.cu (TMEM lane = row + 64 * (token >= 32)); arrivals that the issuing
-//                       thread waits for go to the leader's barriers (remote arrive from rank 1)
+//   warps 0-3 softmax : TMEM lane = row + 64 * (token >= 32); arrivals that the issuing thread waits for go to the
+//                       leader's barriers (remote arrive from rank 1)
 //   warp 4   K loader : per 64-token block the CTA's 32 token rows.  The leader's copies complete on
 //                       the barrier its MMA warp waits on; the peer's copies complete on a barrier of the peer
 //                       and one thread there passes each completion on with a single remote arrive (letting the
@@ -32,8 +32,8 @@
 //   warp 7   V relay  : waits for the local V part, clears the rows of the last page that lie beyond the
 //                       sequence (they may hold NaN and 0 * NaN must not reach O), tells the leader
 // TMEM (512 columns per CTA, allocated as a pair): O = [0,256), S[0] = [256,288), S[1] = [288,320), Q chunks
-// 0..5 = [320,512) (32 columns each); O / S layouts as in mla_tc.cu (the 64-row halves of an M=128 pair
-// instruction have the layout of the M=64 .ws form).
+// 0..5 = [320,512) (32 columns each); element (row r, column c) of an N-wide result
+// (the 64-row half of an M=128 pair instruction) sits in lane r + 64 * (c >= N/2), column c % (N/2).
 //
 // Gathering modes (sparse FP8 decode: 480 threads, sparse prefill: 320 threads).  Each CTA brings only its 32 token
 // rows of a 64-index block into the K ring -- prefill: three warps of 16-byte cp.async copies that arrive on the
@@ -49,6 +49,7 @@
 // index handling of the sparse modes.  Every wait is bounded; on expiry the pair drains and frees
 // its tensor memory.
 #include "kernels.h"
+#include "launch.cuh"
 #include "mla_work.cuh"
 #include "tc_common.cuh"
 
@@ -128,18 +129,6 @@ __device__ __forceinline__ void pst_shared_v4(uint32_t addr, uint4 v) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-// 32 bytes to global memory: one 256-bit store when the address allows it, else two 128-bit stores
-__device__ __forceinline__ void st_global_32B(void* p, const uint32_t (&w)[8]) {
-  if ((reinterpret_cast<uintptr_t>(p) & 31u) == 0) {
-    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
-                 "r"(w[5]), "r"(w[6]), "r"(w[7])
-                 : "memory");
-  } else {
-    reinterpret_cast<uint4*>(p)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-    reinterpret_cast<uint4*>(p)[1] = make_uint4(w[4], w[5], w[6], w[7]);
-  }
-}
-
 __device__ __forceinline__ void mma_pair_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
@@ -210,8 +199,6 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
     g_pair_span[(blockIdx.z * gridDim.x + blockIdx.x) * 2] = (long long)t;
   }
 #endif
-  const Tile tile = make_tile<WM>(P);
-  if (tile.n_work == 0) return;                 // both CTAs of a pair see the same schedule row
   const bool misaligned = (sbase & 1023u) != 0;  // the swizzled tiles need a 1024-byte aligned base
   auto lbar = [&](int i) { return tc::mapa(bar(i), 0); };    // the leader's copy of barrier i
   const float scale_log2 = PREFILL ? P.sp.scale_log2 : p.scale_log2;
@@ -248,8 +235,10 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
   __syncthreads();
   tc::cluster_sync_all();      // barriers of both CTAs exist before anything is sent to them
   tc::tc_fence_after();
+  pdl_wait();                  // the schedule, the queries and the cache may come from the kernel in front of this one
   pdl_allow_dependents();      // a merge kernel launched as a programmatic dependent may become resident now
   const uint32_t tmem = *sTmem;
+  const Tile tile = make_tile<WM>(P);           // both CTAs of a pair see the same schedule row (possibly an empty one)
 
   if (misaligned) {
     // nothing was issued; fall through to the common exit
@@ -1106,6 +1095,13 @@ static bool pair_map_4d(CUtensorMap* m, const void* base, uint64_t d1, uint64_t 
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <auto Kern>
+static cudaError_t launch_pair(const TcParams& P, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, dim3 grid, int threads,
+                               cudaStream_t stream) {
+  if (cudaError_t e = allow_smem<Kern>(ptc::SMEM_BYTES); e != cudaSuccess) return e;
+  return launch_dependent(Kern, grid, threads, ptc::SMEM_BYTES, stream, P, tq, tk, tv);
+}
+
 bool decode_sparse_pair_applies(const DecodeKernelParams& p) { return p.h_k == 1 && p.hq_per_hk == 128 && !p.is_f16; }
 
 cudaError_t launch_decode_sparse_pair(const DecodeKernelParams& p, cudaStream_t stream) {
@@ -1114,15 +1110,7 @@ cudaError_t launch_decode_sparse_pair(const DecodeKernelParams& p, cudaStream_t 
   CUtensorMap tq;
   // q [b][s_q][h_q][576] ; box = 64 heads x 64 columns
   if (!pair_map_4d(&tq, p.q, p.h_q, p.s_q, p.b, p.q_stride_h, p.q_stride_s, p.q_stride_b, 64, 1)) return cudaErrorInvalidValue;
-  auto kern = mla_pair_kernel<false, kSparseDecode>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ptc::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
-  kern<<<dim3(2, p.s_q, p.num_sm_parts), ptc::kSparseDecodeThreads, ptc::SMEM_BYTES, stream>>>(P, tq, tq, tq);   // the K / V maps are not used in this mode
-  return cudaGetLastError();
+  return launch_pair<mla_pair_kernel<false, kSparseDecode>>(P, tq, tq, tq, dim3(2, p.s_q, p.num_sm_parts), ptc::kSparseDecodeThreads, stream);   // the K / V maps are not used in this mode
 }
 
 bool sparse_prefill_pair_applies(const SparsePrefillKernelParams& sp) { return sp.h_q == 128; }
@@ -1136,15 +1124,7 @@ cudaError_t launch_sparse_prefill_pair(const SparsePrefillKernelParams& sp, cuda
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
   const int lanes = max(1, min(sp.s_q, sms / 2));
-  auto kern = mla_pair_kernel<false, kSparsePrefill>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ptc::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
-  kern<<<dim3(2, lanes, 1), ptc::kPrefillThreads, ptc::SMEM_BYTES, stream>>>(P, tq, tq, tq);    // the K / V maps are not used in this mode
-  return cudaGetLastError();
+  return launch_pair<mla_pair_kernel<false, kSparsePrefill>>(P, tq, tq, tq, dim3(2, lanes, 1), ptc::kPrefillThreads, stream);    // the K / V maps are not used in this mode
 }
 
 bool decode_dense_pair_applies(const DecodeKernelParams& p) { return p.hq_per_hk % 128 == 0; }
@@ -1165,25 +1145,8 @@ cudaError_t launch_decode_dense_pair(const DecodeKernelParams& p, cudaStream_t s
   if (!pair_map_4d(&tv, p.kcache, p.h_k, 64, p.num_blocks, p.k_stride_head, p.k_stride_row, p.k_stride_block, 1, 64)) return cudaErrorInvalidValue;
   const int n_hb = p.hq_per_hk / 64;
   const dim3 grid(p.s_q * n_hb, p.h_k, p.num_sm_parts);
-  static bool attr_set[2] = {false, false};      // idempotent, so a race between threads is harmless
-  if (p.is_f16) {
-    auto kern = mla_pair_kernel<true, kDense>;
-    if (!attr_set[1]) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ptc::SMEM_BYTES);
-      if (e != cudaSuccess) return e;
-      attr_set[1] = true;
-    }
-    kern<<<grid, ptc::kThreads, ptc::SMEM_BYTES, stream>>>(P, tq, tk, tv);
-  } else {
-    auto kern = mla_pair_kernel<false, kDense>;
-    if (!attr_set[0]) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ptc::SMEM_BYTES);
-      if (e != cudaSuccess) return e;
-      attr_set[0] = true;
-    }
-    kern<<<grid, ptc::kThreads, ptc::SMEM_BYTES, stream>>>(P, tq, tk, tv);
-  }
-  return cudaGetLastError();
+  if (p.is_f16) return launch_pair<mla_pair_kernel<true, kDense>>(P, tq, tk, tv, grid, ptc::kThreads, stream);
+  return launch_pair<mla_pair_kernel<false, kDense>>(P, tq, tk, tv, grid, ptc::kThreads, stream);
 }
 
 #ifdef FMLA_TRACE

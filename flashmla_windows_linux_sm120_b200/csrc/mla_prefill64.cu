@@ -693,46 +693,7 @@ static cudaError_t launch_tc(const TcParams& P, const CUtensorMap& tq, const CUt
   return cudaGetLastError();
 }
 
-// FMLA_DISABLE_PAIR=1 in the environment keeps the one-CTA-per-64-heads kernel for every shape (A/B runs)
-static bool pair_kernel_enabled() {
-  static const bool on = [] {
-    const char* v = getenv("FMLA_DISABLE_PAIR");
-    return !(v && v[0] == '1');
-  }();
-  return on;
-}
-
-bool decode_dense_merges_in_kernel(const DecodeKernelParams& p) {
-  return p.topk < 0 && decode_dense_pair_applies(p) && pair_kernel_enabled() && p.arrival_counters != nullptr && !p.force_partial;
-}
-
-cudaError_t launch_decode_dense_tc(const DecodeKernelParams& p, cudaStream_t stream) {
-  if (decode_dense_pair_applies(p) && pair_kernel_enabled()) return launch_decode_dense_pair(p, stream);
-  TcParams P = {};
-  P.d = p;
-  CUtensorMap tq, tkv;
-  // q [b][s_q][h_q][576] ; box = 64 heads x 64 columns (heads past h_q read as zero)
-  if (!make_map_4d(&tq, p.q, p.h_q, p.s_q, p.b, p.q_stride_h, p.q_stride_s, p.q_stride_b, 64, 1)) return cudaErrorInvalidValue;
-  // cache [num_blocks][64][h_k][576] addressed as (col, head, row-in-page, page) ; box = 64 rows x 64 columns of one head
-  if (!make_map_4d(&tkv, p.kcache, p.h_k, 64, p.num_blocks, p.k_stride_head, p.k_stride_row, p.k_stride_block, 1, 64))
-    return cudaErrorInvalidValue;
-  const int n_hb = (p.hq_per_hk + 63) / 64;
-  // the tensor maps only move 16-bit elements: one map type serves bf16 and fp16
-  if (p.is_f16) return launch_tc<kDense, true>(P, tq, tkv, dim3(p.s_q * n_hb, p.h_k, p.num_sm_parts), stream);
-  return launch_tc<kDense>(P, tq, tkv, dim3(p.s_q * n_hb, p.h_k, p.num_sm_parts), stream);
-}
-
-cudaError_t launch_decode_sparse_tc(const DecodeKernelParams& p, cudaStream_t stream) {
-  if (decode_sparse_pair_applies(p) && pair_kernel_enabled()) return launch_decode_sparse_pair(p, stream);
-  TcParams P = {};
-  P.d = p;
-  CUtensorMap tq;
-  if (!make_map_4d(&tq, p.q, p.h_q, p.s_q, p.b, p.q_stride_h, p.q_stride_s, p.q_stride_b, 64, 1)) return cudaErrorInvalidValue;
-  return launch_tc<kSparseDecode>(P, tq, tq, dim3((p.hq_per_hk + 63) / 64, p.s_q, p.num_sm_parts), stream);
-}
-
-cudaError_t launch_sparse_prefill_tc(const SparsePrefillKernelParams& sp, cudaStream_t stream) {
-  if (sparse_prefill_pair_applies(sp) && pair_kernel_enabled()) return launch_sparse_prefill_pair(sp, stream);
+cudaError_t launch_sparse_prefill_64(const SparsePrefillKernelParams& sp, cudaStream_t stream) {
   TcParams P = {};
   P.sp = sp;
   CUtensorMap tq;
@@ -752,9 +713,9 @@ extern "C" int fmla_debug_read_trace(long long* host, int n) {
 }
 #endif
 
-cudaError_t set_status_mirror_mla(int* mapped_host_word) { return tc::set_status_mirror(mapped_host_word); }
+cudaError_t set_status_mirror_prefill64(int* mapped_host_word) { return tc::set_status_mirror(mapped_host_word); }
 
-cudaError_t read_decode_tc_status(int* host_status, bool reset) {
+cudaError_t read_prefill64_status(int* host_status, bool reset) {
   cudaError_t e = cudaMemcpyFromSymbol(host_status, g_decode_tc_status, sizeof(int));
   if (e != cudaSuccess) return e;
   if (reset && *host_status != 0) {

@@ -1,4 +1,4 @@
-// Work decomposition shared by the MLA attention kernels (mla_tc.cu, mla_pair.cu): which tile of heads and
+// Work decomposition of the CTA-pair MLA attention kernel (mla_pair.cu; the modes also of mla_few_rows.cu): which tile of heads and
 // which stretch of the split-KV schedule a CTA owns, and the requests / query tokens it walks.
 #pragma once
 

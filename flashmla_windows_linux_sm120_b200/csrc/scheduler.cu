@@ -18,6 +18,7 @@
 //   partition k       = everything between cuts k and k+1; equal cuts give an empty partition (begin_idx = batch)
 // The integer statement of the same algorithm, against which the kernel is checked bit for bit, is
 // oracle/scheduler.py:schedule_cut_ref.
+#include "fmla_common.cuh"
 #include "kernels.h"
 
 namespace fmla {
@@ -34,11 +35,12 @@ struct Cut { int req, off; };
 __global__ void __launch_bounds__(kSchedThreads) get_mla_metadata_kernel(const int* __restrict__ seqlens_k, int batch,
                                                                          int num_sm_parts, int topk, int* __restrict__ md,
                                                                          int* __restrict__ num_splits) {
-  __shared__ int s_scan[kSchedThreads];
+  __shared__ int s_warp[kSchedThreads / 32];
   __shared__ int s_carry;
   __shared__ Cut s_cut[kMaxParts + 2];
   __shared__ unsigned char s_new[kMaxParts + 2];     // cut k differs from cut k-1
   const int tid = threadIdx.x;
+  pdl_allow_dependents();      // the attention kernel may be set up meanwhile; it waits for this kernel before it reads the schedule
   auto len_of = [&](int i) { return topk == -1 ? __ldg(seqlens_k + i) : topk; };
   auto real_blocks = [&](int i) { const int l = len_of(i); return l == 0 ? 0 : (l + kBlockN - 1) / kBlockN; };
   auto cost_of = [&](int i) { return max(real_blocks(i), 1) + kFixedOverheadBlocks; };
@@ -50,18 +52,30 @@ __global__ void __launch_bounds__(kSchedThreads) get_mla_metadata_kernel(const i
     for (int base = 0; base < n; base += kSchedThreads) {
       const int i = base + tid;
       const int v = i < n ? value(i) : 0;
-      s_scan[tid] = v;
-      __syncthreads();
-      for (int off = 1; off < kSchedThreads; off <<= 1) {
-        const int add = tid >= off ? s_scan[tid - off] : 0;
-        __syncthreads();
-        s_scan[tid] += add;
-        __syncthreads();
+      // scan within the warps, then over the warp totals
+      int x = v;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int add = __shfl_up_sync(0xffffffffu, x, off);
+        if ((tid & 31) >= off) x += add;
       }
-      const int carry = s_carry;
-      if (i < n) dst[i] = carry + s_scan[tid] - v;
+      if ((tid & 31) == 31) s_warp[tid >> 5] = x;
       __syncthreads();
-      if (tid == kSchedThreads - 1) s_carry = carry + s_scan[tid];
+      if (tid < 32) {
+        int w = s_warp[tid];
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const int add = __shfl_up_sync(0xffffffffu, w, off);
+          if (tid >= off) w += add;
+        }
+        s_warp[tid] = w;
+      }
+      __syncthreads();
+      const int carry = s_carry;
+      x += carry + (tid >= 32 ? s_warp[(tid >> 5) - 1] : 0);
+      if (i < n) dst[i] = x - v;
+      __syncthreads();
+      if (tid == kSchedThreads - 1) s_carry = x;
       __syncthreads();
     }
     if (tid == 0) dst[n] = s_carry;
