@@ -10,18 +10,17 @@
 // contiguous per load instruction.
 #include "fmla_common.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 #include "tc_common.cuh"
 
 namespace fmla {
 
 constexpr int kCombineWarps = 8;
+constexpr int kPartsInFlight = 4;       // partial rows whose loads a lane issues before it uses the first
 
-// lse_part(i) / o_part(i) address part i of this row.  COHERENT: the partial outputs may have been written by
-// another GPU while this kernel was already resident (peer merge), so they are read with ld.global.cv
-// instead of the non-coherent path, which is undefined for memory modified during the kernel's lifetime.
-template <bool COHERENT = false, class LseAt, class OAt>
-__device__ __forceinline__ void combine_row(int nparts, LseAt lse_at, OAt o_at, float* s_w, __nv_bfloat16* out_row,
-                                            float* lse_out, bool f16 = false) {
+// Weights 2^(lse_i - lse) of the parts of a row -> s_w (whole warp); returns the base-2 LSE of the row.
+template <class LseAt>
+__device__ __forceinline__ float combine_weights(int nparts, LseAt lse_at, float* s_w) {
   const int lane = threadIdx.x & 31;
   float mx = neg_inf();
   for (int i = lane; i < nparts; i += 32) mx = fmaxf(mx, lse_at(i));
@@ -33,37 +32,66 @@ __device__ __forceinline__ void combine_row(int nparts, LseAt lse_at, OAt o_at, 
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
   const float glse = (sum == 0.f || sum != sum) ? pos_inf() : log2f(sum) + mx;
-  if (lane == 0) *lse_out = glse * kLn2;
   for (int i = lane; i < nparts; i += 32) s_w[i] = exp2f(lse_at(i) - glse);
   __syncwarp();
+  return glse;
+}
 
-  float4 acc[4];
+// Weighted sum of the parts over column groups [first, first + NG) of 128 columns (lane = 4 columns of a group), in the
+// order of the parts.  A part with weight 0 is not read: 0 * (Inf or NaN) must not reach the sum.
+// COHERENT: the partial outputs may have been written by another GPU while this kernel was already resident (peer
+// merge), so they are read with ld.global.cv instead of the non-coherent path, which is undefined for memory modified
+// during the kernel's lifetime.
+template <int NG, bool COHERENT, class OAt>
+__device__ __forceinline__ void combine_columns(int nparts, OAt o_at, const float* s_w, __nv_bfloat16* out_row, int first, bool f16) {
+  const int lane = threadIdx.x & 31;
+  float4 acc[NG];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int i = 0; i < nparts; ++i) {
-    const float w = s_w[i];
-    if (w == 0.f) continue;
-    const float4* src = reinterpret_cast<const float4*>(o_at(i));
+  for (int j = 0; j < NG; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i0 = 0; i0 < nparts; i0 += kPartsInFlight) {
+    float4 v[kPartsInFlight][NG];
+    float w[kPartsInFlight];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float4 v = COHERENT ? __ldcv(src + j * 32 + lane) : __ldg(src + j * 32 + lane);
-      acc[j].x += w * v.x;
-      acc[j].y += w * v.y;
-      acc[j].z += w * v.z;
-      acc[j].w += w * v.w;
+    for (int u = 0; u < kPartsInFlight; ++u) {
+      w[u] = i0 + u < nparts ? s_w[i0 + u] : 0.f;
+      if (w[u] == 0.f) continue;
+      const float4* src = reinterpret_cast<const float4*>(o_at(i0 + u)) + first * 32 + lane;
+#pragma unroll
+      for (int j = 0; j < NG; ++j) v[u][j] = COHERENT ? __ldcv(src + j * 32) : __ldg(src + j * 32);
+    }
+#pragma unroll
+    for (int u = 0; u < kPartsInFlight; ++u) {
+      if (w[u] == 0.f) continue;
+#pragma unroll
+      for (int j = 0; j < NG; ++j) {
+        acc[j].x += w[u] * v[u][j].x;
+        acc[j].y += w[u] * v[u][j].y;
+        acc[j].z += w[u] * v[u][j].z;
+        acc[j].w += w[u] * v[u][j].w;
+      }
     }
   }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < NG; ++j) {
     // out_row addresses 16-bit elements: bf16, or fp16 when the queries were fp16
     uint2 packed = f16 ? make_uint2(pack_f16x2(acc[j].x, acc[j].y), pack_f16x2(acc[j].z, acc[j].w))
                        : make_uint2(pack_bf16x2(acc[j].x, acc[j].y), pack_bf16x2(acc[j].z, acc[j].w));
-    *reinterpret_cast<uint2*>(out_row + (j * 32 + lane) * 4) = packed;
+    *reinterpret_cast<uint2*>(out_row + ((first + j) * 32 + lane) * 4) = packed;
   }
 }
 
-// grid (b, ceil(h_k*q_seq_per_hk / 8)); requests with a single part were written
+template <bool COHERENT = false, class LseAt, class OAt>
+__device__ __forceinline__ void combine_row(int nparts, LseAt lse_at, OAt o_at, float* s_w, __nv_bfloat16* out_row,
+                                            float* lse_out) {
+  const float glse = combine_weights(nparts, lse_at, s_w);
+  if ((threadIdx.x & 31) == 0) *lse_out = glse * kLn2;
+  combine_columns<4, COHERENT>(nparts, o_at, s_w, out_row, 0, false);
+}
+
+// grid (b, ceil(h_k*q_seq_per_hk / rows per CTA)); requests with a single part were written
 // in final form by the attention kernel and are skipped (mla_combine.cu:30-32).
+// WPR warps per row, each for 4 / WPR of the row's four 128-column groups.
+template <int WPR>
 __global__ void __launch_bounds__(kCombineWarps * 32) decode_combine_kernel(const __grid_constant__ DecodeKernelParams p) {
   extern __shared__ float s_weights[];  // [8][num_sm_parts]
   pdl_wait();                           // launched as a programmatic dependent of the attention kernel
@@ -73,19 +101,20 @@ __global__ void __launch_bounds__(kCombineWarps * 32) decode_combine_kernel(cons
   if (nparts <= 1) return;
   const int q_seq_per_hk = p.s_q * p.hq_per_hk;
   const int rows = p.h_k * q_seq_per_hk;
-  const int warp = threadIdx.x >> 5;
-  const int r = blockIdx.y * kCombineWarps + warp;
+  const int warp = threadIdx.x >> 5, sub = warp % WPR;
+  const int r = blockIdx.y * (kCombineWarps / WPR) + warp / WPR;
   if (r >= rows) return;
   const int kh = r / q_seq_per_hk, row = r % q_seq_per_hk;
   const int sq = row / p.hq_per_hk, head = kh * p.hq_per_hk + row % p.hq_per_hk;
   const float* lse_base = p.lse_accum + (int64_t)lo * rows + r;
   const float* o_base = p.o_accum + ((int64_t)lo * rows + r) * 512;
   const int64_t part_stride = rows;
-  combine_row(
-      nparts, [&](int i) { return __ldg(lse_base + i * part_stride); },
-      [&](int i) { return o_base + i * part_stride * 512; }, s_weights + warp * p.num_sm_parts,
-      reinterpret_cast<__nv_bfloat16*>(p.out) + batch * p.o_stride_b + sq * p.o_stride_s + head * p.o_stride_h,
-      p.softmax_lse + ((int64_t)batch * p.h_q + head) * p.s_q + sq, p.is_f16 != 0);
+  float* w = s_weights + warp * p.num_sm_parts;
+  const float glse = combine_weights(nparts, [&](int i) { return __ldg(lse_base + i * part_stride); }, w);
+  if (sub == 0 && (threadIdx.x & 31) == 0) p.softmax_lse[((int64_t)batch * p.h_q + head) * p.s_q + sq] = glse * kLn2;
+  combine_columns<4 / WPR, false>(
+      nparts, [&](int i) { return o_base + i * part_stride * 512; }, w,
+      reinterpret_cast<__nv_bfloat16*>(p.out) + batch * p.o_stride_b + sq * p.o_stride_s + head * p.o_stride_h, sub * (4 / WPR), p.is_f16 != 0);
 }
 
 __global__ void __launch_bounds__(kCombineWarps * 32)
@@ -251,24 +280,21 @@ cudaError_t read_merge_status(int* host_status, bool reset) {
   return e;
 }
 
+template <int WPR>
+static cudaError_t launch_decode_combine_wpr(const DecodeKernelParams& p, int rows, cudaStream_t stream) {
+  constexpr int kRows = kCombineWarps / WPR;
+  const size_t smem = sizeof(float) * kCombineWarps * p.num_sm_parts;
+  if (cudaError_t e = allow_dynamic_smem(decode_combine_kernel<WPR>, smem); e != cudaSuccess) return e;
+  return launch_dependent(decode_combine_kernel<WPR>, dim3(p.b, (rows + kRows - 1) / kRows), kCombineWarps * 32, smem, stream, p);
+}
+
 cudaError_t launch_decode_combine(const DecodeKernelParams& p, cudaStream_t stream) {
   const int rows = p.h_k * p.s_q * p.hq_per_hk;
-  dim3 grid(p.b, (rows + kCombineWarps - 1) / kCombineWarps);
-  const size_t smem = sizeof(float) * kCombineWarps * p.num_sm_parts;
-  if (cudaError_t e = allow_dynamic_smem(decode_combine_kernel, smem); e != cudaSuccess) return e;
-  // programmatic dependent launch: the blocks may become resident while the attention kernel drains and start
-  // the moment it has completed (they wait in pdl_wait()), instead of being launched after it
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(kCombineWarps * 32);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, decode_combine_kernel, p);
+  // Few rows with many parts each (4 requests x 16 heads split 37 ways): one warp per row walks its parts one after the
+  // other on a handful of SMs, so a row is spread over four warps as long as that fits on the chip at once
+  // (148 SMs x 64 warps); beyond that the rows alone fill it and four times the CTAs would only cost their launch.
+  if ((int64_t)p.b * rows * 4 <= 148 * 64) return launch_decode_combine_wpr<4>(p, rows, stream);
+  return launch_decode_combine_wpr<1>(p, rows, stream);
 }
 
 cudaError_t launch_combine_partials(const float* lse_accum, const float* o_accum, int num_parts, int rows, void* out,
