@@ -13,32 +13,29 @@
 //   3. dK/dV: one CTA per (128-key tile, head, sequence), walks the queries in blocks of 64
 // Requires h_q == h_k (as flash_mla/flash_mla_interface.py:413-415).
 //
-// Both main kernels use the same roles as the forward: warps 0-3 element-wise (one thread per row of
-// the resident tile = one TMEM lane), warp 4 TMA, warp 5 MMA.  The two first GEMMs of a step write
+// Both main kernels: warps 0-7 element-wise (two threads per row of the resident tile = TMEM lane, one per half of the
+// streamed columns), then a TMA warp and the MMA issuing warps.  The two first GEMMs of a step write
 // fp32 tiles [128 x 64] into tensor memory; the element-wise warps turn them into bf16 P / dS in the
 // same columns; the second GEMMs read those as their A operand straight from tensor memory and the
 // streamed tile, read MN-major, as B.
 // Every mbarrier wait is bounded (tc_common.cuh); a pipeline fault sets a status word and lets the
 // CTA drain and free its tensor memory.
 #include "kernels.h"
+#include "launch.cuh"
 #include "tc_common.cuh"
 #include "tma_host.cuh"
+
+#include <type_traits>
 
 namespace fmla {
 
 namespace dbt {
 constexpr int kResChunk = 128 * 128;              // resident tiles: [128 rows x 64 bf16] chunks
 constexpr int kStgChunk = 64 * 128;               // streamed tiles: [64 rows x 64 bf16] chunks
+constexpr int kEwWarps = 8;                       // element-wise warps (two per 32 accumulator rows)
+constexpr int kDqThreads = (kEwWarps + 3) * 32;   // + TMA + two MMA issuers
+constexpr int kDkvThreads = (kEwWarps + 2) * 32;  // + TMA + MMA issuer
 constexpr int kStages = 3;                        // ring of streamed tiles (the TMEM buffers alternate independently)
-template <int V> struct IC { static constexpr int value = V; };
-// calls f(IC<stage>, IC<buffer>) with compile-time stage (0..2) and buffer (0..1): every combination gets
-// its own straight-line code, so that all descriptors stay a warp-uniform base plus an immediate
-template <typename F>
-__device__ __forceinline__ void dispatch_stage_buffer(int st, int b, F&& f) {
-  if (st == 0) { if (b == 0) f(IC<0>{}, IC<0>{}); else f(IC<0>{}, IC<1>{}); }
-  else if (st == 1) { if (b == 0) f(IC<1>{}, IC<0>{}); else f(IC<1>{}, IC<1>{}); }
-  else { if (b == 0) f(IC<2>{}, IC<0>{}); else f(IC<2>{}, IC<1>{}); }
-}
 template <int D_QK>
 struct Layout {
   static constexpr int NCH = D_QK / 64;
@@ -71,22 +68,35 @@ __device__ long long g_dense_bwd_trace[64 * 16];
 #endif
 
 // ---- 1. delta[h, t] = sum_d dO * O --------------------------------------------------------------
+// Bound by HBM (512 bytes read per row): 16 lanes per row with 16-byte loads, kDeltaRows rows per half warp in flight.
+constexpr int kDeltaRows = 4;
 __global__ void __launch_bounds__(256) dense_bwd_delta_tc_kernel(const __grid_constant__ DenseKernelParams p) {
-  const int warp = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= p.total_q * p.h_q) return;
-  const int t = warp / p.h_q, h = warp % p.h_q;
-  const __nv_bfloat16* o = reinterpret_cast<const __nv_bfloat16*>(p.o) + (int64_t)t * p.o_stride_t + h * p.o_stride_h;
-  const __nv_bfloat16* d = reinterpret_cast<const __nv_bfloat16*>(p.d_o) + (int64_t)t * p.do_stride_t + h * p.do_stride_h;
-  const uint2 ov = *reinterpret_cast<const uint2*>(o + lane * 4);
-  const uint2 dv = *reinterpret_cast<const uint2*>(d + lane * 4);
-  const float2 o0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ov.x));
-  const float2 o1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ov.y));
-  const float2 d0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&dv.x));
-  const float2 d1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&dv.y));
-  float s = o0.x * d0.x + o0.y * d0.y + o1.x * d1.x + o1.y * d1.y;
+  const int group = (blockIdx.x * 256 + threadIdx.x) >> 4, l16 = threadIdx.x & 15;
+  const int64_t rows = (int64_t)p.total_q * p.h_q, first = (int64_t)group * kDeltaRows;
+  uint4 ov[kDeltaRows], dv[kDeltaRows];
 #pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) p.delta[(int64_t)h * p.total_q + t] = s;
+  for (int r = 0; r < kDeltaRows; ++r) {
+    ov[r] = dv[r] = make_uint4(0, 0, 0, 0);
+    if (first + r < rows) {
+      const int t = static_cast<int>((first + r) / p.h_q), h = static_cast<int>((first + r) % p.h_q);
+      ov[r] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.o) + (int64_t)t * p.o_stride_t + h * p.o_stride_h) + l16);
+      dv[r] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.d_o) + (int64_t)t * p.do_stride_t + h * p.do_stride_h) + l16);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kDeltaRows; ++r) {
+    const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&ov[r]);
+    const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(&dv[r]);
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 a = __bfloat1622float2(o2[i]), g = __bfloat1622float2(d2[i]);
+      s += a.x * g.x + a.y * g.y;
+    }
+#pragma unroll
+    for (int off = 8; off >= 1; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (l16 == 0 && first + r < rows) p.delta[(first + r) % p.h_q * p.total_q + (first + r) / p.h_q] = s;
+  }
 }
 
 // Zeroes rows [rows_valid, 64) of a streamed tile of NCHUNK 64-column chunks (whole warp).  Rows past
@@ -102,6 +112,9 @@ __device__ __forceinline__ void zero_stage_tail(unsigned char* tile, int nchunk,
   __syncwarp();
 }
 
+// The instructions of a step exist once: ring stage and buffer come in as run-time bases (warp-uniform), to which the
+// unrolled code adds immediates.  With one unrolled copy per (stage, buffer) each copy came around once in three to six
+// steps and its first MMA waited for the instruction fetch.
 // D[128 x 64] (TMEM column d_col) = A[128 x 64*NCH] (resident, K-major) * B[64 x 64*NCH]^T (streamed, K-major)
 template <int NCH>
 __device__ __forceinline__ void mma_res_stg(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
@@ -118,8 +131,29 @@ __device__ __forceinline__ void mma_tmem_stg(uint32_t d_tmem, uint32_t a_tmem, u
   for (int s = 0; s < 4; ++s) tc::mma_ts(d_tmem, a_tmem + s * 8, tc::desc_advance(desc_b, s * 2048), idesc, (first && s == 0) ? 0u : 1u);
 }
 
+// 32 fp32 columns of an accumulator row -> bf16, times `mul`, as full 32-byte sectors (zeros when nothing was computed)
+__device__ __forceinline__ void store_grad_chunk(uint32_t taddr, bool have, bool row_ok, float mul, __nv_bfloat16* dst) {
+  uint32_t ov[32];
+  if (have) {
+    tc::tmem_ld32(taddr, ov);
+    tc::tmem_wait_ld();
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) ov[i] = 0u;
+  }
+  if (!row_ok) return;
+#pragma unroll
+  for (int q8 = 0; q8 < 2; ++q8) {
+    uint32_t w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      w[i] = pack_bf16x2(__uint_as_float(ov[q8 * 16 + 2 * i]) * mul, __uint_as_float(ov[q8 * 16 + 2 * i + 1]) * mul);
+    st_global_32B(dst + q8 * 16, w);
+  }
+}
+
 // ---- 2. dQ ------------------------------------------------------------------------------------------
-// grid (ceil(max_seqlen_q/128), h_q, batch), 224 threads (warps 0-3 element-wise, 4 TMA, 5 and 6 MMA).
+// grid (ceil(max_seqlen_q/128), h_q, batch), 352 threads (warps 0-7 element-wise, 8 TMA, 9 and 10 MMA).
 // Resident: Q, dO tiles of 128 queries.
 // Per step (64 keys): S = Q K^T and dP = dO V^T into one of two TMEM buffer pairs, dS (bf16) into one of two
 // slots, then dQ += dS K.  TMEM: dQ = [0, D_QK), buffer b: S = [192 + 128 b, +64), dP = [256 + 128 b, +64),
@@ -129,7 +163,7 @@ enum BarQ { Q_RES_FULL = 0, Q_KV_FULL0, Q_KV_EMPTY0 = Q_KV_FULL0 + kStages, Q_SD
 }
 
 template <int D_QK>
-__global__ void __launch_bounds__(224, 1)
+__global__ void __launch_bounds__(dbt::kDqThreads, 1)
 dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_constant__ CUtensorMap tmap_q,
                        const __grid_constant__ CUtensorMap tmap_do, const __grid_constant__ CUtensorMap tmap_k,
                        const __grid_constant__ CUtensorMap tmap_v) {
@@ -147,9 +181,16 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
   const int q0 = __ldg(p.cu_q + b), lq = __ldg(p.cu_q + b + 1) - q0;
   const int k0 = __ldg(p.cu_k + b), lk = __ldg(p.cu_k + b + 1) - k0;
   const int m_base = (gridDim.x - 1 - blockIdx.x) * 128;    // the tiles with the most keys first
-  if (m_base >= lq) return;
+  // The dQ kernel may start while the dK / dV kernel in front of it drains.  One CTA waits for that kernel's end, so that
+  // this kernel ends after it and what follows in the stream sees both.
+  const bool waits = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
+  if (m_base >= lq) {
+    if (waits) pdl_wait();
+    return;
+  }
   if ((sbase & 1023u) != 0) {
     if (tid == 0) tc::report_status(status, 30);
+    if (waits) pdl_wait();
     return;
   }
   int nblk = (lk + 63) >> 6;
@@ -158,41 +199,51 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
     nblk = last_key < 0 ? 0 : min(nblk, (last_key >> 6) + 1);
   }
 
-  if (tid == 0) {
-    for (int i = 0; i < Q_NUM_BARS; ++i) tc::mbar_init(bar(i), (i == Q_DS_FULL0 || i == Q_DS_FULL1) ? 128 : 1);
-    tc::fence_mbar_init();
+  auto load_keys = [&](int j) {
+    const int st = j % kStages, tok = k0 + j * 64;
+    const uint32_t stage = sStg + st * L::kStage;
+    DBT_TRACE_AT(j, 0);
+    tc::mbar_arrive_expect_tx(bar(Q_KV_FULL0 + st), L::kStage);
+#pragma unroll
+    for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(stage + c * kStgChunk, &tmap_k, c * 64, head, tok, bar(Q_KV_FULL0 + st));
+#pragma unroll
+    for (int c = 0; c < 2; ++c) tc::tma_load_3d(stage + L::kStgA + c * kStgChunk, &tmap_v, c * 64, head, tok, bar(Q_KV_FULL0 + st));
+  };
+  if (warp == kEwWarps) {
+    // the thread that makes the barriers starts the first loads at once, before the others have tensor memory
+    if (tc::elect_one()) {
+      // one arrival per element-wise warp
+      for (int i = 0; i < Q_NUM_BARS; ++i) tc::mbar_init(bar(i), (i == Q_DS_FULL0 || i == Q_DS_FULL1) ? kEwWarps : 1);
+      tc::fence_mbar_init();
+      tc::fence_proxy_async_smem();
+      if (nblk > 0) {
+        tc::mbar_arrive_expect_tx(bar(Q_RES_FULL), L::kResA + L::kResB);
+#pragma unroll
+        for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(sQ + c * kResChunk, &tmap_q, c * 64, head, q0 + m_base, bar(Q_RES_FULL));
+#pragma unroll
+        for (int c = 0; c < 2; ++c) tc::tma_load_3d(sDO + c * kResChunk, &tmap_do, c * 64, head, q0 + m_base, bar(Q_RES_FULL));
+        for (int j = 0; j < min(kStages, nblk); ++j) load_keys(j);
+      }
+    }
+    __syncwarp();
   }
-  if (warp == 5) tc::tmem_alloc(sbase + L::MISC_OFF, 512);
+  if (warp == kEwWarps + 1) tc::tmem_alloc(sbase + L::MISC_OFF, 512);
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *sTmem;
   constexpr int TM_DQ = 0, TM_SD = 192, TM_DS = 448;
 
-  if (warp == 4) {
+  if (warp == kEwWarps) {
     // ================================ TMA producer =====================================
-    if (tc::elect_one() && nblk > 0) {
-      tc::mbar_arrive_expect_tx(bar(Q_RES_FULL), L::kResA + L::kResB);
-#pragma unroll
-      for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(sQ + c * kResChunk, &tmap_q, c * 64, head, q0 + m_base, bar(Q_RES_FULL));
-#pragma unroll
-      for (int c = 0; c < 2; ++c) tc::tma_load_3d(sDO + c * kResChunk, &tmap_do, c * 64, head, q0 + m_base, bar(Q_RES_FULL));
+    if (tc::elect_one()) {
       bool alive = true;
-      for (int j = 0; j < nblk && alive; ++j) {
-        const int st = j % kStages;
-        const uint32_t stage = sStg + st * L::kStage;
-        const int tok = k0 + j * 64;
-        alive = tc::mbar_wait(bar(Q_KV_EMPTY0 + st), ((j / kStages) & 1) ^ 1, status, 51);
-        if (!alive) break;
-        DBT_TRACE_AT(j, 0);
-        tc::mbar_arrive_expect_tx(bar(Q_KV_FULL0 + st), L::kStage);
-#pragma unroll
-        for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(stage + c * kStgChunk, &tmap_k, c * 64, head, tok, bar(Q_KV_FULL0 + st));
-#pragma unroll
-        for (int c = 0; c < 2; ++c) tc::tma_load_3d(stage + L::kStgA + c * kStgChunk, &tmap_v, c * 64, head, tok, bar(Q_KV_FULL0 + st));
+      for (int j = kStages; j < nblk && alive; ++j) {
+        alive = tc::mbar_wait(bar(Q_KV_EMPTY0 + j % kStages), ((j / kStages) & 1) ^ 1, status, 51);
+        if (alive) load_keys(j);
       }
     }
-  } else if (warp == 5 || warp == 6) {
+  } else if (warp > kEwWarps) {
     // ================================ MMA issuers =======================================
     constexpr uint32_t idesc_sd = tc::idesc_bf16_f32(128, 64, 0, 0);
     constexpr uint32_t idesc_dq = tc::idesc_bf16_f32(128, D_QK, 0, 1);
@@ -203,10 +254,10 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
     const uint64_t desc_kt = tc::smem_desc_sw128(sStg, kStgChunk, 1024);              // K tile of stage 0, MN-major (B of dQ)
     bool alive = nblk > 0;
     if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_RES_FULL), 0, status, 52));
-    // Two issuing warps: warp 5 the first GEMMs of a step (S, dP), warp 6 the second one (dQ).  Each
+    // Two issuing warps: the first for the first GEMMs of a step (S, dP), the other for the second one (dQ).  Each
     // wait on an mbarrier costs the issuing warp a few hundred cycles in which the tensor pipe would
     // otherwise idle; with two warps the waits of one overlap the instructions of the other.
-    if (warp == 5) {
+    if (warp == kEwWarps + 1) {
       for (int j = 0; j < nblk && alive; ++j) {
         const int st = j % kStages, bf = j & 1;
         // the tile has landed, and the S / dP buffer pair bf is free (the element-wise warps have read step
@@ -218,11 +269,9 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
         tc::tc_fence_after();
         if (lane == 0) DBT_TRACE_AT(j, 2);
         if (tc::elect_one()) {
-          dispatch_stage_buffer(st, bf, [&](auto ST, auto BF) {
-            constexpr int kOff = decltype(ST)::value * L::kStage, kCol = TM_SD + decltype(BF)::value * 128;
-            mma_res_stg<L::NCH>(tmem + kCol, desc_q, tc::desc_advance(desc_k, kOff), idesc_sd);
-            mma_res_stg<2>(tmem + kCol + 64, desc_do, tc::desc_advance(desc_v, kOff), idesc_sd);
-          });
+          const uint32_t off = st * L::kStage, col = tmem + TM_SD + bf * 128;
+          mma_res_stg<L::NCH>(col, desc_q, tc::desc_advance(desc_k, off), idesc_sd);
+          mma_res_stg<2>(col + 64, desc_do, tc::desc_advance(desc_v, off), idesc_sd);
           tc::tc_commit(bar(Q_SD_FULL0 + bf));
           DBT_TRACE_AT(j, 3);
         }
@@ -238,10 +287,7 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
         tc::tc_fence_after();
         if (lane == 0) DBT_TRACE_AT(j, 4);
         if (tc::elect_one()) {
-          dispatch_stage_buffer(st, bf, [&](auto ST, auto BF) {
-            mma_tmem_stg(tmem + TM_DQ, tmem + TM_DS + decltype(BF)::value * 32, tc::desc_advance(desc_kt, decltype(ST)::value * L::kStage),
-                         idesc_dq, j == 0);
-          });
+          mma_tmem_stg(tmem + TM_DQ, tmem + TM_DS + bf * 32, tc::desc_advance(desc_kt, st * L::kStage), idesc_dq, j == 0);
           tc::tc_commit(bar(Q_KV_EMPTY0 + st));
           tc::tc_commit(bar(Q_BUF_FREE0 + bf));
           if (j == nblk - 1) tc::tc_commit(bar(Q_DONE));
@@ -252,16 +298,20 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
     }
   } else {
     // ================================ element-wise / epilogue ==========================
-    const int row = m_base + tid;
+    // Warps w and w + 4 share the TMEM lanes of 32 rows: warp w takes columns [0, 32) of every 64-key block, warp w + 4
+    // the other half.  With four warps (one per scheduler) the chain TMEM load -> exponentials -> dS -> store of a step
+    // outlasted the step's 1344 clk of MMAs, and the tensor pipe waited for it.
+    const int half = warp >> 2, rl = tid & 127;
+    const int row = m_base + rl;
     const bool row_ok = row < lq;
-    const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const float lse2 = row_ok ? __ldg(p.lse + (int64_t)(q0 + row) * p.lse_stride_t + head * p.lse_stride_h) * kLog2e : 0.f;
     const float dl = row_ok ? __ldg(p.delta + (int64_t)head * p.total_q + q0 + row) : 0.f;
     const int limit = !row_ok ? 0 : (p.is_causal ? max(0, min(lk, row + (lk - lq) + 1)) : lk);
     bool alive = true;
     for (int j = 0; j < nblk && alive; ++j) {
       const int st = j & 1;
-      const uint32_t sd_addr = tmem + lane_addr + TM_SD + st * 128;
+      const uint32_t sd_addr = tmem + lane_addr + TM_SD + st * 128 + half * 32;
       // S and dP of this step are there, and the dS slot st is free (it was last read by the dQ
       // instructions of step j-2; dS has slots of its own so that the fp32 buffers are free again as
       // soon as they have been read)
@@ -269,33 +319,36 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
       if (!alive) break;
       if (tid == 0) DBT_TRACE_AT(j, 6);
       tc::tc_fence_after();
-      uint32_t sv[2][32], dp[2][32];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        tc::tmem_ld32(sd_addr + c * 32, sv[c]);
-        tc::tmem_ld32(sd_addr + 64 + c * 32, dp[c]);
-      }
+      uint32_t sv[32], dp[32], pk[16];
+      tc::tmem_ld32(sd_addr, sv);
+      tc::tmem_ld32(sd_addr + 64, dp);
       tc::tmem_wait_ld();
       if (tid == 0) DBT_TRACE_AT(j, 7);
-      const int cnt = limit - j * 64;                          // visible keys of this block: [0, cnt)
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t pk[16];
+      const int cnt = limit - j * 64 - half * 32;              // visible keys of this half block: [0, cnt)
+      const bool all_visible = __all_sync(0xffffffffu, cnt >= 32);
+      // two loops, not a test per element: the compiler makes a branch of each test (40 clk per element measured)
+      auto to_ds = [&](auto masked) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const float p0 = exp2f(fmaf(__uint_as_float(sv[c][2 * i]), p.scale_log2, -lse2));
-          const float p1 = exp2f(fmaf(__uint_as_float(sv[c][2 * i + 1]), p.scale_log2, -lse2));
-          // a select, not a product: masked entries may hold Inf or NaN
-          const float d0 = (c * 32 + 2 * i < cnt) ? p0 * (__uint_as_float(dp[c][2 * i]) - dl) : 0.f;
-          const float d1 = (c * 32 + 2 * i + 1 < cnt) ? p1 * (__uint_as_float(dp[c][2 * i + 1]) - dl) : 0.f;
+          const float p0 = exp2f(fmaf(__uint_as_float(sv[2 * i]), p.scale_log2, -lse2));
+          const float p1 = exp2f(fmaf(__uint_as_float(sv[2 * i + 1]), p.scale_log2, -lse2));
+          float d0 = p0 * (__uint_as_float(dp[2 * i]) - dl);
+          float d1 = p1 * (__uint_as_float(dp[2 * i + 1]) - dl);
+          if constexpr (decltype(masked)::value) {             // a select, not a product: masked entries may hold Inf or NaN
+            d0 = 2 * i < cnt ? d0 : 0.f;
+            d1 = 2 * i + 1 < cnt ? d1 : 0.f;
+          }
           pk[i] = pack_bf16x2(d0, d1);
         }
-        tc::tmem_st16(tmem + lane_addr + TM_DS + st * 32 + c * 16, pk);
-      }
+      };
+      if (all_visible) to_ds(std::false_type{});
+      else to_ds(std::true_type{});
+      tc::tmem_st16(tmem + lane_addr + TM_DS + st * 32 + half * 16, pk);
       if (tid == 0) DBT_TRACE_AT(j, 8);
       tc::tmem_wait_st();
       tc::tc_fence_before();
-      tc::mbar_arrive(bar(Q_DS_FULL0 + st));
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(bar(Q_DS_FULL0 + st));
       if (tid == 0) DBT_TRACE_AT(j, 9);
     }
     bool have = nblk > 0 && alive;
@@ -305,46 +358,32 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
     }
     __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.dq) + (int64_t)(q0 + row) * p.dq_stride_t + head * p.dq_stride_h;
 #pragma unroll 1
-    for (int c = 0; c < D_QK / 32; ++c) {
-      uint32_t ov[32];
-      if (have) {
-        tc::tmem_ld32(tmem + lane_addr + TM_DQ + c * 32, ov);
-        tc::tmem_wait_ld();
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) ov[i] = 0u;
-      }
-      if (row_ok) {
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          uint4 v;
-          v.x = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 0]) * p.scale, __uint_as_float(ov[q4 * 8 + 1]) * p.scale);
-          v.y = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 2]) * p.scale, __uint_as_float(ov[q4 * 8 + 3]) * p.scale);
-          v.z = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 4]) * p.scale, __uint_as_float(ov[q4 * 8 + 5]) * p.scale);
-          v.w = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 6]) * p.scale, __uint_as_float(ov[q4 * 8 + 7]) * p.scale);
-          *reinterpret_cast<uint4*>(orow + c * 32 + q4 * 8) = v;
-        }
-      }
-    }
+    for (int c = half; c < D_QK / 32; c += 2) store_grad_chunk(tmem + lane_addr + TM_DQ + c * 32, have, row_ok, p.scale, orow + c * 32);
   }
 
   tc::tc_fence_before();
   __syncthreads();
-  if (warp == 5) tc::tmem_dealloc(tmem, 512);
+  if (warp == kEwWarps + 1) tc::tmem_dealloc(tmem, 512);
+  if (waits) pdl_wait();
 }
 
 // ---- 3. dK, dV ----------------------------------------------------------------------------------
-// grid (ceil(max_seqlen_k/128), h, batch), 192 threads.  Resident: K, V tiles of 128 keys.
-// Per step (64 queries): S^T = K Q^T into one of two buffers, dP^T = V dO^T into a single buffer
-// (tensor memory has no room for a second one beside dK and dV), P^T over S^T and dS^T over dP^T,
-// then dV += P^T dO and dK += dS^T Q.
-// TMEM: dV = [0,128), dK = [128, 128 + D_QK), S^T buffer b = [320 + 64 b, +64), dP^T = [448, 512).
+// grid (ceil(max_seqlen_k/128), h, batch), 320 threads (warps 0-7 element-wise, 8 TMA, 9 MMA).  Resident: K, V tiles
+// of 128 keys.  Per step (64 queries): S^T = K Q^T, dP^T = V dO^T, P^T and dS^T (bf16), dV += P^T dO, dK += dS^T Q.
+// TMEM: dV = [0,128), dK = [128, 128 + D_QK), S^T = [320,384), dP^T = [384,448), P^T = [448,480), dS^T = [480,512).
+// The 192 columns that dV and dK leave hold the fp32 tiles of ONE step and the bf16 tiles of ONE step: the element-wise
+// warps take S^T and dP^T of step j into registers, which frees those columns for step j+1, and write P^T and dS^T of
+// step j into columns of their own.  The tensor pipe runs S^T(j+1), dP^T(j+1), dV(j), dK(j) back to back while the
+// element-wise work of a step hides behind the 1600 clk of MMAs of its neighbours.  (With the bf16 tiles written over
+// the fp32 ones, two S^T buffers and a single dP^T buffer, dP^T(j+1) had to wait for dK(j) and dK(j) for the
+// element-wise work on dP^T(j).)
 namespace dbt {
-enum BarK { K_RES_FULL = 0, K_QD_FULL0, K_QD_EMPTY0 = K_QD_FULL0 + kStages, K_SD_FULL = K_QD_EMPTY0 + kStages, K_PD_FULL, K_DONE, K_NUM_BARS };
+enum BarK { K_RES_FULL = 0, K_QD_FULL0, K_QD_EMPTY0 = K_QD_FULL0 + kStages, K_S_FULL = K_QD_EMPTY0 + kStages, K_DP_FULL, K_P_FREE, K_DS_FREE,
+            K_S_READ, K_DP_READ, K_P_FULL, K_DS_FULL, K_NUM_BARS };   // K_S_READ and later: one arrival per element-wise warp
 }
 
 template <int D_QK>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(dbt::kDkvThreads, 1)
 dense_bwd_dkdv_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_constant__ CUtensorMap tmap_k,
                          const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_q,
                          const __grid_constant__ CUtensorMap tmap_do) {
@@ -359,6 +398,7 @@ dense_bwd_dkdv_tc_kernel(const __grid_constant__ DenseKernelParams p, const __gr
   volatile int* sAbort = reinterpret_cast<volatile int*>(smem + L::MISC_OFF + 8);   // set by an element-wise thread whose wait expired
   int* status = &g_dense_bwd_tc_status;
 
+  pdl_allow_dependents();      // the dQ kernel needs nothing of this one: its CTAs fill the SMs that run out of key tiles
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int b = blockIdx.z, head = blockIdx.y;
   const int q0 = __ldg(p.cu_q + b), lq = __ldg(p.cu_q + b + 1) - q0;
@@ -374,41 +414,50 @@ dense_bwd_dkdv_tc_kernel(const __grid_constant__ DenseKernelParams p, const __gr
   const int jb_lo = p.is_causal ? min(jb_hi, max(0, n_base - (lk - lq)) >> 6) : 0;
   const int nstep = jb_hi - jb_lo;
 
-  if (tid == 0) {
-    for (int i = 0; i < K_NUM_BARS; ++i) tc::mbar_init(bar(i), i == K_PD_FULL ? 128 : 1);
-    tc::fence_mbar_init();
-    *sAbort = 0;
+  auto load_queries = [&](int j) {
+    const int st = j % kStages, tok = q0 + (jb_lo + j) * 64;
+    const uint32_t stage = sStg + st * L::kStage;
+    tc::mbar_arrive_expect_tx(bar(K_QD_FULL0 + st), L::kStage);
+#pragma unroll
+    for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(stage + c * kStgChunk, &tmap_q, c * 64, head, tok, bar(K_QD_FULL0 + st));
+#pragma unroll
+    for (int c = 0; c < 2; ++c) tc::tma_load_3d(stage + L::kStgA + c * kStgChunk, &tmap_do, c * 64, head, tok, bar(K_QD_FULL0 + st));
+  };
+  if (warp == kEwWarps) {
+    // as in the dQ kernel: barriers and first loads before the others have tensor memory
+    if (tc::elect_one()) {
+      for (int i = 0; i < K_NUM_BARS; ++i) tc::mbar_init(bar(i), i >= K_S_READ ? kEwWarps : 1);
+      tc::fence_mbar_init();
+      tc::fence_proxy_async_smem();
+      *sAbort = 0;
+      if (nstep > 0) {
+        tc::mbar_arrive_expect_tx(bar(K_RES_FULL), L::kResA + L::kResB);
+#pragma unroll
+        for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(sK + c * kResChunk, &tmap_k, c * 64, head, k0 + n_base, bar(K_RES_FULL));
+#pragma unroll
+        for (int c = 0; c < 2; ++c) tc::tma_load_3d(sV + c * kResChunk, &tmap_v, c * 64, head, k0 + n_base, bar(K_RES_FULL));
+        for (int j = 0; j < min(kStages, nstep); ++j) load_queries(j);
+      }
+    }
+    __syncwarp();
   }
-  if (warp == 5) tc::tmem_alloc(sbase + L::MISC_OFF, 512);
+  if (warp == kEwWarps + 1) tc::tmem_alloc(sbase + L::MISC_OFF, 512);
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *sTmem;
-  constexpr int TM_DV = 0, TM_DK = 128, TM_ST = 320, TM_DPT = 448;
+  constexpr int TM_DV = 0, TM_DK = 128, TM_ST = 320, TM_DPT = 384, TM_P = 448, TM_DS = 480;
 
-  if (warp == 4) {
+  if (warp == kEwWarps) {
     // ================================ TMA producer =====================================
-    if (tc::elect_one() && nstep > 0) {
-      tc::mbar_arrive_expect_tx(bar(K_RES_FULL), L::kResA + L::kResB);
-#pragma unroll
-      for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(sK + c * kResChunk, &tmap_k, c * 64, head, k0 + n_base, bar(K_RES_FULL));
-#pragma unroll
-      for (int c = 0; c < 2; ++c) tc::tma_load_3d(sV + c * kResChunk, &tmap_v, c * 64, head, k0 + n_base, bar(K_RES_FULL));
+    if (tc::elect_one()) {
       bool alive = true;
-      for (int j = 0; j < nstep && alive; ++j) {
-        const int st = j % kStages;
-        const uint32_t stage = sStg + st * L::kStage;
-        const int tok = q0 + (jb_lo + j) * 64;
-        alive = tc::mbar_wait(bar(K_QD_EMPTY0 + st), ((j / kStages) & 1) ^ 1, status, 61);
-        if (!alive) break;
-        tc::mbar_arrive_expect_tx(bar(K_QD_FULL0 + st), L::kStage);
-#pragma unroll
-        for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(stage + c * kStgChunk, &tmap_q, c * 64, head, tok, bar(K_QD_FULL0 + st));
-#pragma unroll
-        for (int c = 0; c < 2; ++c) tc::tma_load_3d(stage + L::kStgA + c * kStgChunk, &tmap_do, c * 64, head, tok, bar(K_QD_FULL0 + st));
+      for (int j = kStages; j < nstep && alive; ++j) {
+        alive = tc::mbar_wait(bar(K_QD_EMPTY0 + j % kStages), ((j / kStages) & 1) ^ 1, status, 61);
+        if (alive) load_queries(j);
       }
     }
-  } else if (warp == 5) {
+  } else if (warp == kEwWarps + 1) {
     // ================================ MMA issuer =======================================
     constexpr uint32_t idesc_sd = tc::idesc_bf16_f32(128, 64, 0, 0);
     constexpr uint32_t idesc_dv = tc::idesc_bf16_f32(128, 128, 0, 1);
@@ -421,159 +470,180 @@ dense_bwd_dkdv_tc_kernel(const __grid_constant__ DenseKernelParams p, const __gr
     const uint64_t desc_dot = tc::smem_desc_sw128(sStg + L::kStgA, kStgChunk, 1024);  // dO tile, MN-major (B of dV)
     bool alive = nstep > 0;
     if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(K_RES_FULL), 0, status, 62));
-    // waits for the tile of step j, clears its rows past the end of the sequence, issues S^T(j)
+    // waits (whole warp) for phase `ph` of barrier `i`
+    auto wait = [&](int i, int ph, int code) {
+      if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(i), ph, status, code));
+      return alive;
+    };
+    // S^T of step j, once its tile has landed and S^T of step j-1 has been read; rows past the end of the sequence
+    // are cleared first
     auto issue_st = [&](int j) {
-      const int st = j % kStages, bf = j & 1;
-      alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(K_QD_FULL0 + st), (j / kStages) & 1, status, 63));
-      if (!alive) return;
+      const int st = j % kStages;
+      if (!wait(K_QD_FULL0 + st, (j / kStages) & 1, 63)) return;
       const int rows_valid = lq - (jb_lo + j) * 64;
       if (rows_valid < 64) zero_stage_tail(smem + L::STG_OFF + st * L::kStage, L::NCH + 2, rows_valid, lane);
+      if (!wait(K_S_READ, (j & 1) ^ 1, 64)) return;
       tc::tc_fence_after();
       if (tc::elect_one()) {
-        dispatch_stage_buffer(st, bf, [&](auto ST, auto BF) {
-          mma_res_stg<L::NCH>(tmem + TM_ST + decltype(BF)::value * 64, desc_k, tc::desc_advance(desc_q, decltype(ST)::value * L::kStage), idesc_sd);
-        });
+        mma_res_stg<L::NCH>(tmem + TM_ST, desc_k, tc::desc_advance(desc_q, st * L::kStage), idesc_sd);
+        tc::tc_commit(bar(K_S_FULL));
       }
       __syncwarp();
     };
     auto issue_dpt = [&](int j) {
-      const int st = j % kStages;
+      if (!wait(K_DP_READ, (j & 1) ^ 1, 67)) return;
+      tc::tc_fence_after();
       if (tc::elect_one()) {
-        dispatch_stage_buffer(st, 0, [&](auto ST, auto) {
-          mma_res_stg<2>(tmem + TM_DPT, desc_v, tc::desc_advance(desc_do, decltype(ST)::value * L::kStage), idesc_sd);
-        });
-        tc::tc_commit(bar(K_SD_FULL));
+        mma_res_stg<2>(tmem + TM_DPT, desc_v, tc::desc_advance(desc_do, (j % kStages) * L::kStage), idesc_sd);
+        tc::tc_commit(bar(K_DP_FULL));
       }
       __syncwarp();
     };
     if (alive) issue_st(0);
     if (alive) issue_dpt(0);
     for (int j = 0; j < nstep && alive; ++j) {
-      const int st = j % kStages, bf = j & 1;
-      if (j + 1 < nstep) issue_st(j + 1);
-      if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(K_PD_FULL), j & 1, status, 64));
-      if (!alive) break;
+      const int st = j % kStages;
+      if (j + 1 < nstep) {
+        issue_st(j + 1);
+        issue_dpt(j + 1);
+      }
+      if (!wait(K_P_FULL, j & 1, 68)) break;
       tc::tc_fence_after();
       if (tc::elect_one()) {
-        dispatch_stage_buffer(st, bf, [&](auto ST, auto BF) {
-          constexpr int kOff = decltype(ST)::value * L::kStage;
-          mma_tmem_stg(tmem + TM_DV, tmem + TM_ST + decltype(BF)::value * 64, tc::desc_advance(desc_dot, kOff), idesc_dv, j == 0);
-          mma_tmem_stg(tmem + TM_DK, tmem + TM_DPT, tc::desc_advance(desc_qt, kOff), idesc_dk, j == 0);
-        });
-        if (j + 1 >= nstep) tc::tc_commit(bar(K_DONE));
+        mma_tmem_stg(tmem + TM_DV, tmem + TM_P, tc::desc_advance(desc_dot, st * L::kStage), idesc_dv, j == 0);
+        tc::tc_commit(bar(K_P_FREE));
       }
       __syncwarp();
-      // dP^T of the next step goes into the buffer that the dK instructions above read (the tensor
-      // pipe runs them in order); the stage of step j is handed back right after its last readers
-      if (tc::elect_one()) tc::tc_commit(bar(K_QD_EMPTY0 + st));
+      if (!wait(K_DS_FULL, j & 1, 69)) break;
+      tc::tc_fence_after();
+      if (tc::elect_one()) {
+        mma_tmem_stg(tmem + TM_DK, tmem + TM_DS, tc::desc_advance(desc_qt, st * L::kStage), idesc_dk, j == 0);
+        tc::tc_commit(bar(K_DS_FREE));             // completes after dV of this step: the tensor pipe runs in order
+        tc::tc_commit(bar(K_QD_EMPTY0 + st));
+      }
       __syncwarp();
-      if (j + 1 < nstep) issue_dpt(j + 1);
     }
   } else {
     // ================================ element-wise / epilogue ==========================
-    const int key = n_base + tid;
-    const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
+    // warps w and w + 4 share the TMEM lanes of 32 keys: warp w takes queries [0, 32) of every block, warp w + 4 the rest
+    const int half = warp >> 2, rl = tid & 127;
+    const int key = n_base + rl;
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int shift = lk - lq;                                 // query i sees keys <= i + shift
+    // per-query vectors of a step: lse * log2(e) (threads 0-63) and delta (threads 64-127); each value is loaded one
+    // step ahead, so that no step waits for global memory
+    auto load_vec = [&](int j) {
+      const int i = (jb_lo + j) * 64 + (tid & 63);
+      if (tid >= 128 || i >= lq) return 0.f;
+      return tid < 64 ? __ldg(p.lse + (int64_t)(q0 + i) * p.lse_stride_t + head * p.lse_stride_h) * kLog2e
+                      : __ldg(p.delta + (int64_t)head * p.total_q + q0 + i);
+    };
+    float v_next = nstep > 0 ? load_vec(0) : 0.f;
     bool alive = true;
     for (int j = 0; j < nstep && alive; ++j) {
-      const int jb = jb_lo + j, st = j & 1;
-      // per-query vectors of this step: lse * log2(e) (threads 0-63) and delta (threads 64-127)
-      {
-        const int i = jb * 64 + (tid & 63);
-        float v = 0.f;
-        if (i < lq) {
-          v = tid < 64 ? __ldg(p.lse + (int64_t)(q0 + i) * p.lse_stride_t + head * p.lse_stride_h) * kLog2e
-                       : __ldg(p.delta + (int64_t)head * p.total_q + q0 + i);
-        }
-        sVec[st * 128 + tid] = v;
-      }
-      if (!tc::mbar_wait(bar(K_SD_FULL), j & 1, status, 65)) *sAbort = 1;
-      bar_sync(1, 128);                                        // vectors visible; also keeps the two buffers of sVec apart
-      if (*sAbort) { alive = false; break; }                   // read right after the barrier: the same for all 128 threads
+      const int jb = jb_lo + j, vb = j & 1;
+      if (tid < 128) sVec[vb * 128 + tid] = v_next;
+      if (j + 1 < nstep) v_next = load_vec(j + 1);
+      if (!tc::mbar_wait(bar(K_S_FULL), j & 1, status, 65)) *sAbort = 1;
+      bar_sync(1, kEwWarps * 32);                              // vectors visible; also keeps the two buffers of sVec apart
+      if (*sAbort) { alive = false; break; }                   // read right after the barrier: the same for all threads
       tc::tc_fence_after();
-      uint32_t sv[2][32], dp[2][32];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        tc::tmem_ld32(tmem + lane_addr + TM_ST + st * 64 + c * 32, sv[c]);
-        tc::tmem_ld32(tmem + lane_addr + TM_DPT + c * 32, dp[c]);
-      }
+      uint32_t sv[32], dp[32], pk[16];
+      tc::tmem_ld32(tmem + lane_addr + TM_ST + half * 32, sv);
       tc::tmem_wait_ld();
-      const int c_max = lq - jb * 64;                          // columns (queries) [c_min, c_max) see this key
-      const int c_min = p.is_causal ? key - shift - jb * 64 : 0;
-      const float4* vl = reinterpret_cast<const float4*>(sVec + st * 128);
-      const float4* vd = reinterpret_cast<const float4*>(sVec + st * 128 + 64);
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t pp[16], pd[16];
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(bar(K_S_READ));
+      const int c_max = lq - jb * 64 - half * 32;              // columns (queries) [c_min, c_max) see this key
+      const int c_min = p.is_causal ? key - shift - jb * 64 - half * 32 : 0;
+      const bool all_visible = __all_sync(0xffffffffu, c_min <= 0 && c_max >= 32);
+      const float4* vl = reinterpret_cast<const float4*>(sVec + vb * 128 + half * 32);
+      const float4* vd = reinterpret_cast<const float4*>(sVec + vb * 128 + 64 + half * 32);
+      auto to_p = [&](auto masked) {
 #pragma unroll
         for (int i4 = 0; i4 < 8; ++i4) {
-          const float4 l4 = vl[c * 8 + i4], d4 = vd[c * 8 + i4];
-          const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, ds[4] = {d4.x, d4.y, d4.z, d4.w};
-          float pv[4], dv[4];
+          const float4 l4 = vl[i4];
+          const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const int col = c * 32 + i4 * 4 + e;
-            const bool vis = col >= c_min && col < c_max;
-            const float pe = exp2f(fmaf(__uint_as_float(sv[c][i4 * 4 + e]), p.scale_log2, -ls[e]));
-            // selects, not products: masked entries may hold Inf or NaN
-            pv[e] = vis ? pe : 0.f;
-            dv[e] = vis ? pe * (__uint_as_float(dp[c][i4 * 4 + e]) - ds[e]) : 0.f;
+            const int col = i4 * 4 + e;
+            float pe = exp2f(fmaf(__uint_as_float(sv[col]), p.scale_log2, -ls[e]));
+            if constexpr (decltype(masked)::value) pe = col >= c_min && col < c_max ? pe : 0.f;      // a select: see the dQ kernel
+            sv[col] = __float_as_uint(pe);
           }
-          pp[i4 * 2] = pack_bf16x2(pv[0], pv[1]);
-          pp[i4 * 2 + 1] = pack_bf16x2(pv[2], pv[3]);
-          pd[i4 * 2] = pack_bf16x2(dv[0], dv[1]);
-          pd[i4 * 2 + 1] = pack_bf16x2(dv[2], dv[3]);
+          pk[i4 * 2] = pack_bf16x2(__uint_as_float(sv[i4 * 4]), __uint_as_float(sv[i4 * 4 + 1]));
+          pk[i4 * 2 + 1] = pack_bf16x2(__uint_as_float(sv[i4 * 4 + 2]), __uint_as_float(sv[i4 * 4 + 3]));
         }
-        tc::tmem_st16(tmem + lane_addr + TM_ST + st * 64 + c * 16, pp);
-        tc::tmem_st16(tmem + lane_addr + TM_DPT + c * 16, pd);
-      }
+      };
+      if (all_visible) to_p(std::false_type{});
+      else to_p(std::true_type{});
+      // a wait that gives up here lets the step run on; the flag ends the loop at the next barrier
+      if (!tc::mbar_wait(bar(K_P_FREE), (j & 1) ^ 1, status, 70)) *sAbort = 1;       // dV of step j-1 has read P^T
+      tc::tc_fence_after();
+      __syncwarp();
+      tc::tmem_st16(tmem + lane_addr + TM_P + half * 16, pk);
       tc::tmem_wait_st();
       tc::tc_fence_before();
-      tc::mbar_arrive(bar(K_PD_FULL));
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(bar(K_P_FULL));
+      if (!tc::mbar_wait(bar(K_DP_FULL), j & 1, status, 71)) *sAbort = 1;
+      tc::tc_fence_after();
+      __syncwarp();
+      tc::tmem_ld32(tmem + lane_addr + TM_DPT + half * 32, dp);
+      tc::tmem_wait_ld();
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(bar(K_DP_READ));
+      auto to_ds = [&](auto masked) {
+#pragma unroll
+        for (int i4 = 0; i4 < 8; ++i4) {
+          const float4 d4 = vd[i4];
+          const float ds[4] = {d4.x, d4.y, d4.z, d4.w};
+          float dv[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int col = i4 * 4 + e;
+            dv[e] = __uint_as_float(sv[col]) * (__uint_as_float(dp[col]) - ds[e]);
+            if constexpr (decltype(masked)::value) dv[e] = col >= c_min && col < c_max ? dv[e] : 0.f;
+          }
+          pk[i4 * 2] = pack_bf16x2(dv[0], dv[1]);
+          pk[i4 * 2 + 1] = pack_bf16x2(dv[2], dv[3]);
+        }
+      };
+      if (all_visible) to_ds(std::false_type{});
+      else to_ds(std::true_type{});
+      if (!tc::mbar_wait(bar(K_DS_FREE), (j & 1) ^ 1, status, 72)) *sAbort = 1;      // dK of step j-1 has read dS^T
+      tc::tc_fence_after();
+      __syncwarp();
+      tc::tmem_st16(tmem + lane_addr + TM_DS + half * 16, pk);
+      tc::tmem_wait_st();
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(bar(K_DS_FULL));
     }
     bool have = nstep > 0 && alive;
     if (have) {
-      have = __all_sync(0xffffffffu, tc::mbar_wait(bar(K_DONE), 0, status, 66));
+      have = __all_sync(0xffffffffu, tc::mbar_wait(bar(K_DS_FREE), (nstep - 1) & 1, status, 66));   // the last dK, hence all of them
       tc::tc_fence_after();
     }
     const bool row_ok = key < lk;
     __nv_bfloat16* dv_row = reinterpret_cast<__nv_bfloat16*>(p.dv) + (int64_t)(k0 + key) * p.dv_stride_t + head * p.dv_stride_h;
     __nv_bfloat16* dk_row = reinterpret_cast<__nv_bfloat16*>(p.dk) + (int64_t)(k0 + key) * p.dk_stride_t + head * p.dk_stride_h;
 #pragma unroll 1
-    for (int c = 0; c < (128 + D_QK) / 32; ++c) {
-      uint32_t ov[32];
-      if (have) {
-        tc::tmem_ld32(tmem + lane_addr + c * 32, ov);          // dV columns first, then dK
-        tc::tmem_wait_ld();
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) ov[i] = 0u;
-      }
-      const float mul = c < 4 ? 1.f : p.scale;
-      __nv_bfloat16* dst = c < 4 ? dv_row + c * 32 : dk_row + (c - 4) * 32;
-      if (row_ok) {
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          uint4 v;
-          v.x = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 0]) * mul, __uint_as_float(ov[q4 * 8 + 1]) * mul);
-          v.y = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 2]) * mul, __uint_as_float(ov[q4 * 8 + 3]) * mul);
-          v.z = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 4]) * mul, __uint_as_float(ov[q4 * 8 + 5]) * mul);
-          v.w = pack_bf16x2(__uint_as_float(ov[q4 * 8 + 6]) * mul, __uint_as_float(ov[q4 * 8 + 7]) * mul);
-          *reinterpret_cast<uint4*>(dst + q4 * 8) = v;
-        }
-      }
-    }
+    for (int c = half; c < (128 + D_QK) / 32; c += 2)          // dV columns first, then dK
+      store_grad_chunk(tmem + lane_addr + c * 32, have, row_ok, c < 4 ? 1.f : p.scale, c < 4 ? dv_row + c * 32 : dk_row + (c - 4) * 32);
   }
 
   tc::tc_fence_before();
   __syncthreads();
-  if (warp == 5) tc::tmem_dealloc(tmem, 512);
+  if (warp == kEwWarps + 1) tc::tmem_dealloc(tmem, 512);
 }
 
 // ---- host side ----------------------------------------------------------------------------------
 template <int D_QK>
 static cudaError_t launch_bwd_tc(const DenseKernelParams& p, cudaStream_t stream) {
-  using L = dbt::Layout<D_QK>;
+  using namespace dbt;
+  using L = Layout<D_QK>;
   CUtensorMap q128, do128, k64, v64, k128, v128, q64, do64;
   bool ok = tmah::make_map_thd(&q128, p.q, p.d_qk, p.h_q, p.total_q, p.q_stride_h, p.q_stride_t, 128) &&
             tmah::make_map_thd(&q64, p.q, p.d_qk, p.h_q, p.total_q, p.q_stride_h, p.q_stride_t, 64) &&
@@ -584,17 +654,16 @@ static cudaError_t launch_bwd_tc(const DenseKernelParams& p, cudaStream_t stream
             tmah::make_map_thd(&v128, p.v, p.d_v, p.h_k, p.total_k, p.v_stride_h, p.v_stride_t, 128) &&
             tmah::make_map_thd(&v64, p.v, p.d_v, p.h_k, p.total_k, p.v_stride_h, p.v_stride_t, 64);
   if (!ok) return cudaErrorInvalidValue;
-  auto kq = dense_bwd_dq_tc_kernel<D_QK>;
-  auto kk = dense_bwd_dkdv_tc_kernel<D_QK>;
-  cudaError_t e = cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM_BYTES);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(kk, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM_BYTES);
-  if (e != cudaSuccess) return e;
-  const int rows = p.total_q * p.h_q;
-  dense_bwd_delta_tc_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(p);
-  kk<<<dim3((p.max_seqlen_k + 127) / 128, p.h_q, p.batch), 192, L::SMEM_BYTES, stream>>>(p, k128, v128, q64, do64);
-  kq<<<dim3((p.max_seqlen_q + 127) / 128, p.h_q, p.batch), 224, L::SMEM_BYTES, stream>>>(p, q128, do128, k64, v64);
-  return cudaGetLastError();
+  constexpr auto kq = dense_bwd_dq_tc_kernel<D_QK>;
+  constexpr auto kk = dense_bwd_dkdv_tc_kernel<D_QK>;
+  if (cudaError_t e = allow_smem<kq>(L::SMEM_BYTES); e != cudaSuccess) return e;
+  if (cudaError_t e = allow_smem<kk>(L::SMEM_BYTES); e != cudaSuccess) return e;
+  const int64_t rows = (int64_t)p.total_q * p.h_q;
+  const int64_t per_block = 16 * kDeltaRows;
+  dense_bwd_delta_tc_kernel<<<static_cast<unsigned>((rows + per_block - 1) / per_block), 256, 0, stream>>>(p);
+  kk<<<dim3((p.max_seqlen_k + 127) / 128, p.h_q, p.batch), kDkvThreads, L::SMEM_BYTES, stream>>>(p, k128, v128, q64, do64);
+  if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
+  return launch_dependent(kq, dim3((p.max_seqlen_q + 127) / 128, p.h_q, p.batch), kDqThreads, L::SMEM_BYTES, stream, p, q128, do128, k64, v64);
 }
 
 cudaError_t launch_dense_bwd_tc(const DenseKernelParams& p, cudaStream_t stream) {
