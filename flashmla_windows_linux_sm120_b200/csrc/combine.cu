@@ -40,8 +40,9 @@ __device__ __forceinline__ float combine_weights(int nparts, LseAt lse_at, float
 // Weighted sum of the parts over column groups [first, first + NG) of 128 columns (lane = 4 columns of a group), in the
 // order of the parts.  A part with weight 0 is not read: 0 * (Inf or NaN) must not reach the sum.
 // COHERENT: the partial outputs may have been written by another GPU while this kernel was already resident (peer
-// merge), so they are read with ld.global.cv instead of the non-coherent path, which is undefined for memory modified
-// during the kernel's lifetime.
+// merge), so they are read with ld.global.cv.  Otherwise plain loads: the merge of a decode call is resident, waiting in
+// pdl_wait(), while the attention kernel writes the partials, and the non-coherent path (__ldg) is undefined for memory
+// modified during the kernel's lifetime.
 template <int NG, bool COHERENT, class OAt>
 __device__ __forceinline__ void combine_columns(int nparts, OAt o_at, const float* s_w, __nv_bfloat16* out_row, int first, bool f16) {
   const int lane = threadIdx.x & 31;
@@ -57,7 +58,7 @@ __device__ __forceinline__ void combine_columns(int nparts, OAt o_at, const floa
       if (w[u] == 0.f) continue;
       const float4* src = reinterpret_cast<const float4*>(o_at(i0 + u)) + first * 32 + lane;
 #pragma unroll
-      for (int j = 0; j < NG; ++j) v[u][j] = COHERENT ? __ldcv(src + j * 32) : __ldg(src + j * 32);
+      for (int j = 0; j < NG; ++j) v[u][j] = COHERENT ? __ldcv(src + j * 32) : src[j * 32];
     }
 #pragma unroll
     for (int u = 0; u < kPartsInFlight; ++u) {
@@ -94,9 +95,9 @@ __device__ __forceinline__ void combine_row(int nparts, LseAt lse_at, OAt o_at, 
 template <int WPR>
 __global__ void __launch_bounds__(kCombineWarps * 32) decode_combine_kernel(const __grid_constant__ DecodeKernelParams p) {
   extern __shared__ float s_weights[];  // [8][num_sm_parts]
-  pdl_wait();                           // launched as a programmatic dependent of the attention kernel
+  pdl_wait();                           // launched as a programmatic dependent of the attention kernel: plain loads from here on
   const int batch = blockIdx.x;
-  const int lo = __ldg(p.num_splits + batch), hi = __ldg(p.num_splits + batch + 1);
+  const int lo = p.num_splits[batch], hi = p.num_splits[batch + 1];
   const int nparts = hi - lo;
   if (nparts <= 1) return;
   const int q_seq_per_hk = p.s_q * p.hq_per_hk;
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(kCombineWarps * 32) decode_combine_kernel(cons
   const float* o_base = p.o_accum + ((int64_t)lo * rows + r) * 512;
   const int64_t part_stride = rows;
   float* w = s_weights + warp * p.num_sm_parts;
-  const float glse = combine_weights(nparts, [&](int i) { return __ldg(lse_base + i * part_stride); }, w);
+  const float glse = combine_weights(nparts, [&](int i) { return lse_base[i * part_stride]; }, w);
   if (sub == 0 && (threadIdx.x & 31) == 0) p.softmax_lse[((int64_t)batch * p.h_q + head) * p.s_q + sq] = glse * kLn2;
   combine_columns<4 / WPR, false>(
       nparts, [&](int i) { return o_base + i * part_stride * 512; }, w,

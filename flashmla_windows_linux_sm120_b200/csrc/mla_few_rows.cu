@@ -157,7 +157,10 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
-  pdl_wait();                   // the schedule, the queries and the cache may come from the kernel in front of this one
+  // The schedule, the queries and the cache may come from the kernel in front of this one.  From here on plain loads (not
+  // __ldg, which the compiler may move above the wait and whose path is undefined for memory that is written while this
+  // kernel is resident) read the schedule, the lengths, the block table and the indices; the FP8 records hang on those.
+  pdl_wait();
   pdl_allow_dependents();       // the merge kernel may become resident now
   const uint32_t tmem = *sTmem;
 
@@ -174,8 +177,8 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
   }
   const int tile_heads = min(hq - hb * 64, 64), nrows = ntok * tile_heads, head0 = kh * hq + hb * 64;
   const int* md_row = p.tile_scheduler_metadata + blockIdx.z * 8;
-  const int4 md = __ldg(reinterpret_cast<const int4*>(md_row));
-  const int begin_idx = md.x, begin_block = md.y, end_idx = md.z, end_block = md.w, begin_split = __ldg(md_row + 4);
+  const int4 md = *reinterpret_cast<const int4*>(md_row);
+  const int begin_idx = md.x, begin_block = md.y, end_idx = md.z, end_block = md.w, begin_split = md_row[4];
   const int n_work = begin_idx >= p.b ? 0 : end_idx - begin_idx + 1;
   // dense: query token t of the sequence sees keys below seqlen - (s_q - 1 - t)
   const int lag_first = MODE == kDense && p.is_causal ? p.s_q - 1 - sq0 : 0, lag_last = MODE == kDense && p.is_causal ? p.s_q - sq0 - ntok : 0;
@@ -183,7 +186,7 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
   auto request = [&](int wi) {
     Req r;
     r.batch = begin_idx + wi;
-    r.seqlen = SPARSE ? p.topk : __ldg(p.seqlens_k + r.batch);
+    r.seqlen = SPARSE ? p.topk : p.seqlens_k[r.batch];
     const int total = (r.seqlen + 63) >> 6, seen = r.seqlen - lag_last;
     r.blk_lo = r.batch == begin_idx ? begin_block : 0;
     r.blk_hi = min(r.batch == end_idx ? min(end_block, total) : total, seen > 0 ? (seen + 63) >> 6 : 0);
@@ -216,10 +219,10 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
         ++req;
         if constexpr (SPARSE) continue;
         const int* bt = p.block_table + (int64_t)r.batch * p.block_table_stride_b;
-        int page_next = __ldg(bt + r.blk_lo);
+        int page_next = bt[r.blk_lo];
         for (int blk = r.blk_lo; blk < r.blk_hi && alive; ++blk, ++g) {
           const int page = page_next, full = bar(KV_FULL0 + g % kPageBars);
-          if (blk + 1 < r.blk_hi) page_next = __ldg(bt + blk + 1);
+          if (blk + 1 < r.blk_hi) page_next = bt[blk + 1];
           alive = tc::mbar_wait(bar(ROPE_EMPTY0 + g % L::kRopeSlots), ((g / L::kRopeSlots) & 1) ^ 1, status, 202);
           if (!alive) break;
           // (page g - 4 has left the ring before page g starts to enter it, so its full barrier has turned over)
@@ -259,7 +262,7 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
         if (p.indices_logical) {       // token position of the request -> physical slot through its block table
           const int pos = v;
           v = -1;
-          if (pos >= 0 && pos < __ldg(p.seqlens_k + batch)) v = __ldg(p.block_table + batch * p.block_table_stride_b + (pos >> 6)) * 64 + (pos & 63);
+          if (pos >= 0 && pos < p.seqlens_k[batch]) v = p.block_table[batch * p.block_table_stride_b + (pos >> 6)] * 64 + (pos & 63);
         }
         return (v < 0 || v >= p.num_blocks * 64) ? -1 : v;
       };
@@ -276,7 +279,7 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
       int raw = -1, raw_batch = 0;
       auto read_indices = [&] {        // lanes 0..7: row 8 gw + lane of the next unread block
         if (c_wi >= n_work) return false;
-        raw = __ldg(c_r.idx + c_blk * 64 + gw * 8 + (lane & 7));
+        raw = c_r.idx[c_blk * 64 + gw * 8 + (lane & 7)];
         raw_batch = c_r.batch;
         ++c_blk;
         skip();
@@ -569,8 +572,8 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
       }
 
       // ---- epilogue of this work item ---------------------------------------------------
-      const int lo = __ldg(p.num_splits + r.batch);
-      const bool no_split = !p.force_partial && __ldg(p.num_splits + r.batch + 1) - lo == 1;
+      const int lo = p.num_splits[r.batch];
+      const bool no_split = !p.force_partial && p.num_splits[r.batch + 1] - lo == 1;
       const int64_t slot = lo + (r.batch == begin_idx ? begin_split : 0);
       const int64_t part_row = (slot * p.h_k + kh) * (int64_t)p.s_q * hq + sq0 * hq + hb * 64;      // row 0 of the tile in its partial slot
       bar_sync(1, 128);

@@ -235,7 +235,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
   __syncthreads();
   tc::cluster_sync_all();      // barriers of both CTAs exist before anything is sent to them
   tc::tc_fence_after();
-  pdl_wait();                  // the schedule, the queries and the cache may come from the kernel in front of this one
+  pdl_wait();                  // the schedule, the queries and the cache may come from the kernel in front of this one (loads: mla_work.cuh)
   pdl_allow_dependents();      // a merge kernel launched as a programmatic dependent may become resident now
   const uint32_t tmem = *sTmem;
   const Tile tile = make_tile<WM>(P);           // both CTAs of a pair see the same schedule row (possibly an empty one)
@@ -266,20 +266,20 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
       // the indices of a block are read one block ahead of their use: their latency would otherwise be paid in
       // every turn of this loop
       const int* my_idx = r.idx + 32 * static_cast<int>(rank) + lane;
-      int mine_next = r.blk_lo < r.blk_hi ? __ldg(my_idx + r.blk_lo * 64) : -1, i0_next = -1, i1_next = -1;
+      int mine_next = r.blk_lo < r.blk_hi ? my_idx[r.blk_lo * 64] : -1, i0_next = -1, i1_next = -1;
       if (warp == 4 && r.blk_lo < r.blk_hi) {
-        i0_next = __ldg(r.idx + r.blk_lo * 64 + lane);
-        i1_next = __ldg(r.idx + r.blk_lo * 64 + 32 + lane);
+        i0_next = r.idx[r.blk_lo * 64 + lane];
+        i1_next = r.idx[r.blk_lo * 64 + 32 + lane];
       }
       for (int blk = r.blk_lo; blk < r.blk_hi && alive; ++blk, ++g) {
         const int st = g % kKStages;
         int mine = mine_next;                                                          // row `lane` of this CTA's part
         const int i0 = i0_next, i1 = i1_next;
         if (blk + 1 < r.blk_hi) {
-          mine_next = __ldg(my_idx + (blk + 1) * 64);
+          mine_next = my_idx[(blk + 1) * 64];
           if (warp == 4) {
-            i0_next = __ldg(r.idx + (blk + 1) * 64 + lane);
-            i1_next = __ldg(r.idx + (blk + 1) * 64 + 32 + lane);
+            i0_next = r.idx[(blk + 1) * 64 + lane];
+            i1_next = r.idx[(blk + 1) * 64 + 32 + lane];
           }
         }
         if (mine < 0 || mine >= s_kv) mine = -1;
@@ -329,7 +329,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
       if (p.indices_logical) {       // token position of the request -> physical slot through its block table
         const int pos = v;
         v = -1;
-        if (pos >= 0 && pos < __ldg(p.seqlens_k + batch)) v = __ldg(p.block_table + batch * p.block_table_stride_b + (pos >> 6)) * 64 + (pos & 63);
+        if (pos >= 0 && pos < p.seqlens_k[batch]) v = p.block_table[batch * p.block_table_stride_b + (pos >> 6)] * 64 + (pos & 63);
       }
       return (v < 0 || v >= p.num_blocks * 64) ? -1 : v;
     };
@@ -355,10 +355,10 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
     struct Raw { int mine, t0, t1, batch; };
     auto read_indices = [&](Raw& w) -> bool {
       if (c_wi >= tile.n_work) return false;
-      w.mine = __ldg(c_r.idx + c_blk * 64 + 32 * static_cast<int>(rank) + gw * 8 + (lane & 7));
+      w.mine = c_r.idx[c_blk * 64 + 32 * static_cast<int>(rank) + gw * 8 + (lane & 7)];
       if (publisher) {
-        w.t0 = __ldg(c_r.idx + c_blk * 64 + lane);
-        w.t1 = __ldg(c_r.idx + c_blk * 64 + 32 + lane);
+        w.t0 = c_r.idx[c_blk * 64 + lane];
+        w.t1 = c_r.idx[c_blk * 64 + 32 + lane];
       }
       w.batch = c_r.batch;
       for (int i = 0; i < kDecodeGatherGroups; ++i) advance();
@@ -455,18 +455,18 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
         // 64-row map, whose boxes cover a page in 9 pieces)
         if (pf > 0 && rank == 0) {
           for (int blk = r.blk_lo; blk < min(r.blk_lo + pf, r.blk_hi); ++blk) {
-            const int pg = __ldg(bt + blk);
+            const int pg = bt[blk];
 #pragma unroll
             for (int c = 0; c < 9; ++c) tc::tma_prefetch_l2_4d(&tmap_v64, c * 64, tile.kh, 0, pg);
           }
         }
-        int page_next = __ldg(bt + r.blk_lo);
+        int page_next = bt[r.blk_lo];
         for (int blk = r.blk_lo; blk < r.blk_hi; ++blk, ++g) {
           const int st = g % kKStages;
           const int page = page_next;
-          if (blk + 1 < r.blk_hi) page_next = __ldg(bt + blk + 1);
+          if (blk + 1 < r.blk_hi) page_next = bt[blk + 1];
           if (pf > 0 && rank == 0 && blk + pf < r.blk_hi) {
-            const int pg = __ldg(bt + blk + pf);
+            const int pg = bt[blk + pf];
 #pragma unroll
             for (int c = 0; c < 9; ++c) tc::tma_prefetch_l2_4d(&tmap_v64, c * 64, tile.kh, 0, pg);
           }
@@ -616,7 +616,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
         const int* bt = p.block_table + r.batch * p.block_table_stride_b;
         for (int blk = r.blk_lo; blk < r.blk_hi; ++blk, ++g) {
           const int st = g & 1;
-          const int page = __ldg(bt + blk);
+          const int page = bt[blk];
           alive = tc::mbar_wait(bar(V_EMPTY0 + st), ((g >> 1) & 1) ^ 1, status, 103);
           if (!alive) break;
           FMLA_PTRACE_AT(g, 12);
@@ -1000,7 +1000,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
         bar_sync(1, 128);
         int* sMerge = reinterpret_cast<int*>(smem + MISC_OFF + 16);
         if (tid == 0) {
-          const int lo = __ldg(p.num_splits + r.batch), nsp = __ldg(p.num_splits + r.batch + 1) - lo;
+          const int lo = p.num_splits[r.batch], nsp = p.num_splits[r.batch + 1] - lo;
           const int n_hb = p.hq_per_hk >> 6;
           int* ctr = p.arrival_counters + (((int64_t)r.batch * p.s_q + tile.sq) * p.h_k + tile.kh) * n_hb + tile.hb;
           const bool last = atomicAdd(ctr, 1) == nsp - 1;

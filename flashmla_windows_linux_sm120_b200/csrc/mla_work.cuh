@@ -1,5 +1,7 @@
 // Work decomposition of the CTA-pair MLA attention kernel (mla_pair.cu; the modes also of mla_few_rows.cu): which tile of heads and
 // which stretch of the split-KV schedule a CTA owns, and the requests / query tokens it walks.
+// The kernel is resident while the one that writes the schedule may still run, so schedule and lengths are read with plain
+// loads, after pdl_wait(): __ldg is undefined for memory written meanwhile and may be moved above the wait.
 #pragma once
 
 #include "kernels.h"
@@ -52,9 +54,9 @@ __device__ __forceinline__ Tile make_tile(const TcParams& P) {
     }
     t.head0 = t.kh * p.hq_per_hk + t.hb * 64;
     t.nvalid = min(64, p.hq_per_hk - t.hb * 64);
-    const int4 md = __ldg(reinterpret_cast<const int4*>(p.tile_scheduler_metadata + part * 8));
+    const int4 md = *reinterpret_cast<const int4*>(p.tile_scheduler_metadata + part * 8);
     t.begin_idx = md.x; t.begin_block = md.y; t.end_idx = md.z; t.end_block = md.w;
-    t.begin_split = __ldg(p.tile_scheduler_metadata + part * 8 + 4);
+    t.begin_split = p.tile_scheduler_metadata[part * 8 + 4];
     t.n_work = t.begin_idx >= p.b ? 0 : t.end_idx - t.begin_idx + 1;
   }
   return t;
@@ -75,7 +77,7 @@ __device__ __forceinline__ Work get_work(const TcParams& P, const Tile& t, int i
     w.batch = batch;
     int nblk_total, nblk_visible;
     if constexpr (MODE == kDense) {
-      w.seqlen = __ldg(p.seqlens_k + batch);
+      w.seqlen = p.seqlens_k[batch];
       nblk_total = (w.seqlen + 63) >> 6;
       w.border = p.is_causal ? w.seqlen - (p.s_q - 1 - t.sq) : w.seqlen;
       nblk_visible = w.border > 0 ? (w.border + 63) >> 6 : 0;
@@ -88,8 +90,8 @@ __device__ __forceinline__ Work get_work(const TcParams& P, const Tile& t, int i
     w.blk_lo = batch == t.begin_idx ? t.begin_block : 0;
     w.blk_hi = min(min(batch == t.end_idx ? t.end_block : nblk_total, nblk_total), nblk_visible);
     if (w.blk_hi < w.blk_lo) w.blk_hi = w.blk_lo;
-    const int lo = __ldg(p.num_splits + batch);
-    w.no_split = !p.force_partial && __ldg(p.num_splits + batch + 1) - lo == 1;
+    const int lo = p.num_splits[batch];
+    w.no_split = !p.force_partial && p.num_splits[batch + 1] - lo == 1;
     w.split_slot = lo + (batch == t.begin_idx ? t.begin_split : 0);
   }
   return w;
