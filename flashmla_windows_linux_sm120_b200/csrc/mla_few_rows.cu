@@ -58,8 +58,10 @@ struct Layout {
   static constexpr int M_OFF = X_OFF + 4 * N * 4;          // float [N]: rescale factors, then 1 / l
   static constexpr int MISC_OFF = M_OFF + N * 4;
   static constexpr int VALID_OFF = MISC_OFF + 32;          // sparse modes: 64 validity bits per page in flight
-  static constexpr int SMEM_BYTES = VALID_OFF + kPageBars * 8;
+  static constexpr int ROW_OFF = VALID_OFF + kPageBars * 8;        // int64 [N]: element offset of a row within a request's output
+  static constexpr int SMEM_BYTES = ROW_OFF + N * 8;
   static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB shared memory limit per CTA");
+  static_assert(kPBufs * N * 128 >= 4 * N * (N == 64 ? 16 : 32) * 2, "the P buffers stage the output rows of the four softmax warps");
   static_assert(kVSlots % 2 == 0 && kVSlots >= 16 && kVSlots <= 8 * (kPageBars - 1) + 1, "ring sizes");
 };
 enum Bar { Q_FULL = 0, Q_EMPTY, KV_FULL0, KV_EMPTY0 = KV_FULL0 + kPageBars, ROPE_EMPTY0 = KV_EMPTY0 + kPageBars, S_FULL0 = ROPE_EMPTY0 + 3, S_FULL1,
@@ -103,6 +105,11 @@ __device__ __forceinline__ void tmem_ld_16x256b(uint32_t taddr, uint32_t (&v)[R]
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint4 v) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 // four 8x8 matrices of 16-bit elements, each stored transposed; lane i gives the address of row i % 8 of matrix i / 8
 __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
@@ -128,6 +135,7 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
   auto bar = [&](int i) { return sbase + L::BAR_OFF + i * 8; };
   float* sX = reinterpret_cast<float*>(smem + L::X_OFF);
   float* sM = reinterpret_cast<float*>(smem + L::M_OFF);
+  int64_t* sRow = reinterpret_cast<int64_t*>(smem + L::ROW_OFF);
   volatile uint32_t* sTmem = reinterpret_cast<volatile uint32_t*>(smem + L::MISC_OFF);
   volatile int* sAbort = reinterpret_cast<volatile int*>(smem + L::MISC_OFF + 8);   // set by a softmax thread whose wait expired
   int* status = &g_decode_few_status;
@@ -440,11 +448,15 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
     constexpr int K8 = N / 8;                            // groups of 8 columns
     const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
     const int t4 = lane & 3, tr = lane >> 2;
+    // Where row `tid` of the tile goes: one division per row and CTA (it is read after the barriers of an epilogue).
+    const int my_tok = sq0 + tid / tile_heads, my_head = head0 + tid % tile_heads;
+    if (tid < N) sRow[tid] = my_tok * p.o_stride_s + my_head * p.o_stride_h;
     int g = 0, req = 0;
     bool aborted = false;        // uniform over the 128 softmax threads: only read right after a barrier
     for (int wi = 0; wi < n_work; ++wi) {
       const Req r = request(wi);
       const int nblk = r.blk_hi - r.blk_lo;
+      const int lo = p.num_splits[r.batch], hi = p.num_splits[r.batch + 1];      // here: their latency hides behind the blocks
       // per column of this thread: the scale O^T and l carry (-inf: no visible key yet), and its share of the row sum
       float m_used[K8][2], l_part[K8][2];
 #pragma unroll
@@ -572,8 +584,7 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
       }
 
       // ---- epilogue of this work item ---------------------------------------------------
-      const int lo = p.num_splits[r.batch];
-      const bool no_split = !p.force_partial && p.num_splits[r.batch + 1] - lo == 1;
+      const bool no_split = !p.force_partial && hi - lo == 1;
       const int64_t slot = lo + (r.batch == begin_idx ? begin_split : 0);
       const int64_t part_row = (slot * p.h_k + kh) * (int64_t)p.s_q * hq + sq0 * hq + hb * 64;      // row 0 of the tile in its partial slot
       bar_sync(1, 128);
@@ -599,9 +610,8 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
       if (tid < N) {
         sM[tid] = (l == 0.f || nblk == 0) ? 0.f : 1.f / l;
         if (tid < nrows) {
-          const int tok = tid / tile_heads, head = head0 + tid % tile_heads;
           if (no_split) {
-            p.softmax_lse[((int64_t)r.batch * p.h_q + head) * p.s_q + sq0 + tok] = l == 0.f ? pos_inf() : (log2f(l) + m) * kLn2;
+            p.softmax_lse[((int64_t)r.batch * p.h_q + my_head) * p.s_q + my_tok] = l == 0.f ? pos_inf() : (log2f(l) + m) * kLn2;
           } else {
             p.lse_accum[part_row + tid] = l == 0.f ? neg_inf() : log2f(l) + m;
             if (p.no_split_hint && tid == 0) tc::report_status(status, 41);     // a split request although the caller ruled it out
@@ -616,39 +626,86 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
       }
       bar_sync(1, 128);
       if (*sAbort) { aborted = true; break; }
-      // lane = value column 128 mb + 32 warp + lane, registers = query rows
+      if (no_split) {
+        // 16-bit rows, through the P buffers (free: every P V of the request has completed).  A warp transposes W of its 32 value
+        // columns at a time with stmatrix and stores rows in 16-byte pieces, a full 32-byte sector or two per row.
+        // Scattered from the lanes' columns 4 bytes at a time, 64 unsplit rows took 13 000 clk, against 4 600 now.
+        constexpr int W = N == 64 ? 16 : 32, kPieces = W / 8;
+        const uint32_t stage = sbase + L::P_OFF + warp * (N * W * 2);
+        auto piece_at = [&](int row, int piece) {      // swizzled so that eight rows of one piece fall into different banks
+          return stage + row * (W * 2) + ((piece ^ (W == 16 ? (row >> 2) & 1 : (row >> 1) & 3)) << 4);
+        };
+        float2 inv[K8];
+#pragma unroll
+        for (int k = 0; k < K8; ++k) inv[k] = *reinterpret_cast<const float2*>(sM + 8 * k + 2 * t4);
+        __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + r.batch * p.o_stride_b + warp * 32;
 #pragma unroll 1
-      for (int c = 0; c < 4 * N; c += 16) {
-        const int mb = c / N, row0 = c % N;
-        if (row0 >= nrows) continue;
-        uint32_t ov[16];
-        if (have_o) {
-          tc::tmem_ld16(tmem + lane_addr + TMEM_O + c, ov);
-          tc::tmem_wait_ld();
-        } else {
+        for (int c = 0; c < 512 / 4 / W; ++c) {          // 128 mb + 32 warp + W part
+          const int mb = c / (32 / W), part = c % (32 / W);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) ov[i] = 0u;
-        }
-        const int col = mb * 128 + warp * 32 + lane;
-        if (no_split) {
-          // two rows at a time: even lanes store columns (col, col + 1) of row i, odd lanes columns (col - 1, col) of row i + 1
+          for (int h = 0; h < W / 16; ++h) {
+            uint32_t ov[4 * K8];
+            if (have_o) {
+              tmem_ld_16x256b(tmem + lane_addr + (static_cast<uint32_t>(part * W + h * 16) << 16) + TMEM_O + mb * N, ov);
+              tc::tmem_wait_ld();
+            } else {
 #pragma unroll
-          for (int i = 0; i < 16; i += 2) {
-            const float a = __uint_as_float(ov[i]) * sM[row0 + i], b = __uint_as_float(ov[i + 1]) * sM[row0 + i + 1];
-            const float other = __shfl_xor_sync(0xffffffffu, (lane & 1) ? a : b, 1);
-            const int row = row0 + i + (lane & 1);
-            const uint32_t w = (lane & 1) ? pack_16x2<F16>(other, b) : pack_16x2<F16>(a, other);
-            if (row < nrows) {
-              const int tok = row / tile_heads, head = head0 + row % tile_heads;
-              __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + r.batch * p.o_stride_b + (sq0 + tok) * p.o_stride_s + head * p.o_stride_h;
-              *reinterpret_cast<uint32_t*>(dst + (col & ~1)) = w;
+              for (int i = 0; i < 4 * K8; ++i) ov[i] = 0u;
             }
+            uint32_t pk[2 * K8];
+#pragma unroll
+            for (int k = 0; k < K8; ++k) {
+              pk[2 * k] = pack_16x2<F16>(__uint_as_float(ov[4 * k]) * inv[k].x, __uint_as_float(ov[4 * k + 1]) * inv[k].y);
+              pk[2 * k + 1] = pack_16x2<F16>(__uint_as_float(ov[4 * k + 2]) * inv[k].x, __uint_as_float(ov[4 * k + 3]) * inv[k].y);
+            }
+            const int mrow = lane & 7, mat = lane >> 3;
+#pragma unroll
+            for (int k = 0; k < K8; k += 2)
+              stmatrix_x4_trans(piece_at((k + (mat >> 1)) * 8 + mrow, h * 2 + (mat & 1)), pk[2 * k], pk[2 * k + 1], pk[2 * k + 2], pk[2 * k + 3]);
           }
-        } else {
-          float* dst = p.o_accum + (part_row + row0) * 512 + col;
+          __syncwarp();
+          constexpr int kEach = N * kPieces / 32;
+          uint4 v[kEach];
+          int64_t at[kEach];
+#pragma unroll
+          for (int i = 0; i < kEach; ++i) {
+            const int row = (i * 32 + lane) / kPieces, piece = lane % kPieces;
+            v[i] = ld_shared_v4(piece_at(row, piece));
+            at[i] = sRow[row] + mb * 128 + part * W + piece * 8;
+          }
+#pragma unroll
+          for (int i = 0; i < kEach; ++i)
+            if ((i * 32 + lane) / kPieces < nrows) *reinterpret_cast<uint4*>(out + at[i]) = v[i];
+          __syncwarp();
+        }
+      } else {
+        // fp32 partial: lane = value column 128 mb + 32 warp + lane, registers = query rows
+#pragma unroll 1
+        for (int c = 0; c < 4 * N; c += 16) {
+          const int mb = c / N, row0 = c % N;
+          if (row0 >= nrows) continue;
+          uint32_t ov[16];
+          if (have_o) {
+            tc::tmem_ld16(tmem + lane_addr + TMEM_O + c, ov);
+            tc::tmem_wait_ld();
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) ov[i] = 0u;
+          }
+          // the factors are read before the first store: the compiler keeps a load behind the stores in front of it, and each
+          // store then cost the latency of one (64 rows: 8 700 clk, now 5 200)
+#pragma unroll
+          for (int i = 0; i < 16; i += 4) {
+            const float4 f = *reinterpret_cast<const float4*>(sM + row0 + i);
+            ov[i] = __float_as_uint(__uint_as_float(ov[i]) * f.x);
+            ov[i + 1] = __float_as_uint(__uint_as_float(ov[i + 1]) * f.y);
+            ov[i + 2] = __float_as_uint(__uint_as_float(ov[i + 2]) * f.z);
+            ov[i + 3] = __float_as_uint(__uint_as_float(ov[i + 3]) * f.w);
+          }
+          float* dst = p.o_accum + (part_row + row0) * 512 + mb * 128 + warp * 32 + lane;
 #pragma unroll
           for (int i = 0; i < 16; ++i)
-            if (row0 + i < nrows) dst[i * 512] = __uint_as_float(ov[i]) * sM[row0 + i];
+            if (row0 + i < nrows) dst[i * 512] = __uint_as_float(ov[i]);
         }
       }
       if (nblk > 0) {
