@@ -65,7 +65,7 @@ struct Layout {
   static_assert(kVSlots % 2 == 0 && kVSlots >= 16 && kVSlots <= 8 * (kPageBars - 1) + 1, "ring sizes");
 };
 enum Bar { Q_FULL = 0, Q_EMPTY, KV_FULL0, KV_EMPTY0 = KV_FULL0 + kPageBars, ROPE_EMPTY0 = KV_EMPTY0 + kPageBars, S_FULL0 = ROPE_EMPTY0 + 3, S_FULL1,
-           S_EMPTY0, S_EMPTY1, P_FULL0, P_FULL1, P_EMPTY0, P_EMPTY1, O_FULL, O_EMPTY, NUM_BARS };
+           P_FULL0, P_FULL1, P_EMPTY0, P_EMPTY1, O_FULL, NUM_BARS };
 static_assert(NUM_BARS * 8 <= 256, "barrier area too small");
 constexpr int TMEM_O = 0, TMEM_S = 256;
 constexpr float kRescaleThreshold = 8.0f;         // log2 units; below it O keeps its stale scale
@@ -149,7 +149,7 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
     // a page has landed: with its bytes (TMA), or when every gather warp has stored its rows
     constexpr int kFull = SPARSE ? kGather : 1;
     for (int i = 0; i < NUM_BARS; ++i)
-      tc::mbar_init(bar(i), (i >= S_EMPTY0 && i <= P_FULL1) || i == O_EMPTY ? 4          // one arrival per softmax warp
+      tc::mbar_init(bar(i), i == P_FULL0 || i == P_FULL1 ? 4                             // one arrival per softmax warp
                             : (i >= KV_FULL0 && i < KV_EMPTY0)              ? kFull : 1);
     tc::fence_mbar_init();
     *sAbort = 0;
@@ -371,20 +371,28 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
       const int nblk = r.blk_hi - r.blk_lo;
       if (nblk == 0) continue;
       alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_FULL), req & 1, status, 205));
-      // S^T of block js and O^T of block jp < js are issued in whichever order their inputs become ready, O^T first: it
-      // releases slots of the ring.  One poll reads every barrier of interest, one per lane:
-      //   lane 0 P_FULL(jp)  lane 1 O_EMPTY  lane 2 S_EMPTY(js)  lane 3 KV_FULL(js)
+      // S^T runs one block ahead of O^T; where both could be next, whichever has its inputs first is issued, O^T first: it
+      // releases slots of the ring.  S^T(js) overwrites S^T(js - 2), and O^T(0) what the request before left: the softmax
+      // warps had read both before they arrived on a P_FULL that has been waited for here (P_FULL(js - 2), P_FULL(0)).
+      // A test of a barrier takes about 130 clk and tests of different barriers by different lanes follow one another, so
+      // only what is needed is looked at: with four barriers per poll the warp saw P 550 clk after its last arrival.
       int js = 0, jp = 0, idle = 0;
       while (jp < nblk && alive) {
-        const int gs = g + min(js, nblk - 1), gp = g + jp;
-        int pb = P_FULL0 + gp % L::kPBufs;
-        uint32_t pp = (gp / L::kPBufs) & 1;
-        if (lane == 1) { pb = O_EMPTY; pp = (req & 1) ^ 1; }
-        if (lane == 2) { pb = S_EMPTY0 + (gs & 1); pp = ((gs >> 1) & 1) ^ 1; }
-        if (lane >= 3) { pb = KV_FULL0 + gs % kPageBars; pp = (gs / kPageBars) & 1; }
-        const bool hit = lane < 4 && tc::mbar_test_wait(bar(pb), pp);
-        const uint32_t m = __ballot_sync(0xffffffffu, hit);
-        if (jp < js && (m & 1u) && (jp > 0 || (m & 2u))) {
+        const int gs = g + js, gp = g + jp;
+        const bool want_s = js < nblk && js <= jp + 1, want_p = jp < js;
+        const uint32_t p_full = bar(P_FULL0 + gp % L::kPBufs), kv_full = bar(KV_FULL0 + gs % kPageBars);
+        const uint32_t p_ph = (gp / L::kPBufs) & 1, kv_ph = (gs / kPageBars) & 1;
+        bool go_p = false, go_s = false;
+        if (want_s && want_p) {
+          const uint32_t m = __ballot_sync(0xffffffffu, lane < 2 && tc::mbar_test_wait(lane == 0 ? p_full : kv_full, lane == 0 ? p_ph : kv_ph));
+          go_p = m & 1u;
+          go_s = m & 2u;
+        } else if (want_p) {
+          go_p = alive = __all_sync(0xffffffffu, tc::mbar_wait(p_full, p_ph, status, 207));
+        } else {
+          go_s = alive = __all_sync(0xffffffffu, tc::mbar_wait(kv_full, kv_ph, status, 212));
+        }
+        if (go_p) {
           tc::tc_fence_after();
           if (tc::elect_one()) {
             const uint64_t dp = tc::desc_advance(desc_p, (gp % L::kPBufs) * N * 128);
@@ -402,7 +410,7 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
           slot_p = next_page(slot_p);
           ++jp;
           idle = 0;
-        } else if (js < nblk && (m & 0xcu) == 0xcu) {
+        } else if (go_s) {
           // rows of the last page beyond the sequence may hold anything (NaN included): zeroed so that 0 * garbage
           // cannot reach O^T
           const int rows_valid = SPARSE ? 64 : r.seqlen - (r.blk_lo + js) * 64;
@@ -433,7 +441,7 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
           slot_s = next_page(slot_s);
           ++js;
           idle = 0;
-        } else if (++idle > tc::kSpinLimit) {
+        } else if (alive && ++idle > tc::kSpinLimit) {
           if (lane == 0) tc::report_status(status, 206);
           alive = false;
         }
@@ -474,8 +482,6 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
 #pragma unroll
           for (int i = 0; i < 4 * K8; ++i) sv[i] = 0u;
         }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(bar(S_EMPTY0 + (g & 1)));
         // logits of hidden tokens become -inf (a select: they may hold anything)
         const int blk0 = (r.blk_lo + j) * 64, tok0 = blk0 + warp * 16 + tr;
         if constexpr (SPARSE) {
@@ -710,8 +716,6 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
       }
       if (nblk > 0) {
         tc::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(bar(O_EMPTY));
         ++req;
       }
       bar_sync(1, 128);          // sM and sX are reused by the next request
