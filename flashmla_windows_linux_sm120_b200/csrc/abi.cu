@@ -240,7 +240,7 @@ static int decode_impl(const fmla_decode_params* P, const fmla_peer_push* push, 
   k.tile_scheduler_metadata = a.tile_scheduler_metadata; k.num_sm_parts = a.num_sm_parts; k.num_splits = a.num_splits;
   k.out = a.out; k.o_stride_b = a.o_stride_b; k.o_stride_s = a.o_stride_s; k.o_stride_h = a.o_stride_h;
   k.softmax_lse = a.softmax_lse; k.lse_accum = a.lse_accum; k.o_accum = a.o_accum;
-  k.arrival_counters = (!push && !sparse) ? a.arrival_counters : nullptr;
+  k.arrival_counters = (!push && !sparse && k.hq_per_hk % 128 == 0) ? a.arrival_counters : nullptr;
   k.no_split_hint = (!push && a.no_split_hint) ? 1 : 0;
   if (push) {
     k.force_partial = 1;

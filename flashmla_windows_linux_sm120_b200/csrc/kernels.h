@@ -100,7 +100,7 @@ cudaError_t launch_decode_sparse_tc(const DecodeKernelParams& p, cudaStream_t st
 cudaError_t launch_sparse_prefill_tc(const SparsePrefillKernelParams& p, cudaStream_t stream);
 // read_*_status: reads (and optionally clears) the status word a kernel sets when a bounded wait expires
 // dense decode as a CTA pair (mla_pair.cu): 128 heads per pair, tcgen05 cta_group::2; used by
-// launch_decode_dense_tc whenever the heads per kv head are a multiple of 128
+// launch_decode_dense_tc whenever the heads per kv head are a multiple of 128, or 64 with an even number of query tokens
 bool decode_dense_pair_applies(const DecodeKernelParams& p);
 // true when launch_decode_dense_tc will merge the split partials inside the attention kernel (no merge launch needed)
 bool decode_dense_merges_in_kernel(const DecodeKernelParams& p);

@@ -1,5 +1,5 @@
-// Which kernel runs an MLA attention call: the CTA pair (mla_pair.cu) where 128 heads share a kv head -- its two CTAs read
-// every cached token once for all of them -- and otherwise one CTA per at most 64 query rows (mla_few_rows.cu), or per 64
+// Which kernel runs an MLA attention call: the CTA pair (mla_pair.cu) where 128 heads share a kv head, or the 64 heads of two
+// query tokens -- its two CTAs read every cached token once for all of them -- and otherwise one CTA per at most 64 query rows (mla_few_rows.cu), or per 64
 // heads of the sparse prefill (mla_prefill64.cu).
 #include "kernels.h"
 

@@ -3,7 +3,8 @@
 // gathering modes differ in how the K rows reach shared memory and where the V operand comes from (further down).
 //
 // The pair owns 128 query heads of one (query token, kv head, partition): CTA r of the pair (cluster rank r)
-// owns heads 64r .. 64r+63, i.e. the Q tile, the S tile, the P tile and the O accumulator of those heads.
+// owns heads 64r .. 64r+63, i.e. the Q tile, the S tile, the P tile and the O accumulator of those heads.  (Dense decode with
+// 64 heads and an even number of query tokens: CTA r owns the heads of query token 2i + r.)
 // One thread of the leader (rank 0) issues every MMA for both SMs:
 //   S = Q K^T   36 x tcgen05.mma.cta_group::2 m128n64k16: the B operand (64 tokens x 576) is split along N, so
 //               each CTA stages only ITS 32 token rows of a page (36 KB) -- the pair reads a page for S once
@@ -1127,7 +1128,10 @@ cudaError_t launch_sparse_prefill_pair(const SparsePrefillKernelParams& sp, cuda
   return launch_pair<mla_pair_kernel<false, kSparsePrefill>>(P, tq, tq, tq, dim3(2, lanes, 1), ptc::kPrefillThreads, stream);    // the K / V maps are not used in this mode
 }
 
-bool decode_dense_pair_applies(const DecodeKernelParams& p) { return p.hq_per_hk % 128 == 0; }
+// Two 64-row tiles that read the same pages: the halves of 128 heads, or the 64 heads of two consecutive query tokens, which
+// one CTA each (mla_few_rows.cu) would read twice: 64 heads, two tokens, 16 requests of 16 000 tokens 140 us against 82 us
+// here, 4 of 200 tokens 18.5 against 16.2; no shape in between the other way.
+bool decode_dense_pair_applies(const DecodeKernelParams& p) { return p.hq_per_hk % 128 == 0 || (p.hq_per_hk == 64 && p.s_q % 2 == 0); }
 
 cudaError_t launch_decode_dense_pair(const DecodeKernelParams& p, cudaStream_t stream) {
   TcParams P = {};

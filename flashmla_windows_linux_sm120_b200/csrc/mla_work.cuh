@@ -80,7 +80,9 @@ __device__ __forceinline__ Work get_work(const TcParams& P, const Tile& t, int i
       w.seqlen = p.seqlens_k[batch];
       nblk_total = (w.seqlen + 63) >> 6;
       w.border = p.is_causal ? w.seqlen - (p.s_q - 1 - t.sq) : w.seqlen;
-      nblk_visible = w.border > 0 ? (w.border + 63) >> 6 : 0;
+      // with 64 heads the two CTAs of a pair hold consecutive query tokens and walk the blocks that the later one sees
+      const int seen = p.is_causal && p.hq_per_hk == 64 ? w.seqlen - (p.s_q - 1 - (t.sq | 1)) : w.border;
+      nblk_visible = seen > 0 ? (seen + 63) >> 6 : 0;
       w.idx = nullptr;
     } else {
       w.seqlen = p.topk; w.border = p.topk;
