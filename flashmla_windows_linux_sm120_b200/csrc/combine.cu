@@ -16,22 +16,24 @@
 namespace fmla {
 
 constexpr int kCombineWarps = 8;
-constexpr int kPartsInFlight = 4;       // partial rows whose loads a lane issues before it uses the first
 
 // Weights 2^(lse_i - lse) of the parts of a row -> s_w (whole warp); returns the base-2 LSE of the row.
 template <class LseAt>
 __device__ __forceinline__ float combine_weights(int nparts, LseAt lse_at, float* s_w) {
   const int lane = threadIdx.x & 31;
   float mx = neg_inf();
+#pragma unroll 1
   for (int i = lane; i < nparts; i += 32) mx = fmaxf(mx, lse_at(i));
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
   if (mx == neg_inf()) mx = 0.f;
   float sum = 0.f;
+#pragma unroll 1
   for (int i = lane; i < nparts; i += 32) sum += exp2f(lse_at(i) - mx);
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
   const float glse = (sum == 0.f || sum != sum) ? pos_inf() : log2f(sum) + mx;
+#pragma unroll 1
   for (int i = lane; i < nparts; i += 32) s_w[i] = exp2f(lse_at(i) - glse);
   __syncwarp();
   return glse;
@@ -39,16 +41,21 @@ __device__ __forceinline__ float combine_weights(int nparts, LseAt lse_at, float
 
 // Weighted sum of the parts over column groups [first, first + NG) of 128 columns (lane = 4 columns of a group), in the
 // order of the parts.  A part with weight 0 is not read: 0 * (Inf or NaN) must not reach the sum.
+// The loads of 4 / NG parts are in flight at a time: four 16-byte loads per lane.  With four parts of four groups each the merge
+// needed 98 registers, too many to wait beside an attention CTA, and 1024 of its CTAs (64 requests x 128 heads) took three
+// and a half waves.
 // COHERENT: the partial outputs may have been written by another GPU while this kernel was already resident (peer
 // merge), so they are read with ld.global.cv.  Otherwise plain loads: the merge of a decode call is resident, waiting in
 // pdl_wait(), while the attention kernel writes the partials, and the non-coherent path (__ldg) is undefined for memory
 // modified during the kernel's lifetime.
 template <int NG, bool COHERENT, class OAt>
 __device__ __forceinline__ void combine_columns(int nparts, OAt o_at, const float* s_w, __nv_bfloat16* out_row, int first, bool f16) {
+  constexpr int kPartsInFlight = 4 / NG;
   const int lane = threadIdx.x & 31;
   float4 acc[NG];
 #pragma unroll
   for (int j = 0; j < NG; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
   for (int i0 = 0; i0 < nparts; i0 += kPartsInFlight) {
     float4 v[kPartsInFlight][NG];
     float w[kPartsInFlight];
