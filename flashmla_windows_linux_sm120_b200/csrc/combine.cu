@@ -298,10 +298,15 @@ static cudaError_t launch_decode_combine_wpr(const DecodeKernelParams& p, int ro
 
 cudaError_t launch_decode_combine(const DecodeKernelParams& p, cudaStream_t stream) {
   const int rows = p.h_k * p.s_q * p.hq_per_hk;
+  int dev = 0, sms = 0;
+  if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
+  if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); e != cudaSuccess) return e;
   // Few rows with many parts each (4 requests x 16 heads split 37 ways): one warp per row walks its parts one after the
   // other on a handful of SMs, so a row is spread over four warps as long as that fits on the chip at once
-  // (148 SMs x 64 warps); beyond that the rows alone fill it and four times the CTAs would only cost their launch.
-  if ((int64_t)p.b * rows * 4 <= 148 * 64) return launch_decode_combine_wpr<4>(p, rows, stream);
+  // (64 warps per SM); beyond that the rows alone fill it and four times the CTAs would only cost their launch.  Device time
+  // of decode steps, 24 shapes each with 16 / 32 / 64 heads and 48 with 128: one warp always 2.7 / 4.8 / 4.8 / 0 % more than
+  // this rule, four always 0 / 0 / 0.8 / 3 % more.
+  if ((int64_t)p.b * rows * 4 <= (int64_t)sms * 64) return launch_decode_combine_wpr<4>(p, rows, stream);
   return launch_decode_combine_wpr<1>(p, rows, stream);
 }
 
