@@ -241,8 +241,9 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
   const uint32_t tmem = *sTmem;
   const Tile tile = make_tile<WM>(P);           // both CTAs of a pair see the same schedule row (possibly an empty one)
 
-  if (misaligned) {
-    // nothing was issued; fall through to the common exit
+  if (misaligned || tile.n_work == 0) {
+    // nothing was issued; fall through to the common exit.  (The work of an empty schedule row must not be asked for: its
+    // request is p.b, past the lengths, the indices and num_splits.)
   } else if ((warp == 4 || warp >= 8) && WM == kSparsePrefill) {
     // ================================ Q and K loader, sparse prefill ===================
     // The CTA's 32 token rows of a block (32 x 1152 bytes) are gathered with 16-byte cp.async copies by three warps

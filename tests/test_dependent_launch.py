@@ -26,6 +26,17 @@ def test_no_invariant_loads_of_what_the_kernel_in_front_writes():
         assert all("rec" in arg for arg in re.findall(r"__ldg\(([^;]*);", text)), name
 
 
+def test_an_empty_schedule_row_asks_for_no_work():
+    """begin_idx of an empty row is the batch size: reading that request's length or split count is out of range.  Such a CTA
+    has to stay (it waits for the kernel in front), so both decode kernels leave every role out instead."""
+    for name, guard in (("mla_pair.cu", "if (misaligned || tile.n_work == 0) {"), ("mla_few_rows.cu", "if (n_work == 0 || misaligned) {")):
+        with open(os.path.join(CSRC, name)) as f:
+            text = f.read()
+        kernel = text[text.index("pdl_wait();"):]
+        assert guard in kernel
+        assert not re.search(r"get_work<|request\(0\)", kernel[:kernel.index(guard)])
+
+
 def _lengths(kind):
     return {"even": [700] * 12, "one_long": [70] * 11 + [6400], "other_long": [3000] + [1] * 10 + [0]}[kind]
 
