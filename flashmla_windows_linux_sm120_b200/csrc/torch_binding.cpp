@@ -71,6 +71,14 @@ at::Tensor new_tensor(at::IntArrayRef shape, const at::Tensor& like, at::ScalarT
 }
 void* stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
+// Gives up the GIL for the allocations and launches of a call: an allocation may synchronise and a launch waits while the
+// stream's queue is full, and what it waits for may be a host callback that needs the GIL.  Python objects are read before,
+// and tensors are declared outside its scope (the last reference to one may go through Python).
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 PyObject* pair(at::Tensor a, at::Tensor b) {
   PyObject* list = PyList_New(2);
   PyList_SET_ITEM(list, 0, THPVariable_Wrap(std::move(a)));
@@ -115,16 +123,22 @@ PyObject* metadata(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     require(lens.is_contiguous(), "seqlens_k must be contiguous");
     require(lens.scalar_type() == at::kInt, "seqlens_k must have dtype int32");
     if (sparse) require(a[3] != Py_None, "num_heads_q must be provided when topk is provided");
-    int parts = 0;
-    check(fmla_get_num_sm_parts(lens.get_device(), as_int(a[1]), as_int(a[2]), a[3] != Py_None ? as_int(a[3]) : 0, truth(a[4]), sparse,
-                                &parts));
-    const int64_t b = lens.size(0);
+    const int q_per_hk = as_int(a[1]), h_k = as_int(a[2]), h_q = a[3] != Py_None ? as_int(a[3]) : 0;
+    const bool fp8 = truth(a[4]);
     const int topk = sparse ? as_int(a[5]) : -1;
-    const c10::cuda::CUDAGuard guard(lens.device());
-    at::Tensor md = new_tensor({parts, 8}, lens, at::kInt), ns = new_tensor({b + 1}, lens, at::kInt);
-    check(fmla_get_mla_metadata(static_cast<const int32_t*>(lens.const_data_ptr()), static_cast<int>(b), parts, topk,
-                                static_cast<int32_t*>(md.mutable_data_ptr()), static_cast<int32_t*>(ns.mutable_data_ptr()),
-                                stream_of(lens)));
+    const int64_t b = lens.size(0);
+    int parts = 0;
+    at::Tensor md, ns;
+    {
+      const NoGil nogil;
+      check(fmla_get_num_sm_parts(lens.get_device(), q_per_hk, h_k, h_q, fp8, sparse, &parts));
+      const c10::cuda::CUDAGuard guard(lens.device());
+      md = new_tensor({parts, 8}, lens, at::kInt);
+      ns = new_tensor({b + 1}, lens, at::kInt);
+      check(fmla_get_mla_metadata(static_cast<const int32_t*>(lens.const_data_ptr()), static_cast<int>(b), parts, topk,
+                                  static_cast<int32_t*>(md.mutable_data_ptr()), static_cast<int32_t*>(ns.mutable_data_ptr()),
+                                  stream_of(lens)));
+    }
     PyObject* list = PyList_New(3);
     PyList_SET_ITEM(list, 0, THPVariable_Wrap(std::move(md)));
     PyList_SET_ITEM(list, 1, THPVariable_Wrap(std::move(ns)));
@@ -182,11 +196,8 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     require(!(qt == at::kHalf && (sparse || fp8)),
             "flashmla_b200: unsupported configuration: float16 queries are supported for the dense (float16 cache) decode only");
 
-    const c10::cuda::CUDAGuard guard(q.device());
-    at::Tensor out = new_tensor({b, s_q, h_q, dv}, q, qt), lse = new_tensor({b, h_q, s_q}, q, at::kFloat);
     // scratch of the split requests: fp32 partial outputs, then their log-sum-exps
     const int64_t parts = md.size(0), rows = (b + parts) * s_q * h_q;
-    at::Tensor accum = new_tensor({rows * (dv + 1)}, q, at::kFloat);
     fmla_decode_params p = {};
     p.b = static_cast<int32_t>(b); p.s_q = static_cast<int32_t>(s_q); p.h_q = static_cast<int32_t>(h_q);
     p.h_k = static_cast<int32_t>(h_k); p.d = static_cast<int32_t>(d); p.d_v = static_cast<int32_t>(dv);
@@ -206,14 +217,22 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     }
     p.tile_scheduler_metadata = static_cast<const int32_t*>(md.const_data_ptr()); p.num_sm_parts = static_cast<int32_t>(parts);
     p.num_splits = static_cast<const int32_t*>(ns.const_data_ptr());
-    p.out = out.mutable_data_ptr(); p.o_stride_b = out.stride(0); p.o_stride_s = out.stride(1); p.o_stride_h = out.stride(2);
-    p.softmax_lse = static_cast<float*>(lse.mutable_data_ptr());
-    p.o_accum = static_cast<float*>(accum.mutable_data_ptr()); p.lse_accum = p.o_accum + rows * dv;
     p.arrival_counters = reinterpret_cast<int32_t*>(integer(a[14]));
     p.no_split_hint = truth(a[15]);
     p.profile_event_begin = reinterpret_cast<void*>(integer(a[11]));
     p.profile_event_end = reinterpret_cast<void*>(integer(a[12]));
-    check(fmla_fwd_kvcache_mla(&p, stream_of(q)));
+    at::Tensor out, lse, accum;
+    {
+      const NoGil nogil;
+      const c10::cuda::CUDAGuard guard(q.device());
+      out = new_tensor({b, s_q, h_q, dv}, q, qt);
+      lse = new_tensor({b, h_q, s_q}, q, at::kFloat);
+      accum = new_tensor({rows * (dv + 1)}, q, at::kFloat);
+      p.out = out.mutable_data_ptr(); p.o_stride_b = out.stride(0); p.o_stride_s = out.stride(1); p.o_stride_h = out.stride(2);
+      p.softmax_lse = static_cast<float*>(lse.mutable_data_ptr());
+      p.o_accum = static_cast<float*>(accum.mutable_data_ptr()); p.lse_accum = p.o_accum + rows * dv;
+      check(fmla_fwd_kvcache_mla(&p, stream_of(q)));
+    }
     return pair(std::move(out), std::move(lse));
   });
 }
@@ -232,9 +251,6 @@ PyObject* sparse_prefill(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     require(kv.size(2) == q.size(2), "q and kv head dims differ");
     require(idx.size(0) == q.size(0) && idx.size(1) == kv.size(1), "indices must be [s_q, h_kv, topk]");
     const int64_t s_q = q.size(0), h_q = q.size(1), dv = integer(a[4]);
-    const c10::cuda::CUDAGuard guard(q.device());
-    at::Tensor out = new_tensor({s_q, h_q, dv}, q, at::kBFloat16), mx = new_tensor({s_q, h_q}, q, at::kFloat),
-               lse = new_tensor({s_q, h_q}, q, at::kFloat);
     fmla_sparse_prefill_params p = {};
     p.s_q = static_cast<int32_t>(s_q); p.s_kv = static_cast<int32_t>(kv.size(0)); p.h_q = static_cast<int32_t>(h_q);
     p.h_kv = static_cast<int32_t>(kv.size(1)); p.d_qk = static_cast<int32_t>(q.size(2)); p.d_v = static_cast<int32_t>(dv);
@@ -243,10 +259,18 @@ PyObject* sparse_prefill(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     p.q = q.const_data_ptr(); p.q_stride_s = q.stride(0); p.q_stride_h = q.stride(1);
     p.kv = kv.const_data_ptr(); p.kv_stride_s = kv.stride(0); p.kv_stride_h = kv.stride(1);
     p.indices = static_cast<const int32_t*>(idx.const_data_ptr()); p.indices_stride_s = idx.stride(0); p.indices_stride_h = idx.stride(1);
-    p.out = out.mutable_data_ptr();
-    p.max_logits = static_cast<float*>(mx.mutable_data_ptr());
-    p.lse = static_cast<float*>(lse.mutable_data_ptr());
-    check(fmla_sparse_prefill_fwd(&p, stream_of(q)));
+    at::Tensor out, mx, lse;
+    {
+      const NoGil nogil;
+      const c10::cuda::CUDAGuard guard(q.device());
+      out = new_tensor({s_q, h_q, dv}, q, at::kBFloat16);
+      mx = new_tensor({s_q, h_q}, q, at::kFloat);
+      lse = new_tensor({s_q, h_q}, q, at::kFloat);
+      p.out = out.mutable_data_ptr();
+      p.max_logits = static_cast<float*>(mx.mutable_data_ptr());
+      p.lse = static_cast<float*>(lse.mutable_data_ptr());
+      check(fmla_sparse_prefill_fwd(&p, stream_of(q)));
+    }
     PyObject* list = pair(std::move(out), std::move(mx));
     PyObject* l = THPVariable_Wrap(std::move(lse));
     PyList_Append(list, l);
@@ -260,27 +284,31 @@ PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   return guarded(nargs, 3, [&]() -> PyObject* {
     const at::Tensor& kv = tensor(a[0], "kv");
     require(kv.is_cuda() && kv.scalar_type() == at::kBFloat16 && kv.dim() > 0 && kv.size(-1) == 576, "kv must be CUDA bf16 [..., 576]");
-    const at::Tensor flat = kv.dim() == 2 ? kv : kv.reshape({-1, 576});
-    require(flat.stride(1) == 1, "kv rows must be contiguous");
-    const c10::cuda::CUDAGuard guard(kv.device());
-    at::Tensor cache;
-    if (a[1] == Py_None) {
-      std::vector<int64_t> shape(kv.sizes().begin(), kv.sizes().end());
-      shape.back() = 656;
-      cache = new_tensor(shape, kv, at::kFloat8_e4m3fn);
-    } else {
-      cache = tensor(a[1], "cache");
-    }
-    const bool plain = cache.element_size() == 1 && cache.is_contiguous() && cache.dim() > 0 && cache.size(-1) == 656;
-    const at::Tensor records = plain ? cache : cache.view(at::kByte).reshape({-1, 656});
+    const at::Tensor* given = a[1] != Py_None ? &tensor(a[1], "cache") : nullptr;
     const int32_t* slots = nullptr;
     if (a[2] != Py_None) {
       const at::Tensor& s = tensor(a[2], "dst_slots");
       require(s.is_cuda() && s.scalar_type() == at::kInt && s.is_contiguous(), "dst_slots must be a contiguous CUDA int32 tensor");
       slots = static_cast<const int32_t*>(s.const_data_ptr());
     }
-    check(fmla_quantize_kv_fp8(flat.const_data_ptr(), flat.stride(0), static_cast<int>(flat.size(0)), slots, records.mutable_data_ptr(),
-                               plain ? 656 : records.stride(0), stream_of(kv)));
+    at::Tensor flat, cache, records;
+    {
+      const NoGil nogil;
+      flat = kv.dim() == 2 ? kv : kv.reshape({-1, 576});
+      require(flat.stride(1) == 1, "kv rows must be contiguous");
+      const c10::cuda::CUDAGuard guard(kv.device());
+      if (!given) {
+        std::vector<int64_t> shape(kv.sizes().begin(), kv.sizes().end());
+        shape.back() = 656;
+        cache = new_tensor(shape, kv, at::kFloat8_e4m3fn);
+      } else {
+        cache = *given;
+      }
+      const bool plain = cache.element_size() == 1 && cache.is_contiguous() && cache.dim() > 0 && cache.size(-1) == 656;
+      records = plain ? cache : cache.view(at::kByte).reshape({-1, 656});
+      check(fmla_quantize_kv_fp8(flat.const_data_ptr(), flat.stride(0), static_cast<int>(flat.size(0)), slots, records.mutable_data_ptr(),
+                                 plain ? 656 : records.stride(0), stream_of(kv)));
+    }
     if (a[1] == Py_None) return THPVariable_Wrap(std::move(cache));
     Py_INCREF(a[1]);
     return a[1];
