@@ -11,6 +11,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <Python.h>
@@ -21,6 +22,8 @@
 #include <vector>
 
 namespace {
+
+struct PythonErrorSet {};      // thrown where a Python call has failed and set the error
 
 void require(bool cond, const char* msg) {
   if (!cond) throw std::runtime_error(msg);
@@ -40,14 +43,14 @@ const at::Tensor& tensor(PyObject* o, const char* name) {
 int64_t integer(PyObject* o) {
   if (!PyLong_Check(o)) {                      // what int() takes: 16.0, a numpy or tensor scalar
     PyObject* whole = PyNumber_Long(o);
-    if (!whole) throw std::runtime_error("");
+    if (!whole) throw PythonErrorSet();
     const int64_t v = PyLong_AsLongLong(whole);
     Py_DECREF(whole);
-    if (v == -1 && PyErr_Occurred()) throw std::runtime_error("");
+    if (v == -1 && PyErr_Occurred()) throw PythonErrorSet();
     return v;
   }
   const int64_t v = PyLong_AsLongLong(o);
-  if (v == -1 && PyErr_Occurred()) throw std::runtime_error("");
+  if (v == -1 && PyErr_Occurred()) throw PythonErrorSet();
   return v;
 }
 int as_int(PyObject* o) {
@@ -57,12 +60,12 @@ int as_int(PyObject* o) {
 }
 double real(PyObject* o) {
   const double v = PyFloat_AsDouble(o);
-  if (v == -1.0 && PyErr_Occurred()) throw std::runtime_error("");
+  if (v == -1.0 && PyErr_Occurred()) throw PythonErrorSet();
   return v;
 }
 bool truth(PyObject* o) {
   const int v = PyObject_IsTrue(o);
-  if (v < 0) throw std::runtime_error("");
+  if (v < 0) throw PythonErrorSet();
   return v != 0;
 }
 
@@ -86,7 +89,8 @@ PyObject* pair(at::Tensor a, at::Tensor b) {
   return list;
 }
 
-// Runs `f`, turning a C++ exception into a Python RuntimeError (an error that Python raised inside `f` stays as it is).
+// Runs `f`, turning a C++ exception into the Python one that torch makes of it: torch.OutOfMemoryError for a failed
+// allocation, IndexError and the like for torch's own errors, RuntimeError for the messages above.
 template <class F>
 PyObject* guarded(Py_ssize_t nargs, Py_ssize_t want, F&& f) {
   if (nargs != want) {
@@ -95,10 +99,9 @@ PyObject* guarded(Py_ssize_t nargs, Py_ssize_t want, F&& f) {
   }
   try {
     return f();
-  } catch (const c10::Error& e) {
-    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
-  } catch (const std::exception& e) {
-    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (const PythonErrorSet&) {
+  } catch (...) {
+    torch::translate_exception_to_python(std::current_exception());
   }
   return nullptr;
 }

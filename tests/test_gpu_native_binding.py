@@ -72,3 +72,24 @@ def test_two_threads_decode_on_their_own_streams():
     for k in range(2):
         for out, lse in results[k]:
             assert torch.equal(out.cpu(), expected[k][0]) and torch.equal(lse.cpu(), expected[k][1])
+
+
+def test_errors_keep_their_types():
+    from flashmla_windows_linux_sm120_b200 import cuda_sm100
+    one = dict(dtype=torch.bfloat16, device="cuda")
+    n = 1 << 23                                          # an output of half a terabyte: refused before anything is launched
+    q, kv = torch.zeros((1, 64, 576), **one).expand(n, 64, 576), torch.zeros((1, 1, 576), **one)
+    idx = torch.zeros((1, 1, 64), dtype=torch.int32, device="cuda").expand(n, 1, 64)
+    with pytest.raises(torch.OutOfMemoryError):
+        cuda_sm100.sparse_prefill_fwd(q, kv, idx, 1.0)
+    with pytest.raises(IndexError):                      # a tensor without dimensions, where the batch is asked for
+        cuda_sm100.get_mla_decoding_metadata(torch.tensor(5, dtype=torch.int32, device="cuda"), 128, 1)
+    lens = torch.tensor([64], dtype=torch.int32, device="cuda")
+    with pytest.raises(TypeError):
+        cuda_sm100.get_mla_decoding_metadata(lens, None, 1)
+    with pytest.raises(RuntimeError, match="seqlens_k must have dtype int32"):
+        cuda_sm100.get_mla_decoding_metadata(lens.long(), 128, 1)
+    md, ns = cuda_sm100.get_mla_decoding_metadata(lens, 128, 1)
+    q, cache, table = torch.zeros((1, 1, 128, 576), **one), torch.zeros((1, 64, 1, 576), **one), torch.zeros((1, 1), dtype=torch.int32, device="cuda")
+    with pytest.raises(RuntimeError, match="head_size_v == 512"):
+        cuda_sm100.fwd_kvcache_mla(q, cache, 256, lens, table, 1.0, False, md, ns)
