@@ -9,6 +9,7 @@
 #include "../../include/flashmla_b200.h"
 
 #include <ATen/ATen.h>
+#include <c10/core/InferenceMode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -136,6 +137,9 @@ PyObject* metadata(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       const NoGil nogil;
       check(fmla_get_num_sm_parts(lens.get_device(), q_per_hk, h_k, h_q, fp8, sparse, &parts));
       const c10::cuda::CUDAGuard guard(lens.device());
+      // ordinary tensors under torch.inference_mode() too: what is known of a plan holds until an in-place write to it, which
+      // only their version counter tells
+      const c10::InferenceMode ordinary(false);
       md = new_tensor({parts, 8}, lens, at::kInt);
       ns = new_tensor({b + 1}, lens, at::kInt);
       check(fmla_get_mla_metadata(static_cast<const int32_t*>(lens.const_data_ptr()), static_cast<int>(b), parts, topk,

@@ -53,7 +53,7 @@ def get_mla_decoding_metadata(seqlens_k: torch.Tensor, num_q_tokens_per_head_k: 
                               topk: Optional[int] = None) -> List[torch.Tensor]:
     """csrc/pybind.cpp:383-428.  Returns [tile_scheduler_metadata int32[num_sm_parts, 8], num_splits int32[b+1]]."""
     md, ns, whole = _native.metadata(seqlens_k, num_q_tokens_per_head_k, h_k, h_q, is_fp8_kvcache, topk)
-    if whole is not None and not ns.is_inference():
+    if whole is not None:
         ns._fmla_no_split, ns._fmla_no_split_version = whole, ns._version
     return [md, ns]
 
@@ -86,11 +86,14 @@ def fwd_kvcache_mla(q: torch.Tensor, kcache: torch.Tensor, head_size_v: int, seq
 def _no_request_is_split(num_splits: torch.Tensor) -> bool:
     """True when the schedule is known to give every request to one partition: the merge kernel is then not launched.
     A sparse schedule is a function of numbers the host has (batch, topk, partitions), so get_mla_decoding_metadata
-    says so on the tensor it returns; an in-place write to that tensor withdraws it.  The lengths of a dense batch are
-    on the device, and reading the outcome back costs a synchronisation per plan (40 us against the 2 us of a merge
-    kernel that finds nothing to do): it counts as not known."""
-    known = getattr(num_splits, "_fmla_no_split", False)
-    return known and getattr(num_splits, "_fmla_no_split_version", None) in (None, num_splits._version)
+    says so on the tensor it returns.  An in-place write to that tensor withdraws it, and a copy that carries the mark
+    (deepcopy, pickle, torch.save) never has its version; a write that torch cannot see (through .data, or by a kernel of
+    the caller's) leaves it, and the attention kernel then reports device status 41.  The lengths of a dense batch are on
+    the device, and reading the outcome back costs a synchronisation per plan (40 us) against 1 to 3 us of a merge kernel
+    that finds nothing to do: it counts as not known."""
+    if not getattr(num_splits, "_fmla_no_split", False) or num_splits.is_inference():
+        return False
+    return getattr(num_splits, "_fmla_no_split_version", None) in (None, num_splits._version)
 
 
 def sparse_prefill_fwd(q: torch.Tensor, kv: torch.Tensor, indices: torch.Tensor, sm_scale: float,
