@@ -117,6 +117,15 @@ bool uniform_schedule_splits_nothing(int64_t b, int64_t len, int64_t parts) {
   return true;
 }
 
+// the same for the test that holds it against the oracle's statement of the schedule: b, len, parts -> bool
+PyObject* splits_nothing(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  return guarded(nargs, 3, [&]() -> PyObject* {
+    const int64_t b = integer(a[0]), len = integer(a[1]), parts = integer(a[2]);
+    require(b > 0 && len >= 0 && parts > 0, "b and parts must be positive, len non-negative");
+    return PyBool_FromLong(uniform_schedule_splits_nothing(b, len, parts));
+  });
+}
+
 // seqlens_k, num_q_tokens_per_head_k, h_k, h_q | None, is_fp8, topk | None -> [metadata, num_splits, no request is split]
 // (the last one None where it depends on lengths that only the device has)
 PyObject* metadata(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
@@ -327,6 +336,7 @@ PyCFunction fast() {
   return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(F));
 }
 PyMethodDef methods[] = {{"metadata", fast<metadata>(), METH_FASTCALL, nullptr},
+                         {"splits_nothing", fast<splits_nothing>(), METH_FASTCALL, nullptr},
                          {"decode", fast<decode>(), METH_FASTCALL, nullptr},
                          {"sparse_prefill", fast<sparse_prefill>(), METH_FASTCALL, nullptr},
                          {"quantize", fast<quantize>(), METH_FASTCALL, nullptr},
