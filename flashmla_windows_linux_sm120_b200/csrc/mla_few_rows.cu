@@ -31,6 +31,7 @@
 #include "launch.cuh"
 #include "mla_work.cuh"
 #include "tc_common.cuh"
+#include "tma_host.cuh"
 
 #include <cuda.h>
 #include <cuda_fp8.h>
@@ -728,27 +729,6 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
 }
 
 // ---- host side ----------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-// 16-bit tensor [d3][d2][d1][576] with element strides s1, s2, s3; box {64, b1, b2, 1}
-static bool few_map_4d(CUtensorMap* m, const void* base, uint64_t d1, uint64_t d2, uint64_t d3, int64_t s1, int64_t s2, int64_t s3, uint32_t b1,
-                       uint32_t b2) {
-  static EncodeTiledFn enc = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess) f = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(f);
-  }();
-  if (!enc) return false;
-  cuuint64_t dims[4] = {576, d1, d2, d3};
-  cuuint64_t strides[3] = {static_cast<cuuint64_t>(s1) * 2, static_cast<cuuint64_t>(s2) * 2, static_cast<cuuint64_t>(s3) * 2};
-  cuuint32_t box[4] = {64, b1, b2, 1};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <int MODE, int N, bool F16 = false>
 static cudaError_t launch_few(const FewParams& P, const CUtensorMap& tq, const CUtensorMap& tkv, dim3 grid, cudaStream_t stream) {
   constexpr auto kern = mla_few_rows_kernel<MODE, N, F16>;
@@ -768,8 +748,8 @@ cudaError_t launch_decode_few_rows(const DecodeKernelParams& p, cudaStream_t str
   const int n = rows <= 16 ? 16 : rows <= 32 ? 32 : 64;
   CUtensorMap tq, tkv;
   // q [b][s_q][h_q][576]; cache [num_blocks][64][h_k][576] as (col, head, row in page, page), one map type for bf16 and fp16
-  if (!few_map_4d(&tq, p.q, p.h_q, p.s_q, p.b, p.q_stride_h, p.q_stride_s, p.q_stride_b, fold ? p.hq_per_hk : n, 1)) return cudaErrorInvalidValue;
-  if (!few_map_4d(&tkv, p.kcache, p.h_k, 64, p.num_blocks, p.k_stride_head, p.k_stride_row, p.k_stride_block, 1, 64)) return cudaErrorInvalidValue;
+  if (!tmah::make_map_4d(&tq, p.q, p.h_q, p.s_q, p.b, p.q_stride_h, p.q_stride_s, p.q_stride_b, fold ? p.hq_per_hk : n, 1)) return cudaErrorInvalidValue;
+  if (!tmah::make_map_4d(&tkv, p.kcache, p.h_k, 64, p.num_blocks, p.k_stride_head, p.k_stride_row, p.k_stride_block, 1, 64)) return cudaErrorInvalidValue;
   const dim3 grid(tiles, p.h_k, p.num_sm_parts);
   if (p.is_f16) {
     if (n == 16) return launch_few<kDense, 16, true>(P, tq, tkv, grid, stream);
@@ -786,7 +766,7 @@ cudaError_t launch_decode_sparse_few_rows(const DecodeKernelParams& p, cudaStrea
   P.d = p;
   const int rows = p.hq_per_hk < 64 ? p.hq_per_hk : 64, n = rows <= 16 ? 16 : rows <= 32 ? 32 : 64;
   CUtensorMap tq;
-  if (!few_map_4d(&tq, p.q, p.h_q, p.s_q, p.b, p.q_stride_h, p.q_stride_s, p.q_stride_b, n, 1)) return cudaErrorInvalidValue;
+  if (!tmah::make_map_4d(&tq, p.q, p.h_q, p.s_q, p.b, p.q_stride_h, p.q_stride_s, p.q_stride_b, n, 1)) return cudaErrorInvalidValue;
   const dim3 grid(p.s_q * ((p.hq_per_hk + 63) / 64), 1, p.num_sm_parts);
   if (n == 16) return launch_few<kSparseDecode, 16>(P, tq, tq, grid, stream);      // the cache is not read through a map
   if (n == 32) return launch_few<kSparseDecode, 32>(P, tq, tq, grid, stream);

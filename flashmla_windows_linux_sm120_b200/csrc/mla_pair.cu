@@ -53,6 +53,7 @@
 #include "launch.cuh"
 #include "mla_work.cuh"
 #include "tc_common.cuh"
+#include "tma_host.cuh"
 
 #include <cuda.h>
 #include <cuda_fp8.h>
@@ -551,9 +552,6 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
             // (its commit goes to both): both V stages are free
             const int kst = vg % kKStages, vst = vg & 1;
             FMLA_PTRACE_AT(vg, 12);
-#ifdef FMLA_EXP_NO_FWD          // timing experiment only: results are wrong
-            tc::mbar_arrive(bar(V_LAND0 + vst));
-#else
             tc::mbar_arrive_expect_tx(bar(V_LAND0 + vst), kVStageBytes);      // 16 KB from this CTA, 16 KB from the peer
 #pragma unroll
             for (int d = 0; d < 2; ++d) {
@@ -569,7 +567,6 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
                              : "memory");
               }
             }
-#endif
             ++vg;
             did = true;
             if (vg == v_end) {
@@ -622,17 +619,12 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
           alive = tc::mbar_wait(bar(V_EMPTY0 + st), ((g >> 1) & 1) ^ 1, status, 103);
           if (!alive) break;
           FMLA_PTRACE_AT(g, 12);
-#ifdef FMLA_EXP_NO_V_LOAD      // timing experiment only: results are wrong
-          tc::mbar_arrive(bar(V_LAND0 + st));
-          (void)page;
-#else
           tc::mbar_arrive_expect_tx(bar(V_LAND0 + st), kVStageBytes);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int chunk = (i >> 1) * 4 + 2 * static_cast<int>(rank) + (i & 1);     // value columns 64*chunk ..
             tc::tma_load_4d(sV + st * kVStageBytes + i * kChunkBytes, &tmap_v64, chunk * 64, tile.kh, 0, page, bar(V_LAND0 + st));
           }
-#endif
         }
       }
     }
@@ -756,9 +748,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
             tc::tc_fence_after();
             if (lane == 0) { FMLA_PTRACE_AT(gp, 4); FMLA_GTRACE_AT(gp, 0, 5); }
             if (tc::elect_one()) {
-#ifndef FMLA_EXP_NO_PV         // timing experiment only: results are wrong
               pv_block_pair(tmem + TMEM_O, tc::desc_advance(desc_p, stp * kChunkBytes), tc::desc_advance(desc_v, stp * kVStageBytes), idesc_o, jp == 0);
-#endif
               commit_both(V_EMPTY0 + stp);
               commit_both(P_EMPTY0 + stp);
               FMLA_PTRACE_AT(gp, 5);
@@ -1070,33 +1060,6 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
 }
 
 // ---- host side ----------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn pair_encode_fn() {
-  static EncodeTiledFn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess) f = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(f);
-  }();
-  return fn;
-}
-
-// 16-bit tensor [d3][d2][d1][d0=576] with element strides s1,s2,s3 ; box {64, b1, b2, 1}
-static bool pair_map_4d(CUtensorMap* m, const void* base, uint64_t d1, uint64_t d2, uint64_t d3, int64_t s1, int64_t s2, int64_t s3,
-                        uint32_t b1, uint32_t b2) {
-  EncodeTiledFn enc = pair_encode_fn();
-  if (!enc) return false;
-  cuuint64_t dims[4] = {576, d1, d2, d3};
-  cuuint64_t strides[3] = {static_cast<cuuint64_t>(s1) * 2, static_cast<cuuint64_t>(s2) * 2, static_cast<cuuint64_t>(s3) * 2};
-  cuuint32_t box[4] = {64, b1, b2, 1};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <auto Kern>
 static cudaError_t launch_pair(const TcParams& P, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, dim3 grid, int threads,
                                cudaStream_t stream) {
@@ -1111,7 +1074,7 @@ cudaError_t launch_decode_sparse_pair(const DecodeKernelParams& p, cudaStream_t 
   P.d = p;
   CUtensorMap tq;
   // q [b][s_q][h_q][576] ; box = 64 heads x 64 columns
-  if (!pair_map_4d(&tq, p.q, p.h_q, p.s_q, p.b, p.q_stride_h, p.q_stride_s, p.q_stride_b, 64, 1)) return cudaErrorInvalidValue;
+  if (!tmah::make_map_4d(&tq, p.q, p.h_q, p.s_q, p.b, p.q_stride_h, p.q_stride_s, p.q_stride_b, 64, 1)) return cudaErrorInvalidValue;
   return launch_pair<mla_pair_kernel<false, kSparseDecode>>(P, tq, tq, tq, dim3(2, p.s_q, p.num_sm_parts), ptc::kSparseDecodeThreads, stream);   // the K / V maps are not used in this mode
 }
 
@@ -1122,7 +1085,7 @@ cudaError_t launch_sparse_prefill_pair(const SparsePrefillKernelParams& sp, cuda
   P.sp = sp;
   CUtensorMap tq;
   // q [s_q][h_q][576] as (col, head, token, 1)
-  if (!pair_map_4d(&tq, sp.q, sp.h_q, sp.s_q, 1, sp.q_stride_h, sp.q_stride_s, sp.q_stride_s * sp.s_q, 64, 1)) return cudaErrorInvalidValue;
+  if (!tmah::make_map_4d(&tq, sp.q, sp.h_q, sp.s_q, 1, sp.q_stride_h, sp.q_stride_s, sp.q_stride_s * sp.s_q, 64, 1)) return cudaErrorInvalidValue;
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
   const int lanes = max(1, min(sp.s_q, sms / 2));
@@ -1144,10 +1107,10 @@ cudaError_t launch_decode_dense_pair(const DecodeKernelParams& p, cudaStream_t s
   P.d.l2_prefetch_dist = prefetch;
   CUtensorMap tq, tk, tv;
   // q [b][s_q][h_q][576] ; box = 64 heads x 64 columns
-  if (!pair_map_4d(&tq, p.q, p.h_q, p.s_q, p.b, p.q_stride_h, p.q_stride_s, p.q_stride_b, 64, 1)) return cudaErrorInvalidValue;
+  if (!tmah::make_map_4d(&tq, p.q, p.h_q, p.s_q, p.b, p.q_stride_h, p.q_stride_s, p.q_stride_b, 64, 1)) return cudaErrorInvalidValue;
   // cache [num_blocks][64][h_k][576] addressed as (col, head, row-in-page, page): boxes of 32 rows (K part) and 64 rows (V part)
-  if (!pair_map_4d(&tk, p.kcache, p.h_k, 64, p.num_blocks, p.k_stride_head, p.k_stride_row, p.k_stride_block, 1, 32)) return cudaErrorInvalidValue;
-  if (!pair_map_4d(&tv, p.kcache, p.h_k, 64, p.num_blocks, p.k_stride_head, p.k_stride_row, p.k_stride_block, 1, 64)) return cudaErrorInvalidValue;
+  if (!tmah::make_map_4d(&tk, p.kcache, p.h_k, 64, p.num_blocks, p.k_stride_head, p.k_stride_row, p.k_stride_block, 1, 32)) return cudaErrorInvalidValue;
+  if (!tmah::make_map_4d(&tv, p.kcache, p.h_k, 64, p.num_blocks, p.k_stride_head, p.k_stride_row, p.k_stride_block, 1, 64)) return cudaErrorInvalidValue;
   const int n_hb = p.hq_per_hk / 64;
   const dim3 grid(p.s_q * n_hb, p.h_k, p.num_sm_parts);
   if (p.is_f16) return launch_pair<mla_pair_kernel<true, kDense>>(P, tq, tk, tv, grid, ptc::kThreads, stream);

@@ -28,7 +28,7 @@ struct Work {
 
 // Which tile and which stretch of the schedule a CTA owns.
 struct Tile {
-  int sq, hb, kh, head0, nvalid;
+  int sq, hb, kh, head0;
   int begin_idx, end_idx, begin_block, end_block, begin_split;
   int n_work;
 };
@@ -40,7 +40,7 @@ __device__ __forceinline__ Tile make_tile(const TcParams& P) {
     // persistent over query tokens: this CTA takes tokens blockIdx.y, blockIdx.y + gridDim.y, ... so that the
     // Q load and the output stores of one token overlap with the blocks of its neighbours
     t.hb = blockIdx.x; t.sq = blockIdx.y; t.kh = 0;
-    t.head0 = t.hb * 64; t.nvalid = 64;
+    t.head0 = t.hb * 64;
     t.begin_idx = t.end_idx = 0; t.begin_block = 0; t.end_block = P.sp.topk / 64; t.begin_split = 0;
     t.n_work = (P.sp.s_q - static_cast<int>(blockIdx.y) + static_cast<int>(gridDim.y) - 1) / static_cast<int>(gridDim.y);
   } else {
@@ -53,7 +53,6 @@ __device__ __forceinline__ Tile make_tile(const TcParams& P) {
       t.hb = blockIdx.x; t.sq = blockIdx.y; t.kh = 0; part = blockIdx.z;
     }
     t.head0 = t.kh * p.hq_per_hk + t.hb * 64;
-    t.nvalid = min(64, p.hq_per_hk - t.hb * 64);
     const int4 md = *reinterpret_cast<const int4*>(p.tile_scheduler_metadata + part * 8);
     t.begin_idx = md.x; t.begin_block = md.y; t.end_idx = md.z; t.end_block = md.w;
     t.begin_split = p.tile_scheduler_metadata[part * 8 + 4];
