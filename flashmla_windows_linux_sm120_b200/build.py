@@ -3,7 +3,7 @@
 ``python flashmla_windows_linux_sm120_b200/build.py`` (run as a script, so that a stale library cannot block its own rebuild) compiles
 ``csrc/*.cu`` into ``flashmla_windows_linux_sm120_b200/lib/libflashmla_b200.so`` and the torch marshalling module
 ``csrc/torch_binding.cpp`` into ``lib/_fmla_torch.so``, which finds the library beside it.
-Objects are rebuilt only when a source or header is newer.
+Objects are rebuilt only when a source or header is newer, the module also when torch or Python is another one.
 """
 from __future__ import annotations
 
@@ -85,10 +85,16 @@ def build(force: bool = False, verbose: bool = False) -> str:
 def _build_binding(force: bool) -> None:
     src = os.path.join(CSRC, "torch_binding.cpp")
     header = os.path.join(INCLUDE_DIR, "flashmla_b200.h")
-    if not force and os.path.exists(BINDING_PATH) and os.path.getmtime(BINDING_PATH) >= _newest([src, header]):
-        return
     # torch is located, not imported: importing it takes longer than this compilation
     torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    # the module holds on to the ABI of one torch and one Python
+    with open(os.path.join(torch_dir, "version.py")) as f:
+        built_for = f"{sys.version}\n{torch_dir}\n{f.read()}"
+    stamp = os.path.join(OBJ_DIR, "_fmla_torch.built_for")
+    if not force and os.path.exists(BINDING_PATH) and os.path.getmtime(BINDING_PATH) >= _newest([src, header]) and os.path.exists(stamp):
+        with open(stamp) as f:
+            if f.read() == built_for:
+                return
     cuda_home = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", src, "-o", BINDING_PATH,
            "-I", sysconfig.get_paths()["include"], "-I", os.path.join(torch_dir, "include"),
@@ -99,6 +105,8 @@ def _build_binding(force: bool) -> None:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"building {BINDING_PATH} failed:\n{r.stdout}\n{r.stderr}")
+    with open(stamp, "w") as f:
+        f.write(built_for)
 
 
 if __name__ == "__main__":
