@@ -6,14 +6,17 @@
 // with N = 16, 32 or 64, the smallest that holds the tile's rows.  What bounds the path is the cache stream (1152 bytes
 // per token against 2 * 1088 * rows FLOP), so the layout serves the loads in flight:
 //   * Q takes N x 1152 bytes of shared memory instead of 72 KB: the rest is a ring of 8 KB slots (64 tokens x 64
-//     columns) filled and released slot by slot -- 22 + 3 slots for N = 16 (2.8 pages in flight), 20 + 2 for N = 32,
+//     columns) filled slot by slot behind the pages that P V has finished with -- 22 + 3 slots for N = 16 (2.8 pages in flight), 20 + 2 for N = 32,
 //     16 + 2 for N = 64.  Two whole-page stages, each held from the start of its load to the end of its P V, left the
 //     memory idle half of the time (61 requests x 6000 tokens, 16 heads: 117 us against 63 us at the copy bandwidth).
 //   * several query tokens share a CTA and with it the page (s_q * heads <= 64: the cache is read once per step, not
 //     once per query token).
-//   * an output column lives in one TMEM lane: every store of a warp covers 32 consecutive columns of a row.  With one
-//     row per lane the partial tile of a split request (64 rows x 2 KB) took 10 000 clk to leave the SM, more than
-//     everything else a CTA does for a short request.
+//   * an output column lives in one TMEM lane: a warp's store to a partial covers 32 consecutive columns of a row (64 rows of
+//     2 KB leave the SM in 5 200 clk; with one row per lane they took 10 000).  Rows of whole requests are transposed on the
+//     way out (stmatrix) and leave in 16-byte pieces: 4 600 clk for 64 of them.
+// Two neighbouring 64-head tiles that read the same pages belong to the CTA pair instead (mla_pair.cu).  Reading pages beyond
+// the ring into L2 ahead of their loads was measured slower throughout (six pages ahead, in the steady state or at the start
+// of a request only: 100 shapes with 16 heads 6 and 5 %, with 64 heads 4 and 3 %).
 // Warps: 0-3 softmax and epilogue, 4 TMA, 5 MMA, 6-13 gather (sparse), which read the 656-byte records of a 64-index block
 // into registers one block ahead, de-quantise (bf16(fp32(e4m3) * scale)) and store them into the slots in the layout TMA
 // produces.  An invalid index leaves a zero row and a cleared validity bit.
@@ -375,8 +378,8 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
       // S^T runs one block ahead of O^T; where both could be next, whichever has its inputs first is issued, O^T first: it
       // releases slots of the ring.  S^T(js) overwrites S^T(js - 2), and O^T(0) what the request before left: the softmax
       // warps had read both before they arrived on a P_FULL that has been waited for here (P_FULL(js - 2), P_FULL(0)).
-      // A test of a barrier takes about 130 clk and tests of different barriers by different lanes follow one another, so
-      // only what is needed is looked at: with four barriers per poll the warp saw P 550 clk after its last arrival.
+      // Only what is needed is looked at: with four barriers per poll, one per lane, the warp saw P 550 clk after its last
+      // arrival, now 375 (64 heads, two query tokens, 16 x 16 000 tokens: 143 -> 140 us; 8 to 64 rows 2 % of a step).
       int js = 0, jp = 0, idle = 0;
       while (jp < nblk && alive) {
         const int gs = g + js, gp = g + jp;

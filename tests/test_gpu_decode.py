@@ -243,8 +243,8 @@ def _device_status(reset=True):
 @pytest.mark.parametrize("h_q,b", [(128, 21), (64, 42)])
 def test_no_merge_kernel_when_no_request_is_split(h_q, b):
     """Requests of equal cost (2 blocks + 5 of overhead) whose number makes the pitch of the cuts equal to that
-    cost: the schedule splits none of them, the binding reads that back once (remembered on the metadata tensor)
-    and the merge kernel is not launched.  Same results."""
+    cost: the schedule splits none of them, which the binding knows from the batch, topk and the number of partitions
+    (noted on the num_splits tensor), and the merge kernel is not launched.  Same results."""
     fm = _api()
     t = gen.DecodeCase(b=b, s_q=1, s_k=600, is_varlen=True, topk=128, h_q=h_q)
     d = gen.make_decode_case(t)
@@ -253,7 +253,7 @@ def test_no_merge_kernel_when_no_request_is_split(h_q, b):
     lens = d.cache_seqlens.cuda()
     md, ns = fm.get_mla_metadata(lens, t.s_q * t.h_q, 1, t.h_q, True, t.topk)
     assert int(ns[t.b]) == t.b                      # no request is split
-    for _ in range(2):                              # the second call uses the remembered answer
+    for _ in range(2):
         out, lse = fm.flash_mla_with_kvcache(d.q.cuda(), kq.cuda(), d.block_table.cuda(), lens, t.dv, md, ns,
                                              is_fp8_kvcache=True, indices=d.indices.cuda())
         torch.cuda.synchronize()
