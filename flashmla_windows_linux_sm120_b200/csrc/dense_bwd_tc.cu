@@ -663,7 +663,20 @@ static cudaError_t launch_bwd_tc(const DenseKernelParams& p, cudaStream_t stream
   dense_bwd_delta_tc_kernel<<<static_cast<unsigned>((rows + per_block - 1) / per_block), 256, 0, stream>>>(p);
   kk<<<dim3((p.max_seqlen_k + 127) / 128, p.h_q, p.batch), kDkvThreads, L::SMEM_BYTES, stream>>>(p, k128, v128, q64, do64);
   if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
-  return launch_dependent(kq, dim3((p.max_seqlen_q + 127) / 128, p.h_q, p.batch), kDqThreads, L::SMEM_BYTES, stream, p, q128, do128, k64, v64);
+  const dim3 grid((p.max_seqlen_q + 127) / 128, p.h_q, p.batch);
+  // dQ written over Q or dO (which its own kernel reads tile by tile, before it writes) must wait until dK / dV has read them
+  const auto overlaps = [&](const void* x, int d, int64_t stride_t, int64_t stride_h) {
+    const auto end = [&](const void* base, int dim, int64_t st, int64_t sh) {
+      return reinterpret_cast<uintptr_t>(base) + 2 * ((p.total_q - 1) * st + (p.h_q - 1) * sh + dim);
+    };
+    return reinterpret_cast<uintptr_t>(p.dq) < end(x, d, stride_t, stride_h) &&
+           reinterpret_cast<uintptr_t>(x) < end(p.dq, p.d_qk, p.dq_stride_t, p.dq_stride_h);
+  };
+  if (overlaps(p.q, p.d_qk, p.q_stride_t, p.q_stride_h) || overlaps(p.d_o, p.d_v, p.do_stride_t, p.do_stride_h)) {
+    kq<<<grid, kDqThreads, L::SMEM_BYTES, stream>>>(p, q128, do128, k64, v64);
+    return cudaGetLastError();
+  }
+  return launch_dependent(kq, grid, kDqThreads, L::SMEM_BYTES, stream, p, q128, do128, k64, v64);
 }
 
 cudaError_t launch_dense_bwd_tc(const DenseKernelParams& p, cudaStream_t stream) {
