@@ -39,7 +39,7 @@ def test_a_full_launch_queue_stops_no_other_thread():
     ticker.join()
     torch.cuda.synchronize()
     assert waited > 0.3, "the launch queue never filled"
-    assert max(gaps) < 0.15, max(gaps)
+    assert max(gaps) < 0.25, max(gaps)
 
 
 def test_two_threads_decode_on_their_own_streams():
