@@ -88,7 +88,7 @@ void ensure_status_mirror(int dev) {
     return;
   }
   int* w = static_cast<int*>(dptr);
-  if (fmla::set_status_mirror_prefill64(w) != cudaSuccess || fmla::set_status_mirror_pair(w) != cudaSuccess ||
+  if (fmla::set_status_mirror_tile64(w) != cudaSuccess || fmla::set_status_mirror_pair(w) != cudaSuccess ||
       fmla::set_status_mirror_few_rows(w) != cudaSuccess ||
       fmla::set_status_mirror_merge(w) != cudaSuccess ||
       fmla::set_status_mirror_dense_fwd(w) != cudaSuccess || fmla::set_status_mirror_dense_bwd(w) != cudaSuccess) {
@@ -408,7 +408,7 @@ int fmla_device_status(int* status_host, int reset) {
   cudaError_t e = fmla::read_decode_pair_status(status_host, reset != 0);
   if (e != cudaSuccess) return cuda_fail(e, "reading the device status word");
   int other_status = 0;
-  e = fmla::read_prefill64_status(&other_status, reset != 0);
+  e = fmla::read_tile64_status(&other_status, reset != 0);
   if (e != cudaSuccess) return cuda_fail(e, "reading the device status word");
   if (*status_host == 0) *status_host = other_status;
   int few_status = 0;

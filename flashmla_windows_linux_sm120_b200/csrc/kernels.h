@@ -106,7 +106,7 @@ bool decode_dense_pair_applies(const DecodeKernelParams& p);
 bool decode_dense_merges_in_kernel(const DecodeKernelParams& p);
 cudaError_t launch_decode_dense_pair(const DecodeKernelParams& p, cudaStream_t stream);
 cudaError_t read_decode_pair_status(int* host_status, bool reset);
-// at most 64 query rows per CTA (mla_few_rows.cu): every head count the pair kernel does not take
+// at most 64 query rows per CTA (mla_few_rows.cu): what the other two do not take
 cudaError_t launch_decode_few_rows(const DecodeKernelParams& p, cudaStream_t stream);
 cudaError_t launch_decode_sparse_few_rows(const DecodeKernelParams& p, cudaStream_t stream);
 cudaError_t read_decode_few_rows_status(int* host_status, bool reset);
@@ -114,10 +114,12 @@ cudaError_t set_status_mirror_few_rows(int* mapped_host_word);
 // sparse decode and sparse prefill as CTA pairs (mla_pair.cu): 128 heads
 bool decode_sparse_pair_applies(const DecodeKernelParams& p);
 cudaError_t launch_decode_sparse_pair(const DecodeKernelParams& p, cudaStream_t stream);
-// sparse prefill, one CTA per 64 heads (mla_prefill64.cu)
+// one CTA per 64 heads (mla_tile64.cu): sparse prefill; dense decode where several 64-row tiles read the same pages
+bool decode_dense_tile64_applies(const DecodeKernelParams& p);
+cudaError_t launch_decode_dense_tile64(const DecodeKernelParams& p, cudaStream_t stream);
 cudaError_t launch_sparse_prefill_64(const SparsePrefillKernelParams& sp, cudaStream_t stream);
-cudaError_t read_prefill64_status(int* host_status, bool reset);
-cudaError_t set_status_mirror_prefill64(int* mapped_host_word);
+cudaError_t read_tile64_status(int* host_status, bool reset);
+cudaError_t set_status_mirror_tile64(int* mapped_host_word);
 bool sparse_prefill_pair_applies(const SparsePrefillKernelParams& sp);
 cudaError_t launch_sparse_prefill_pair(const SparsePrefillKernelParams& sp, cudaStream_t stream);
 // Merge of split partials for a decode call (reads num_splits; skips unsplit requests).

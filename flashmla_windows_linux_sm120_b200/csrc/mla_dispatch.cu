@@ -1,6 +1,7 @@
 // Which kernel runs an MLA attention call: the CTA pair (mla_pair.cu) where 128 heads share a kv head, or the 64 heads of two
-// query tokens -- its two CTAs read every cached token once for all of them -- and otherwise one CTA per at most 64 query rows (mla_few_rows.cu), or per 64
-// heads of the sparse prefill (mla_prefill64.cu).
+// query tokens -- its two CTAs read every cached token once for all of them.  Otherwise one CTA per 64 heads (mla_tile64.cu) for
+// the sparse prefill and where several such tiles of a dense decode read the same pages, or per at most 64 query rows
+// (mla_few_rows.cu).
 #include "kernels.h"
 
 #include <cstdlib>
@@ -22,6 +23,7 @@ bool decode_dense_merges_in_kernel(const DecodeKernelParams& p) {
 
 cudaError_t launch_decode_dense_tc(const DecodeKernelParams& p, cudaStream_t stream) {
   if (decode_dense_pair_applies(p) && pair_kernel_enabled()) return launch_decode_dense_pair(p, stream);
+  if (decode_dense_tile64_applies(p)) return launch_decode_dense_tile64(p, stream);
   return launch_decode_few_rows(p, stream);
 }
 

@@ -14,7 +14,7 @@
 //   * an output column lives in one TMEM lane: a warp's store to a partial covers 32 consecutive columns of a row (64 rows of
 //     2 KB leave the SM in 5 200 clk; with one row per lane they took 10 000).  Rows of whole requests are transposed on the
 //     way out (stmatrix) and leave in 16-byte pieces: 4 600 clk for 64 of them.
-// Two neighbouring 64-head tiles that read the same pages belong to the CTA pair instead (mla_pair.cu).  Reading pages beyond
+// 64-head tiles that read the same pages belong to the CTA pair (two of them, mla_pair.cu) or to mla_tile64.cu instead.  Reading pages beyond
 // the ring into L2 ahead of their loads was measured slower throughout (six pages ahead, in the steady state or at the start
 // of a request only: 100 shapes with 16 heads 6 and 5 %, with 64 heads 4 and 3 %).
 // Warps: 0-3 softmax and epilogue, 4 TMA, 5 MMA, 6-13 gather (sparse), which read the 656-byte records of a 64-index block

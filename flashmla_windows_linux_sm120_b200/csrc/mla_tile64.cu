@@ -1,21 +1,28 @@
-// Sparse MLA prefill forward for 64 heads per CTA on sm_100a (tcgen05 / TMA / tensor memory): top-k row indices into
-// kv[s_kv, 576], rows gathered with cp.async by eight producer warps.  128 heads take the CTA pair (mla_pair.cu).
+// MLA attention for 64 query rows per CTA on sm_100a (tcgen05 / TMA / tensor memory), the rows being the rows of an M = 64 tile:
+//   kSparsePrefill sparse prefill forward with 64 heads: top-k row indices into kv[s_kv, 576], rows gathered with cp.async by
+//                  eight producer warps.  128 heads take the CTA pair (mla_pair.cu).
+//   kDense         dense split-KV decode where several 64-row tiles read the same pages and no pair takes them: three or more
+//                  query tokens of 64 heads, 96 or 192 heads.  Whichever tile is first pulls a page into L2 (six ahead), the others
+//                  find it there, and what counts is how long a page is held: 3 350 clk per page here, 3 900 with the transposed
+//                  products of mla_few_rows.cu and 64 rows.
 //
-// One CTA = the 64-head tile of one query token at a time.
-//   warps 0-3 softmax : TMEM S -> registers, mask, running max / sum (base 2), P (bf16) -> shared
+// One CTA = the 64-head tile of one query token (at a time).
+//   warps 0-3 softmax : TMEM S -> registers, mask, running max / sum (base 2), P (16 bits) -> shared
 //                       memory, lazy rescale of O in TMEM, final 1/l normalisation and stores
-//   warp 4   TMA      : Q tile (9 boxes of 64 rows x 64 cols)
+//   warp 4   TMA      : Q tile (9 boxes of 64 rows x 64 cols); kDense also the pages (9 boxes) into the two stages
 //   warp 5   MMA      : S = Q K^T  (36 x tcgen05.mma.ws m64n64k16)  -> TMEM S[stage]
 //                       O += P V   ( 8 x tcgen05.mma.ws m64n256k16) -> TMEM O
 //                       V is the first 512 columns of the same K tile, read MN-major
-//   warps 6-13 gather : write K rows in the layout TMA produces (64-column chunks of 128-byte rows, 128-byte swizzle)
-// The transposed products of mla_few_rows.cu were measured slower in this use (333 query tokens, top-k 512: 105 us against
+//   warps 6-13 gather : kSparsePrefill; write K rows in the layout TMA produces (64-column chunks of 128-byte rows, 128-byte
+//                       swizzle)
+// The transposed products were measured slower in the prefill too (333 query tokens, top-k 512: 105 us against
 // 64 us): with 64 heads they need the same shared memory, and the cp.async gather, not the page stream, sets the pace.
 // TMEM map (512 columns allocated): O = [0,256) (two N=256 halves of 128 columns),
 // S[0] = [256,288), S[1] = [288,320).  In the M=64 weight-stationary layout element
 // (row r, col c) of an N-wide result sits in lane r + 64*(c >= N/2), column c % (N/2).
 //
-// Semantics follow csrc/sm100/prefill/sparse/fwd.cu:399-417, 438-445, 677-679 of the reference.
+// Semantics follow the reference kernels: sparse prefill csrc/sm100/prefill/sparse/fwd.cu:399-417, 438-445, 677-679; decode
+// borders / split outputs / LSE conventions csrc/sm90/decode/dense/splitkv_mla.cu:948-957, 1022-1042, 1237-1269.
 // Every mbarrier wait is bounded (tc_common.cuh); a pipeline fault sets a status word and lets the
 // CTA drain and free its tensor memory.
 #include "kernels.h"
@@ -44,17 +51,18 @@ static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB shared memory limit per 
 static_assert(NUM_BARS * 8 <= 128, "barrier area too small");
 constexpr float kRescaleThreshold = 8.0f;         // log2 units; below it O keeps its stale scale
 constexpr int kGatherThreads = 256;               // 8 gather warps
-constexpr int kThreads = 192 + kGatherThreads;
+constexpr int threads(int mode) { return 192 + (mode == kDense ? 0 : kGatherThreads); }
+constexpr int kPrefetchDist = 6;                  // cache pages pulled into L2 ahead of the stage loads
 }  // namespace dtc
 
-__device__ int g_prefill64_status = 0;
+__device__ int g_tile64_status = 0;
 
 // Optional timeline of the first blocks of CTA (0,0,0), compiled in with -DFMLA_TRACE only.
 #ifdef FMLA_TRACE
-__device__ long long g_prefill64_trace[64 * 16];
+__device__ long long g_tile64_trace[64 * 16];
 #define FMLA_TRACE_AT(blk, slot)                                                          \
   do {                                                                                     \
-    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (blk) < 64) g_prefill64_trace[(blk) * 16 + (slot)] = clock64(); \
+    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && (blk) < 64) g_tile64_trace[(blk) * 16 + (slot)] = clock64(); \
   } while (0)
 #else
 #define FMLA_TRACE_AT(blk, slot) do {} while (0)
@@ -77,9 +85,11 @@ __device__ __forceinline__ void s_block(uint32_t tmem, uint64_t desc_q, uint64_t
                     tc::desc_advance(desc_k, ST * kTileBytes + c * kChunkBytes + s * 32), idesc, (c | s) ? 1u : 0u);
 }
 
-// grid (h_q / 64, min(s_q, SMs / (h_q / 64))): persistent over the query tokens
-__global__ void __launch_bounds__(dtc::kThreads, 1)
-mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUtensorMap tmap_q) {
+// kDense: grid (s_q * ceil(hq_per_hk / 64), h_k, parts); kSparsePrefill: grid (h_q / 64, min(s_q, SMs / (h_q / 64))), persistent
+// over the query tokens
+template <int MODE, bool F16>
+__global__ void __launch_bounds__(dtc::threads(MODE), 1)
+mla_tile64_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kv) {
   using namespace dtc;
   extern __shared__ __align__(1024) unsigned char smem[];
   const uint32_t sbase = smem_u32(smem);
@@ -89,17 +99,17 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
   volatile uint32_t* sTmem = reinterpret_cast<volatile uint32_t*>(smem + MISC_OFF);
   volatile int* sAbort = reinterpret_cast<volatile int*>(smem + MISC_OFF + 8);   // set by a softmax thread whose wait expired
   volatile uint32_t* sValid = reinterpret_cast<volatile uint32_t*>(smem + MISC_OFF + 16);   // [stage][token half]: 32 validity bits
-  int* status = &g_prefill64_status;
+  int* status = &g_tile64_status;
+
+  const DecodeKernelParams& p = P.d;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const Tile tile = make_tile<kSparsePrefill>(P);
-  if ((sbase & 1023u) != 0) {   // the swizzled tiles need a 1024-byte aligned base
-    if (tid == 0) tc::report_status(status, 30);
-    return;
-  }
-  const float scale_log2 = P.sp.scale_log2;
-  // arrivals per filled stage: one per gather thread (by hardware) and one per gather warp
-  constexpr int kKvFullCount = kGatherThreads + kGatherThreads / 32;
+  const bool misaligned = (sbase & 1023u) != 0;      // the swizzled tiles need a 1024-byte aligned base
+  if (misaligned && tid == 0) tc::report_status(status, 30);
+  const float scale_log2 = MODE == kSparsePrefill ? P.sp.scale_log2 : p.scale_log2;
+  // arrivals per filled stage: one (with a byte count) from the TMA thread, or one per gather thread (by hardware) and one
+  // per gather warp
+  constexpr int kKvFullCount = MODE == kDense ? 1 : kGatherThreads + kGatherThreads / 32;
 
   if (tid == 0) {
     tc::mbar_init(bar(Q_FULL), 1);
@@ -124,28 +134,59 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *sTmem;
+  if constexpr (MODE == kDense) {
+    pdl_wait();                 // the schedule, the queries and the cache may come from the kernel in front of this one (loads: mla_work.cuh)
+    pdl_allow_dependents();     // the merge kernel may become resident now
+  }
+  const Tile tile = make_tile<MODE>(P);
 
-  if (warp == 4) {
+  if (misaligned || tile.n_work == 0) {
+    // nothing to do
+  } else if (warp == 4) {
     // ================================ TMA producer =====================================
     if (tc::elect_one()) {
       tc::prefetch_tensormap(&tmap_q);
-      int req = 0;
+      if constexpr (MODE == kDense) tc::prefetch_tensormap(&tmap_kv);
+      int g = 0, req = 0;
       bool alive = true;
       for (int wi = 0; wi < tile.n_work && alive; ++wi) {
-        const Work r = get_work<kSparsePrefill>(P, tile, wi);
+        const Work r = get_work<MODE>(P, tile, wi);
         if (r.blk_hi == r.blk_lo) continue;
         alive = tc::mbar_wait(bar(Q_EMPTY), (req & 1) ^ 1, status, 1);
         if (!alive) break;
         tc::mbar_arrive_expect_tx(bar(Q_FULL), kTileBytes);
 #pragma unroll
         for (int c = 0; c < 9; ++c)
-          tc::tma_load_4d(sQ + c * kChunkBytes, &tmap_q, c * 64, tile.head0, r.batch, 0, bar(Q_FULL));
+          tc::tma_load_4d(sQ + c * kChunkBytes, &tmap_q, c * 64, tile.head0, MODE == kDense ? tile.sq : r.batch, MODE == kDense ? r.batch : 0, bar(Q_FULL));
         ++req;
+        if constexpr (MODE == kDense) {
+          const int* bt = p.block_table + r.batch * p.block_table_stride_b;
+          // pages kPrefetchDist steps ahead are pulled into L2 while the two shared-memory stages are busy, so that the load
+          // that later fills a stage sees L2 latency instead of HBM latency
+          auto prefetch = [&](int blk) {
+            const int pg = bt[blk];
+#pragma unroll
+            for (int c = 0; c < 9; ++c) tc::tma_prefetch_l2_4d(&tmap_kv, c * 64, tile.kh, 0, pg);
+          };
+          for (int blk = r.blk_lo; blk < min(r.blk_lo + kPrefetchDist, r.blk_hi); ++blk) prefetch(blk);
+          int page_next = bt[r.blk_lo];
+          for (int blk = r.blk_lo; blk < r.blk_hi; ++blk, ++g) {
+            const int st = g & 1, page = page_next;
+            if (blk + 1 < r.blk_hi) page_next = bt[blk + 1];
+            if (blk + kPrefetchDist < r.blk_hi) prefetch(blk + kPrefetchDist);
+            alive = tc::mbar_wait(bar(KV_EMPTY0 + st), ((g >> 1) & 1) ^ 1, status, 2);
+            if (!alive) break;
+            tc::mbar_arrive_expect_tx(bar(KV_FULL0 + st), kTileBytes);
+#pragma unroll
+            for (int c = 0; c < 9; ++c)
+              tc::tma_load_4d(sKV + st * kTileBytes + c * kChunkBytes, &tmap_kv, c * 64, tile.kh, 0, page, bar(KV_FULL0 + st));
+          }
+        }
       }
     }
   } else if (warp >= 6) {
     // ================================ gather producers =================================
-    {
+    if constexpr (MODE == kSparsePrefill) {
       // Eight gather warps, eight rows each, all on the same block.  For each row the 32 lanes copy
       // consecutive 16-byte pieces (pieces lane, lane+32 and, for 8 lanes, lane+64 of the 72):
       // coalesced cp.async with a handful of address instructions per row.
@@ -157,7 +198,7 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
       int g = 0;
       bool alive = true;
       for (int wi = 0; wi < tile.n_work && alive; ++wi) {
-        const Work r = get_work<kSparsePrefill>(P, tile, wi);
+        const Work r = get_work<MODE>(P, tile, wi);
         for (int blk = r.blk_lo; blk < r.blk_hi && alive; ++blk, ++g) {
           const int st = g & 1;
           int my_idx = __ldg(r.idx + blk * 64 + gw * 8 + (lane & 7));
@@ -191,8 +232,8 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
     }
   } else if (warp == 5) {
     // ================================ MMA issuer =======================================
-    constexpr uint32_t idesc_s = tc::idesc_bf16_f32(64, 64, 0, 0);
-    constexpr uint32_t idesc_o = tc::idesc_bf16_f32(64, 256, 0, 1);
+    constexpr uint32_t idesc_s = tc::idesc_bf16_f32(64, 64, 0, 0, F16);
+    constexpr uint32_t idesc_o = tc::idesc_bf16_f32(64, 256, 0, 1, F16);
     // descriptors of the operand bases; per-MMA addresses are constant offsets added to the low word
     const uint64_t desc_q = tc::smem_desc_sw128(sQ, 16, 1024);             // A of S: K-major
     const uint64_t desc_k = tc::smem_desc_sw128(sKV, 16, 1024);            // B of S: K-major (stage 0)
@@ -231,7 +272,7 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
       __syncwarp();
     };
     for (int wi = 0; wi < tile.n_work && alive; ++wi) {
-      const Work r = get_work<kSparsePrefill>(P, tile, wi);
+      const Work r = get_work<MODE>(P, tile, wi);
       const int nblk = r.blk_hi - r.blk_lo;
       if (nblk == 0) continue;
       alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_FULL), req & 1, status, 5));
@@ -259,7 +300,20 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
           ++jp;
           did = true;
         } else if (js < nblk && (m & 0xcu) == 0xcu) {
-          tc::fence_proxy_async_smem();   // rows written by cp.async -> tensor pipe
+          if constexpr (MODE == kSparsePrefill) {
+            tc::fence_proxy_async_smem();   // rows written by cp.async -> tensor pipe
+          } else {
+            // rows of the last page beyond the sequence may hold anything (NaN included) and 0 * NaN must not reach O
+            const int rows_valid = r.seqlen - (r.blk_lo + js) * 64;
+            if (rows_valid < 64) {
+              for (int i = lane; i < (64 - rows_valid) * 64; i += 32) {
+                const int row = rows_valid + (i >> 6), c16 = i & 63;
+                *reinterpret_cast<uint4*>(smem + KV_OFF + st * kTileBytes + (c16 >> 3) * kChunkBytes + row * 128 + (c16 & 7) * 16) = make_uint4(0, 0, 0, 0);
+              }
+              tc::fence_proxy_async_smem();
+              __syncwarp();
+            }
+          }
           tc::tc_fence_after();
           if (lane == 0) FMLA_TRACE_AT(gi, 2);
           if (tc::elect_one()) {
@@ -294,7 +348,7 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
     int g = 0, req = 0;
     bool aborted = false;        // uniform over the 128 softmax threads: only read right after a bar_sync
     for (int wi = 0; wi < tile.n_work; ++wi) {
-      const Work r = get_work<kSparsePrefill>(P, tile, wi);
+      const Work r = get_work<MODE>(P, tile, wi);
       const int nblk = r.blk_hi - r.blk_lo;
       float m_run = neg_inf();     // running maximum (base-2 scaled logits)
       float m_used = 0.f;          // the maximum O and l are currently scaled with
@@ -307,7 +361,7 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
           if (tid == 0) FMLA_TRACE_AT(g, 6);
           tc::tc_fence_after();
           tc::tmem_ld32(tmem + lane_addr + TMEM_S + st * 32, sv);
-          vbits = sValid[st * 2 + th];
+          if constexpr (MODE == kSparsePrefill) vbits = sValid[st * 2 + th];
           tc::tmem_wait_ld();
           tc::tc_fence_before();
         } else {
@@ -318,6 +372,10 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
         tc::mbar_arrive(bar(S_EMPTY0 + st));
         if (tid == 0) FMLA_TRACE_AT(g, 7);
 
+        if constexpr (MODE == kDense) {
+          const int tok0 = (r.blk_lo + j) * 64 + th * 32;
+          if (tok0 + 32 > r.border) vbits = tok0 >= r.border ? 0u : (0xffffffffu >> (32 - (r.border - tok0)));
+        }
         // masked logits become -inf (a select: they may hold anything); the maximum is taken over the raw
         // logits in four independent chains and scaled once (the scale is positive)
         if (vbits != 0xffffffffu) {
@@ -378,7 +436,7 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
           const float p0 = exp2f(fmaf(__uint_as_float(sv[2 * i]), scale_log2, -m_used));
           const float p1 = exp2f(fmaf(__uint_as_float(sv[2 * i + 1]), scale_log2, -m_used));
           rs4[i & 3] += p0 + p1;
-          pk[i] = pack_bf16x2(p0, p1);
+          pk[i] = pack_16x2<F16>(p0, p1);
         }
         l_part += (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
         if (!pv_done && !tc::mbar_wait(bar(P_EMPTY), (g & 1) ^ 1, status, 9)) *sAbort = 1;
@@ -410,7 +468,13 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
       }
       // Every store is one full 32-byte sector (each thread writes its own row: 16-byte stores made the load/store unit handle
       // twice as many half-filled ones).
-      __nv_bfloat16* o_row = reinterpret_cast<__nv_bfloat16*>(P.sp.out) + ((int64_t)r.batch * P.sp.h_q + head) * 512;
+      const bool row_ok = MODE == kSparsePrefill || r_row < p.hq_per_hk - tile.hb * 64;
+      const int q_seq_per_hk = MODE == kSparsePrefill ? 0 : p.s_q * p.hq_per_hk;
+      // row of the partial slot of a split request: (kv head, query token, head)
+      const int64_t part_row = MODE == kSparsePrefill ? 0 : ((int64_t)r.split_slot * p.h_k + tile.kh) * q_seq_per_hk + tile.sq * p.hq_per_hk + tile.hb * 64 + r_row;
+      __nv_bfloat16* o_row = MODE == kSparsePrefill
+          ? reinterpret_cast<__nv_bfloat16*>(P.sp.out) + ((int64_t)r.batch * P.sp.h_q + head) * 512
+          : reinterpret_cast<__nv_bfloat16*>(p.out) + r.batch * p.o_stride_b + tile.sq * p.o_stride_s + head * p.o_stride_h;
 #pragma unroll 1
       for (int c = 0; c < 8; ++c) {
         uint32_t cur[32];
@@ -422,13 +486,24 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
           for (int i = 0; i < 32; ++i) cur[i] = 0u;
         }
         const int col = (c >> 2) * 256 + th * 128 + (c & 3) * 32;
+        if (!row_ok) continue;
+        if (MODE == kSparsePrefill || r.no_split) {
 #pragma unroll
-        for (int q8 = 0; q8 < 2; ++q8) {
-          uint32_t w[8];
+          for (int q8 = 0; q8 < 2; ++q8) {
+            uint32_t w[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            w[i] = pack_bf16x2(__uint_as_float(cur[q8 * 16 + 2 * i]) * inv, __uint_as_float(cur[q8 * 16 + 2 * i + 1]) * inv);
-          st_global_32B(o_row + col + q8 * 16, w);
+            for (int i = 0; i < 8; ++i)
+              w[i] = pack_16x2<F16>(__uint_as_float(cur[q8 * 16 + 2 * i]) * inv, __uint_as_float(cur[q8 * 16 + 2 * i + 1]) * inv);
+            st_global_32B(o_row + col + q8 * 16, w);
+          }
+        } else {
+#pragma unroll
+          for (int q8 = 0; q8 < 4; ++q8) {
+            uint32_t w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i] = __float_as_uint(__uint_as_float(cur[q8 * 8 + i]) * inv);
+            st_global_32B(p.o_accum + part_row * 512 + col + q8 * 8, w);
+          }
         }
       }
       if (nblk > 0) {
@@ -436,10 +511,17 @@ mla_prefill64_kernel(const __grid_constant__ TcParams P, const __grid_constant__
         tc::mbar_arrive(bar(O_EMPTY));
         ++req;
       }
-      if (th == 0) {
-        const int64_t o = (int64_t)r.batch * P.sp.h_q + head;
-        P.sp.max_logits[o] = inv == 0.f ? neg_inf() : m_run;
-        P.sp.lse[o] = inv == 0.f ? neg_inf() : log2f(l) + m_used;
+      if (th == 0 && row_ok) {
+        if constexpr (MODE == kSparsePrefill) {
+          const int64_t o = (int64_t)r.batch * P.sp.h_q + head;
+          P.sp.max_logits[o] = inv == 0.f ? neg_inf() : m_run;
+          P.sp.lse[o] = inv == 0.f ? neg_inf() : log2f(l) + m_used;
+        } else if (r.no_split) {
+          p.softmax_lse[((int64_t)r.batch * p.h_q + head) * p.s_q + tile.sq] = inv == 0.f ? pos_inf() : (log2f(l) + m_used) * kLn2;
+        } else {
+          p.lse_accum[part_row] = inv == 0.f ? neg_inf() : log2f(l) + m_used;
+          if (p.no_split_hint && tid == 0) tc::report_status(status, 41);     // a split request although the caller ruled it out
+        }
       }
     }
   }
@@ -461,25 +543,50 @@ cudaError_t launch_sparse_prefill_64(const SparsePrefillKernelParams& sp, cudaSt
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
   const int n_hb = sp.h_q / 64;
   const int lanes = max(1, min(sp.s_q, sms / n_hb));
-  if (cudaError_t e = allow_smem<mla_prefill64_kernel>(dtc::SMEM_BYTES); e != cudaSuccess) return e;
-  mla_prefill64_kernel<<<dim3(n_hb, lanes, 1), dtc::kThreads, dtc::SMEM_BYTES, stream>>>(P, tq);
+  constexpr auto kern = mla_tile64_kernel<kSparsePrefill, false>;
+  if (cudaError_t e = allow_smem<kern>(dtc::SMEM_BYTES); e != cudaSuccess) return e;
+  kern<<<dim3(n_hb, lanes, 1), dtc::threads(kSparsePrefill), dtc::SMEM_BYTES, stream>>>(P, tq, tq);      // no page is read through a map
   return cudaGetLastError();
+}
+
+template <bool F16>
+static cudaError_t launch_dense_tile64(const TcParams& P, const CUtensorMap& tq, const CUtensorMap& tkv, dim3 grid, cudaStream_t stream) {
+  constexpr auto kern = mla_tile64_kernel<kDense, F16>;
+  if (cudaError_t e = allow_smem<kern>(dtc::SMEM_BYTES); e != cudaSuccess) return e;
+  return launch_dependent(kern, grid, dtc::threads(kDense), dtc::SMEM_BYTES, stream, P, tq, tkv);
+}
+
+// Several 64-row tiles read the same pages (and the pair does not apply, mla_dispatch.cu).  Against mla_few_rows.cu, device time:
+// 64 heads x 3 tokens, 16 requests of 16 000 tokens 188 -> 158 us, 64 of 4 000 179 -> 153, 128 of 1 000 115 -> 102, 16 of 1 000
+// 34.6 -> 35.5, one of 1 000 21.6 -> 23.3; 96 and 192 heads, one and two tokens, alike.  The lengths are on the device, so the
+// line is drawn for the larger calls.
+bool decode_dense_tile64_applies(const DecodeKernelParams& p) { return p.hq_per_hk >= 64 && p.s_q * ((p.hq_per_hk + 63) / 64) > 1; }
+
+cudaError_t launch_decode_dense_tile64(const DecodeKernelParams& p, cudaStream_t stream) {
+  TcParams P = {};
+  P.d = p;
+  CUtensorMap tq, tkv;
+  // q [b][s_q][h_q][576], box of 64 heads (heads past h_q read as zero); cache [num_blocks][64][h_k][576] as (col, head, row in page, page)
+  if (!tmah::make_map_4d(&tq, p.q, p.h_q, p.s_q, p.b, p.q_stride_h, p.q_stride_s, p.q_stride_b, 64, 1)) return cudaErrorInvalidValue;
+  if (!tmah::make_map_4d(&tkv, p.kcache, p.h_k, 64, p.num_blocks, p.k_stride_head, p.k_stride_row, p.k_stride_block, 1, 64)) return cudaErrorInvalidValue;
+  const dim3 grid(p.s_q * ((p.hq_per_hk + 63) / 64), p.h_k, p.num_sm_parts);
+  return p.is_f16 ? launch_dense_tile64<true>(P, tq, tkv, grid, stream) : launch_dense_tile64<false>(P, tq, tkv, grid, stream);
 }
 
 #ifdef FMLA_TRACE
 extern "C" int fmla_debug_read_trace(long long* host, int n) {
-  return (int)cudaMemcpyFromSymbol(host, g_prefill64_trace, sizeof(long long) * n);
+  return (int)cudaMemcpyFromSymbol(host, g_tile64_trace, sizeof(long long) * n);
 }
 #endif
 
-cudaError_t set_status_mirror_prefill64(int* mapped_host_word) { return tc::set_status_mirror(mapped_host_word); }
+cudaError_t set_status_mirror_tile64(int* mapped_host_word) { return tc::set_status_mirror(mapped_host_word); }
 
-cudaError_t read_prefill64_status(int* host_status, bool reset) {
-  cudaError_t e = cudaMemcpyFromSymbol(host_status, g_prefill64_status, sizeof(int));
+cudaError_t read_tile64_status(int* host_status, bool reset) {
+  cudaError_t e = cudaMemcpyFromSymbol(host_status, g_tile64_status, sizeof(int));
   if (e != cudaSuccess) return e;
   if (reset && *host_status != 0) {
     const int zero = 0;
-    e = cudaMemcpyToSymbol(g_prefill64_status, &zero, sizeof(int));
+    e = cudaMemcpyToSymbol(g_tile64_status, &zero, sizeof(int));
   }
   return e;
 }
