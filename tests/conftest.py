@@ -10,6 +10,10 @@ if ROOT not in sys.path:
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200)")
+    # The first exp of a process that torch splits over several CPU threads is now and then off by 1e-4 (12 of 250 processes, always
+    # that call, never with one thread); after one small exp on this thread it was not (0 of 250).  The oracle is held to 1e-6.
+    import torch
+    torch.exp(torch.zeros(64))
 
 
 @pytest.fixture(autouse=True)
