@@ -119,14 +119,14 @@ __device__ __forceinline__ void combine_row(int nparts, LseAt lse_at, OAt o_at, 
 // WPR warps per row, each for 4 / WPR of the row's four 128-column groups; with more than four, a CTA takes one row and every four
 // warps a share of its parts.
 constexpr int combine_warps(int wpr) { return wpr > kCombineWarps ? wpr : kCombineWarps; }
-template <int WPR>
+template <int WPR, bool SHARED>
 __global__ void __launch_bounds__(combine_warps(WPR) * 32) decode_combine_kernel(const __grid_constant__ DecodeKernelParams p) {
   extern __shared__ float s_weights[];  // [8][num_sm_parts]
   pdl_wait();                           // launched as a programmatic dependent of the attention kernel: plain loads from here on
   const int batch = blockIdx.x;
   int lo = p.num_splits[batch], hi = p.num_splits[batch + 1];
-  if (p.sub_split) {
-    const int k = sub_splits(p);
+  if constexpr (SHARED) {
+    const int k = sub_splits<false>(p);
     lo *= k;
     hi *= k;
   }
@@ -343,12 +343,12 @@ cudaError_t read_merge_status(int* host_status, bool reset) {
   return e;
 }
 
-template <int WPR>
+template <int WPR, bool SHARED>
 static cudaError_t launch_decode_combine_wpr(const DecodeKernelParams& p, int rows, cudaStream_t stream) {
   constexpr int kWarps = combine_warps(WPR), kRows = kWarps / WPR;
   const size_t smem = sizeof(float) * kWarps * p.num_sm_parts;
-  if (cudaError_t e = allow_dynamic_smem(decode_combine_kernel<WPR>, smem); e != cudaSuccess) return e;
-  return launch_dependent(decode_combine_kernel<WPR>, dim3(p.b, (rows + kRows - 1) / kRows), kWarps * 32, smem, stream, p);
+  if (cudaError_t e = allow_dynamic_smem(decode_combine_kernel<WPR, SHARED>, smem); e != cudaSuccess) return e;
+  return launch_dependent(decode_combine_kernel<WPR, SHARED>, dim3(p.b, (rows + kRows - 1) / kRows), kWarps * 32, smem, stream, p);
 }
 
 cudaError_t launch_decode_combine(const DecodeKernelParams& p, cudaStream_t stream) {
@@ -361,11 +361,16 @@ cudaError_t launch_decode_combine(const DecodeKernelParams& p, cudaStream_t stre
   // (64 warps per SM); beyond that the rows alone fill it and four times the CTAs would only cost their launch.  Device time
   // of decode steps, 24 shapes each with 16 / 32 / 64 heads and 48 with 128: one warp always 2.7 / 4.8 / 4.8 / 0 % more than
   // this rule, four always 0 / 0 / 0.8 / 3 % more.
-  const bool many = p.sub_split && p.num_sm_parts >= 8 * p.b;
-  if (many && (int64_t)p.b * rows * 16 <= (int64_t)sms * 64) return launch_decode_combine_wpr<16>(p, rows, stream);
-  if (many && (int64_t)p.b * rows * 8 <= (int64_t)sms * 64) return launch_decode_combine_wpr<8>(p, rows, stream);
-  if ((int64_t)p.b * rows * 4 <= (int64_t)sms * 64) return launch_decode_combine_wpr<4>(p, rows, stream);
-  return launch_decode_combine_wpr<1>(p, rows, stream);
+  // Where rows of the schedule may be shared a request has more parts still: while eight rows of the schedule and more fall on a request,
+  // 16 warps per row as long as they fill half of the chip at most, or 8.  At most four -> this rule: 16 heads, 4 x 1 024 tokens
+  // 17.5 -> 13.4 us, 16 x 1 000 17.2 -> 15.4; 64 heads, 1 x 8 000 30.0 -> 21.7, 8 x 3 000 26.2 -> 23.3, 12 x 600 19.6 -> 19.2.  16 warps on more than half of
+  // the chip: 8 x 3 000 25.1, 8 x 400 (few parts) 21.7 -> 23.0.  With the line at 32 rows of the schedule 16 x 1 000 stays at 17.2.
+  const int64_t all = (int64_t)p.b * rows, room = (int64_t)sms * 64;
+  if (!p.sub_split) return all * 4 <= room ? launch_decode_combine_wpr<4, false>(p, rows, stream) : launch_decode_combine_wpr<1, false>(p, rows, stream);
+  const bool many = p.num_sm_parts >= 8 * p.b;
+  if (many && all * 32 <= room) return launch_decode_combine_wpr<16, true>(p, rows, stream);
+  if (many && all * 8 <= room) return launch_decode_combine_wpr<8, true>(p, rows, stream);
+  return all * 4 <= room ? launch_decode_combine_wpr<4, true>(p, rows, stream) : launch_decode_combine_wpr<1, true>(p, rows, stream);
 }
 
 template <int WPR>

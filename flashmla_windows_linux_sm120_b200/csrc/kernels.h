@@ -111,8 +111,10 @@ cudaError_t launch_sparse_prefill_tc(const SparsePrefillKernelParams& p, cudaStr
 // launch_decode_dense_tc whenever the heads per kv head are a multiple of 128, or 64 with an even number of query tokens
 bool decode_dense_pair_applies(const DecodeKernelParams& p);
 // true when launch_decode_dense_tc will merge the split partials inside the attention kernel (no merge launch needed)
-bool decode_splits_rows_further(const DecodeKernelParams& p);
 bool decode_dense_merges_in_kernel(const DecodeKernelParams& p);
+// true when the kernel for at most 64 rows may share out the rows of the schedule further: a request that the schedule leaves whole may
+// then have partials too, and the merge kernel has to follow
+bool decode_splits_rows_further(const DecodeKernelParams& p);
 cudaError_t launch_decode_dense_pair(const DecodeKernelParams& p, cudaStream_t stream);
 cudaError_t read_decode_pair_status(int* host_status, bool reset);
 // at most 64 query rows per CTA (mla_few_rows.cu): what the other two do not take

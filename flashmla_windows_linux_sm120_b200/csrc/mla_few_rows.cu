@@ -37,8 +37,16 @@
 
 #include <cuda.h>
 #include <cuda_fp8.h>
+#include <type_traits>
 
 namespace fmla {
+
+// What a CTA works on where the rows of the schedule are shared (share_of_row), laid out as a row is.
+struct alignas(16) RowShare {
+  int4 row;                    // first request and block, last request and block
+  int split;                   // first split of the first request
+  int share;                   // k, and part v of c of the request's blocks: k | v << 8 | c << 16
+};
 
 namespace frt {
 constexpr int kSlot = 64 * 128;                   // 64 tokens x 64 columns of 16 bits
@@ -67,7 +75,8 @@ struct Layout {
   static constexpr int MISC_OFF = M_OFF + N * 4;
   static constexpr int VALID_OFF = MISC_OFF + 32;          // sparse modes: 64 validity bits per page in flight
   static constexpr int ROW_OFF = VALID_OFF + kPageBars * 8;        // int64 [N]: element offset of a row within a request's output
-  static constexpr int SMEM_BYTES = ROW_OFF + N * 8;
+  static constexpr int SHARE_OFF = ROW_OFF + N * 8;
+  static constexpr int SMEM_BYTES = SHARE_OFF + sizeof(RowShare);
   static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB shared memory limit per CTA");
   static_assert(kPBufs * N * 128 >= 4 * N * (N == 64 ? 16 : 32) * 2, "the P buffers stage the output rows of the four softmax warps");
   static_assert(kVSlots % 2 == 0 && kVSlots >= 16 && kVSlots <= 8 * (kPageBars - 1) + 1, "ring sizes");
@@ -135,8 +144,47 @@ __device__ __forceinline__ bool bar_any(int id, bool x) {
   return r != 0;
 }
 
-// grid (row tiles, h_k, parts)
-template <int MODE, int N, bool F16>
+// What this CTA works on with k > 1 CTAs to a row of the schedule.  A CTA works on one request of the row: each request gets CTAs in
+// proportion to its blocks, one at least; where there are more requests than CTAs the first takes them all.
+__device__ __noinline__ void share_of_row(const DecodeKernelParams& p, int k, int lag_last, RowShare* out) {
+  const int* md = p.tile_scheduler_metadata + blockIdx.z / k * 8;
+  RowShare s = {*reinterpret_cast<const int4*>(md), md[4], k | 1 << 16};
+  const int u = blockIdx.z % k, n = s.row.z - s.row.x + 1;
+  if (s.row.x >= p.b || n > k) {
+    if (u > 0) s.row.x = p.b;
+    *out = s;
+    return;
+  }
+  struct Blocks { int lo, hi; };
+  auto blocks = [&](int i) {       // as `request` in the kernel
+    const int batch = s.row.x + i, len = p.topk >= 0 ? p.topk : p.seqlens_k[batch], total = (len + 63) >> 6, seen = len - lag_last;
+    Blocks r = {i == 0 ? s.row.y : 0, min(i == n - 1 ? min(s.row.w, total) : total, seen > 0 ? (seen + 63) >> 6 : 0)};
+    r.hi = max(r.hi, r.lo);
+    return r;
+  };
+  const Blocks r0 = blocks(0), r1 = blocks(n - 1);       // (their lengths are on the way together)
+  auto of = [&](int i) { return i == 0 ? r0 : i == n - 1 ? r1 : blocks(i); };
+  int total = 0, seen = 0, first = 0, w = 0, next = 0;
+  for (int i = 0; i < n; ++i) { const Blocks r = of(i); total += r.hi - r.lo; }
+  Blocks r;
+  for (;; ++w) {
+    r = of(w);
+    seen += r.hi - r.lo;
+    next = w == n - 1 ? k : min(max(total > 0 ? (k * seen + total / 2) / total : 0, first + 1), k - (n - 1 - w));
+    if (u < next) break;
+    first = next;
+  }
+  const int v = u - first, c = next - first, len = r.hi - r.lo;
+  s.row = make_int4(s.row.x + w, r.lo + len * v / c, s.row.x + w, r.lo + len * (v + 1) / c);
+  if (w > 0) s.split = 0;
+  s.share = k | v << 8 | c << 16;
+  *out = s;
+}
+
+// grid (row tiles, h_k, parts).  SHARED: rows of the schedule may be shared, which the schedule tells.  Calls in which none can be take the
+// other form: with one for all they were 0.7 to 2 us slower (64 heads, top-k 2048, 30 requests 42.4 -> 44.2, 140 x 1 000 tokens 63.8 ->
+// 65.4).
+template <int MODE, int N, bool F16, bool SHARED>
 __global__ void __launch_bounds__(frt::threads(MODE), 1)
 mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kv) {
   using namespace frt;
@@ -149,7 +197,7 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
   int64_t* sRow = reinterpret_cast<int64_t*>(smem + L::ROW_OFF);
   volatile uint32_t* sTmem = reinterpret_cast<volatile uint32_t*>(smem + L::MISC_OFF);
   volatile int* sAbort = reinterpret_cast<volatile int*>(smem + L::MISC_OFF + 8);   // set by a softmax thread whose wait expired
-  int* sSub = reinterpret_cast<int*>(smem + L::MISC_OFF + 16);      // sub_k, sub_v and sub_c for the epilogue (registers)
+  RowShare* sShare = reinterpret_cast<RowShare*>(smem + L::SHARE_OFF);
   int* status = &g_decode_few_status;
   const DecodeKernelParams& p = P.d;
   constexpr bool SPARSE = MODE == kSparseDecode;
@@ -196,14 +244,25 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
     hb = blockIdx.x % n_hb;
   }
   const int tile_heads = min(hq - hb * 64, 64), nrows = ntok * tile_heads, head0 = kh * hq + hb * 64;
-  const int sub_k = p.sub_split ? sub_splits(p) : 1;
-  const int* md_row = p.tile_scheduler_metadata + blockIdx.z / sub_k * 8;
-  const int4 md = *reinterpret_cast<const int4*>(md_row);
-  int begin_idx = md.x, begin_block = md.y, end_idx = md.z, end_block = md.w, begin_split = md_row[4];
-  int n_work = begin_idx >= p.b ? 0 : end_idx - begin_idx + 1;
-  int sub_v = 0, sub_c = 1;      // this CTA's share of the blocks of a request: part sub_v of sub_c
   // dense: query token t of the sequence sees keys below seqlen - (s_q - 1 - t)
   const int lag_first = MODE == kDense && p.is_causal ? p.s_q - 1 - sq0 : 0, lag_last = MODE == kDense && p.is_causal ? p.s_q - sq0 - ntok : 0;
+  const int* md_row = p.tile_scheduler_metadata + blockIdx.z * 8;
+  if constexpr (SHARED) {
+    if (tid == 0) {
+      const int4 own = *reinterpret_cast<const int4*>(md_row);      // on the way together with what tells k
+      const int split = md_row[4], k = sub_splits<true>(p);
+      if (k == 1) *sShare = {own, split, 1 | 1 << 16};
+      else share_of_row(p, k, lag_last, sShare);
+    }
+    __syncthreads();
+    // One load for either case, from an address that is the same for all threads: where the row came out of a branch, or out of the
+    // loops of share_of_row, the compiler took the loops of every role for divergent (32 heads, 7 x 22 000 tokens 47.7 -> 49.7 us).
+    md_row = reinterpret_cast<const int*>(sShare);
+  }
+  const int4 md = *reinterpret_cast<const int4*>(md_row);
+  const int begin_split = md_row[4];
+  const int begin_idx = md.x, begin_block = md.y, end_idx = md.z, end_block = md.w;
+  const int n_work = begin_idx >= p.b ? 0 : end_idx - begin_idx + 1;
   struct Req { int batch, seqlen, blk_lo, blk_hi; const int* idx; };
   auto request = [&](int wi) {
     Req r;
@@ -216,35 +275,6 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
     r.idx = SPARSE ? p.indices + r.batch * p.indices_stride_b + sq0 * p.indices_stride_s : nullptr;
     return r;
   };
-  if (sub_k > 1 && n_work > 0) {
-    // a CTA works on one request of the row: each of them gets CTAs in proportion to its blocks, one at least
-    const int u = blockIdx.z % sub_k;
-    if (n_work <= sub_k) {
-      const Req r0 = request(0), r1 = request(n_work - 1);       // (their lengths are on the way together)
-      auto of = [&](int i) { return i == 0 ? r0 : i == n_work - 1 ? r1 : request(i); };
-      int total = 0, seen = 0, first = 0, w = 0, next = 0;
-      for (int i = 0; i < n_work; ++i) { const Req r = of(i); total += r.blk_hi - r.blk_lo; }
-      for (;; ++w) {
-        const Req r = of(w);
-        seen += r.blk_hi - r.blk_lo;
-        next = w == n_work - 1 ? sub_k : min(max(total > 0 ? (sub_k * seen + total / 2) / total : 0, first + 1), sub_k - (n_work - 1 - w));
-        if (u < next) break;
-        first = next;
-      }
-      sub_v = u - first;
-      sub_c = next - first;
-      const Req r = of(w);
-      const int len = r.blk_hi - r.blk_lo;
-      if (w > 0) begin_split = 0;
-      n_work = 1;
-      begin_idx = end_idx = r.batch;
-      begin_block = r.blk_lo + len * sub_v / sub_c;
-      end_block = r.blk_lo + len * (sub_v + 1) / sub_c;
-    } else if (u > 0) {
-      n_work = 0;                                    // more requests than CTAs: the first takes them all
-    }
-  }
-  if (tid == 0) *sSub = sub_k | sub_v << 8 | sub_c << 16;      // read after the barrier of an epilogue
   const bool misaligned = (sbase & 1023u) != 0;      // the swizzled tiles need a 1024-byte aligned base
   if (misaligned && tid == 0) tc::report_status(status, 30);
 
@@ -637,9 +667,10 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
 
       // ---- epilogue of this work item ---------------------------------------------------
       bar_sync(1, 128);
-      const int shares = *sSub & 0xff, share = *sSub >> 8 & 0xff, given = *sSub >> 16;
-      const bool no_split = !p.force_partial && hi - lo == 1 && shares == 1;
-      const int64_t slot = static_cast<int64_t>(lo + (r.batch == begin_idx ? begin_split : 0)) * shares + share;
+      int k = 1, share = 0, given = 1;
+      if constexpr (SHARED) { k = sShare->share & 0xff; share = sShare->share >> 8 & 0xff; given = sShare->share >> 16; }
+      const bool no_split = !p.force_partial && hi - lo == 1 && k == 1;
+      const int64_t slot = static_cast<int64_t>(lo + (r.batch == begin_idx ? begin_split : 0)) * k + share;
       const int64_t part_row = (slot * p.h_k + kh) * (int64_t)p.s_q * hq + sq0 * hq + hb * 64;      // row 0 of the tile in its partial slot
       if (*sAbort) aborted = true;
       if (aborted) break;
@@ -667,8 +698,8 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
             p.softmax_lse[((int64_t)r.batch * p.h_q + my_head) * p.s_q + my_tok] = l == 0.f ? pos_inf() : (log2f(l) + m) * kLn2;
           } else {
             p.lse_accum[part_row + tid] = l == 0.f ? neg_inf() : log2f(l) + m;
-            if (share == 0)                                // slots of this request that no CTA has been given
-              for (int i = given; i < shares; ++i) p.lse_accum[part_row + (int64_t)i * p.h_k * p.s_q * hq + tid] = neg_inf();
+            if (SHARED && share == 0)                      // slots of this request that no CTA has been given
+              for (int i = given; i < k; ++i) p.lse_accum[part_row + (int64_t)i * p.h_k * p.s_q * hq + tid] = neg_inf();
             if (p.no_split_hint && tid == 0) tc::report_status(status, 41);     // a split request although the caller ruled it out
           }
         }
@@ -733,7 +764,7 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
             if ((i * 32 + lane) / kPieces < nrows) *reinterpret_cast<uint4*>(out + at[i]) = v[i];
           __syncwarp();
         }
-      } else if (have_o || shares == 1) {                  // (the merge does not read the rows of a part with -inf)
+      } else {
         // fp32 partial: lane = value column 128 mb + 32 warp + lane, registers = query rows
 #pragma unroll 1
         for (int c = 0; c < 4 * N; c += 16) {
@@ -779,9 +810,12 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
 // ---- host side ----------------------------------------------------------------------------------
 template <int MODE, int N, bool F16 = false>
 static cudaError_t launch_few(const FewParams& P, const CUtensorMap& tq, const CUtensorMap& tkv, dim3 grid, cudaStream_t stream) {
-  constexpr auto kern = mla_few_rows_kernel<MODE, N, F16>;
-  if (cudaError_t e = allow_smem<kern>(frt::Layout<N>::SMEM_BYTES); e != cudaSuccess) return e;
-  return launch_dependent(kern, grid, frt::threads(MODE), frt::Layout<N>::SMEM_BYTES, stream, P, tq, tkv);
+  auto launch = [&](auto shared) {
+    constexpr auto kern = mla_few_rows_kernel<MODE, N, F16, decltype(shared)::value>;
+    if (cudaError_t e = allow_smem<kern>(frt::Layout<N>::SMEM_BYTES); e != cudaSuccess) return e;
+    return launch_dependent(kern, grid, frt::threads(MODE), frt::Layout<N>::SMEM_BYTES, stream, P, tq, tkv);
+  };
+  return P.d.sub_split ? launch(std::true_type{}) : launch(std::false_type{});
 }
 
 cudaError_t launch_decode_few_rows(const DecodeKernelParams& p, cudaStream_t stream) {

@@ -110,19 +110,29 @@ __device__ __forceinline__ Work get_work(const TcParams& P, const Tile& t, int i
 // CTAs per row of the schedule.  With no more requests than rows the schedule takes at least six blocks per row (the slack that lets
 // equal requests fall one per row), so a small batch leaves most rows empty: 7 requests of 2 000 tokens occupy 34 of 148.  Each
 // row is then shared by as many CTAs as there are empty rows for (the rows in use come first), as far as the partials fit the
-// b + num_sm_parts slots; slot i of num_splits becomes the slots k i .. k i + k - 1.  Only where the schedule splits most requests
-// anyway: the merge is then paid for.  Attention and merge kernel find the same k from the schedule alone, with loads that do
-// not wait for one another (a count of the rows, with its barrier, cost 1.5 us in the two kernels).
-constexpr int kMaxSubSplits = 6;        // a row of more than six blocks comes with k <= 3
+// b + num_sm_parts slots; slot i of num_splits becomes the slots k i .. k i + k - 1.  Only where the schedule has more than two parts per
+// request on average: the merge is then paid for.  Attention and merge kernel find the same k from the schedule alone.
+// Unshared -> shared: 16 heads, 4 x 1 024 tokens 16.1 -> 13.5 us, 16 x 1 000 19.8 -> 15.2; 64 heads, 1 x 8 000 25.0 -> 22.0, 24 x 1 500 29.6 ->
+// 24.3; sparse, 64 heads, top-k 2048, 1 request 24.5 -> 17.5, 5 of two tokens, top-k 512, 24.2 -> 16.6.
+// Seven would take a schedule of at most a seventh of the rows, and the rows of that have six blocks.
+constexpr int kMaxSubSplits = 6;
 constexpr int kMaxPartsPerRequest = 64;      // on average: 1 x 8 000 tokens, 64 heads: 21.3 us with 44 parts, 26.3 with 132
+// AT_ONCE: everything is asked for at once; otherwise first what rules most schedules out.  The words are the same for all CTAs, and as
+// soon as many warps ask for them they queue up: one thread of each attention CTA reads them at once, the warps of the merge
+// one after the other (all of them at once: 32 x 500 tokens, 32 heads, 22.2 -> 22.8 us, past the L1 cache 23.9).
+template <bool AT_ONCE>
 __device__ __forceinline__ int sub_splits(const DecodeKernelParams& p) {
-  const int slots = p.num_splits[p.b];
+  const int slots = p.num_splits[p.b], room = min(p.b + p.num_sm_parts, kMaxPartsPerRequest * p.b);
+  int first[kMaxSubSplits + 1];      // the request of the first row that has to be empty for k = i
+  first[2] = p.tile_scheduler_metadata[p.num_sm_parts / 2 * 8];
+  if (!AT_ONCE && (slots <= 2 * p.b || first[2] < p.b)) return 1;
+#pragma unroll
+  for (int i = 3; i <= kMaxSubSplits; ++i) first[i] = p.tile_scheduler_metadata[p.num_sm_parts / i * 8];
   int k = 1;
 #pragma unroll
   for (int i = 2; i <= kMaxSubSplits; ++i)
-    if (p.tile_scheduler_metadata[p.num_sm_parts / i * 8] >= p.b) k = i;
-  if (slots <= 2 * p.b) return 1;
-  return max(1, min(k, min((p.b + p.num_sm_parts) / slots, kMaxPartsPerRequest * p.b / slots)));
+    if (first[i] >= p.b && i * slots <= room) k = i;
+  return slots > 2 * p.b ? k : 1;
 }
 
 }  // namespace fmla
