@@ -18,9 +18,11 @@ namespace fmla {
 
 constexpr int kCombineWarps = 8;
 
-// Weights 2^(lse_i - lse) of the parts of a row -> s_w (whole warp); returns the base-2 LSE of the row.
+// Weights 2^(lse_i - lse) of the parts of a row -> s_w (whole warp); returns the base-2 LSE of the row.  A NaN among the parts gives NaN
+// outputs and, for requests that the schedule splits, +inf.  keep_nan: what one CTA gives for the whole row, NaN; for rows that the
+// schedule, or the caller, knows as whole.
 template <class LseAt>
-__device__ __forceinline__ float combine_weights(int nparts, LseAt lse_at, float* s_w) {
+__device__ __forceinline__ float combine_weights(int nparts, LseAt lse_at, float* s_w, bool keep_nan = false) {
   const int lane = threadIdx.x & 31;
   float mx = neg_inf();
 #pragma unroll 1
@@ -33,7 +35,7 @@ __device__ __forceinline__ float combine_weights(int nparts, LseAt lse_at, float
   for (int i = lane; i < nparts; i += 32) sum += exp2f(lse_at(i) - mx);
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-  const float glse = (sum == 0.f || sum != sum) ? pos_inf() : log2f(sum) + mx;
+  const float glse = (sum == 0.f || (sum != sum && !keep_nan)) ? pos_inf() : log2f(sum) + mx;
 #pragma unroll 1
   for (int i = lane; i < nparts; i += 32) s_w[i] = exp2f(lse_at(i) - glse);
   __syncwarp();
@@ -125,6 +127,7 @@ __global__ void __launch_bounds__(combine_warps(WPR) * 32) decode_combine_kernel
   pdl_wait();                           // launched as a programmatic dependent of the attention kernel: plain loads from here on
   const int batch = blockIdx.x;
   int lo = p.num_splits[batch], hi = p.num_splits[batch + 1];
+  const bool whole = hi - lo == 1;      // in the schedule
   if constexpr (SHARED) {
     const int k = sub_splits<false>(p);
     lo *= k;
@@ -146,7 +149,7 @@ __global__ void __launch_bounds__(combine_warps(WPR) * 32) decode_combine_kernel
   const float* o_base = p.o_accum + ((int64_t)lo * rows + r) * 512;
   const int64_t part_stride = rows;
   float* w = s_weights + warp * p.num_sm_parts;
-  const float glse = combine_weights(nparts, [&](int i) { return lse_base[i * part_stride]; }, w);
+  const float glse = combine_weights(nparts, [&](int i) { return lse_base[i * part_stride]; }, w, SHARED && whole);
   if (sub == 0 && (threadIdx.x & 31) == 0) p.softmax_lse[((int64_t)batch * p.h_q + head) * p.s_q + sq] = glse * kLn2;
   combine_columns<4 / kGroups, false, kShares>(
       nparts, [&](int i) { return o_base + i * part_stride * 512; }, w,
@@ -164,7 +167,7 @@ __global__ void __launch_bounds__(kCombineWarps * 32) sparse_prefill_combine_ker
   const int64_t first = (int64_t)blockIdx.x * p.per * p.h_q + head;
   pdl_wait();                           // launched as a programmatic dependent of the attention kernel: plain loads from here on
   float* w = s_weights + warp * p.per;
-  const float glse = combine_weights(p.per, [&](int i) { return p.lse_accum[first + (int64_t)i * p.h_q]; }, w);
+  const float glse = combine_weights(p.per, [&](int i) { return p.lse_accum[first + (int64_t)i * p.h_q]; }, w, true);
   const int64_t out_row = (int64_t)(p.whole + blockIdx.x) * p.h_q + head;
   if (sub == 0) {
     float mx = neg_inf();
