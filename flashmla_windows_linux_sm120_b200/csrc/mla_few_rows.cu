@@ -302,6 +302,7 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
         const int* bt = p.block_table + (int64_t)r.batch * p.block_table_stride_b;
         int page_next = bt[r.blk_lo];
         const bool ahead = r.blk_hi - r.blk_lo >= kPrefetchBlocks && p.k_stride_row == 576;
+        const char* kv_head = reinterpret_cast<const char*>(p.kcache) + kh * p.k_stride_head * 2;
         for (int blk = r.blk_lo; blk < r.blk_hi && alive; ++blk, ++g) {
           const int page = page_next, full = bar(KV_FULL0 + g % kPageBars);
           if (blk + 1 < r.blk_hi) page_next = bt[blk + 1];
@@ -311,7 +312,9 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
           tc::mbar_arrive_expect_tx(full, kPageBytes);
           tc::tma_load_4d(sbase + L::R_OFF + (g % L::kRopeSlots) * kSlot, &tmap_kv, 512, kh, 0, page, full);
           // the next page, as one piece: the tiles read it 128 bytes of a row at a time, and their slots are only free a page later
-          if (ahead && blk + 1 < r.blk_hi) prefetch_l2(reinterpret_cast<const char*>(p.kcache) + page_next * p.k_stride_block * 2, kPageBytes);
+          // (an entry of the block table that is no page: the loads read zeros there, a bare address would be one past the cache)
+          if (ahead && blk + 1 < r.blk_hi && static_cast<unsigned>(page_next) < static_cast<unsigned>(p.num_blocks))
+            prefetch_l2(kv_head + page_next * p.k_stride_block * 2, kPageBytes);
 #pragma unroll 1
           for (int c = 0; c < 8 && alive; ++c) {
             const int n = g * 8 + c;               // chunk n takes the slot of chunk n - kVSlots, i.e. of page (n - kVSlots) / 8
