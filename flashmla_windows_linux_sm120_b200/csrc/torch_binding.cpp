@@ -316,6 +316,7 @@ fmla_dense_params dense_params(PyObject* const* a) {
   require(cu_q.is_contiguous() && cu_k.is_contiguous(), "cumulative seqlens must be contiguous");
   fmla_dense_params p = {};
   p.batch = static_cast<int32_t>(cu_q.size(0) - 1);
+  require(cu_k.numel() >= cu_q.size(0), "cumulative_seqlen_kv is shorter than cumulative_seqlen_q");      // the kernels read as many of both
   require(k.size(0) == v.size(0) && k.size(1) == v.size(1) && k.size(2) == q.size(2), "k shape mismatch");
   require(o.size(0) == q.size(0) && o.size(1) == q.size(1) && o.size(2) == v.size(2), "o shape mismatch");
   require(lse.size(0) == q.size(0) && lse.size(1) == q.size(1), "lse must be [total_q, h_q]");

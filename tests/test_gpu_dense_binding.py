@@ -61,3 +61,15 @@ def test_backward_refuses():
         bwd(dq=torch.empty((69, 2, 192), dtype=torch.bfloat16, device="cuda"))
     with pytest.raises(RuntimeError, match="must be bfloat16"):
         bwd(d_o=torch.zeros((70, 2, 128), device="cuda"))
+
+
+def test_short_cumulative_lengths():
+    """The kernels read batch + 1 entries of both (more keys' entries than that are never looked at)."""
+    a = _args()
+    want = _fwd(a)
+    with pytest.raises(RuntimeError, match="cumulative_seqlen_kv is shorter"):
+        _fwd(dict(a, cu_k=a["cu_k"][:1]))
+    with pytest.raises(RuntimeError, match="cumulative_seqlen_kv is shorter"):
+        _fwd(dict(a, cu_q=torch.tensor([0, 30, 70], dtype=torch.int32, device="cuda")))
+    longer = torch.tensor([0, 70, 10 ** 6], dtype=torch.int32, device="cuda")
+    assert all(torch.equal(x, y) for x, y in zip(_fwd(dict(a, cu_k=longer)), want))
