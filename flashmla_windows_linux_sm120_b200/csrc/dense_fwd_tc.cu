@@ -34,6 +34,7 @@
 #include "tc_common.cuh"
 #include "tma_host.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace fmla {
@@ -561,18 +562,29 @@ static cudaError_t launch_fwd_tc(DenseKernelParams p, const CUtensorMap& tq, con
   p.tiles_outer = p.is_causal && (int64_t)p.total_k * p.h_k * (p.d_qk + p.d_v) * 2 <= (64 << 20);
   const int64_t ctas = (int64_t)((p.max_seqlen_q + 255) / 256) * p.h_q * p.batch;
   if (ctas > INT32_MAX) return cudaErrorInvalidConfiguration;
-  // Taking CTAs over pays from some two CTAs per SM on; below, its longer code costs what it saves.  Device time in a graph, plain ->
-  // taking over: 128 CTAs (4 sequences of 1000 tokens, 8 heads, 192/128) 24.6 -> 26.3 us, 192 (6 of 500 to 1000, 8 heads, 128/128)
-  // 21.9 -> 23.7, 256 (8 of 500 to 1000, 8 heads) 27.6 -> 28.6, 320 (4 of 1000 to 1200, 16 heads, 192/128) 76.4 -> 75.8, 512 (2 of 1000
-  // to 2000, 32 heads) 72.5 -> 69.0, 768 (3 of 1129 to 1950) 99.8 -> 92.3, 4096 (8 of 300 to 900, 128 heads, 192/128) 304 -> 276.
-  constexpr int kTakeOverCtas = 320;
+  // Taking CTAs over pays from nearly two CTAs with rows per SM on; below, its longer code costs what it saves.  Sequences shorter than the
+  // longest leave CTAs without rows, which count for nothing here: no more than (total_q / 256 + batch) per head have some.  Device
+  // time in a graph, plain -> taking over: 128 CTAs (4 sequences of 1000 tokens, 8 heads, 192/128) 24.6 -> 26.3 us, 192 (6 of 500 to 1000, 8
+  // heads, 128/128) 21.9 -> 23.7, 256 (8 of 500 to 1000, 8 heads) 27.6 -> 28.6; 480 of which 208 have rows (1500, 700, 300, 100 and 20
+  // tokens, 16 heads, 192/128, causal) 32.4 -> 34.8, 448 of which 160 (1000 and 6 of 30, 16 heads) 23.7 -> 25.4; 288 (9 of 250, 32 heads) 24.5 -> 21.8,
+  // 288 (3 of 700) 33.7 -> 31.7, 320 (20 of 256, 16 heads) 35.8 -> 30.7, 768 (3 of 1129 to 1950, 128/128) 103.4 -> 98.2, 16384 of which 560
+  // (16384 and 255 of 128, 4 heads) 863 -> 574.
+  // With long tiles the loop, some 3 % slower at 192/128, outweighs the borders.  192/128, tiles of 8 blocks (16 of 1024, 16 heads, no
+  // mask) 199 -> 191, 16 blocks (4 of 2048, 24 heads) 282 -> 275, 32 (8 of 4096) 1293 -> 1302, 64 (4 of 8192) 2455 -> 2524; with a causal
+  // mask, which halves them, 16 of 2048 437 -> 411, 4 of 8192 1318 -> 1352; at 128/128 1194 -> 1151.
+  int dev = 0, sms = 0;
+  if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
+  if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); e != cudaSuccess) return e;
+  const int64_t with_rows = std::min<int64_t>(ctas, (static_cast<int64_t>(p.total_q / 256) + p.batch) * p.h_q);
+  const int64_t keys = p.total_k / p.batch / (p.is_causal ? 2 : 1);
+  const bool takes_over = with_rows * 8 >= sms * 15 && (D_QK == 128 || keys <= 2048);
   auto launch = [&](auto take_over) {
     constexpr auto kern = dense_fwd_tc_kernel<D_QK, decltype(take_over)::value>;
     if (cudaError_t e = allow_smem<kern>(L::SMEM_BYTES); e != cudaSuccess) return e;
     kern<<<static_cast<unsigned>(ctas), dft::threads(decltype(take_over)::value), L::SMEM_BYTES, stream>>>(p, tq, tk, tv);
     return cudaGetLastError();
   };
-  return ctas >= kTakeOverCtas ? launch(std::true_type{}) : launch(std::false_type{});
+  return takes_over ? launch(std::true_type{}) : launch(std::false_type{});
 }
 
 cudaError_t launch_dense_fwd_tc(const DenseKernelParams& p, cudaStream_t stream) {
