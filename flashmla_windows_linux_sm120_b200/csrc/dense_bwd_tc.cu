@@ -9,8 +9,8 @@
 // with floating-point reduce-adds in a launch-dependent order, every output here is produced by
 // exactly one CTA in a fixed order, so dQ, dK and dV are bitwise reproducible.  Three kernels:
 //   1. delta pre-pass                         (FmhaKernelBwdSumOdO's job)
-//   2. dQ:    one CTA per (128-query tile, head, sequence), walks the keys in blocks of 128
-//   3. dK/dV: one CTA per (128-key tile, head, sequence), walks the queries in blocks of 128
+//   2. dQ:    one CTA per (128-query tile, head, sequence), walks the keys in blocks of 128, or of 64 (dense_bwd_steps64.cuh)
+//   3. dK/dV: one CTA per (128-key tile, head, sequence), walks the queries in blocks of 128, or of 64
 // Requires h_q == h_k (as flash_mla/flash_mla_interface.py:413-415).
 //
 // Both main kernels: warps 0-7 element-wise (two threads per row of the resident tile = TMEM lane, one per half of the
@@ -689,25 +689,49 @@ dense_bwd_dkdv_tc_kernel(const __grid_constant__ DenseKernelParams p, const __gr
   if (warp == kEwWarps + 1) tc::tmem_dealloc(tmem, 512);
 }
 
+}  // namespace fmla
+
+#include "dense_bwd_steps64.cuh"
+
+namespace fmla {
+
 // ---- host side ----------------------------------------------------------------------------------
+// Kernels and shared memory of either step
+template <int D_QK, bool STEPS64>
+struct BwdForm {
+  static constexpr auto kq = dense_bwd_dq_tc_kernel<D_QK>;
+  static constexpr auto kk = dense_bwd_dkdv_tc_kernel<D_QK>;
+  static constexpr int kSmem = dbt::Layout<D_QK>::SMEM_BYTES, kStep = 128;
+};
 template <int D_QK>
+struct BwdForm<D_QK, true> {
+  static constexpr auto kq = dense_bwd_dq_tc64_kernel<D_QK>;
+  static constexpr auto kk = dense_bwd_dkdv_tc64_kernel<D_QK>;
+  static constexpr int kSmem = dbt64::Layout<D_QK>::SMEM_BYTES, kStep = 64;
+};
+
+template <int D_QK, bool STEPS64>
 static cudaError_t launch_bwd_tc(const DenseKernelParams& p, cudaStream_t stream) {
   using namespace dbt;
-  using L = Layout<D_QK>;
-  CUtensorMap tq, tdo, tk, tv;
-  bool ok = tmah::make_map_thd(&tq, p.q, p.d_qk, p.h_q, p.total_q, p.q_stride_h, p.q_stride_t, 128) &&
-            tmah::make_map_thd(&tdo, p.d_o, p.d_v, p.h_q, p.total_q, p.do_stride_h, p.do_stride_t, 128) &&
-            tmah::make_map_thd(&tk, p.k, p.d_qk, p.h_k, p.total_k, p.k_stride_h, p.k_stride_t, 128) &&
-            tmah::make_map_thd(&tv, p.v, p.d_v, p.h_k, p.total_k, p.v_stride_h, p.v_stride_t, 128);
-  if (!ok) return cudaErrorInvalidValue;
-  constexpr auto kq = dense_bwd_dq_tc_kernel<D_QK>;
-  constexpr auto kk = dense_bwd_dkdv_tc_kernel<D_QK>;
-  if (cudaError_t e = allow_smem<kq>(L::SMEM_BYTES); e != cudaSuccess) return e;
-  if (cudaError_t e = allow_smem<kk>(L::SMEM_BYTES); e != cudaSuccess) return e;
+  using Form = BwdForm<D_QK, STEPS64>;
+  // of each tensor a map for resident tiles and one for streamed tiles
+  CUtensorMap q, d_o, k, v, q_step, do_step, k_step, v_step;
+  auto maps = [&](CUtensorMap& tile, CUtensorMap& step, const void* x, int d, int heads, int tokens, int64_t stride_h, int64_t stride_t) {
+    if (!tmah::make_map_thd(&tile, x, d, heads, tokens, stride_h, stride_t, 128)) return false;
+    if (Form::kStep == 128) { step = tile; return true; }
+    return tmah::make_map_thd(&step, x, d, heads, tokens, stride_h, stride_t, Form::kStep);
+  };
+  if (!(maps(q, q_step, p.q, p.d_qk, p.h_q, p.total_q, p.q_stride_h, p.q_stride_t) && maps(d_o, do_step, p.d_o, p.d_v, p.h_q, p.total_q, p.do_stride_h, p.do_stride_t) &&
+        maps(k, k_step, p.k, p.d_qk, p.h_k, p.total_k, p.k_stride_h, p.k_stride_t) && maps(v, v_step, p.v, p.d_v, p.h_k, p.total_k, p.v_stride_h, p.v_stride_t)))
+    return cudaErrorInvalidValue;
+  constexpr auto kq = Form::kq;
+  constexpr auto kk = Form::kk;
+  if (cudaError_t e = allow_smem<kq>(Form::kSmem); e != cudaSuccess) return e;
+  if (cudaError_t e = allow_smem<kk>(Form::kSmem); e != cudaSuccess) return e;
   const int64_t rows = (int64_t)p.total_q * p.h_q;
   const int64_t per_block = 16 * kDeltaRows;
   dense_bwd_delta_tc_kernel<<<static_cast<unsigned>((rows + per_block - 1) / per_block), 256, 0, stream>>>(p);
-  kk<<<dim3((p.max_seqlen_k + 127) / 128, p.h_q, p.batch), kDkvThreads, L::SMEM_BYTES, stream>>>(p, tk, tv, tq, tdo);
+  kk<<<dim3((p.max_seqlen_k + 127) / 128, p.h_q, p.batch), kDkvThreads, Form::kSmem, stream>>>(p, k, v, q_step, do_step);
   if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
   const dim3 grid((p.max_seqlen_q + 127) / 128, p.h_q, p.batch);
   // dQ written over Q or dO (which its own kernel reads tile by tile, before it writes) must wait until dK / dV has read them
@@ -719,15 +743,22 @@ static cudaError_t launch_bwd_tc(const DenseKernelParams& p, cudaStream_t stream
            reinterpret_cast<uintptr_t>(x) < end(p.dq, p.d_qk, p.dq_stride_t, p.dq_stride_h);
   };
   if (overlaps(p.q, p.d_qk, p.q_stride_t, p.q_stride_h) || overlaps(p.d_o, p.d_v, p.do_stride_t, p.do_stride_h)) {
-    kq<<<grid, kDqThreads, L::SMEM_BYTES, stream>>>(p, tq, tdo, tk, tv);
+    kq<<<grid, kDqThreads, Form::kSmem, stream>>>(p, q, d_o, k_step, v_step);
     return cudaGetLastError();
   }
-  return launch_dependent(kq, grid, kDqThreads, L::SMEM_BYTES, stream, p, tq, tdo, tk, tv);
+  return launch_dependent(kq, grid, kDqThreads, Form::kSmem, stream, p, q, d_o, k_step, v_step);
 }
 
 cudaError_t launch_dense_bwd_tc(const DenseKernelParams& p, cudaStream_t stream) {
-  if (p.d_qk == 192) return launch_bwd_tc<192>(p, stream);
-  return launch_bwd_tc<128>(p, stream);
+  // Steps of 64 rows for short sequences: the last step of 128 works for up to 127 rows in vain, and with a causal mask tiles walk half of
+  // a sequence.  By the mean length, which is what the host has; steps of 64 -> steps of 128, at this length and a multiple of a step or
+  // half of one beyond it.  Causal, 16 heads, 192/128: 64 tokens 50.9 -> 62.1 us, 320 50.4 -> 57.8, 704 62.2 -> 69.1, 1088 79.7 -> 84.1, 1344 60.2 ->
+  // 61.5, 1500 71.8 -> 70.6, 2000 112.7 -> 106.6; 64 heads, 128/128: 320 170 -> 185, 704 204 -> 211, 1088 258 -> 255, 1500 222 -> 209.  Without a mask, 64
+  // heads, 128/128: 64 tokens 186 -> 214, 320 209 -> 213, 384 207 -> 193, 512 216 -> 195; 192/128: 320 233 -> 241, 384 233 -> 219, 512 240 -> 220.
+  const int64_t mean = (static_cast<int64_t>(p.total_q) + p.total_k) / (2 * static_cast<int64_t>(p.batch));
+  const bool short_sequences = mean <= (p.is_causal ? 1088 : 352);
+  if (p.d_qk == 192) return short_sequences ? launch_bwd_tc<192, true>(p, stream) : launch_bwd_tc<192, false>(p, stream);
+  return short_sequences ? launch_bwd_tc<128, true>(p, stream) : launch_bwd_tc<128, false>(p, stream);
 }
 
 #ifdef FMLA_TRACE

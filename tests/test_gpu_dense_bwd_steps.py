@@ -1,0 +1,51 @@
+"""Dense backward with steps of 64 and of 128 streamed rows: sequences beside a long one take the longer steps, by themselves the
+shorter ones, and their gradients are the same bit for bit, at every edge of either step and whatever lies beside them."""
+import pytest
+import torch
+
+from test_gpu_unsplit_plans import _kernels
+
+pytestmark = pytest.mark.gpu
+
+
+def _grads(x, lens_q, lens_k, causal, names):
+    from flashmla_windows_linux_sm120_b200 import cuda_sm100
+    d = x["q"].shape[2]
+    cu_q, cu_k = (torch.tensor([0, *n], device="cuda").cumsum(0).to(torch.int32) for n in (lens_q, lens_k))
+    args = (int(causal), d ** -0.5, max(lens_q), max(lens_k))
+    o, lse = torch.empty_like(x["d_o"]), torch.empty(x["q"].shape[:2][::-1], device="cuda").T
+    cuda_sm100.dense_prefill_fwd(None, x["q"], x["k"], x["v"], cu_q, cu_k, o, lse, *args)
+    grads = [torch.empty_like(x[n]) for n in "qkv"]
+    work = torch.empty(4 * lse.numel() + 256, dtype=torch.uint8, device="cuda")
+    call = lambda: cuda_sm100.dense_prefill_bwd(work, x["d_o"], x["q"], x["k"], x["v"], o, lse, cu_q, cu_k, *grads, *args)      # noqa: E731
+    call()
+    with _kernels(names):
+        call()
+    return grads
+
+
+@pytest.mark.parametrize("d", [192, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_same_gradients(d, causal):
+    lens_q = [1, 2, 15, 16, 17, 63, 64, 65, 100, 127, 128, 129, 191, 192, 193, 256, 257, 320, 5]
+    lens_k = [3, 2, 17, 16, 15, 65, 64, 63, 128, 130, 127, 129, 192, 190, 257, 256, 300, 320, 333]
+    h, long = 3, len(lens_q) * 1100
+    g = torch.Generator(device="cuda").manual_seed(d)
+    r = lambda n, w: torch.randn((n, h, w), device="cuda", dtype=torch.bfloat16, generator=g)       # noqa: E731
+    short = dict(q=r(sum(lens_q), d), k=r(sum(lens_k), d), v=r(sum(lens_k), 128), d_o=r(sum(lens_q), 128))
+    beside = {n: torch.cat([t, r(long, t.shape[2])]) for n, t in short.items()}
+    names, names_long = [], []
+    want = _grads(short, lens_q, lens_k, causal, names)
+    got = _grads(beside, lens_q + [long], lens_k + [long], causal, names_long)
+    assert sum("tc64_kernel" in n for n in names) == 2 and not any("tc64_kernel" in n for n in names_long), (names, names_long)
+    for n, a, b in zip("qkv", want, got):
+        assert torch.equal(a, b[:a.shape[0]]), n
+
+
+@pytest.mark.parametrize("causal,mean,steps64", [(True, 1088, True), (True, 1090, False), (False, 352, True), (False, 354, False)])
+def test_rule(causal, mean, steps64):
+    g = torch.Generator(device="cuda").manual_seed(mean)
+    x = {n: torch.randn((2 * mean, 1, w), device="cuda", dtype=torch.bfloat16, generator=g) for n, w in (("q", 128), ("k", 128), ("v", 128), ("d_o", 128))}
+    names = []
+    _grads(x, [mean - 100, mean + 100], [mean + 30, mean - 30], causal, names)
+    assert any("tc64_kernel" in n for n in names) == steps64, names
