@@ -65,6 +65,10 @@ cudaError_t launch_decode_sparse_tc(const DecodeKernelParams& p, cudaStream_t st
 // Whole -> cut: 128 heads, top-k 2048, 1 / 12 / 37 / 100 tokens 44.7 -> 16.8, 45.2 -> 26.8, 46.5 -> 38.3, 91.4 -> 80.7 us; top-k 1024, 24 / 37
 // tokens 27.1 -> 26.4, 27.8 -> 28.5; 64 heads, top-k 2048, 1 / 37 / 333 tokens 63.2 -> 16.4, 63.5 -> 30.7, 183 -> 154; top-k 512, 1 / 37
 // tokens 20.5 -> 14.3, 20.5 -> 20.5.  (All blocks on one line, cut anywhere: 60 tokens, 128 heads, top-k 2048 53.7 -> 61.3.)
+// At its line the rule takes what is worth nothing either way.  64 heads, top-k 512, one round of whole tokens in front, whole -> cut: 37 left
+// over (four parts of two blocks, taken) 37.0 -> 34.5; 38, 44, 50, 62 and 74 (three and two parts, refused) 37.0 -> 36.8, 36.8 -> 37.0, 36.8 ->
+// 36.9, 37.0 -> 36.9, 37.4 -> 37.7; two rounds in front 37: 53.7 -> 53.2, 50: 53.3 -> 54.9.  Top-k 1024, 38 to 74 (taken) 65.8 -> 56.4 to 59.6.  128 heads, top-k
+// 1024, 74 in front, 18 (refused) 50.7 -> 47.1, 25: 50.9 -> 50.8, 31: 51.0 -> 51.2.
 void plan_sparse_prefill(SparsePrefillKernelParams& sp, int sms, bool can_split) {
   const int cap = std::max(1, sms / (sp.h_q / 64)), nblk = sp.topk / 64;      // pairs for 128 heads, CTAs per 64-head tile otherwise
   sp.units = std::min(sp.s_q, cap);

@@ -111,7 +111,9 @@ __device__ __forceinline__ Work get_work(const TcParams& P, const Tile& t, int i
 // equal requests fall one per row), so a small batch leaves most rows empty: 7 requests of 2 000 tokens occupy 34 of 148.  Each
 // row is then shared by as many CTAs as there are empty rows for (the rows in use come first), as far as the partials fit the
 // b + num_sm_parts slots; slot i of num_splits becomes the slots k i .. k i + k - 1.  Only where the schedule has more than two parts per
-// request on average: the merge is then paid for.  Attention and merge kernel find the same k from the schedule alone.
+// request on average: the merge is then paid for (from more than three on 16 x 1 000 tokens, 16 heads, stay at 20.2 us instead of 15.3; from
+// more than one on 64 heads, 30 x top-k 512 would take 21.8 instead of 28.9, but one request of 100 tokens 11.4 instead of 9.7).
+// Attention and merge kernel find the same k from the schedule alone.
 // Unshared -> shared: 16 heads, 4 x 1 024 tokens 16.1 -> 13.5 us, 16 x 1 000 19.8 -> 15.2; 64 heads, 1 x 8 000 25.0 -> 22.0, 24 x 1 500 29.6 ->
 // 24.3; sparse, 64 heads, top-k 2048, 1 request 24.5 -> 17.5, 5 of two tokens, top-k 512, 24.2 -> 16.6.
 // Seven would take a schedule of at most a seventh of the rows, and the rows of that have six blocks.
