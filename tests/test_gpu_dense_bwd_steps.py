@@ -1,5 +1,5 @@
 """Dense backward with steps of 64 and of 128 streamed rows: sequences beside a long one take the longer steps, by themselves the
-shorter ones, and their gradients are the same bit for bit, at every edge of either step and whatever lies beside them."""
+shorter ones, and their gradients are the same bit for bit, at every edge of either step and with NaN and Inf on either side."""
 import pytest
 import torch
 
@@ -29,17 +29,23 @@ def _grads(x, lens_q, lens_k, causal, names):
 def test_same_gradients(d, causal):
     lens_q = [1, 2, 15, 16, 17, 63, 64, 65, 100, 127, 128, 129, 191, 192, 193, 256, 257, 320, 5]
     lens_k = [3, 2, 17, 16, 15, 65, 64, 63, 128, 130, 127, 129, 192, 190, 257, 256, 300, 320, 333]
-    h, long = 3, len(lens_q) * 1100
+    h, between, long = 3, 70, len(lens_q) * 2400
     g = torch.Generator(device="cuda").manual_seed(d)
     r = lambda n, w: torch.randn((n, h, w), device="cuda", dtype=torch.bfloat16, generator=g)       # noqa: E731
     short = dict(q=r(sum(lens_q), d), k=r(sum(lens_k), d), v=r(sum(lens_k), 128), d_o=r(sum(lens_q), 128))
-    beside = {n: torch.cat([t, r(long, t.shape[2])]) for n, t in short.items()}
+    beside = {}
+    for n, value in (("q", float("nan")), ("k", float("nan")), ("v", float("inf")), ("d_o", float("inf"))):
+        parts = short[n].split(lens_q if n in ("q", "d_o") else lens_k)
+        poison = torch.full((between, h, short[n].shape[2]), value, dtype=torch.bfloat16, device="cuda")
+        beside[n] = torch.cat([t for part in parts for t in (part, poison)] + [r(long, poison.shape[2])])
     names, names_long = [], []
     want = _grads(short, lens_q, lens_k, causal, names)
-    got = _grads(beside, lens_q + [long], lens_k + [long], causal, names_long)
+    with_poison = [[x for n in lens for x in (n, between)] + [long] for lens in (lens_q, lens_k)]
+    got = _grads(beside, *with_poison, causal, names_long)
     assert sum("tc64_kernel" in n for n in names) == 2 and not any("tc64_kernel" in n for n in names_long), (names, names_long)
-    for n, a, b in zip("qkv", want, got):
-        assert torch.equal(a, b[:a.shape[0]]), n
+    for n, a, b, lens in zip("qkv", want, got, (lens_q, lens_k, lens_k)):
+        pieces = b.split([x for m in lens for x in (m, between)] + [long])[0:-1:2]
+        assert torch.equal(a, torch.cat(pieces)), n
 
 
 @pytest.mark.parametrize("causal,mean,steps64", [(True, 1088, True), (True, 1090, False), (False, 352, True), (False, 354, False)])

@@ -1,5 +1,5 @@
-"""CTA pairs that walk several requests or query tokens: the first product of the next one is issued before the last of the one in
-front, from either stage, with requests of one block and without any, and parts of requests in between."""
+"""CTA pairs that walk several requests or query tokens: requests and tokens of one block and of several, requests without any, and
+parts of requests in between, so that every border follows work of every length on either stage of the rings."""
 import pytest
 import torch
 
