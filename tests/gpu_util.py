@@ -50,3 +50,31 @@ def assert_out_lse(out, lse, ref_out, ref_lse, out_cos=OUT_COS, what: str = "") 
     assert check_is_allclose("out", out, ref_out, abs_tol=OUT_ABS, rel_tol=OUT_REL, cos_diff_tol=out_cos)
     assert check_is_allclose("lse", lse, ref_lse, abs_tol=LSE_ABS, rel_tol=LSE_REL)
     return assert_target_bounds(out, lse, ref_out, ref_lse, what)
+
+
+def kernel_names(call):
+    """(Mangled) names of the kernels that `call` launches, from the nodes of a graph that it is captured into: nothing here depends on a
+    profiler's window."""
+    from cuda.bindings import driver
+
+    def ok(result):
+        assert result[0] == driver.CUresult.CUDA_SUCCESS, result[0]
+        return result[1] if len(result) == 2 else result[1:]
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call()                                           # what a first call sets up is not part of the graph
+    torch.cuda.current_stream().wait_stream(side)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    names = []
+    for node in ok(driver.cuGraphGetNodes(raw, ok(driver.cuGraphGetNodes(raw, 0))[1]))[0]:
+        if ok(driver.cuGraphNodeGetType(node)) == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            params = ok(driver.cuGraphKernelNodeGetParams(node))
+            name = ok(driver.cuFuncGetName(params.func)) if int(params.func) else ok(driver.cuKernelGetName(params.kern))
+            names.append(name.decode())
+    return names

@@ -3,12 +3,13 @@ shorter ones, and their gradients are the same bit for bit, at every edge of eit
 import pytest
 import torch
 
-from test_gpu_unsplit_plans import _kernels
+from gpu_util import kernel_names
 
 pytestmark = pytest.mark.gpu
 
 
-def _grads(x, lens_q, lens_k, causal, names):
+def _grads(x, lens_q, lens_k, causal):
+    """dq, dk, dv, and whether they come from steps of 64 rows."""
     from flashmla_windows_linux_sm120_b200 import cuda_sm100
     d = x["q"].shape[2]
     cu_q, cu_k = (torch.tensor([0, *n], device="cuda").cumsum(0).to(torch.int32) for n in (lens_q, lens_k))
@@ -18,10 +19,10 @@ def _grads(x, lens_q, lens_k, causal, names):
     grads = [torch.empty_like(x[n]) for n in "qkv"]
     work = torch.empty(4 * lse.numel() + 256, dtype=torch.uint8, device="cuda")
     call = lambda: cuda_sm100.dense_prefill_bwd(work, x["d_o"], x["q"], x["k"], x["v"], o, lse, cu_q, cu_k, *grads, *args)      # noqa: E731
+    main = ["tc64_kernel" in n for n in kernel_names(call) if "dense_bwd_dq" in n or "dense_bwd_dkdv" in n]
+    assert len(main) == 2 and main[0] == main[1]
     call()
-    with _kernels(names):
-        call()
-    return grads
+    return grads, main[0]
 
 
 @pytest.mark.parametrize("d", [192, 128])
@@ -38,11 +39,10 @@ def test_same_gradients(d, causal):
         parts = short[n].split(lens_q if n in ("q", "d_o") else lens_k)
         poison = torch.full((between, h, short[n].shape[2]), value, dtype=torch.bfloat16, device="cuda")
         beside[n] = torch.cat([t for part in parts for t in (part, poison)] + [r(long, poison.shape[2])])
-    names, names_long = [], []
-    want = _grads(short, lens_q, lens_k, causal, names)
+    want, steps64 = _grads(short, lens_q, lens_k, causal)
     with_poison = [[x for n in lens for x in (n, between)] + [long] for lens in (lens_q, lens_k)]
-    got = _grads(beside, *with_poison, causal, names_long)
-    assert sum("tc64_kernel" in n for n in names) == 2 and not any("tc64_kernel" in n for n in names_long), (names, names_long)
+    got, steps64_beside = _grads(beside, *with_poison, causal)
+    assert steps64 and not steps64_beside
     for n, a, b, lens in zip("qkv", want, got, (lens_q, lens_k, lens_k)):
         pieces = b.split([x for m in lens for x in (m, between)] + [long])[0:-1:2]
         assert torch.equal(a, torch.cat(pieces)), n
@@ -52,6 +52,4 @@ def test_same_gradients(d, causal):
 def test_rule(causal, mean, steps64):
     g = torch.Generator(device="cuda").manual_seed(mean)
     x = {n: torch.randn((2 * mean, 1, w), device="cuda", dtype=torch.bfloat16, generator=g) for n, w in (("q", 128), ("k", 128), ("v", 128), ("d_o", 128))}
-    names = []
-    _grads(x, [mean - 100, mean + 100], [mean + 30, mean - 30], causal, names)
-    assert any("tc64_kernel" in n for n in names) == steps64, names
+    assert _grads(x, [mean - 100, mean + 100], [mean + 30, mean - 30], causal)[1] == steps64

@@ -3,15 +3,15 @@ sequence is longer than the others, and not those of long tiles at 192/128."""
 import pytest
 import torch
 
-from test_gpu_unsplit_plans import _kernels
+from gpu_util import kernel_names
 
 pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("lens,h,d,causal,want", [
-    ([1500, 700, 300, 100, 20], 16, 192, True, "false"), ([1000] + [30] * 6, 16, 128, False, "false"), ([256] * 20, 16, 192, True, "true"), ([256] * 9, 32, 128, True, "true"),
-    ([256] * 8, 32, 128, True, "false"), ([16384] + [128] * 255, 1, 192, True, "true"), ([2048] * 8, 8, 192, False, "true"), ([4200] * 4, 8, 192, False, "false"),
-    ([4200] * 4, 8, 192, True, "false"), ([4096] * 4, 8, 192, True, "true"), ([4200] * 4, 8, 128, False, "true")])
+    ([1500, 700, 300, 100, 20], 16, 192, True, False), ([1000] + [30] * 6, 16, 128, False, False), ([256] * 20, 16, 192, True, True), ([256] * 9, 32, 128, True, True),
+    ([256] * 8, 32, 128, True, False), ([16384] + [128] * 255, 1, 192, True, True), ([2048] * 8, 8, 192, False, True), ([4200] * 4, 8, 192, False, False),
+    ([4200] * 4, 8, 192, True, False), ([4096] * 4, 8, 192, True, True), ([4200] * 4, 8, 128, False, True)])
 def test_form(lens, h, d, causal, want):
     import flashmla_windows_linux_sm120_b200 as fm
     if torch.cuda.get_device_properties(0).multi_processor_count != 148:
@@ -19,9 +19,6 @@ def test_form(lens, h, d, causal, want):
     n = sum(lens)
     q, k, v = (torch.zeros((n, h, w), dtype=torch.bfloat16, device="cuda") for w in (d, d, 128))
     cu = torch.tensor([0, *lens], device="cuda").cumsum(0).to(torch.int32)
-    names = []
     with torch.no_grad():
-        fm.flash_attn_varlen_func(q, k, v, cu, cu, max(lens), max(lens), causal=causal)
-        with _kernels(names):
-            fm.flash_attn_varlen_func(q, k, v, cu, cu, max(lens), max(lens), causal=causal)
-    assert [n.split(">")[0].split(", ")[-1] for n in names if "dense_fwd_tc_kernel" in n] == [want]
+        names = kernel_names(lambda: fm.flash_attn_varlen_func(q, k, v, cu, cu, max(lens), max(lens), causal=causal))
+    assert [f"dense_fwd_tc_kernelILi{d}ELb{int(want)}E" in n for n in names if "dense_fwd_tc_kernel" in n] == [True], names

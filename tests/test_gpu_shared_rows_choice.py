@@ -1,9 +1,11 @@
 """Which decode calls of at most 64 rows look for rows of the schedule to share: the others run a kernel without it."""
+import re
+
 import pytest
 import torch
 
+from gpu_util import kernel_names
 from oracle import scheduler
-from test_gpu_unsplit_plans import _kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -15,11 +17,8 @@ def _ctas_per_row(md, ns, parts):
 
 
 def _few_rows_forms(call):
-    call()
-    names = []
-    with _kernels(names):
-        call()
-    return [n.split(">")[0].split(", ")[-1] for n in names if "mla_few_rows_kernel" in n]
+    """Whether the attention kernel of each call is the form that looks for rows to share."""
+    return [m.group(1) == "1" for m in (re.search(r"mla_few_rows_kernelILi\d+ELi\d+ELb[01]ELb([01])E", n) for n in kernel_names(call)) if m]
 
 
 @pytest.mark.parametrize("b,h_q,s_q,topk", [(1, 16, 1, 64), (1, 64, 1, 2048), (5, 64, 2, 512), (8, 16, 1, 512), (16, 16, 1, 512), (16, 64, 1, 128), (20, 96, 1, 1024),
@@ -35,10 +34,10 @@ def test_sparse(b, h_q, s_q, topk):
     plan = md, ns.clone()                                # (a copy: nothing is known of it, so that unsplit plans come here too)
     table = torch.zeros((b, 2), dtype=torch.int32, device="cuda")
     forms = _few_rows_forms(lambda: fm.flash_mla_with_kvcache(q, cache, table, lens, 512, *plan, is_fp8_kvcache=True, indices=idx))
-    assert forms == ["true" if k > 1 else "false"], k
+    assert forms == [k > 1], k
 
 
-@pytest.mark.parametrize("b,h_q,width,want", [(4, 16, 16, "true"), (4, 16, 8, "true"), (4, 16, 7, "false"), (48, 16, 16, "true"), (49, 16, 16, "false"), (148, 16, 16, "false")])
+@pytest.mark.parametrize("b,h_q,width,want", [(4, 16, 16, True), (4, 16, 8, True), (4, 16, 7, False), (48, 16, 16, True), (49, 16, 16, False), (148, 16, 16, False)])
 def test_dense(b, h_q, width, want):
     import flashmla_windows_linux_sm120_b200 as fm
     cache = torch.zeros((2, 64, 1, 576), dtype=torch.bfloat16, device="cuda")
