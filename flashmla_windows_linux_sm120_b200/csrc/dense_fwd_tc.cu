@@ -221,7 +221,7 @@ dense_fwd_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_co
       tc::prefetch_tensormap(&tmap_q);
       tc::prefetch_tensormap(&tmap_k);
       tc::prefetch_tensormap(&tmap_v);
-      for (int i = 0; i < NUM_BARS; ++i)
+      for (int i = 0; i < (kTakeOver ? NUM_BARS : CLAIMED); ++i)
         tc::mbar_init(bar(i), (i == P_FULL0 || i == P_FULL1) ? kSoftmaxWarps / 2 : i == TILE_EMPTY ? kSoftmaxWarps + 2 : 1);
       tc::fence_mbar_init();
       tc::fence_proxy_async_smem();
