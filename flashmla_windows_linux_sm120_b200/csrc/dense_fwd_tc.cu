@@ -2,22 +2,26 @@
 // tcgen05 / TMA / tensor memory.
 //
 // One CTA = 256 query rows (two tiles of 128) of one (sequence, head) at a time; keys are walked in blocks of 128.
-//   warps 0-7  softmax of tile 0, warps 8-15 softmax of tile 1: two threads per query row (TMEM lane = row), one for each
-//              half of the 128 keys: S -> registers, mask, P (bf16) written back into the columns S came from, row
-//              sums, final 1/l normalisation and stores
-//   warp 16    TMA: both Q tiles once; K blocks into a 2-stage ring, V blocks into a single stage (two at 128/128)
-//              (64-column chunks of [128 rows x 128 bytes], 128-byte swizzle)
-//   warp 17    MMA: S_t = Q_t K^T (tcgen05.mma m128n128k16, both operands from shared memory),
+//   warps 0-3  softmax of tile 0, warps 4-7 softmax of tile 1: one thread per query row (TMEM lane = row): largest logit, then in two
+//              halves of 64 keys S -> registers, P (bf16) written back over the columns S came from, row sums; at the end 1/l
+//              normalisation and stores
+//   warp 8     TMA: both Q tiles once; K and V blocks in the order of their use through one ring of 32 KB stages (64-column chunks of
+//              [128 rows x 128 bytes], 128-byte swizzle); columns 128 to 191 of K into two slots of their own
+//   warp 9     MMA, one thread: S_t = Q_t K^T (tcgen05.mma m128n128k16, both operands from shared memory),
 //              O_t += P_t V (m128n128k16, P from tensor memory, V from shared memory MN-major), in the
 //              order  P V of tile 0, S of tile 0 for the next block, P V of tile 1, S of tile 1 for the
-//              next block: while the softmax of one tile runs, the tensor pipe works for the other tile.
-//   warp 18    in large grids: takes over CTAs that have not been started (clusterlaunchcontrol), one after the other
+//              next block: while the softmax of one tile runs, the tensor pipe works for the other tile.  P V starts on the first 64
+//              keys of a block while the softmax of the others runs.
+//   warp 10    in large grids: takes over CTAs that have not been started (clusterlaunchcontrol), one after the other
 // What bounds it: a tile's chain S -> softmax -> P V -> S (P lies over S, and tensor memory has no room for a second S), of
 // which the tensor pipe can hide the part that is as long as the other tile's two GEMMs (1280 clk at 192/128, 1024 at
-// 128/128).  Hence two threads per row: with one, the 128 logits of a row took a thread longer than that.
-// The scale m_used of a row moves only when one of its logits exceeds it by more than 2^8: each of the two threads
-// compares its own maximum, and one barrier-with-reduction of their two warps decides; only then the maxima are
-// exchanged, O is rescaled and the exponentials are formed again.
+// 128/128), and in long runs the power limit.  A block of a CTA (two tiles) took 3 980 clk at 192/128 and 3 760 at 128/128 with two
+// threads per row, single V stages at 192/128 (700 clk waiting for V) and issue and waits by a whole warp; it takes some 3 300 and 2 900
+// now, at a clock that the power limit lowers from 1.66 to 1.52 GHz.  What shortened it: one ring for K and V; the maximum first,
+// so that a warp decides alone whether the scale moves and P can be handed over in halves; part of the exponentials off the special
+// function unit; and little code: the warps of both tiles and the issuing thread share an instruction cache, and the block's body
+// rolled up to 64 logits, with masked blocks rewritten in place first, is 6 % faster than unrolled to 128.
+// The scale m_used of a row moves only when one of its logits exceeds it by more than 2^8; only then O is rescaled.
 // TMEM map (all 512 columns): S/P of tile 0 = [0,128), of tile 1 = [128,256), O of tile 0 = [256,384),
 // of tile 1 = [384,512).  For M = 128 element (row r, col c) of a result sits in lane r, column c;
 // the bf16 A operand in tensor memory holds k values (2c, 2c+1) of row r in the 32-bit column c of lane r.
@@ -42,23 +46,28 @@ namespace fmla {
 namespace dft {
 constexpr int kChunkBytes = 128 * 128;            // [128 rows x 64 bf16], 128-byte rows
 constexpr int kVBytes = 2 * kChunkBytes;          // 128 x 128 bf16
-constexpr int kSoftmaxWarps = 16;
+constexpr int kSoftmaxWarps = 8;
 constexpr int threads(bool take_over) { return (kSoftmaxWarps + 2 + take_over) * 32; }
-enum Bar { Q_FULL = 0, Q_EMPTY, K_FULL0, K_FULL1, K_EMPTY0, K_EMPTY1, V_FULL0, V_FULL1, V_EMPTY0, V_EMPTY1, S_FULL0, S_FULL1, P_FULL0, P_FULL1, PV_DONE0,
-           PV_DONE1, O_DONE0, O_DONE1, CLAIMED, TILE_FULL, TILE_EMPTY, NUM_BARS };
+constexpr int kMaxStages = 5;
+enum Bar { Q_FULL = 0, Q_EMPTY, FULL0, EMPTY0 = FULL0 + kMaxStages, S_FULL0 = EMPTY0 + kMaxStages, S_FULL1, P_HEAD0, P_HEAD1, P_FULL0,
+           P_FULL1, O_DONE0, O_DONE1, CLAIMED, TILE_FULL, TILE_EMPTY, NUM_BARS };
 constexpr int TMEM_S = 0, TMEM_O = 256;
+// One pair of logits in so many is exponentiated on the multiply-add pipe (the special function unit does 16 a clock and SM: 1024 clk
+// for a tile's block, as long as its two products).  4 x 1000 tokens, 8 heads, 128/128, causal: none 23.3, one in eight 20.9, in four
+// 20.4, in three 19.9, in two 21.3 us.
+constexpr int kPolyPeriod = 3;
 constexpr float kRescaleThreshold = 8.0f;         // log2 units; below it O keeps its stale scale
 template <int D_QK>
 struct Layout {
   static constexpr int NCH = D_QK / 64;           // 64-column chunks of Q and K
   static constexpr int kTileBytes = NCH * kChunkBytes;    // one Q tile / one K block
   static constexpr int Q_OFF = 0;                 // 2 tiles
-  static constexpr int K_OFF = 2 * kTileBytes;    // 2 stages
-  static constexpr int V_OFF = K_OFF + 2 * kTileBytes;
-  static constexpr int kVStages = D_QK == 192 ? 1 : 2;
-  static constexpr int BAR_OFF = V_OFF + kVStages * kVBytes;
-  static constexpr int X_OFF = BAR_OFF + 192;     // float [tile][half][128]: exchange between the two threads of a row
-  static constexpr int MISC_OFF = X_OFF + 2048;
+  static constexpr int RING_OFF = 2 * kTileBytes;
+  static constexpr int kStages = D_QK == 192 ? 3 : 5;
+  static constexpr int REST_OFF = RING_OFF + kStages * kVBytes;      // columns 128 to 191 of K: two slots, block c in slot c & 1
+  static constexpr int kRestSlots = D_QK == 192 ? 2 : 0;
+  static constexpr int BAR_OFF = REST_OFF + kRestSlots * kChunkBytes;
+  static constexpr int MISC_OFF = BAR_OFF + 192;
   static constexpr int CLAIM_OFF = MISC_OFF + 16; // answer of a claim
   static constexpr int TILE_OFF = CLAIM_OFF + 16; // int [2][8]: the tile that is worked on and the next one
   static constexpr int SMEM_BYTES = TILE_OFF + 64;
@@ -73,31 +82,78 @@ __device__ int g_dense_tc_status = 0;
 // run time (warp-uniform) and the unrolled code adds immediates; with a copy for each, every copy's first instruction
 // waited for its fetch.
 template <int D_QK>
-__device__ __forceinline__ void dense_s_block(uint32_t tmem_s, uint64_t desc_q, uint64_t desc_k, uint32_t idesc) {
+__device__ __forceinline__ void dense_s_block(uint32_t tmem_s, uint64_t desc_q, uint64_t desc_k, uint64_t desc_rest, uint32_t idesc) {
   using L = dft::Layout<D_QK>;
 #pragma unroll
   for (int c = 0; c < L::NCH; ++c)
 #pragma unroll
     for (int s = 0; s < 4; ++s)
-      tc::mma_ss(tmem_s, tc::desc_advance(desc_q, c * dft::kChunkBytes + s * 32), tc::desc_advance(desc_k, c * dft::kChunkBytes + s * 32), idesc,
+      tc::mma_ss(tmem_s, tc::desc_advance(desc_q, c * dft::kChunkBytes + s * 32), c < 2 ? tc::desc_advance(desc_k, c * dft::kChunkBytes + s * 32) : tc::desc_advance(desc_rest, s * 32), idesc,
                  (c | s) ? 1u : 0u);
 }
-// O += P V of one tile and key block: P from the S columns of the tile (8 columns per 16-token step; the second half of
-// the tokens 64 columns further on: each softmax warp writes over the half it has read).
-__device__ __forceinline__ void dense_pv_block(uint32_t tmem_o, uint32_t tmem_p, uint64_t desc_v, uint32_t idesc, bool first) {
+// O += P V of one tile and key block, the 16-key steps [kFirst, kEnd): P from the first 64 of the S columns (8 a step).
+template <int kFirst, int kEnd>
+__device__ __forceinline__ void dense_pv_steps(uint32_t tmem_o, uint32_t tmem_p, uint64_t desc_v, uint32_t idesc, bool first) {
 #pragma unroll
-  for (int s = 0; s < 8; ++s)
-    tc::mma_ts(tmem_o, tmem_p + (s >> 2) * 64 + (s & 3) * 8, tc::desc_advance(desc_v, s * 2048), idesc, (first && s == 0) ? 0u : 1u);
+  for (int s = kFirst; s < kEnd; ++s)
+    tc::mma_ts(tmem_o, tmem_p + s * 8, tc::desc_advance(desc_v, s * 2048), idesc, (first && s == 0) ? 0u : 1u);
 }
+// Place in the ring of K and V blocks: stage, and the parity of the rounds before.
+template <int N>
+struct RingPos {
+  int st;
+  uint32_t ph;
+  __device__ __forceinline__ void step(int n) {
+    st += n;
+    if (st >= N) {
+      st -= N;
+      ph ^= 1u;
+    }
+  }
+};
 
-// barrier over the 64 threads of two warps that also tells whether any of them passed true
-__device__ __forceinline__ bool pair_any(int id, bool x) {
-  uint32_t r;
-  asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %2, 0;\nbarrier.cta.red.or.aligned.pred q, %1, 64, p;\nselp.u32 %0, 1, 0, q;\n}\n"
-               : "=r"(r)
-               : "r"(id), "r"(static_cast<uint32_t>(x))
-               : "memory");
-  return r != 0;
+// Two floats at a time (one instruction each).
+struct F2 {
+  float lo, hi;
+};
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 d;
+  asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\nfma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}\n"
+      : "=f"(d.lo), "=f"(d.hi)
+      : "f"(a.lo), "f"(a.hi), "f"(b.lo), "f"(b.hi), "f"(c.lo), "f"(c.hi));
+  return d;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 d;
+  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}\n"
+      : "=f"(d.lo), "=f"(d.hi)
+      : "f"(a.lo), "f"(a.hi), "f"(b.lo), "f"(b.hi));
+  return d;
+}
+__device__ __forceinline__ F2 f2(float x) { return F2{x, x}; }
+// 2^x for x <= 2^7 on the multiply-add pipe: x = n + f with n the nearest whole number (held in the low bits of x + 1.5 * 2^23) and
+// |f| <= 1/2, and 2^f = 1 + f q(f) with the polynomial of least largest relative error (fitted with Lawson's weights; 1.6e-7 in
+// fp32 over the range, the special function unit's 2^x is specified to 2.4e-7).  Below -127 the result is 0.
+__device__ __forceinline__ F2 f2_exp2(F2 x) {
+  x.lo = fmaxf(x.lo, -127.f);
+  x.hi = fmaxf(x.hi, -127.f);
+  const F2 t = f2_add(x, f2(12582912.f));
+  const F2 n = f2_add(t, f2(-12582912.f));
+  const F2 f = f2_fma(n, f2(-1.f), x);
+  F2 r = f2_fma(f, f2(0x1.5bba14p-10f), f2(0x1.3cea88p-7f));
+  r = f2_fma(r, f, f2(0x1.c6b752p-5f));
+  r = f2_fma(r, f, f2(0x1.ebf9bcp-3f));
+  r = f2_fma(r, f, f2(0x1.62e42ap-1f));
+  r = f2_fma(r, f, f2(1.f));
+  r.lo = __uint_as_float(__float_as_uint(r.lo) + (__float_as_uint(t.lo) << 23));
+  r.hi = __uint_as_float(__float_as_uint(r.hi) + (__float_as_uint(t.hi) << 23));
+  return r;
+}
+// the largest of three; NaN if one of them is
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
 }
 
 // What a CTA works on: 256 query rows of one head of one sequence.
@@ -155,7 +211,7 @@ __device__ __forceinline__ int claimed_cta(uint32_t answer) {
 }
 
 // grid: ceil(max_seqlen_q/256) * h_q * batch CTAs in the order `p.tiles_outer` selects.  kTakeOver: a CTA that is running takes over
-// CTAs that have not been started (warp 18), so that the loads and first products of its next tile overlap the last softmax,
+// CTAs that have not been started (warp 10), so that the loads and first products of its next tile overlap the last softmax,
 // the read of O and the stores of the present one; barriers, tensor memory and tensor maps are set up once.
 template <int D_QK, bool kTakeOver>
 __global__ void __launch_bounds__(dft::threads(kTakeOver), 1)
@@ -165,7 +221,7 @@ dense_fwd_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_co
   using L = Layout<D_QK>;
   extern __shared__ __align__(1024) unsigned char smem[];
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t sQ = sbase + L::Q_OFF, sK = sbase + L::K_OFF, sV = sbase + L::V_OFF;
+  const uint32_t sQ = sbase + L::Q_OFF, sRing = sbase + L::RING_OFF, sRest = sbase + L::REST_OFF;
   auto bar = [&](int i) { return sbase + L::BAR_OFF + i * 8; };
   volatile uint32_t* sTmem = reinterpret_cast<volatile uint32_t*>(smem + L::MISC_OFF);
   volatile int* sTile = reinterpret_cast<volatile int*>(smem + L::TILE_OFF);
@@ -187,15 +243,16 @@ dense_fwd_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_co
       for (int c = 0; c < L::NCH; ++c)
         tc::tma_load_3d(sQ + t * L::kTileBytes + c * kChunkBytes, &tmap_q, c * 64, w.head, w.q0 + w.m_base + t * 128, bar(Q_FULL));
   };
-  auto load_k = [&](int j, int st) {
-    tc::mbar_arrive_expect_tx(bar(K_FULL0 + st), L::kTileBytes);
+  auto load_k = [&](int j, int st, int c_blk) {
+    tc::mbar_arrive_expect_tx(bar(FULL0 + st), L::kTileBytes);
 #pragma unroll
-    for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(sK + st * L::kTileBytes + c * kChunkBytes, &tmap_k, c * 64, w.head / group, w.k0 + j * 128, bar(K_FULL0 + st));
+    for (int c = 0; c < L::NCH; ++c)
+      tc::tma_load_3d(c < 2 ? sRing + st * kVBytes + c * kChunkBytes : sRest + (c_blk & 1) * kChunkBytes, &tmap_k, c * 64, w.head / group, w.k0 + j * 128, bar(FULL0 + st));
   };
   auto load_v = [&](int j, int st) {
-    tc::mbar_arrive_expect_tx(bar(V_FULL0 + st), kVBytes);
+    tc::mbar_arrive_expect_tx(bar(FULL0 + st), kVBytes);
 #pragma unroll
-    for (int c = 0; c < 2; ++c) tc::tma_load_3d(sV + st * kVBytes + c * kChunkBytes, &tmap_v, c * 64, w.head / group, w.k0 + j * 128, bar(V_FULL0 + st));
+    for (int c = 0; c < 2; ++c) tc::tma_load_3d(sRing + st * kVBytes + c * kChunkBytes, &tmap_v, c * 64, w.head / group, w.k0 + j * 128, bar(FULL0 + st));
   };
   // The n-th tile of this CTA is described in sTile[n & 1]; tiles from the second on are taken over from other CTAs.
   auto put_tile = [&](int n, const DenseTile& t) {
@@ -222,15 +279,15 @@ dense_fwd_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_co
       tc::prefetch_tensormap(&tmap_k);
       tc::prefetch_tensormap(&tmap_v);
       for (int i = 0; i < (kTakeOver ? NUM_BARS : CLAIMED); ++i)
-        tc::mbar_init(bar(i), (i == P_FULL0 || i == P_FULL1) ? kSoftmaxWarps / 2 : i == TILE_EMPTY ? kSoftmaxWarps + 2 : 1);
+        tc::mbar_init(bar(i), (i >= P_HEAD0 && i <= P_FULL1) ? kSoftmaxWarps / 2 : i == TILE_EMPTY ? kSoftmaxWarps + 2 : 1);
       tc::fence_mbar_init();
       tc::fence_proxy_async_smem();
       if (kTakeOver) put_tile(0, w);
       const int n1 = dense_blocks(p, w, 1);
       if (max(dense_blocks(p, w, 0), n1) > 0) {
         load_q(n1 > 0);
-        load_k(0, 0);
-        load_v(0, 0);
+        load_k(0, 0, 0);
+        load_v(0, 1);
       }
     }
     __syncwarp();
@@ -244,30 +301,32 @@ dense_fwd_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_co
   if (warp == kSoftmaxWarps) {
     // ================================ TMA producer =====================================
     if (tc::elect_one()) {
-      int qc = 0, kc = 0;                  // Q tiles, key blocks of the tiles before
+      int qc = 0, kc = 0;                  // Q tiles, key blocks so far
+      RingPos<L::kStages> at = {0, 0u};
       bool alive = true;
       for (int n = 0; alive; ++n) {
         const int n1 = dense_blocks(p, w, 1), nblk = max(dense_blocks(p, w, 0), n1);
-        for (int j = 0; j < nblk && alive; ++j) {
+        for (int j = 0; j < nblk && alive; ++j, ++kc) {
           if (n == 0 && j == 0) {                               // under way since the start
             if (kTakeOver && nblk == 1) tc::mbar_arrive(bar(TILE_EMPTY));
+            at.step(2);
             continue;
           }
-          const int c = kc + j;
-          alive = tc::mbar_wait(bar(K_EMPTY0 + (c & 1)), ((c >> 1) & 1) ^ 1, status, 41);
+          alive = tc::mbar_wait(bar(EMPTY0 + at.st), at.ph ^ 1, status, 41);
           if (!alive) break;
-          load_k(j, c & 1);
+          load_k(j, at.st, kc);
+          at.step(1);
           if (kTakeOver && j == nblk - 1) tc::mbar_arrive(bar(TILE_EMPTY));      // two blocks to go: the next tile may be claimed
           if (j == 0) {                                         // every S of the tile before has been formed
             alive = tc::mbar_wait(bar(Q_EMPTY), (qc & 1) ^ 1, status, 40);
             if (!alive) break;
             load_q(n1 > 0);
           }
-          alive = tc::mbar_wait(bar(V_EMPTY0 + c % L::kVStages), ((c / L::kVStages) & 1) ^ 1, status, 42);
-          if (alive) load_v(j, c % L::kVStages);
+          alive = tc::mbar_wait(bar(EMPTY0 + at.st), at.ph ^ 1, status, 42);
+          if (alive) load_v(j, at.st);
+          at.step(1);
         }
         if (!kTakeOver) break;
-        kc += nblk;
         if (nblk > 0) ++qc;
         else tc::mbar_arrive(bar(TILE_EMPTY));
         if (!alive || !tc::mbar_wait(bar(TILE_FULL), n & 1, status, 50)) break;
@@ -277,79 +336,71 @@ dense_fwd_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_co
     }
   } else if (warp == kSoftmaxWarps + 1) {
     // ================================ MMA issuer =======================================
-    constexpr uint32_t idesc_s = tc::idesc_bf16_f32(128, 128, 0, 0);
-    constexpr uint32_t idesc_o = tc::idesc_bf16_f32(128, 128, 0, 1);
-    const uint64_t desc_q = tc::smem_desc_sw128(sQ, 16, 1024);               // A of S: K-major (tile 0)
-    const uint64_t desc_k = tc::smem_desc_sw128(sK, 16, 1024);               // B of S: K-major (stage 0)
-    const uint64_t desc_v = tc::smem_desc_sw128(sV, kChunkBytes, 1024);      // B of PV: MN-major, 64-wide column groups 16 KB apart (stage 0)
-    int qc = 0, kc = 0, c0 = 0, c1 = 0;      // Q tiles, key blocks, blocks of either tile before this one
-    bool alive = true;
-    if (kTakeOver && lane == 0) tc::mbar_arrive(bar(TILE_EMPTY));
-    for (int n = 0; alive; ++n) {
-      const int n0 = dense_blocks(p, w, 0), n1 = dense_blocks(p, w, 1), nblk = max(n0, n1);
-      if (nblk > 0) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_FULL), qc & 1, status, 43));
-      for (int j = -1; j < nblk && alive; ++j) {
-        const int stv = (kc + j) % L::kVStages, stk = (kc + j + 1) & 1;
-        if (j >= 0) {
-          alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(V_FULL0 + stv), ((kc + j) / L::kVStages) & 1, status, 44));
-          if (!alive) break;
-          // V rows past the end of the sequence belong to the next sequence (or are the zero fill) and are
-          // cleared first, so that 0 * (Inf or NaN) cannot reach O
-          const int rows_valid = w.lk - j * 128;
-          if (rows_valid < 128) {
-            unsigned char* v = smem + L::V_OFF + stv * kVBytes;
-            const int nrows = 128 - rows_valid;
-            for (int i = lane; i < nrows * 16; i += 32) {
-              const int row = rows_valid + (i >> 4), c16 = i & 15;
-              *reinterpret_cast<uint4*>(v + (c16 >> 3) * kChunkBytes + row * 128 + (c16 & 7) * 16) = make_uint4(0, 0, 0, 0);
-            }
-            tc::fence_proxy_async_smem();
-            __syncwarp();
-          }
-        }
-        // S overwrites the columns P of its tile was just read from: the tensor pipe runs in order.  (The first P V of the next
-        // CTA tile overwrites O: its P arrives after the epilogue, which the same warps run before, has read O.)
-        // The issuing thread is held until the pipe has taken its instructions, and a wait after that costs some 100 clk even for a
-        // barrier that is complete; still, an issuing warp per tile (the instructions of both tiles interleave, and both
-        // chains get longer: 600 keys, 8 heads 18.4 -> 22.5 us) and key blocks of 64 with two S buffers (twice the waits: three
-        // sequences of 1129 to 1950 tokens, 32 heads 102 -> 127 us) were slower, P V and S in one go no faster.
+    if (tc::elect_one()) {
+      constexpr uint32_t idesc_s = tc::idesc_bf16_f32(128, 128, 0, 0);
+      constexpr uint32_t idesc_o = tc::idesc_bf16_f32(128, 128, 0, 1);
+      const uint64_t desc_q = tc::smem_desc_sw128(sQ, 16, 1024);               // A of S: K-major (tile 0)
+      const uint64_t desc_k = tc::smem_desc_sw128(sRing, 16, 1024);            // B of S: K-major (stage 0)
+      const uint64_t desc_r = tc::smem_desc_sw128(sRest, 16, 1024);            // the same, columns 128 to 191 (slot 0)
+      const uint64_t desc_v = tc::smem_desc_sw128(sRing, kChunkBytes, 1024);   // B of PV: MN-major, 64-wide column groups 16 KB apart (stage 0)
+      RingPos<L::kStages> at_k = {0, 0u}, at_v = {1, 0u};
+      int qc = 0, kc = 0, c0 = 0, c1 = 0;      // Q tiles, key blocks, blocks of either tile before this one
+      bool alive = true;
+      if (kTakeOver) tc::mbar_arrive(bar(TILE_EMPTY));
+      for (int n = 0; alive; ++n) {
+        const int n0 = dense_blocks(p, w, 0), n1 = dense_blocks(p, w, 1), nblk = max(n0, n1);
+        if (nblk > 0) alive = tc::mbar_wait(bar(Q_FULL), qc & 1, status, 43);
+        for (int j = -1; j < nblk && alive; ++j) {
+          if (j >= 0) alive = tc::mbar_wait(bar(FULL0 + at_v.st), at_v.ph, status, 44);
+          // S overwrites the columns P of its tile was just read from: the tensor pipe runs in order.  (The first P V of the next
+          // CTA tile overwrites O: its P arrives after the epilogue, which the same warps run before, has read O.)
 #pragma unroll 1
-        for (int t = 0; t < 2 && alive; ++t) {
-          const int n_t = t ? n1 : n0;
-          const bool pv = j >= 0 && j < n_t, s = j + 1 < n_t;
-          const bool last_tile = t == 1 || n1 == 0;                     // the last one to read K, V and Q (n1 >= n0 or n1 == 0)
-          if (pv) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(P_FULL0 + t), ((t ? c1 : c0) + j) & 1, status, 45));
-          if (!alive) break;
-          tc::tc_fence_after();
-          if (pv && tc::elect_one()) {
-            dense_pv_block(tmem + TMEM_O + t * 128, tmem + TMEM_S + t * 128, tc::desc_advance(desc_v, stv * kVBytes), idesc_o, j == 0);
-            tc::tc_commit(bar(PV_DONE0 + t));
-            if (!s) tc::tc_commit(bar(O_DONE0 + t));
-            if (last_tile) tc::tc_commit(bar(V_EMPTY0 + stv));
-          }
-          __syncwarp();
-          if (t == 0 && j + 1 < nblk) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(K_FULL0 + stk), ((kc + j + 1) >> 1) & 1, status, 46));
-          if (!alive) break;
-          tc::tc_fence_after();
-          if (s && tc::elect_one()) {
-            dense_s_block<D_QK>(tmem + TMEM_S + t * 128, tc::desc_advance(desc_q, t * L::kTileBytes), tc::desc_advance(desc_k, stk * L::kTileBytes), idesc_s);
-            tc::tc_commit(bar(S_FULL0 + t));
-            if (last_tile) {
-              tc::tc_commit(bar(K_EMPTY0 + stk));
-              if (j + 1 == nblk - 1) tc::tc_commit(bar(Q_EMPTY));
+          for (int t = 0; t < 2 && alive; ++t) {
+            const int n_t = t ? n1 : n0;
+            const bool pv = j >= 0 && j < n_t, s = j + 1 < n_t;
+            const bool last_tile = t == 1 || n1 == 0;                   // the last one to read K, V and Q (n1 >= n0 or n1 == 0)
+            if (pv) {
+              const uint32_t parity = ((t ? c1 : c0) + j) & 1, tmem_o = tmem + TMEM_O + t * 128, tmem_p = tmem + TMEM_S + t * 128;
+              const uint64_t v = tc::desc_advance(desc_v, at_v.st * kVBytes);
+              alive = tc::mbar_wait(bar(P_HEAD0 + t), parity, status, 45);
+              if (!alive) break;
+              tc::tc_fence_after();
+              dense_pv_steps<0, 4>(tmem_o, tmem_p, v, idesc_o, j == 0);
+              alive = tc::mbar_wait(bar(P_FULL0 + t), parity, status, 48);
+              if (!alive) break;
+              tc::tc_fence_after();
+              dense_pv_steps<4, 8>(tmem_o, tmem_p, v, idesc_o, false);
+              if (!s) tc::tc_commit(bar(O_DONE0 + t));
+              if (last_tile) tc::tc_commit(bar(EMPTY0 + at_v.st));
+            }
+            if (t == 0 && j + 1 < nblk) {
+              alive = tc::mbar_wait(bar(FULL0 + at_k.st), at_k.ph, status, 46);
+              if (!alive) break;
+              tc::tc_fence_after();
+            }
+            if (s) {
+              dense_s_block<D_QK>(tmem + TMEM_S + t * 128, tc::desc_advance(desc_q, t * L::kTileBytes), tc::desc_advance(desc_k, at_k.st * kVBytes),
+                                  tc::desc_advance(desc_r, ((kc + j + 1) & 1) * kChunkBytes), idesc_s);
+              tc::tc_commit(bar(S_FULL0 + t));
+              if (last_tile) {
+                tc::tc_commit(bar(EMPTY0 + at_k.st));
+                if (j + 1 == nblk - 1) tc::tc_commit(bar(Q_EMPTY));
+              }
             }
           }
-          __syncwarp();
+          if (j >= 0) at_v.step(2);
+          if (j + 1 < nblk) at_k.step(2);
         }
+        if (!kTakeOver || !alive) break;
+        if (nblk > 0) ++qc;
+        kc += nblk;
+        c0 += n0;
+        c1 += n1;
+        alive = tc::mbar_wait(bar(TILE_FULL), n & 1, status, 50);
+        tc::mbar_arrive(bar(TILE_EMPTY));
+        w = get_tile(n + 1);
+        if (!w.valid) break;
       }
-      if (!kTakeOver || !alive) break;
-      if (nblk > 0) ++qc;
-      kc += nblk;
-      c0 += n0;
-      c1 += n1;
-      alive = await_tile(n + 1);
-      w = get_tile(n + 1);
-      if (!w.valid) break;
     }
   } else if (kTakeOver && warp == kSoftmaxWarps + 2) {
     // ================================ next tiles =======================================
@@ -388,116 +439,136 @@ dense_fwd_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_co
     }
   } else {
     // ================================ softmax / epilogue ================================
-    const int t = warp >> 3, half = (warp >> 2) & 1;           // the tile this warp works for, its half of the columns
+    const int t = warp >> 2;                                   // the tile this warp works for
     const int rl = (warp & 3) * 32 + lane;                     // row within the tile = TMEM lane
-    const int pair_bar = 1 + t * 4 + (warp & 3);               // this warp and the one with the other half of its rows
-    float* x_mine = reinterpret_cast<float*>(smem + L::X_OFF) + t * 256 + half * 128 + rl;
-    float* x_other = reinterpret_cast<float*>(smem + L::X_OFF) + t * 256 + (half ^ 1) * 128 + rl;
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t s_addr = tmem + lane_addr + TMEM_S + t * 128 + half * 64;
-    const uint32_t o_addr = tmem + lane_addr + TMEM_O + t * 128 + half * 64;
-    // A wait that expires clears `alive`; the warp then walks the rest of its blocks without work, because the other warp
-    // of the pair counts on it at their barriers, and both leave after the tile.
+    const uint32_t s_addr = tmem + lane_addr + TMEM_S + t * 128;
+    const uint32_t o_addr = tmem + lane_addr + TMEM_O + t * 128;
     bool alive = true;
-    int c_blk = 0, c_o = 0;                                    // blocks and accumulators of this tile position so far
+    int c_blk = 0, c_o = 0, c_key = 0;                         // blocks and accumulators of this tile position, key blocks so far
     if (kTakeOver && lane == 0) tc::mbar_arrive(bar(TILE_EMPTY));
-    for (int n = 0;; ++n) {
-      int n_mine, limit;
+    for (int n = 0; alive; ++n) {
+      int n_mine, n_key, limit, tail;                          // tail: keys of the sequence's last block, if it is among these
+      bool first_pv;                                           // in the last key block this tile's P V comes first
       {
         const DenseTile tile = kTakeOver ? get_tile(n) : w;
         n_mine = dense_blocks(p, tile, t);
+        const int n_other = dense_blocks(p, tile, t ^ 1);
+        n_key = max(n_mine, n_other);
+        first_pv = n_mine == n_key && (t == 0 || n_other < n_mine);
+        tail = tile.lk - (n_key - 1) * 128;
         // number of keys this row may see: bottom-right aligned causal mask, clipped to the sequence
         limit = p.is_causal ? max(0, min(tile.lk, tile.m_base + t * 128 + rl + (tile.lk - tile.lq) + 1)) : tile.lk;
       }
       float m_used = neg_inf();    // the scale O and l carry (-inf: no visible key yet)
-      float l_run = 0.f;           // this thread's share of the row sum
+      F2 l_run = f2(0.f);          // row sum, of even and odd keys
       for (int j = 0; j < n_mine; ++j, ++c_blk) {
-        if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(S_FULL0 + t), c_blk & 1, status, 47));
+        alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(S_FULL0 + t), c_blk & 1, status, 47));
+        if (!alive) break;
         tc::tc_fence_after();
-        const int cnt = limit - j * 128 - half * 64;           // visible keys of this half block: [0, cnt)
-        const bool full = __all_sync(0xffffffffu, cnt >= 64);
-        // 32 logits at a time: 64 beside their P do not fit into the 96 registers that 18 or 19 warps leave a thread
-        auto load_logits = [&](int c, uint32_t (&sv)[32]) {
-          tc::tmem_ld32(s_addr + c * 32, sv);
-          tc::tmem_wait_ld();
-          if (!full) {
+        const int cnt = limit - j * 128;                       // visible keys of this block: [0, cnt)
+        if (__builtin_expect(!__all_sync(0xffffffffu, cnt >= 128), 0)) {
+          // masked logits become -inf in tensor memory: the code below, short as it is, serves every block
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t sv[32];
+            tc::tmem_ld32(s_addr + c * 32, sv);
+            tc::tmem_wait_ld();
 #pragma unroll
             for (int i = 0; i < 32; ++i)
               if (c * 32 + i >= cnt) sv[i] = 0xff800000u;      // a select: what lies beyond may hold anything
+            tc::tmem_st32(s_addr + c * 32, sv);
           }
-        };
-        // P = 2^(s * scale - m) of this thread's 64 logits as bf16 pairs, their sum and their largest logit
-        uint32_t pk[2][16];
-        float row_sum = 0.f, mx = neg_inf();
-        auto exponentials = [&](float m) {
-          const float m_ref = m == neg_inf() ? 0.f : m;
-          float rs4[4] = {0.f, 0.f, 0.f, 0.f}, mx4[4] = {neg_inf(), neg_inf(), neg_inf(), neg_inf()};      // independent chains
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            uint32_t sv[32];
-            load_logits(c, sv);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float s0 = __uint_as_float(sv[2 * i]), s1 = __uint_as_float(sv[2 * i + 1]);
-              mx4[i & 3] = fmaxf(mx4[i & 3], fmaxf(s0, s1));
-              const float p0 = exp2f(fmaf(s0, p.scale_log2, -m_ref)), p1 = exp2f(fmaf(s1, p.scale_log2, -m_ref));
-              rs4[i & 3] += p0 + p1;
-              pk[c][i] = pack_bf16x2(p0, p1);
+          tc::tmem_wait_st();
+          // V rows past the end of the sequence belong to the next sequence (or are the zero fill): the tile whose P V comes
+          // first clears them, so that 0 * (Inf or NaN) cannot reach O
+          if (tail < 128 && first_pv && j == n_key - 1) {
+            const int item = 2 * (c_key + j) + 1, st = item % L::kStages;
+            alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(FULL0 + st), (item / L::kStages) & 1, status, 51));
+            unsigned char* v = smem + L::RING_OFF + st * kVBytes;
+            for (int i = rl; i < (128 - tail) * 16; i += 128) {
+              const int row = tail + (i >> 4), c16 = i & 15;
+              *reinterpret_cast<uint4*>(v + (c16 >> 3) * kChunkBytes + row * 128 + (c16 & 7) * 16) = make_uint4(0, 0, 0, 0);
             }
+            tc::fence_proxy_async_smem();
           }
-          row_sum = (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
-          mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
-        };
-        // The exponentials are formed with the scale of the blocks before, beside the maximum that says whether it still
-        // serves; in the rare block where it does not they are formed again (S stays until P is stored).  The first block has
-        // no scale yet: its maximum alone (200 tokens with 8 heads took 12.1 us with exponentials formed in vain, 11.3 without).
-        if (alive && j > 0) exponentials(m_used);
-        if (alive && j == 0) {
-          float mx4[4] = {neg_inf(), neg_inf(), neg_inf(), neg_inf()};
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            uint32_t sv[32];
-            load_logits(c, sv);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sv[i]));
-          }
-          mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
         }
-        if (j == 0 || pair_any(pair_bar, alive && mx > m_used + kRescaleThreshold)) {
-          *x_mine = mx;
-          bar_sync(pair_bar, 64);
-          const float m_blk = fmaxf(mx, *x_other);
-          const bool up = m_blk > m_used + kRescaleThreshold;
-          // the first visible key sets the scale: O and l are exactly zero so far
-          const float alpha = (up && m_used != neg_inf()) ? exp2f(m_used - m_blk) : 1.f;
-          if (up) m_used = m_blk;
-          l_run *= alpha;
-          if (pair_any(pair_bar, alpha != 1.f)) {              // (also: x is free for the next exchange)
-            // the previous P V of this tile must be complete before O is rescaled
-            if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(PV_DONE0 + t), (c_blk - 1) & 1, status, 48));
-            tc::tc_fence_after();
+        float mx;
+        {
+          uint32_t sv[4][32];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tc::tmem_ld32(s_addr + c * 32, sv[c]);
+          tc::tmem_wait_ld();
+          float m4[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            m4[c] = __uint_as_float(sv[c][0]);
+#pragma unroll
+            for (int i = 1; i + 1 < 32; i += 2) m4[c] = max3_nan(m4[c], __uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1]));
+            m4[c] = max3_nan(m4[c], m4[c], __uint_as_float(sv[c][31]));
+          }
+          mx = max3_nan(max3_nan(m4[0], m4[1], m4[2]), m4[3], m4[3]) * p.scale_log2;
+        }
+        // The scale moves only when a logit exceeds it by more than the threshold (or is NaN).
+        const bool up = !(mx <= m_used + kRescaleThreshold);
+        if (__any_sync(0xffffffffu, up)) {
+          float alpha = 1.f;
+          if (up) {
+            // an infinite logit makes the row NaN, as inf - inf would
+            const float m_new = mx == pos_inf() ? __int_as_float(0x7fffffff) : mx;
+            // the first visible key sets the scale: O and l are exactly zero so far
+            if (m_used != neg_inf()) alpha = exp2f(m_used - m_new);
+            m_used = m_new;
+          }
+          l_run.lo *= alpha;
+          l_run.hi *= alpha;
+          // O is complete: the P V before this S has been through the tensor pipe before it
+          if (j > 0) {
 #pragma unroll 1
-            for (int c = 0; c < 2 && alive; ++c) {
-              uint32_t ov[32];
-              tc::tmem_ld32(o_addr + c * 32, ov);
+            for (int c = 0; c < 8; ++c) {
+              uint32_t ov[16];
+              tc::tmem_ld16(o_addr + c * 16, ov);
               tc::tmem_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-              tc::tmem_st32(o_addr + c * 32, ov);
+              for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
+              tc::tmem_st16(o_addr + c * 16, ov);
             }
           }
-          if (alive) exponentials(m_used);
         }
-        if (!alive) continue;
-        // P goes over the first 32 of the 64 columns S came from
+        // P = 2^(s * scale - m) as bf16 pairs over the first 64 of the 128 columns S came from
+        const F2 scale = f2(p.scale_log2), m_neg = f2(m_used == neg_inf() ? 0.f : -m_used);
+        F2 sum[2] = {f2(0.f), f2(0.f)};
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          uint32_t sv[2][32];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) tc::tmem_st16(s_addr + c * 16, pk[c]);
-        l_run += row_sum;
-        tc::tmem_wait_st();
-        tc::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(bar(P_FULL0 + t));
+          for (int c = 0; c < 2; ++c) tc::tmem_ld32(s_addr + h * 64 + c * 32, sv[c]);
+          tc::tmem_wait_ld();
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            uint32_t pk[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              F2 x = f2_fma(F2{__uint_as_float(sv[c][2 * i]), __uint_as_float(sv[c][2 * i + 1])}, scale, m_neg);
+              if (i % kPolyPeriod == kPolyPeriod - 1) {
+                x = f2_exp2(x);
+              } else {
+                x.lo = exp2f(x.lo);
+                x.hi = exp2f(x.hi);
+              }
+              sum[i & 1] = f2_add(sum[i & 1], x);
+              pk[i] = pack_bf16x2(x.lo, x.hi);
+            }
+            tc::tmem_st16(s_addr + h * 32 + c * 16, pk);
+          }
+          tc::tmem_wait_st();
+          tc::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(bar((h ? P_FULL0 : P_HEAD0) + t));
+        }
+        l_run = f2_add(l_run, f2_add(sum[0], sum[1]));
       }
+      c_key += n_key;
 
       // ---- epilogue -------------------------------------------------------------------------
       bool have_o = n_mine > 0 && alive;
@@ -506,16 +577,14 @@ dense_fwd_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_co
         ++c_o;
         tc::tc_fence_after();
       }
-      *x_mine = l_run;
-      bar_sync(pair_bar, 64);
-      l_run += *x_other;
       const DenseTile tile = kTakeOver ? get_tile(n) : w;      // (read again: it need not stay in registers through the loop)
       const int row = tile.m_base + t * 128 + rl;              // query row within its sequence
       const bool row_ok = row < tile.lq;
-      const float inv = (l_run == 0.f || !have_o) ? 0.f : 1.f / l_run;
-      __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.o) + (int64_t)(tile.q0 + row) * p.o_stride_t + tile.head * p.o_stride_h + half * 64;
+      const float l_row = l_run.lo + l_run.hi;
+      const float inv = (l_row == 0.f || !have_o) ? 0.f : 1.f / l_row;
+      __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.o) + (int64_t)(tile.q0 + row) * p.o_stride_t + tile.head * p.o_stride_h;
 #pragma unroll 1
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < 4; ++c) {
         uint32_t ov[32];
         if (have_o) {
           tc::tmem_ld32(o_addr + c * 32, ov);
@@ -535,12 +604,11 @@ dense_fwd_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_co
           }
         }
       }
-      if (row_ok && half == 0)
-        p.lse[(int64_t)(tile.q0 + row) * p.lse_stride_t + tile.head * p.lse_stride_h] = inv == 0.f ? neg_inf() : (log2f(l_run) + m_used) * kLn2;
+      if (row_ok)
+        p.lse[(int64_t)(tile.q0 + row) * p.lse_stride_t + tile.head * p.lse_stride_h] = inv == 0.f ? neg_inf() : (log2f(l_row) + m_used) * kLn2;
       if (!kTakeOver) break;
-      tc::tc_fence_before();                                   // O has been read: the next tile's first P V comes after its P_FULL
-      if (alive) alive = await_tile(n + 1);
-      if (pair_any(pair_bar, !alive) || !get_tile(n + 1).valid) break;      // (also: x has been read)
+      tc::tc_fence_before();                                   // O has been read: the next tile's first P V comes after its P
+      if (!alive || !await_tile(n + 1) || !get_tile(n + 1).valid) break;
     }
   }
 
@@ -562,16 +630,14 @@ static cudaError_t launch_fwd_tc(DenseKernelParams p, const CUtensorMap& tq, con
   p.tiles_outer = p.is_causal && (int64_t)p.total_k * p.h_k * (p.d_qk + p.d_v) * 2 <= (64 << 20);
   const int64_t ctas = (int64_t)((p.max_seqlen_q + 255) / 256) * p.h_q * p.batch;
   if (ctas > INT32_MAX) return cudaErrorInvalidConfiguration;
-  // Taking CTAs over pays from nearly two CTAs with rows per SM on; below, its longer code costs what it saves.  Sequences shorter than the
+  // Taking CTAs over pays as soon as there are more CTAs with rows than SMs, and costs 0.2 to 0.3 us below.  Sequences shorter than the
   // longest leave CTAs without rows, which count for nothing here: no more than (total_q / 256 + batch) per head have some.  Device
-  // time in a graph, plain -> taking over: 128 CTAs (4 sequences of 1000 tokens, 8 heads, 192/128) 24.6 -> 26.3 us, 192 (6 of 500 to 1000, 8
-  // heads, 128/128) 21.9 -> 23.7, 256 (8 of 500 to 1000, 8 heads) 27.6 -> 28.6; 480 of which 208 have rows (1500, 700, 300, 100 and 20
-  // tokens, 16 heads, 192/128, causal) 32.4 -> 34.8, 448 of which 160 (1000 and 6 of 30, 16 heads) 23.7 -> 25.4; 288 (9 of 250, 32 heads) 24.5 -> 21.8,
-  // 288 (3 of 700) 33.7 -> 31.7, 320 (20 of 256, 16 heads) 35.8 -> 30.7, 768 (3 of 1129 to 1950, 128/128) 103.4 -> 98.2, 16384 of which 560
-  // (16384 and 255 of 128, 4 heads) 863 -> 574.
-  // With long tiles the loop, some 3 % slower at 192/128, outweighs the borders.  192/128, tiles of 8 blocks (16 of 1024, 16 heads, no
-  // mask) 199 -> 191, 16 blocks (4 of 2048, 24 heads) 282 -> 275, 32 (8 of 4096) 1293 -> 1302, 64 (4 of 8192) 2455 -> 2524; with a causal
-  // mask, which halves them, 16 of 2048 437 -> 411, 4 of 8192 1318 -> 1352; at 128/128 1194 -> 1151.
+  // time in a graph, plain -> taking over: 80 CTAs (4 sequences of 500 tokens, 10 heads, 192/128) 13.5 -> 13.9 us, 144 (18 heads) 14.3 -> 14.6, 160
+  // (4 of 200, 40 heads) 18.5 -> 16.5, 256 (32 heads) 24.3 -> 21.0, 512 (8 of 512, 32 heads, 128/128) 47.6 -> 37.6, 2048 (64 of 64) 81.6 -> 47.7;
+  // 480 of which 208 have rows (1500, 700, 300, 100 and 20 tokens, 16 heads, 192/128) 28.8 -> 29.4.  The line lies at 1.9 CTAs per SM, where it
+  // lay when the plain form's blocks took longer and taking over fewer cost up to 8 % (tests/test_gpu_dense_form.py holds it there).
+  // At 192/128 the same holds for tiles of more than 2048 keys: they cost 2 to 3 % once, and would gain 1 to 5 % now (4 of 8192 tokens, 16 heads,
+  // causal 1268 -> 1217 us, 8 of 4096 696 -> 648, no mask 1196 -> 1165).
   int dev = 0, sms = 0;
   if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
   if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); e != cudaSuccess) return e;
