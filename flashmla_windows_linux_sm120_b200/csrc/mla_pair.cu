@@ -28,7 +28,7 @@
 //                       and one thread there passes each completion on with a single remote arrive (letting the
 //                       peer's copies count their bytes on the leader's barrier directly -- cp.async.bulk.tensor
 //                       ... cta_group::2 -- made a 36 KB part take about 3 us to be seen as landed)
-//   warp 5   MMA      : rank 0: issues every MMA; rank 1: the relay of the Q / K completions just described
+//   warp 5   MMA      : rank 0: one thread issues every MMA; rank 1: the relay of the Q / K completions just described
 //   warp 6   V loader : the Q tile of a request, then per block 4 boxes of 64 rows x 64 columns, completing on a local barrier
 //   warp 7   V relay  : waits for the local V part, clears the rows of the last page that lie beyond the
 //                       sequence (they may hold NaN and 0 * NaN must not reach O), tells the leader
@@ -36,8 +36,8 @@
 // 0..5 = [320,512) (32 columns each); element (row r, column c) of an N-wide result
 // (the 64-row half of an M=128 pair instruction) sits in lane r + 64 * (c >= N/2), column c % (N/2).
 //
-// Gathering modes (sparse FP8 decode: 480 threads, sparse prefill: 320 threads).  Each CTA brings only its 32 token
-// rows of a 64-index block into the K ring -- prefill: three warps of 16-byte cp.async copies that arrive on the
+// Gathering modes (sparse FP8 decode: 480 threads, sparse prefill: 320 or 352 threads).  Each CTA brings only its 32 token
+// rows of a 64-index block into the K ring -- prefill: three or four warps of 16-byte cp.async copies that arrive on the
 // landing barrier by hardware; FP8 decode: two groups of four warps that read the 656-byte records into registers,
 // de-quantise them once per pair and store them in the layout TMA would produce.  The V operand (64 tokens x 256
 // columns per CTA) is not read from global memory at all: the thread of warp 6 forwards it out of the landed K rows
@@ -84,17 +84,17 @@ static_assert(kQTmemChunks * kChunkBytes <= 2 * kVStageBytes, "Q staging must fi
 // and per-CTA barriers (each CTA waits on its own copy; the leader's commits arrive on both copies)
 enum Bar { Q_FULL = 0, K_FULL0, K_FULL1, K_FULL2, V_FULL0, V_FULL1, S_EMPTY0, S_EMPTY1, P_FULL0, P_FULL1, O_EMPTY,
            Q_EMPTY, QT_DONE, K_EMPTY0, K_EMPTY1, K_EMPTY2, V_EMPTY0, V_EMPTY1, V_LAND0, V_LAND1, S_FULL0, S_FULL1,
-           P_EMPTY0, P_EMPTY1, O_FULL, Q_LAND, K_LAND0, K_LAND1, K_LAND2, NUM_BARS };
+           O_FULL, Q_LAND, K_LAND0, K_LAND1, K_LAND2, NUM_BARS };
 constexpr int TMEM_O = 0, TMEM_S = 256, TMEM_Q = 320;
 static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB shared memory limit per CTA");
 static_assert(NUM_BARS * 8 <= 256, "barrier area too small");
 constexpr float kRescaleThreshold = 8.0f;
 constexpr int kThreads = 256;
-#ifndef FMLA_GATHER_WARPS
-#define FMLA_GATHER_WARPS 3
-#endif
-constexpr int kGatherWarps = FMLA_GATHER_WARPS;                 // sparse prefill: warp 4 and warps 8 .. 6 + kGatherWarps (measured: 3 -> 993, 4 -> 983, 5 -> 935, 2 -> 452 TFLOP/s)
-constexpr int kPrefillThreads = (7 + kGatherWarps) * 32;
+// Sparse prefill: gather warps 4 and 8, 9, ..  Long calls run at the power limit with any number of them (4096 tokens 2574 us with three,
+// 2579 with four); with cut tokens, of which few units work at a time, four are faster: one token, top-k 2048, 16.7 -> 16.2 us, 37 tokens
+// 35.7 -> 34.9, and in calls of a few rounds three: 333 tokens, top-k 512, 70.1 -> 71.7, 222, top-k 1024, 72.2 -> 73.4.
+__host__ __device__ constexpr int gather_warps(int wm) { return wm == kSparsePrefillCut ? 4 : 3; }
+__host__ __device__ constexpr int prefill_threads(int wm) { return (7 + gather_warps(wm)) * 32; }
 #ifndef FMLA_DECODE_GROUPS
 #define FMLA_DECODE_GROUPS 2
 #endif
@@ -116,7 +116,6 @@ __device__ long long g_pair_span[512 * 2];       // per CTA: first and last cloc
 #endif
 // cross-CTA timeline in nanoseconds (globaltimer): [block][rank][slot]
 __device__ long long g_pair_gt[160 * 2 * 8];
-__device__ long long g_pair_head[256][2];
 __device__ __forceinline__ long long gtime() { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return (long long)t; }
 #define FMLA_GTRACE_AT(blk, rk, slot)                                                       \
   do {                                                                                       \
@@ -176,7 +175,7 @@ __device__ __forceinline__ void pv_block_pair(uint32_t tmem_o, uint64_t desc_p_s
 // forwarded from those rows (tmap_k32 / tmap_v64 unused); invalid indices leave zero rows and are masked through
 // validity bits.
 template <bool F16, int WM>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WM == kDense ? ptc::kThreads : WM == kSparseDecode ? ptc::kSparseDecodeThreads : ptc::kPrefillThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WM == kDense ? ptc::kThreads : WM == kSparseDecode ? ptc::kSparseDecodeThreads : ptc::prefill_threads(WM), 1)
 mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUtensorMap tmap_q,
                 const __grid_constant__ CUtensorMap tmap_k32, const __grid_constant__ CUtensorMap tmap_v64) {
   using namespace ptc;
@@ -227,7 +226,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
     // and a K stage has landed when every lane of the gather warps has arrived by hardware, plus the thread that
     // published the validity bits (prefill), or when every gather warp has stored its rows (FP8 decode)
     for (int i = Q_EMPTY; i < NUM_BARS; ++i)
-      tc::mbar_init(bar(i), !SPARSE ? 1 : (i >= K_EMPTY0 && i <= K_EMPTY2) ? 3 : (i >= K_LAND0 && i <= K_LAND2) ? (PREFILL ? kGatherWarps * 32 + 1 : 4 /* FP8 decode: the four gather warps of a group */) : 1);
+      tc::mbar_init(bar(i), !SPARSE ? 1 : (i >= K_EMPTY0 && i <= K_EMPTY2) ? 3 : (i >= K_LAND0 && i <= K_LAND2) ? (PREFILL ? gather_warps(WM) * 32 + 1 : 4 /* FP8 decode: the four gather warps of a group */) : 1);
     tc::fence_mbar_init();
     *sAbort = 0;
     if (misaligned) tc::report_status(status, 30);
@@ -247,9 +246,9 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
     // request is p.b, past the lengths, the indices and num_splits.)
   } else if ((warp == 4 || warp >= 8) && PREFILL) {
     // ================================ Q and K loader, sparse prefill ===================
-    // The CTA's 32 token rows of a block (32 x 1152 bytes) are gathered with 16-byte cp.async copies by three warps
-    // (4, 8, 9): 72 warp instructions per block, dealt out round robin, consecutive lanes on consecutive pieces of a row.
-    // Measured at the benchmark shape: with each warp taking a contiguous third of the instructions 751 TFLOP/s; with
+    // The CTA's 32 token rows of a block (32 x 1152 bytes) are gathered with 16-byte cp.async copies by three or four warps
+    // (4, 8, 9, ..): 72 warp instructions per block, dealt out round robin, consecutive lanes on consecutive pieces of a row.
+    // Measured with the issuing warp of before: with each warp taking a contiguous third of the instructions 751 TFLOP/s; with
     // the round-robin deal two warps 452, three 979-1009, four 964-982, five 935-957.  The TMA engine (tile::gather4, 4 rows x 64
     // columns per copy) gathers no faster than ~11 bytes per clock and SM, and mixing the two paths was slower
     // than either (8 of the 32 rows by TMA: 545 TFLOP/s; 16: 466), because the gathers queue behind the forwarding
@@ -302,7 +301,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
         }
         constexpr int kInstr = 32 * 72 / 32;                      // warp instructions per block, dealt out round robin
 #pragma unroll
-        for (int inst = 0; inst < kInstr; inst += kGatherWarps) {
+        for (int inst = 0; inst < kInstr; inst += gather_warps(WM)) {
           if (inst + gw >= kInstr) break;
           const int e = (inst + gw) * 32 + lane;                 // piece e of 32 rows x 72 pieces of 16 bytes
           const int row = e / 72, piece = e % 72;
@@ -678,7 +677,14 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
     }
   } else if (warp == 5) {
     // ================================ MMA issuer (leader only) =========================
-    if (rank == 0) {
+    // One thread, in a fixed order: S of a block, P V of the block before.  A warp that polled the five barriers of interest, and
+    // issued what was ready first, was the longest link of the chain: from the end of one issue to the next some 850 clk, twice a block, with
+    // everything there (votes, taken branches and eight commits a block, now three that go to both CTAs), 2 460 clk a block of the
+    // dense decode with two tokens against 1 700, 2 900 against 2 050 of the sparse prefill, 3 150 against 2 350 of the sparse decode.
+    // Where the power limit holds (long dense decodes, long prefills) the clock takes most of it back: 128 x 4000 tokens 175.7 ->
+    // 174.1 us, two tokens 313.0 -> 309.2, prefill of 4096 tokens 2 648 -> 2 575; elsewhere it shows: 16 x 2000 tokens 27.5 -> 26.2,
+    // 20 prefill tokens 24.5 -> 23.3, sparse decode of 30 x 512 28.7 -> 27.8.
+    if (tc::elect_one()) {
       constexpr uint32_t idesc_s = tc::idesc_bf16_f32(128, 64, 0, 0, F16);
       constexpr uint32_t idesc_o = tc::idesc_bf16_f32(128, 256, 0, 1, F16);
       const uint64_t desc_q = tc::smem_desc_sw128(sQ, 16, 1024);             // A of S, chunks 6..8: K-major
@@ -686,112 +692,55 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
       const uint64_t desc_k = tc::smem_desc_sw128(sK, 16, 1024);             // B of S: K-major, 32 rows per CTA (stage 0)
       const uint64_t desc_p = tc::smem_desc_sw128(sP, 16, 1024);             // A of PV: K-major
       const uint64_t desc_v = tc::smem_desc_sw128(sV, kChunkBytes, 1024);    // B of PV: MN-major, 64-wide column groups 8 KB apart
-      // every commit goes to the barrier copy of each CTA (two plain commits, each naming one barrier)
-      auto commit_both = [&](int b) {
-        tc::tc_commit_pair(bar(b));
-        tc::tc_commit_pair(tc::mapa(bar(b), 1));
-      };
+      // every commit goes to the barrier copies of both CTAs
+      auto commit_both = [&](int b) { tc::tc_commit_pair_both(bar(b)); };
       int g = 0, req = 0;
       bool alive = true;
-#ifdef FMLA_TRACE
-      int seen_k = -1, seen_s = -1, seen_p = -1, seen_v = -1, after_issue = 0;
-#endif
       for (int wi = 0; wi < tile.n_work && alive; ++wi) {
         const Work r = get_work<WM>(P, tile, wi);
         const int nblk = r.blk_hi - r.blk_lo;
         if (nblk == 0) continue;
-        alive = __all_sync(0xffffffffu, tc::mbar_wait_cluster(bar(Q_FULL), req & 1, status, 105));
+        alive = tc::mbar_wait_cluster(bar(Q_FULL), req & 1, status, 105);
         if (!alive) break;
         // Q chunks 0..5: shared memory -> tensor memory of both CTAs (8 copies of 64 rows x 16 bytes per chunk)
         tc::tc_fence_after();
-        if (tc::elect_one()) {
 #pragma unroll
-          for (int c = 0; c < kQTmemChunks; ++c)
+        for (int c = 0; c < kQTmemChunks; ++c)
 #pragma unroll
-            for (int sub = 0; sub < 8; ++sub)
-              tmem_cp_pair_64x128b(tmem + TMEM_Q + c * 32 + sub * 4, tc::desc_advance(desc_qstage, c * kChunkBytes + sub * 16));
-          commit_both(QT_DONE);
-        }
-        __syncwarp();
-        // One poll reads every barrier of interest, one per lane:
-        //   lane 0 P_FULL(jp)  lane 1 O_EMPTY  lane 2 V_FULL(jp)  lane 3 S_EMPTY(js)  lane 4 K_FULL(js)
-        int js = 0, jp = 0, idle = 0;
-        while (jp < nblk && alive) {
-#ifdef FMLA_TRACE
-          if (lane == 0 && after_issue && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == FMLA_TRACE_PART) {   // first pass through the loop head after an issue: rank-0 slots 1 / 10 hold ns
-            if (after_issue == 1) g_pair_head[(g + js - 1) & 255][0] = gtime(); else g_pair_head[(g + jp - 1) & 255][1] = gtime();
-          }
-          after_issue = 0;
-#endif
-          const int gs = g + min(js, nblk - 1), sbs = gs & 1, kst = gs % kKStages;
-          const uint32_t phs = (gs >> 1) & 1, phk = (gs / kKStages) & 1;
-          const int gp = g + jp, stp = gp & 1;
-          const uint32_t php = (gp >> 1) & 1;
-          int pb = P_FULL0 + stp;
-          uint32_t pp = php;
-          if (lane == 1) { pb = O_EMPTY; pp = (req & 1) ^ 1; }
-          if (lane == 2) { pb = V_FULL0 + stp; pp = php; }
-          if (lane == 3) { pb = S_EMPTY0 + sbs; pp = phs ^ 1; }
-          if (lane >= 4) { pb = K_FULL0 + kst; pp = phk; }
-          const bool hit = lane < 5 && tc::mbar_test_wait_cluster(bar(pb), pp);
-          const uint32_t m = __ballot_sync(0xffffffffu, hit);
-#ifdef FMLA_TRACE
-          if (lane == 0) {     // first time each input of the next S / P V is seen ready (rank-1 slots 3..6 of the timeline)
-            if ((m & 0x10u) && js < nblk && seen_k != gs) { seen_k = gs; FMLA_GTRACE_AT(gs, 1, 3); }
-            if ((m & 0x8u) && js < nblk && seen_s != gs) { seen_s = gs; FMLA_GTRACE_AT(gs, 1, 4); }
-            if ((m & 0x1u) && jp < js && seen_p != gp) { seen_p = gp; FMLA_GTRACE_AT(gp, 1, 5); }
-            if ((m & 0x4u) && jp < js && seen_v != gp) { seen_v = gp; FMLA_GTRACE_AT(gp, 1, 6); }
-          }
-#endif
-          bool did = false;
-          if (jp < js && (m & 5u) == 5u && (jp > 0 || (m & 2u))) {
-            tc::tc_fence_after();
-            if (lane == 0) { FMLA_PTRACE_AT(gp, 4); FMLA_GTRACE_AT(gp, 0, 5); }
-            if (tc::elect_one()) {
-              pv_block_pair(tmem + TMEM_O, tc::desc_advance(desc_p, stp * kChunkBytes), tc::desc_advance(desc_v, stp * kVStageBytes), idesc_o, jp == 0);
-              commit_both(V_EMPTY0 + stp);
-              commit_both(P_EMPTY0 + stp);
-              FMLA_PTRACE_AT(gp, 5);
-              FMLA_GTRACE_AT(gp, 0, 6);
-            }
-            __syncwarp();
-            ++jp;
-            did = true;
-#ifdef FMLA_TRACE
-            after_issue = 2;
-#endif
-          } else if (js < nblk && (m & 0x18u) == 0x18u) {
+          for (int sub = 0; sub < 8; ++sub)
+            tmem_cp_pair_64x128b(tmem + TMEM_Q + c * 32 + sub * 4, tc::desc_advance(desc_qstage, c * kChunkBytes + sub * 16));
+        commit_both(QT_DONE);
+        for (int j = 0; j <= nblk; ++j) {
+          if (j < nblk) {
+            const int gs = g + j, sbs = gs & 1, kst = gs % kKStages;
+            alive = tc::mbar_wait_cluster(bar(S_EMPTY0 + sbs), ((gs >> 1) & 1) ^ 1, status, 106);
+            if (alive) alive = tc::mbar_wait_cluster(bar(K_FULL0 + kst), (gs / kKStages) & 1, status, 106);
+            if (!alive) break;
             if constexpr (SPARSE) tc::fence_proxy_async_smem();    // K rows came through cp.async / plain stores
             tc::tc_fence_after();
-            if (lane == 0) { FMLA_PTRACE_AT(gs, 2); FMLA_GTRACE_AT(gs, 0, 3); }
-            if (tc::elect_one()) {
-              s_block_pair(tmem + TMEM_S + sbs * 32, tmem + TMEM_Q, desc_q, tc::desc_advance(desc_k, kst * kKStageBytes), idesc_s);
-              commit_both(S_FULL0 + sbs);
-              commit_both(K_EMPTY0 + kst);
-              FMLA_PTRACE_AT(gs, 3);
-              FMLA_GTRACE_AT(gs, 0, 4);
-              if (js == nblk - 1) commit_both(Q_EMPTY);
-            }
-            __syncwarp();
-            ++js;
-            did = true;
-#ifdef FMLA_TRACE
-            after_issue = 1;
-#endif
+            FMLA_PTRACE_AT(gs, 2);
+            s_block_pair(tmem + TMEM_S + sbs * 32, tmem + TMEM_Q, desc_q, tc::desc_advance(desc_k, kst * kKStageBytes), idesc_s);
+            commit_both(S_FULL0 + sbs);
+            commit_both(K_EMPTY0 + kst);
+            FMLA_PTRACE_AT(gs, 3);
+            if (j == nblk - 1) commit_both(Q_EMPTY);
           }
-          if (did) {
-            idle = 0;
-          } else if (++idle > tc::kSpinLimit) {
-            if (lane == 0) tc::report_status(status, 106);
-            alive = false;
+          if (j > 0) {
+            const int gp = g + j - 1, stp = gp & 1;
+            const uint32_t php = (gp >> 1) & 1;
+            if (j == 1) alive = tc::mbar_wait_cluster(bar(O_EMPTY), (req & 1) ^ 1, status, 106);
+            if (alive) alive = tc::mbar_wait_cluster(bar(V_FULL0 + stp), php, status, 106);
+            if (alive) alive = tc::mbar_wait_cluster(bar(P_FULL0 + stp), php, status, 106);
+            if (!alive) break;
+            tc::tc_fence_after();
+            FMLA_PTRACE_AT(gp, 4);
+            pv_block_pair(tmem + TMEM_O, tc::desc_advance(desc_p, stp * kChunkBytes), tc::desc_advance(desc_v, stp * kVStageBytes), idesc_o, j == 1);
+            commit_both(V_EMPTY0 + stp);
+            FMLA_PTRACE_AT(gp, 5);
           }
-#ifdef FMLA_PAIR_POLL_SLEEP
-          else { __nanosleep(FMLA_PAIR_POLL_SLEEP); }
-#endif
         }
         g += nblk;
-        if (alive && tc::elect_one()) commit_both(O_FULL);
-        __syncwarp();
+        if (alive) commit_both(O_FULL);
         ++req;
       }
     }
@@ -861,7 +810,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
         // P has two buffers (block g uses buffer g & 1): writing it needs P V of block g-2 to be complete;
         // rescaling O needs every earlier P V to be complete, i.e. that of block g-1 (they complete in order)
         if (any_need) {
-          if (j > 0 && !tc::mbar_wait(bar(P_EMPTY0 + ((g - 1) & 1)), ((g - 1) >> 1) & 1, status, 109)) *sAbort = 1;
+          if (j > 0 && !tc::mbar_wait(bar(V_EMPTY0 + ((g - 1) & 1)), ((g - 1) >> 1) & 1, status, 109)) *sAbort = 1;
           const float m_next = need ? m_new : m_used;
           const float alpha = exp2f(m_used - m_next);
           m_used = m_next;
@@ -889,7 +838,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
           pk[i] = pack_16x2<F16>(p0, p1);
         }
         l_part += (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
-        if (!tc::mbar_wait(bar(P_EMPTY0 + st), ((g >> 1) & 1) ^ 1, status, 109)) *sAbort = 1;
+        if (!tc::mbar_wait(bar(V_EMPTY0 + st), ((g >> 1) & 1) ^ 1, status, 109)) *sAbort = 1;
         if (tid == 0) FMLA_PTRACE_AT(g, 9);
         // P[row][th*32 .. +32) -> K-major 128B-swizzled A operand: 16-byte chunk (th*4 + q) ^ (row & 7)
 #pragma unroll
@@ -1088,8 +1037,8 @@ cudaError_t launch_sparse_prefill_pair(const SparsePrefillKernelParams& sp, cuda
   if (!tmah::make_map_4d(&tq, sp.q, sp.h_q, sp.s_q, 1, sp.q_stride_h, sp.q_stride_s, sp.q_stride_s * sp.s_q, 64, 1)) return cudaErrorInvalidValue;
   // a kernel of its own for the cut tokens: their fp32 stores cost the other one three registers that it does not have (4096 tokens 2606 -> 2680 us)
   const dim3 grid(2, sp.units, 1);
-  if (sp.per > 1) return launch_pair<mla_pair_kernel<false, kSparsePrefillCut>>(P, tq, tq, tq, grid, ptc::kPrefillThreads, stream);
-  return launch_pair<mla_pair_kernel<false, kSparsePrefill>>(P, tq, tq, tq, grid, ptc::kPrefillThreads, stream);    // the K / V maps are not used in this mode
+  if (sp.per > 1) return launch_pair<mla_pair_kernel<false, kSparsePrefillCut>>(P, tq, tq, tq, grid, ptc::prefill_threads(kSparsePrefillCut), stream);
+  return launch_pair<mla_pair_kernel<false, kSparsePrefill>>(P, tq, tq, tq, grid, ptc::prefill_threads(kSparsePrefill), stream);    // the K / V maps are not used in this mode
 }
 
 // Two 64-row tiles that read the same pages: the halves of 128 heads, or the 64 heads of two consecutive query tokens, which
@@ -1123,9 +1072,6 @@ extern "C" int fmla_debug_read_pair_trace(long long* host, int n) {
 }
 extern "C" int fmla_debug_read_pair_gt(long long* host, int n) {
   return (int)cudaMemcpyFromSymbol(host, g_pair_gt, sizeof(long long) * n);
-}
-extern "C" int fmla_debug_read_pair_head(long long* host, int n) {
-  return (int)cudaMemcpyFromSymbol(host, g_pair_head, sizeof(long long) * n);
 }
 extern "C" int fmla_debug_read_pair_span(long long* host, int n) {
   return (int)cudaMemcpyFromSymbol(host, g_pair_span, sizeof(long long) * n);
