@@ -93,7 +93,7 @@ constexpr int kThreads = 256;
 // Sparse prefill: gather warps 4 and 8, 9, ..  Long calls run at the power limit with any number of them (4096 tokens 2574 us with three,
 // 2579 with four); with cut tokens, of which few units work at a time, four are faster: one token, top-k 2048, 16.7 -> 16.2 us, 37 tokens
 // 35.7 -> 34.9, and in calls of a few rounds three: 333 tokens, top-k 512, 70.1 -> 71.7, 222, top-k 1024, 72.2 -> 73.4.
-__host__ __device__ constexpr int gather_warps(int wm) { return wm == kSparsePrefillCut ? 4 : 3; }
+__host__ __device__ constexpr int gather_warps(int wm) { return 4; }
 __host__ __device__ constexpr int prefill_threads(int wm) { return (7 + gather_warps(wm)) * 32; }
 #ifndef FMLA_DECODE_GROUPS
 #define FMLA_DECODE_GROUPS 2
@@ -267,7 +267,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
       const Work r = get_work<WM>(P, tile, wi);
       // the indices of a block are read one block ahead of their use: their latency would otherwise be paid in
       // every turn of this loop
-      const int* my_idx = r.idx + 32 * static_cast<int>(rank) + lane;
+      const int* my_idx = r.idx + 32 * static_cast<int>(rank) + gw * 8 + (lane & 7);
       int mine_next = r.blk_lo < r.blk_hi ? my_idx[r.blk_lo * 64] : -1, i0_next = -1, i1_next = -1;
       if (warp == 4 && r.blk_lo < r.blk_hi) {
         i0_next = r.idx[r.blk_lo * 64 + lane];
@@ -275,7 +275,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
       }
       for (int blk = r.blk_lo; blk < r.blk_hi && alive; ++blk, ++g) {
         const int st = g % kKStages;
-        int mine = mine_next;                                                          // row `lane` of this CTA's part
+        int mine = mine_next;                                                          // row 8 gw + lane of this CTA's part (lanes 0..7)
         const int i0 = i0_next, i1 = i1_next;
         if (blk + 1 < r.blk_hi) {
           mine_next = my_idx[(blk + 1) * 64];
@@ -299,16 +299,16 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
           sValid[(g % 6) * 2 + 1] = b1;
           tc::mbar_arrive(bar(K_LAND0 + st));
         }
-        constexpr int kInstr = 32 * 72 / 32;                      // warp instructions per block, dealt out round robin
+        const uint32_t lane_dst = dst + (lane >> 3) * kKChunkBytes + gw * 8 * 128;
 #pragma unroll
-        for (int inst = 0; inst < kInstr; inst += gather_warps(WM)) {
-          if (inst + gw >= kInstr) break;
-          const int e = (inst + gw) * 32 + lane;                 // piece e of 32 rows x 72 pieces of 16 bytes
-          const int row = e / 72, piece = e % 72;
-          const int idx = __shfl_sync(0xffffffffu, mine, row);
+        for (int rr = 0; rr < 8; ++rr) {                          // row 8 gw + rr: 72 pieces of 16 bytes
+          const int idx = __shfl_sync(0xffffffffu, mine, rr);
           const bool ok = idx >= 0;
-          const char* src = kvb + (ok ? (int64_t)idx * row_bytes + piece * 16 : 0);
-          cp_async16(dst + (piece >> 3) * kKChunkBytes + row * 128 + (((piece & 7) ^ (row & 7)) << 4), src, ok);
+          const char* src = kvb + (ok ? (int64_t)idx * row_bytes + lane * 16 : 0);
+          const uint32_t d = lane_dst + rr * 128 + (((lane & 7) ^ rr) << 4);
+          cp_async16(d, src, ok);
+          cp_async16(d + 4 * kKChunkBytes, src + (ok ? 512 : 0), ok);
+          if (lane < 8) cp_async16(d + 8 * kKChunkBytes, src + (ok ? 1024 : 0), ok);
         }
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar(K_LAND0 + st)) : "memory");
       }

@@ -45,7 +45,7 @@ constexpr int BAR_OFF = P_OFF + kChunkBytes;      // mbarriers
 constexpr int MX_OFF = BAR_OFF + 128;             // float [3][128] exchange (2 for row maxima, 1 for row sums)
 constexpr int MISC_OFF = MX_OFF + 1536;           // tmem base, abort flag, token validity masks
 constexpr int SMEM_BYTES = MISC_OFF + 64;         // misc words
-enum Bar { Q_FULL = 0, Q_EMPTY, KV_FULL0, KV_FULL1, KV_EMPTY0, KV_EMPTY1, S_FULL0, S_FULL1, S_EMPTY0, S_EMPTY1, P_FULL, P_EMPTY, O_FULL, O_EMPTY, NUM_BARS };
+enum Bar { Q_FULL = 0, Q_EMPTY, KV_FULL0, KV_FULL1, KV_EMPTY0, KV_EMPTY1, S_FULL0, S_FULL1, P_FULL, O_FULL, O_EMPTY, NUM_BARS };
 constexpr int TMEM_O = 0, TMEM_S = 256;
 static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB shared memory limit per CTA");
 static_assert(NUM_BARS * 8 <= 128, "barrier area too small");
@@ -71,18 +71,22 @@ __device__ long long g_tile64_trace[64 * 16];
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint4 v) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-// The 36 S = Q K^T instructions of one block in stage ST, as straight-line code whose descriptors are
-// a warp-uniform base plus an immediate.  (Two unrolled copies, one per stage, still fit the instruction cache
-// here and were measured faster than one copy with a run-time stage base: 686 vs 641 TFLOP/s on the sparse prefill.)
-template <int ST>
-__device__ __forceinline__ void s_block(uint32_t tmem, uint64_t desc_q, uint64_t desc_k, uint32_t idesc) {
+// The 36 S = Q K^T instructions of one block, as straight-line code whose descriptors are a base plus an immediate.
+__device__ __forceinline__ void s_block(uint32_t tmem_s, uint64_t desc_q, uint64_t desc_k, uint32_t idesc) {
   using namespace dtc;
 #pragma unroll
   for (int c = 0; c < 9; ++c)
 #pragma unroll
     for (int s = 0; s < 4; ++s)
-      tc::mma_ws_ss(tmem + TMEM_S + ST * 32, tc::desc_advance(desc_q, c * kChunkBytes + s * 32),
-                    tc::desc_advance(desc_k, ST * kTileBytes + c * kChunkBytes + s * 32), idesc, (c | s) ? 1u : 0u);
+      tc::mma_ws_ss(tmem_s, tc::desc_advance(desc_q, c * kChunkBytes + s * 32), tc::desc_advance(desc_k, c * kChunkBytes + s * 32), idesc, (c | s) ? 1u : 0u);
+}
+__device__ __forceinline__ void pv_block(uint32_t tmem_o, uint64_t desc_p, uint64_t desc_v, uint32_t idesc, bool first) {
+  using namespace dtc;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+      tc::mma_ws_ss(tmem_o + h * 128, tc::desc_advance(desc_p, s * 32), tc::desc_advance(desc_v, h * 4 * kChunkBytes + s * 2048), idesc, (first && s == 0) ? 0u : 1u);
 }
 
 // kDense: grid (s_q * ceil(hq_per_hk / 64), h_k, parts); kSparsePrefillCut: grid (h_q / 64, units), persistent over query
@@ -120,12 +124,9 @@ mla_tile64_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CU
     tc::mbar_init(bar(KV_EMPTY1), 1);
     tc::mbar_init(bar(S_FULL0), 1);
     tc::mbar_init(bar(S_FULL1), 1);
-    tc::mbar_init(bar(S_EMPTY0), 128);
-    tc::mbar_init(bar(S_EMPTY1), 128);
-    tc::mbar_init(bar(P_FULL), 128);
-    tc::mbar_init(bar(P_EMPTY), 1);
+    tc::mbar_init(bar(P_FULL), 4);         // one arrival per softmax warp
     tc::mbar_init(bar(O_FULL), 1);
-    tc::mbar_init(bar(O_EMPTY), 128);
+    tc::mbar_init(bar(O_EMPTY), 4);
     tc::fence_mbar_init();
     *sAbort = 0;
   }
@@ -230,114 +231,60 @@ mla_tile64_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CU
     }
   } else if (warp == 5) {
     // ================================ MMA issuer =======================================
-    constexpr uint32_t idesc_s = tc::idesc_bf16_f32(64, 64, 0, 0, F16);
-    constexpr uint32_t idesc_o = tc::idesc_bf16_f32(64, 256, 0, 1, F16);
-    // descriptors of the operand bases; per-MMA addresses are constant offsets added to the low word
-    const uint64_t desc_q = tc::smem_desc_sw128(sQ, 16, 1024);             // A of S: K-major
-    const uint64_t desc_k = tc::smem_desc_sw128(sKV, 16, 1024);            // B of S: K-major (stage 0)
-    const uint64_t desc_p = tc::smem_desc_sw128(sP, 16, 1024);             // A of PV: K-major
-    const uint64_t desc_v = tc::smem_desc_sw128(sKV, kChunkBytes, 1024);   // B of PV: MN-major, 64-wide column groups 8 KB apart
-    int g = 0, req = 0;
-    bool alive = true;
-    // both issue helpers are called by the whole warp; one elected thread issues
-    auto issue_pv = [&](int gi, bool first_of_request) {
-      const int st = gi & 1;
-      tc::tc_fence_after();
-      if (lane == 0) FMLA_TRACE_AT(gi, 4);
-      // elect.sync (not a lane-id test) selects the issuing thread: only then does the compiler keep
-      // the descriptors in uniform registers, which halves the per-instruction issue cost
-      if (tc::elect_one()) {
-        // the stage index is resolved by a branch so that every descriptor below is a warp-uniform
-        // base plus an immediate
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (st == 0) {
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-              tc::mma_ws_ss(tmem + TMEM_O + h * 128, tc::desc_advance(desc_p, s * 32),
-                            tc::desc_advance(desc_v, h * 4 * kChunkBytes + s * 2048), idesc_o, (first_of_request && s == 0) ? 0u : 1u);
-          } else {
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-              tc::mma_ws_ss(tmem + TMEM_O + h * 128, tc::desc_advance(desc_p, s * 32),
-                            tc::desc_advance(desc_v, kTileBytes + h * 4 * kChunkBytes + s * 2048), idesc_o, (first_of_request && s == 0) ? 0u : 1u);
-          }
-        }
-        tc::tc_commit(bar(KV_EMPTY0 + st));
-        tc::tc_commit(bar(P_EMPTY));
-        FMLA_TRACE_AT(gi, 5);
-      }
-      __syncwarp();
-    };
-    for (int wi = 0; wi < tile.n_work && alive; ++wi) {
-      const Work r = get_work<MODE>(P, tile, wi);
-      const int nblk = r.blk_hi - r.blk_lo;
-      if (nblk == 0) continue;
-      alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_FULL), req & 1, status, 5));
-      // S of block js and P V of block jp < js are issued in whichever order their inputs become
-      // ready; P V goes first when both are possible: it releases a cache stage and the next load
-      // depends on that.  One poll reads all barriers of interest at once, one per lane, and a ballot
-      // shares the result:  lane 0 P_FULL(jp)   lane 1 O_EMPTY   lane 2 S_EMPTY(js)   lane 3 KV_FULL(js)
-      // The S instructions of a block are issued from one straight-line site per stage (splitting
-      // them into several separately issued groups more than doubled the time of S: the tensor
-      // pipe drains in every gap).
-      int js = 0, jp = 0, idle = 0;
-      while (jp < nblk && alive) {
-        const int gi = g + min(js, nblk - 1), st = gi & 1;
-        const uint32_t ph = (gi >> 1) & 1;
-        int pb = P_FULL;
-        uint32_t pp = (g + jp) & 1;
-        if (lane == 1) { pb = O_EMPTY; pp = (req & 1) ^ 1; }
-        if (lane == 2) { pb = S_EMPTY0 + st; pp = ph ^ 1; }
-        if (lane >= 3) { pb = KV_FULL0 + st; pp = ph; }
-        const bool hit = lane < 4 && tc::mbar_test_wait(bar(pb), pp);
-        const uint32_t m = __ballot_sync(0xffffffffu, hit);
-        bool did = false;
-        if (jp < js && (m & 1u) && (jp > 0 || (m & 2u))) {
-          issue_pv(g + jp, jp == 0);
-          ++jp;
-          did = true;
-        } else if (js < nblk && (m & 0xcu) == 0xcu) {
-          if constexpr (MODE == kSparsePrefillCut) {
-            tc::fence_proxy_async_smem();   // rows written by cp.async -> tensor pipe
-          } else {
-            // rows of the last page beyond the sequence may hold anything (NaN included) and 0 * NaN must not reach O
-            const int rows_valid = r.seqlen - (r.blk_lo + js) * 64;
-            if (rows_valid < 64) {
-              for (int i = lane; i < (64 - rows_valid) * 64; i += 32) {
-                const int row = rows_valid + (i >> 6), c16 = i & 63;
-                *reinterpret_cast<uint4*>(smem + KV_OFF + st * kTileBytes + (c16 >> 3) * kChunkBytes + row * 128 + (c16 & 7) * 16) = make_uint4(0, 0, 0, 0);
-              }
-              tc::fence_proxy_async_smem();
-              __syncwarp();
-            }
-          }
-          tc::tc_fence_after();
-          if (lane == 0) FMLA_TRACE_AT(gi, 2);
-          if (tc::elect_one()) {
-            if (st == 0) s_block<0>(tmem, desc_q, desc_k, idesc_s);
-            else s_block<1>(tmem, desc_q, desc_k, idesc_s);
+    // One thread.  A warp that polled four barriers, shared the outcome by a vote and slept between polls took 8 % longer, and with
+    // it went the arrivals of 128 threads on each of S_EMPTY, P_FULL and O_EMPTY (one per warp now, or none): 333 tokens, top-k 512, 50.4 ->
+    // 47.7 us, 4096, top-k 2048, 1717 -> 1605; dense, 64 heads x 3 tokens, 16 x 16 000 156.5 -> 143.9.
+    if (tc::elect_one()) {
+      constexpr uint32_t idesc_s = tc::idesc_bf16_f32(64, 64, 0, 0, F16);
+      constexpr uint32_t idesc_o = tc::idesc_bf16_f32(64, 256, 0, 1, F16);
+      const uint64_t desc_q = tc::smem_desc_sw128(sQ, 16, 1024);             // A of S: K-major
+      const uint64_t desc_k = tc::smem_desc_sw128(sKV, 16, 1024);            // B of S: K-major (stage 0)
+      const uint64_t desc_p = tc::smem_desc_sw128(sP, 16, 1024);             // A of PV: K-major
+      const uint64_t desc_v = tc::smem_desc_sw128(sKV, kChunkBytes, 1024);   // B of PV: MN-major, 64-wide column groups 8 KB apart (stage 0)
+      int g = 0, req = 0;
+      bool alive = true;
+      for (int wi = 0; wi < tile.n_work && alive; ++wi) {
+        const Work r = get_work<MODE>(P, tile, wi);
+        const int nblk = r.blk_hi - r.blk_lo;
+        if (nblk == 0) continue;
+        alive = tc::mbar_wait(bar(Q_FULL), req & 1, status, 5);
+        // S of block js and P V of block jp < js are issued in whichever order their inputs become ready; P V goes first
+        // when both are possible: it releases a cache stage and the next load depends on that.  (That the stage of block js is
+        // filled says that P V of block js - 2 is complete, so its S has been read and the S buffer is free.)
+        int js = 0, jp = 0, idle = 0;
+        while (jp < nblk && alive) {
+          const int gs = g + js, gp = g + jp;
+          if (jp < js && tc::mbar_test_wait(bar(P_FULL), gp & 1)) {
+            if (jp == 0) alive = tc::mbar_wait(bar(O_EMPTY), (req & 1) ^ 1, status, 6);
+            if (!alive) break;
+            const int st = gp & 1;
+            tc::tc_fence_after();
+            FMLA_TRACE_AT(gp, 4);
+            pv_block(tmem + TMEM_O, desc_p, tc::desc_advance(desc_v, st * kTileBytes), idesc_o, jp == 0);
+            tc::tc_commit(bar(KV_EMPTY0 + st));
+            FMLA_TRACE_AT(gp, 5);
+            ++jp;
+            idle = 0;
+          } else if (js < nblk && tc::mbar_test_wait(bar(KV_FULL0 + (gs & 1)), (gs >> 1) & 1)) {
+            const int st = gs & 1;
+            if constexpr (MODE == kSparsePrefillCut) tc::fence_proxy_async_smem();   // rows written by cp.async -> tensor pipe
+            tc::tc_fence_after();
+            FMLA_TRACE_AT(gs, 2);
+            s_block(tmem + TMEM_S + st * 32, desc_q, tc::desc_advance(desc_k, st * kTileBytes), idesc_s);
             tc::tc_commit(bar(S_FULL0 + st));
-            FMLA_TRACE_AT(gi, 3);
+            FMLA_TRACE_AT(gs, 3);
             if (js == nblk - 1) tc::tc_commit(bar(Q_EMPTY));
+            ++js;
+            idle = 0;
+          } else if (++idle > tc::kSpinLimit) {
+            tc::report_status(status, 6);
+            alive = false;
           }
-          __syncwarp();
-          ++js;
-          did = true;
         }
-        if (did) {
-          idle = 0;
-        } else if (++idle > tc::kSpinLimit) {
-          if (lane == 0) tc::report_status(status, 6);
-          alive = false;
-        } else {
-          __nanosleep(20);   // a tight poll would take issue slots from the softmax warp on this scheduler
-        }
+        g += nblk;
+        if (alive) tc::tc_commit(bar(O_FULL));
+        ++req;
       }
-      g += nblk;
-      if (alive && tc::elect_one()) tc::tc_commit(bar(O_FULL));
-      __syncwarp();
-      ++req;
     }
   } else if (warp < 4) {
     // ================================ softmax / epilogue ================================
@@ -367,10 +314,16 @@ mla_tile64_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CU
 #pragma unroll
           for (int i = 0; i < 32; ++i) sv[i] = 0u;
         }
-        tc::mbar_arrive(bar(S_EMPTY0 + st));
         if (tid == 0) FMLA_TRACE_AT(g, 7);
 
         if constexpr (MODE == kDense) {
+          // Rows of the last page beyond the sequence may hold anything (NaN included) and 0 * NaN must not reach O.  Their logits,
+          // which S has been formed with by now, are masked.
+          const int rows_valid = r.seqlen - (r.blk_lo + j) * 64;
+          for (int i = tid; i < (64 - rows_valid) * 64; i += 128) {
+            const int row = rows_valid + (i >> 6), c16 = i & 63;
+            *reinterpret_cast<uint4*>(smem + KV_OFF + st * kTileBytes + (c16 >> 3) * kChunkBytes + row * 128 + (c16 & 7) * 16) = make_uint4(0, 0, 0, 0);
+          }
           const int tok0 = (r.blk_lo + j) * 64 + th * 32;
           if (tok0 + 32 > r.border) vbits = tok0 >= r.border ? 0u : (0xffffffffu >> (32 - (r.border - tok0)));
         }
@@ -405,9 +358,10 @@ mla_tile64_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CU
         }
         m_run = m_new;
         const bool any_need = __any_sync(0xffffffffu, need);
+        auto before_done = [&] { return g == 0 || tc::mbar_wait(bar(KV_EMPTY0 + (st ^ 1)), ((g - 1) >> 1) & 1, status, 9); };     // P V of the block before
         bool pv_done = false;    // the previous P V must be complete before O is rescaled and before P is overwritten
         if (any_need) {
-          if (!tc::mbar_wait(bar(P_EMPTY), (g & 1) ^ 1, status, 9)) *sAbort = 1;
+          if (!before_done()) *sAbort = 1;
           pv_done = true;
           const float m_next = need ? m_new : m_used;
           const float alpha = exp2f(m_used - m_next);
@@ -437,7 +391,7 @@ mla_tile64_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CU
           pk[i] = pack_16x2<F16>(p0, p1);
         }
         l_part += (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
-        if (!pv_done && !tc::mbar_wait(bar(P_EMPTY), (g & 1) ^ 1, status, 9)) *sAbort = 1;
+        if (!pv_done && !before_done()) *sAbort = 1;
         if (tid == 0) FMLA_TRACE_AT(g, 9);
         // P[row][th*32 .. +32) -> K-major 128B-swizzled A operand: 16-byte chunk (th*4 + q) ^ (row & 7)
 #pragma unroll
@@ -445,7 +399,9 @@ mla_tile64_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CU
           st_shared_v4(sP + r_row * 128 + ((((th * 4 + q4) ^ (r_row & 7))) << 4),
                        make_uint4(pk[q4 * 4], pk[q4 * 4 + 1], pk[q4 * 4 + 2], pk[q4 * 4 + 3]));
         tc::fence_proxy_async_smem();
-        tc::mbar_arrive(bar(P_FULL));
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(bar(P_FULL));
         if (tid == 0) FMLA_TRACE_AT(g, 11);
       }
 
@@ -506,7 +462,8 @@ mla_tile64_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CU
       }
       if (nblk > 0) {
         tc::tc_fence_before();
-        tc::mbar_arrive(bar(O_EMPTY));
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(bar(O_EMPTY));
         ++req;
       }
       if (th == 0 && row_ok) {
