@@ -98,39 +98,6 @@ __device__ __forceinline__ void dense_pv_steps(uint32_t tmem_o, uint32_t tmem_p,
   for (int s = kFirst; s < kEnd; ++s)
     tc::mma_ts(tmem_o, tmem_p + s * 8, tc::desc_advance(desc_v, s * 2048), idesc, (first && s == 0) ? 0u : 1u);
 }
-// Place in the ring of K and V blocks: stage, and the parity of the rounds before.
-template <int N>
-struct RingPos {
-  int st;
-  uint32_t ph;
-  __device__ __forceinline__ void step(int n) {
-    st += n;
-    if (st >= N) {
-      st -= N;
-      ph ^= 1u;
-    }
-  }
-};
-
-// Two floats at a time (one instruction each).
-struct F2 {
-  float lo, hi;
-};
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-  F2 d;
-  asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\nfma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}\n"
-      : "=f"(d.lo), "=f"(d.hi)
-      : "f"(a.lo), "f"(a.hi), "f"(b.lo), "f"(b.hi), "f"(c.lo), "f"(c.hi));
-  return d;
-}
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-  F2 d;
-  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}\n"
-      : "=f"(d.lo), "=f"(d.hi)
-      : "f"(a.lo), "f"(a.hi), "f"(b.lo), "f"(b.hi));
-  return d;
-}
-__device__ __forceinline__ F2 f2(float x) { return F2{x, x}; }
 // 2^x for x <= 2^7 on the multiply-add pipe: x = n + f with n the nearest whole number (held in the low bits of x + 1.5 * 2^23) and
 // |f| <= 1/2, and 2^f = 1 + f q(f) with the polynomial of least largest relative error (fitted with Lawson's weights; 1.6e-7 in
 // fp32 over the range, the special function unit's 2^x is specified to 2.4e-7).  Below -127 the result is 0.
@@ -302,7 +269,7 @@ dense_fwd_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_co
     // ================================ TMA producer =====================================
     if (tc::elect_one()) {
       int qc = 0, kc = 0;                  // Q tiles, key blocks so far
-      RingPos<L::kStages> at = {0, 0u};
+      tc::RingPos<L::kStages> at = {0, 0u};
       bool alive = true;
       for (int n = 0; alive; ++n) {
         const int n1 = dense_blocks(p, w, 1), nblk = max(dense_blocks(p, w, 0), n1);
@@ -343,7 +310,7 @@ dense_fwd_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid_co
       const uint64_t desc_k = tc::smem_desc_sw128(sRing, 16, 1024);            // B of S: K-major (stage 0)
       const uint64_t desc_r = tc::smem_desc_sw128(sRest, 16, 1024);            // the same, columns 128 to 191 (slot 0)
       const uint64_t desc_v = tc::smem_desc_sw128(sRing, kChunkBytes, 1024);   // B of PV: MN-major, 64-wide column groups 16 KB apart (stage 0)
-      RingPos<L::kStages> at_k = {0, 0u}, at_v = {1, 0u};
+      tc::RingPos<L::kStages> at_k = {0, 0u}, at_v = {1, 0u};
       int qc = 0, kc = 0, c0 = 0, c1 = 0;      // Q tiles, key blocks, blocks of either tile before this one
       bool alive = true;
       if (kTakeOver) tc::mbar_arrive(bar(TILE_EMPTY));

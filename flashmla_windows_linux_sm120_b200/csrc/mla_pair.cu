@@ -36,8 +36,8 @@
 // 0..5 = [320,512) (32 columns each); element (row r, column c) of an N-wide result
 // (the 64-row half of an M=128 pair instruction) sits in lane r + 64 * (c >= N/2), column c % (N/2).
 //
-// Gathering modes (sparse FP8 decode: 480 threads, sparse prefill: 320 or 352 threads).  Each CTA brings only its 32 token
-// rows of a 64-index block into the K ring -- prefill: three or four warps of 16-byte cp.async copies that arrive on the
+// Gathering modes (sparse FP8 decode: 480 threads, sparse prefill: 352 threads).  Each CTA brings only its 32 token
+// rows of a 64-index block into the K ring -- prefill: four warps of 16-byte cp.async copies that arrive on the
 // landing barrier by hardware; FP8 decode: two groups of four warps that read the 656-byte records into registers,
 // de-quantise them once per pair and store them in the layout TMA would produce.  The V operand (64 tokens x 256
 // columns per CTA) is not read from global memory at all: the thread of warp 6 forwards it out of the landed K rows
@@ -90,11 +90,8 @@ static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB shared memory limit per 
 static_assert(NUM_BARS * 8 <= 256, "barrier area too small");
 constexpr float kRescaleThreshold = 8.0f;
 constexpr int kThreads = 256;
-// Sparse prefill: gather warps 4 and 8, 9, ..  Long calls run at the power limit with any number of them (4096 tokens 2574 us with three,
-// 2579 with four); with cut tokens, of which few units work at a time, four are faster: one token, top-k 2048, 16.7 -> 16.2 us, 37 tokens
-// 35.7 -> 34.9, and in calls of a few rounds three: 333 tokens, top-k 512, 70.1 -> 71.7, 222, top-k 1024, 72.2 -> 73.4.
-__host__ __device__ constexpr int gather_warps(int wm) { return 4; }
-__host__ __device__ constexpr int prefill_threads(int wm) { return (7 + gather_warps(wm)) * 32; }
+constexpr int kGatherWarps = 4;                   // sparse prefill: warps 4 and 8 .. 10, eight rows each
+constexpr int kPrefillThreads = (7 + kGatherWarps) * 32;
 #ifndef FMLA_DECODE_GROUPS
 #define FMLA_DECODE_GROUPS 2
 #endif
@@ -175,7 +172,7 @@ __device__ __forceinline__ void pv_block_pair(uint32_t tmem_o, uint64_t desc_p_s
 // forwarded from those rows (tmap_k32 / tmap_v64 unused); invalid indices leave zero rows and are masked through
 // validity bits.
 template <bool F16, int WM>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WM == kDense ? ptc::kThreads : WM == kSparseDecode ? ptc::kSparseDecodeThreads : ptc::prefill_threads(WM), 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WM == kDense ? ptc::kThreads : WM == kSparseDecode ? ptc::kSparseDecodeThreads : ptc::kPrefillThreads, 1)
 mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUtensorMap tmap_q,
                 const __grid_constant__ CUtensorMap tmap_k32, const __grid_constant__ CUtensorMap tmap_v64) {
   using namespace ptc;
@@ -226,7 +223,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
     // and a K stage has landed when every lane of the gather warps has arrived by hardware, plus the thread that
     // published the validity bits (prefill), or when every gather warp has stored its rows (FP8 decode)
     for (int i = Q_EMPTY; i < NUM_BARS; ++i)
-      tc::mbar_init(bar(i), !SPARSE ? 1 : (i >= K_EMPTY0 && i <= K_EMPTY2) ? 3 : (i >= K_LAND0 && i <= K_LAND2) ? (PREFILL ? gather_warps(WM) * 32 + 1 : 4 /* FP8 decode: the four gather warps of a group */) : 1);
+      tc::mbar_init(bar(i), !SPARSE ? 1 : (i >= K_EMPTY0 && i <= K_EMPTY2) ? 3 : (i >= K_LAND0 && i <= K_LAND2) ? (PREFILL ? kGatherWarps * 32 + 1 : 4 /* FP8 decode: the four gather warps of a group */) : 1);
     tc::fence_mbar_init();
     *sAbort = 0;
     if (misaligned) tc::report_status(status, 30);
@@ -246,13 +243,14 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
     // request is p.b, past the lengths, the indices and num_splits.)
   } else if ((warp == 4 || warp >= 8) && PREFILL) {
     // ================================ Q and K loader, sparse prefill ===================
-    // The CTA's 32 token rows of a block (32 x 1152 bytes) are gathered with 16-byte cp.async copies by three or four warps
-    // (4, 8, 9, ..): 72 warp instructions per block, dealt out round robin, consecutive lanes on consecutive pieces of a row.
-    // Measured with the issuing warp of before: with each warp taking a contiguous third of the instructions 751 TFLOP/s; with
-    // the round-robin deal two warps 452, three 979-1009, four 964-982, five 935-957.  The TMA engine (tile::gather4, 4 rows x 64
-    // columns per copy) gathers no faster than ~11 bytes per clock and SM, and mixing the two paths was slower
-    // than either (8 of the 32 rows by TMA: 545 TFLOP/s; 16: 466), because the gathers queue behind the forwarding
-    // copies in the TMA engine.  Each lane's copies arrive on the landing barrier by hardware (arrive.noinc).
+    // The CTA's 32 token rows of a block (32 x 1152 bytes) are gathered with 16-byte cp.async copies by four warps (4, 8 .. 10), eight
+    // rows each, three copies a row.  What bounds a gather is the instructions in front of each copy: a deal of the 72 warp
+    // instructions of a block over three warps, piece by piece, cost some 30 instructions a copy (a division, a shuffle and a 64-bit
+    // product) and 1 980 clk a block; by rows the addresses follow from one product a row (74 tokens, top-k 512, 18.1 -> 16.7 us, 4096 of
+    // top-k 2048, which run at the power limit, 2 575 -> 2 558).  The TMA engine (tile::gather4, 4 rows x 64
+    // columns per copy) gathers no faster than ~11 bytes per clock and SM (cp.async alone: up to 67), and mixing the two paths was slower
+    // than either, because the gathers queue behind the forwarding copies in the TMA engine.  Each lane's copies arrive on the
+    // landing barrier by hardware (arrive.noinc).
     // Nothing else of the block is read from global memory: the value operand of both CTAs is put together from
     // these rows by shared-memory copies (warp 6), which also loads Q: the gather runs ahead into the next query
     // token while the current one drains.  Warp 4 publishes the validity bits of the 64 indices.  An index outside
@@ -787,14 +785,18 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
           for (int i = 0; i < 32; ++i)
             if (!((vbits >> i) & 1u)) sv[i] = 0xff800000u;
         }
-        float mx4[4] = {neg_inf(), neg_inf(), neg_inf(), neg_inf()};
+        float mx4[4];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sv[i]));
-        float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
+        for (int c = 0; c < 4; ++c) {
+          mx4[c] = fmaxf(__uint_as_float(sv[c * 8]), __uint_as_float(sv[c * 8 + 1]));
+#pragma unroll
+          for (int i = 2; i < 8; i += 2) mx4[c] = max3(mx4[c], __uint_as_float(sv[c * 8 + i]), __uint_as_float(sv[c * 8 + i + 1]));
+        }
+        float mx = fmaxf(max3(mx4[0], mx4[1], mx4[2]), mx4[3]) * scale_log2;
         float* xch = sMx + (j & 1) * 128;
         xch[tid] = mx;
         bar_sync(1, 128);
-        if (*sAbort) { aborted = true; break; }
+        const bool stop = *sAbort != 0;      // (looked at later: nothing here waits for the load)
         if (tid == 0) FMLA_PTRACE_AT(g, 8);
         mx = fmaxf(mx, xch[tid ^ 64]);
         const float m_new = fmaxf(m_run, mx);
@@ -828,16 +830,19 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
           tc::tmem_wait_st();
           tc::tc_fence_before();
         }
-        float rs4[4] = {0.f, 0.f, 0.f, 0.f};
+        F2 sum[2] = {f2(0.f), f2(0.f)};
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const float p0 = exp2f(fmaf(__uint_as_float(sv[2 * i]), scale_log2, -m_used));
-          const float p1 = exp2f(fmaf(__uint_as_float(sv[2 * i + 1]), scale_log2, -m_used));
-          rs4[i & 3] += p0 + p1;
-          pk[i] = pack_16x2<F16>(p0, p1);
+          F2 x = f2_fma(F2{__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])}, f2(scale_log2), f2(-m_used));
+          x.lo = exp2f(x.lo);
+          x.hi = exp2f(x.hi);
+          sum[i & 1] = f2_add(sum[i & 1], x);
+          pk[i] = pack_16x2<F16>(x.lo, x.hi);
         }
-        l_part += (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
+        sum[0] = f2_add(sum[0], sum[1]);
+        l_part += sum[0].lo + sum[0].hi;
+        if (stop) { aborted = true; break; }
         if (!tc::mbar_wait(bar(V_EMPTY0 + st), ((g >> 1) & 1) ^ 1, status, 109)) *sAbort = 1;
         if (tid == 0) FMLA_PTRACE_AT(g, 9);
         // P[row][th*32 .. +32) -> K-major 128B-swizzled A operand: 16-byte chunk (th*4 + q) ^ (row & 7)
@@ -1037,8 +1042,8 @@ cudaError_t launch_sparse_prefill_pair(const SparsePrefillKernelParams& sp, cuda
   if (!tmah::make_map_4d(&tq, sp.q, sp.h_q, sp.s_q, 1, sp.q_stride_h, sp.q_stride_s, sp.q_stride_s * sp.s_q, 64, 1)) return cudaErrorInvalidValue;
   // a kernel of its own for the cut tokens: their fp32 stores cost the other one three registers that it does not have (4096 tokens 2606 -> 2680 us)
   const dim3 grid(2, sp.units, 1);
-  if (sp.per > 1) return launch_pair<mla_pair_kernel<false, kSparsePrefillCut>>(P, tq, tq, tq, grid, ptc::prefill_threads(kSparsePrefillCut), stream);
-  return launch_pair<mla_pair_kernel<false, kSparsePrefill>>(P, tq, tq, tq, grid, ptc::prefill_threads(kSparsePrefill), stream);    // the K / V maps are not used in this mode
+  if (sp.per > 1) return launch_pair<mla_pair_kernel<false, kSparsePrefillCut>>(P, tq, tq, tq, grid, ptc::kPrefillThreads, stream);
+  return launch_pair<mla_pair_kernel<false, kSparsePrefill>>(P, tq, tq, tq, grid, ptc::kPrefillThreads, stream);    // the K / V maps are not used in this mode
 }
 
 // Two 64-row tiles that read the same pages: the halves of 128 heads, or the 64 heads of two consecutive query tokens, which

@@ -95,6 +95,25 @@ __device__ __forceinline__ bool mbar_wait2(uint32_t bar_a, uint32_t par_a, uint3
   return ok;
 }
 
+// Place in a ring of N stages: stage, and the parity of the rounds before.
+template <int N>
+struct RingPos {
+  int st;
+  uint32_t ph;
+  __device__ __forceinline__ void step(int n) {
+    st += n;
+    if (n <= N) {
+      if (st >= N) {
+        st -= N;
+        ph ^= 1u;
+      }
+    } else {
+      ph ^= static_cast<uint32_t>(st / N) & 1u;
+      st %= N;
+    }
+  }
+};
+
 // ---- TMA ------------------------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tensormap(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];\n" ::"l"(tmap) : "memory");
@@ -173,6 +192,17 @@ __device__ __forceinline__ void mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
       "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+__device__ __forceinline__ void mma_ws_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.ws.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, 0;\n}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// shared memory -> tensor memory, 64 rows x 16 bytes per instruction, rows 0..31 into lanes 0..31 and 64..95, rows 32..63 into lanes
+// 32..63 and 96..127: what an M = 64 operand A takes
+__device__ __forceinline__ void tmem_cp_64x128b(uint32_t taddr, uint64_t desc) {
+  asm volatile("tcgen05.cp.cta_group::1.64x128b.warpx2::02_13 [%0], %1;\n" ::"r"(taddr), "l"(desc) : "memory");
 }
 __device__ __forceinline__ void mma_ws_ss(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
