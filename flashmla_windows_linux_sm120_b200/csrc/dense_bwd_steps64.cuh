@@ -31,17 +31,17 @@ struct Layout {
 };
 }  // namespace dbt64
 
-// Zeroes rows [rows_valid, 64) of a streamed tile of NCHUNK 64-column chunks (whole warp).  Rows past
+// Zeroes rows [rows_valid, 64) of a streamed tile of NCHUNK 64-column chunks (the element-wise threads, before they hand over the P
+// or dS that meets these rows).  Rows past
 // the end of a sequence hold the next sequence's data or the TMA zero fill; they meet exact zeros of
-// P / dS in the second GEMMs, and 0 * (Inf or NaN) must not reach the accumulators.
-__device__ __forceinline__ void zero_stage_tail(unsigned char* tile, int nchunk, int rows_valid, int lane) {
+// P / dS in the second GEMMs, and 0 * (Inf or NaN) must not reach the accumulators.  What the first GEMMs make of them is masked.
+__device__ __forceinline__ void zero_stage_tail(unsigned char* tile, int nchunk, int rows_valid, int tid) {
   const int nrows = 64 - rows_valid;
-  for (int i = lane; i < nrows * nchunk * 8; i += 32) {
+  for (int i = tid; i < nrows * nchunk * 8; i += dbt64::kEwWarps * 32) {
     const int row = rows_valid + i / (nchunk * 8), c16 = i % (nchunk * 8);
     *reinterpret_cast<uint4*>(tile + (c16 >> 3) * dbt64::kStgChunk + row * 128 + (c16 & 7) * 16) = make_uint4(0, 0, 0, 0);
   }
   tc::fence_proxy_async_smem();
-  __syncwarp();
 }
 
 // The instructions of a step exist once: ring stage and buffer come in as run-time bases (warp-uniform), to which the
@@ -163,41 +163,35 @@ dense_bwd_dq_tc64_kernel(const __grid_constant__ DenseKernelParams p, const __gr
     const uint64_t desc_v = tc::smem_desc_sw128(sStg + L::kStgA, 16, 1024);           // V tile of stage 0, K-major (B of dP)
     const uint64_t desc_kt = tc::smem_desc_sw128(sStg, kStgChunk, 1024);              // K tile of stage 0, MN-major (B of dQ)
     bool alive = nblk > 0;
-    if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_RES_FULL), 0, status, 52));
-    // Two issuing warps: the first for the first GEMMs of a step (S, dP), the other for the second one (dQ).  Each
-    // wait on an mbarrier costs the issuing warp a few hundred cycles in which the tensor pipe would
-    // otherwise idle; with two warps the waits of one overlap the instructions of the other.
-    if (warp == kEwWarps + 1) {
-      for (int j = 0; j < nblk && alive; ++j) {
-        const int st = j % kStages, bf = j & 1;
-        // the tile has landed, and the S / dP buffer pair bf is free (the element-wise warps have read step
-        // j-2 out of it)
-        alive = tc::mbar_wait2(bar(Q_KV_FULL0 + st), (j / kStages) & 1, bar(Q_DS_FULL0 + bf), ((j >> 1) & 1) ^ 1, status, 54);
-        if (!alive) break;
-        // K rows past the end of the sequence must be exact zeros for dQ += dS K
-        if (lk - j * 64 < 64) zero_stage_tail(smem + L::STG_OFF + st * L::kStage, L::NCH, lk - j * 64, lane);
-        tc::tc_fence_after();
-        if (tc::elect_one()) {
+    // Two issuing threads: the first for the first GEMMs of a step (S, dP), the other for the second one (dQ); the waits of one
+    // overlap the instructions of the other.
+    if (tc::elect_one()) {
+      if (warp == kEwWarps + 1) {
+        if (alive) alive = tc::mbar_wait(bar(Q_RES_FULL), 0, status, 52);
+        for (int j = 0; j < nblk && alive; ++j) {
+          const int st = j % kStages, bf = j & 1;
+          // the tile has landed, and the S / dP buffer pair bf is free (the element-wise warps have read step
+          // j-2 out of it)
+          alive = tc::mbar_wait(bar(Q_KV_FULL0 + st), (j / kStages) & 1, status, 54);
+          if (alive) alive = tc::mbar_wait(bar(Q_DS_FULL0 + bf), ((j >> 1) & 1) ^ 1, status, 54);
+          if (!alive) break;
+          tc::tc_fence_after();
           const uint32_t off = st * L::kStage, col = tmem + TM_SD + bf * 128;
           mma_res_stg64<L::NCH>(col, desc_q, tc::desc_advance(desc_k, off), idesc_sd);
           mma_res_stg64<2>(col + 64, desc_do, tc::desc_advance(desc_v, off), idesc_sd);
           tc::tc_commit(bar(Q_SD_FULL0 + bf));
         }
-        __syncwarp();
-      }
-    } else {
-      for (int j = 0; j < nblk && alive; ++j) {
-        const int st = j % kStages, bf = j & 1;
-        alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_DS_FULL0 + bf), (j >> 1) & 1, status, 53));
-        if (!alive) break;
-        tc::tc_fence_after();
-        if (tc::elect_one()) {
+      } else {
+        for (int j = 0; j < nblk && alive; ++j) {
+          const int st = j % kStages, bf = j & 1;
+          alive = tc::mbar_wait(bar(Q_DS_FULL0 + bf), (j >> 1) & 1, status, 53);
+          if (!alive) break;
+          tc::tc_fence_after();
           mma_tmem_stg64(tmem + TM_DQ, tmem + TM_DS + bf * 32, tc::desc_advance(desc_kt, st * L::kStage), idesc_dq, j == 0);
           tc::tc_commit(bar(Q_KV_EMPTY0 + st));
           tc::tc_commit(bar(Q_BUF_FREE0 + bf));
           if (j == nblk - 1) tc::tc_commit(bar(Q_DONE));
         }
-        __syncwarp();
       }
     }
   } else {
@@ -228,14 +222,14 @@ dense_bwd_dq_tc64_kernel(const __grid_constant__ DenseKernelParams p, const __gr
       tc::tmem_wait_ld();
       const int cnt = limit - j * 64 - half * 32;              // visible keys of this half block: [0, cnt)
       const bool all_visible = __all_sync(0xffffffffu, cnt >= 32);
+      row_exp2(sv, p.scale_log2, [&](int) { return f2(-lse2); });
       // two loops, not a test per element: the compiler makes a branch of each test (40 clk per element measured)
       auto to_ds = [&](auto masked) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const float p0 = exp2f(fmaf(__uint_as_float(sv[2 * i]), p.scale_log2, -lse2));
-          const float p1 = exp2f(fmaf(__uint_as_float(sv[2 * i + 1]), p.scale_log2, -lse2));
-          float d0 = p0 * (__uint_as_float(dp[2 * i]) - dl);
-          float d1 = p1 * (__uint_as_float(dp[2 * i + 1]) - dl);
+          const F2 d = f2_mul(F2{__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])},
+                              f2_add(F2{__uint_as_float(dp[2 * i]), __uint_as_float(dp[2 * i + 1])}, f2(-dl)));
+          float d0 = d.lo, d1 = d.hi;
           if constexpr (decltype(masked)::value) {             // a select, not a product: masked entries may hold Inf or NaN
             d0 = 2 * i < cnt ? d0 : 0.f;
             d1 = 2 * i + 1 < cnt ? d1 : 0.f;
@@ -245,6 +239,8 @@ dense_bwd_dq_tc64_kernel(const __grid_constant__ DenseKernelParams p, const __gr
       };
       if (all_visible) to_ds(std::false_type{});
       else to_ds(std::true_type{});
+      // K rows past the end of the sequence must be exact zeros for dQ += dS K
+      if (lk - j * 64 < 64) zero_stage_tail(smem + L::STG_OFF + j % kStages * L::kStage, L::NCH, lk - j * 64, tid);
       tc::tmem_st16(tmem + lane_addr + TM_DS + st * 32 + half * 16, pk);
       tc::tmem_wait_st();
       tc::tc_fence_before();
@@ -368,60 +364,39 @@ dense_bwd_dkdv_tc64_kernel(const __grid_constant__ DenseKernelParams p, const __
     const uint64_t desc_do = tc::smem_desc_sw128(sStg + L::kStgA, 16, 1024);          // dO tile of stage 0, K-major (B of dP^T)
     const uint64_t desc_qt = tc::smem_desc_sw128(sStg, kStgChunk, 1024);              // Q tile, MN-major (B of dK)
     const uint64_t desc_dot = tc::smem_desc_sw128(sStg + L::kStgA, kStgChunk, 1024);  // dO tile, MN-major (B of dV)
-    bool alive = nstep > 0;
-    if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(K_RES_FULL), 0, status, 62));
-    // waits (whole warp) for phase `ph` of barrier `i`
-    auto wait = [&](int i, int ph, int code) {
-      if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(i), ph, status, code));
-      return alive;
-    };
-    // S^T of step j, once its tile has landed and S^T of step j-1 has been read; rows past the end of the sequence
-    // are cleared first
-    auto issue_st = [&](int j) {
-      const int st = j % kStages;
-      if (!wait(K_QD_FULL0 + st, (j / kStages) & 1, 63)) return;
-      const int rows_valid = lq - (jb_lo + j) * 64;
-      if (rows_valid < 64) zero_stage_tail(smem + L::STG_OFF + st * L::kStage, L::NCH + 2, rows_valid, lane);
-      if (!wait(K_S_READ, (j & 1) ^ 1, 64)) return;
-      tc::tc_fence_after();
-      if (tc::elect_one()) {
-        mma_res_stg64<L::NCH>(tmem + TM_ST, desc_k, tc::desc_advance(desc_q, st * L::kStage), idesc_sd);
-        tc::tc_commit(bar(K_S_FULL));
+    if (tc::elect_one() && nstep > 0) {
+      bool alive = tc::mbar_wait(bar(K_RES_FULL), 0, status, 62);
+      auto wait = [&](int i, int ph, int code) {
+        if (alive) alive = tc::mbar_wait(bar(i), ph, status, code);
+        return alive;
+      };
+      // step j = -1 issues the first GEMMs of step 0 (the instructions of a step exist once)
+      for (int j = -1; j < nstep && alive; ++j) {
+        if (j + 1 < nstep) {                           // S^T and dP^T of the next step, once those of this one have been read
+          const int st = (j + 1) % kStages;
+          if (!wait(K_QD_FULL0 + st, ((j + 1) / kStages) & 1, 63)) break;
+          if (!wait(K_S_READ, j & 1, 64)) break;
+          tc::tc_fence_after();
+          mma_res_stg64<L::NCH>(tmem + TM_ST, desc_k, tc::desc_advance(desc_q, st * L::kStage), idesc_sd);
+          tc::tc_commit(bar(K_S_FULL));
+          if (!wait(K_DP_READ, j & 1, 67)) break;
+          tc::tc_fence_after();
+          mma_res_stg64<2>(tmem + TM_DPT, desc_v, tc::desc_advance(desc_do, st * L::kStage), idesc_sd);
+          tc::tc_commit(bar(K_DP_FULL));
+        }
+        if (j >= 0) {
+          const int st = j % kStages;
+          if (!wait(K_P_FULL, j & 1, 68)) break;
+          tc::tc_fence_after();
+          mma_tmem_stg64(tmem + TM_DV, tmem + TM_P, tc::desc_advance(desc_dot, st * L::kStage), idesc_dv, j == 0);
+          tc::tc_commit(bar(K_P_FREE));
+          if (!wait(K_DS_FULL, j & 1, 69)) break;
+          tc::tc_fence_after();
+          mma_tmem_stg64(tmem + TM_DK, tmem + TM_DS, tc::desc_advance(desc_qt, st * L::kStage), idesc_dk, j == 0);
+          tc::tc_commit(bar(K_DS_FREE));               // completes after dV of this step: the tensor pipe runs in order
+          tc::tc_commit(bar(K_QD_EMPTY0 + st));
+        }
       }
-      __syncwarp();
-    };
-    auto issue_dpt = [&](int j) {
-      if (!wait(K_DP_READ, (j & 1) ^ 1, 67)) return;
-      tc::tc_fence_after();
-      if (tc::elect_one()) {
-        mma_res_stg64<2>(tmem + TM_DPT, desc_v, tc::desc_advance(desc_do, (j % kStages) * L::kStage), idesc_sd);
-        tc::tc_commit(bar(K_DP_FULL));
-      }
-      __syncwarp();
-    };
-    if (alive) issue_st(0);
-    if (alive) issue_dpt(0);
-    for (int j = 0; j < nstep && alive; ++j) {
-      const int st = j % kStages;
-      if (j + 1 < nstep) {
-        issue_st(j + 1);
-        issue_dpt(j + 1);
-      }
-      if (!wait(K_P_FULL, j & 1, 68)) break;
-      tc::tc_fence_after();
-      if (tc::elect_one()) {
-        mma_tmem_stg64(tmem + TM_DV, tmem + TM_P, tc::desc_advance(desc_dot, st * L::kStage), idesc_dv, j == 0);
-        tc::tc_commit(bar(K_P_FREE));
-      }
-      __syncwarp();
-      if (!wait(K_DS_FULL, j & 1, 69)) break;
-      tc::tc_fence_after();
-      if (tc::elect_one()) {
-        mma_tmem_stg64(tmem + TM_DK, tmem + TM_DS, tc::desc_advance(desc_qt, st * L::kStage), idesc_dk, j == 0);
-        tc::tc_commit(bar(K_DS_FREE));             // completes after dV of this step: the tensor pipe runs in order
-        tc::tc_commit(bar(K_QD_EMPTY0 + st));
-      }
-      __syncwarp();
     }
   } else {
     // ================================ element-wise / epilogue ==========================
@@ -430,19 +405,20 @@ dense_bwd_dkdv_tc64_kernel(const __grid_constant__ DenseKernelParams p, const __
     const int key = n_base + rl;
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int shift = lk - lq;                                 // query i sees keys <= i + shift
-    // per-query vectors of a step: lse * log2(e) (threads 0-63) and delta (threads 64-127); each value is loaded one
-    // step ahead, so that no step waits for global memory
+    // per-query vectors of a step: -lse * log2(e) (threads 0-63) and -delta (threads 64-127); each value is loaded one
+    // step ahead and not touched before the next, so that no step waits for global memory
+    const float* vec = tid < 64 ? p.lse + (int64_t)q0 * p.lse_stride_t + head * p.lse_stride_h : p.delta + (int64_t)head * p.total_q + q0;
+    const int64_t vec_stride = tid < 64 ? p.lse_stride_t : 1;
+    const float vec_mul = tid < 64 ? -kLog2e : -1.f;
     auto load_vec = [&](int j) {
       const int i = (jb_lo + j) * 64 + (tid & 63);
-      if (tid >= 128 || i >= lq) return 0.f;
-      return tid < 64 ? __ldg(p.lse + (int64_t)(q0 + i) * p.lse_stride_t + head * p.lse_stride_h) * kLog2e
-                      : __ldg(p.delta + (int64_t)head * p.total_q + q0 + i);
+      return tid < 128 && i < lq ? __ldg(vec + i * vec_stride) : 0.f;
     };
     float v_next = nstep > 0 ? load_vec(0) : 0.f;
     bool alive = true;
     for (int j = 0; j < nstep && alive; ++j) {
       const int jb = jb_lo + j, vb = j & 1;
-      if (tid < 128) sVec[vb * 128 + tid] = v_next;
+      if (tid < 128) sVec[vb * 128 + tid] = v_next * vec_mul;
       if (j + 1 < nstep) v_next = load_vec(j + 1);
       if (!tc::mbar_wait(bar(K_S_FULL), j & 1, status, 65)) *sAbort = 1;
       bar_sync(1, kEwWarps * 32);                              // vectors visible; also keeps the two buffers of sVec apart
@@ -459,26 +435,26 @@ dense_bwd_dkdv_tc64_kernel(const __grid_constant__ DenseKernelParams p, const __
       const bool all_visible = __all_sync(0xffffffffu, c_min <= 0 && c_max >= 32);
       const float4* vl = reinterpret_cast<const float4*>(sVec + vb * 128 + half * 32);
       const float4* vd = reinterpret_cast<const float4*>(sVec + vb * 128 + 64 + half * 32);
+      row_exp2(sv, p.scale_log2, [&](int i) {
+        const float4 l4 = vl[i >> 1];
+        return i & 1 ? F2{l4.z, l4.w} : F2{l4.x, l4.y};
+      });
       auto to_p = [&](auto masked) {
 #pragma unroll
-        for (int i4 = 0; i4 < 8; ++i4) {
-          const float4 l4 = vl[i4];
-          const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int col = i4 * 4 + e;
-            float pe = exp2f(fmaf(__uint_as_float(sv[col]), p.scale_log2, -ls[e]));
-            if constexpr (decltype(masked)::value) pe = col >= c_min && col < c_max ? pe : 0.f;      // a select: see the dQ kernel
-            sv[col] = __float_as_uint(pe);
+        for (int i = 0; i < 16; ++i) {
+          if constexpr (decltype(masked)::value) {             // a select: see the dQ kernel
+            if (!(2 * i >= c_min && 2 * i < c_max)) sv[2 * i] = 0u;
+            if (!(2 * i + 1 >= c_min && 2 * i + 1 < c_max)) sv[2 * i + 1] = 0u;
           }
-          pk[i4 * 2] = pack_bf16x2(__uint_as_float(sv[i4 * 4]), __uint_as_float(sv[i4 * 4 + 1]));
-          pk[i4 * 2 + 1] = pack_bf16x2(__uint_as_float(sv[i4 * 4 + 2]), __uint_as_float(sv[i4 * 4 + 3]));
+          pk[i] = pack_bf16x2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1]));
         }
       };
       if (all_visible) to_p(std::false_type{});
       else to_p(std::true_type{});
       // a wait that gives up here lets the step run on; the flag ends the loop at the next barrier
       if (!tc::mbar_wait(bar(K_P_FREE), (j & 1) ^ 1, status, 70)) *sAbort = 1;       // dV of step j-1 has read P^T
+      // the last step: rows past the end of the sequence must be exact zeros for dV and dK
+      if (lq - jb * 64 < 64) zero_stage_tail(smem + L::STG_OFF + j % kStages * L::kStage, L::NCH + 2, lq - jb * 64, tid);
       tc::tc_fence_after();
       __syncwarp();
       tc::tmem_st16(tmem + lane_addr + TM_P + half * 16, pk);
@@ -498,16 +474,18 @@ dense_bwd_dkdv_tc64_kernel(const __grid_constant__ DenseKernelParams p, const __
 #pragma unroll
         for (int i4 = 0; i4 < 8; ++i4) {
           const float4 d4 = vd[i4];
-          const float ds[4] = {d4.x, d4.y, d4.z, d4.w};
-          float dv[4];
+          const F2 minus_d[2] = {{d4.x, d4.y}, {d4.z, d4.w}};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int col = i4 * 4 + e;
-            dv[e] = __uint_as_float(sv[col]) * (__uint_as_float(dp[col]) - ds[e]);
-            if constexpr (decltype(masked)::value) dv[e] = col >= c_min && col < c_max ? dv[e] : 0.f;
+          for (int e = 0; e < 2; ++e) {
+            const int col = i4 * 4 + e * 2;
+            F2 dv = f2_mul(F2{__uint_as_float(sv[col]), __uint_as_float(sv[col + 1])},
+                           f2_add(F2{__uint_as_float(dp[col]), __uint_as_float(dp[col + 1])}, minus_d[e]));
+            if constexpr (decltype(masked)::value) {
+              dv.lo = col >= c_min && col < c_max ? dv.lo : 0.f;
+              dv.hi = col + 1 >= c_min && col + 1 < c_max ? dv.hi : 0.f;
+            }
+            pk[i4 * 2 + e] = pack_bf16x2(dv.lo, dv.hi);
           }
-          pk[i4 * 2] = pack_bf16x2(dv[0], dv[1]);
-          pk[i4 * 2 + 1] = pack_bf16x2(dv[2], dv[3]);
         }
       };
       if (all_visible) to_ds(std::false_type{});

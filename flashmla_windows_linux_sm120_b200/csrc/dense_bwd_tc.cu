@@ -23,6 +23,12 @@
 // N = 128.  Hence steps of 128 streamed rows, which also halve the waits, barriers and TMEM round trips per row.  Against
 // steps of 64 (8 sequences of 1 k to 8 k tokens, 128 heads, 192/128, causal, under the power cap at 1.65 to 1.7 GHz): dK/dV and
 // dQ together 32.6 -> 29.5 ms, forward and backward 41.9 -> 39.3 ms.
+// The GEMMs are issued by single threads (waits, votes and branches of whole warps left the tensor pipe idle), the element-wise
+// warps clear what lies past the end of a sequence, and the second GEMM on the wide tile goes chunk by chunk of its columns, each
+// followed by the load of that chunk for the step after next: with one release for the whole tile the next loads came 500 clk late at
+// 192/128.  A step of dK/dV at 192/128 took 3 900 clk and takes 3 480; the element-wise warps (1 300 clk for P, 650 for dS) now set the
+// pace.  Sixteen of them, with half the columns each, were no faster.  4 x 1 000 tokens, 8 heads, 192/128, causal (steps of 64) 72.0 ->
+// 64.2 us, 6 x 1 000, 8 heads, 128/128, no mask 121.8 -> 109.4, 2 x 4 096, 32 heads, no mask 1 916 -> 1 863.
 // Every mbarrier wait is bounded (tc_common.cuh); a pipeline fault sets a status word and lets the
 // CTA drain and free its tensor memory.
 #include "kernels.h"
@@ -36,6 +42,7 @@ namespace fmla {
 
 namespace dbt {
 constexpr int kChunk = 128 * 128;                 // every tile: [128 rows x 64 bf16] chunks, 128-byte swizzled rows
+constexpr int kMaxChunks = 3;
 constexpr int kEwWarps = 8;                       // element-wise warps (two per 32 accumulator rows)
 constexpr int kDqThreads = (kEwWarps + 3) * 32;   // + TMA + two MMA issuers
 constexpr int kDkvThreads = (kEwWarps + 2) * 32;  // + TMA + MMA issuer
@@ -107,35 +114,39 @@ __global__ void __launch_bounds__(256) dense_bwd_delta_tc_kernel(const __grid_co
 // 16-row steps that the valid rows of a streamed tile reach: what lies beyond is neither multiplied nor accumulated
 __device__ __forceinline__ int k_steps(int rows_valid) { return (min(rows_valid, 128) + 15) >> 4; }
 
-// Zeroes the rows from rows_valid to the end of its 16-row step in a streamed tile of NCHUNK 64-column chunks (whole warp).
+// Zeroes the rows from rows_valid to the end of its 16-row step in a streamed tile of NCHUNK 64-column chunks (the element-wise
+// threads, before they hand over the P or dS that meets these rows).
 // Rows past the end of a sequence hold the next sequence's data or the TMA zero fill; they meet exact zeros of
-// P / dS in the second GEMMs, and 0 * (Inf or NaN) must not reach the accumulators.
-__device__ __forceinline__ void zero_tail(unsigned char* tile, int nchunk, int rows_valid, int lane) {
+// P / dS in the second GEMMs, and 0 * (Inf or NaN) must not reach the accumulators.  What the first GEMMs make of them is masked.
+__device__ __forceinline__ void zero_tail(unsigned char* tile, int nchunk, int rows_valid, int tid) {
   const int nrows = k_steps(rows_valid) * 16 - rows_valid;
-  for (int i = lane; i < nrows * nchunk * 8; i += 32) {
+  for (int i = tid; i < nrows * nchunk * 8; i += dbt::kEwWarps * 32) {
     const int row = rows_valid + i / (nchunk * 8), c16 = i % (nchunk * 8);
     *reinterpret_cast<uint4*>(tile + (c16 >> 3) * dbt::kChunk + row * 128 + (c16 & 7) * 16) = make_uint4(0, 0, 0, 0);
   }
   tc::fence_proxy_async_smem();
-  __syncwarp();
 }
 
 // The instructions of a step exist once: ring stage and buffer come in as run-time bases (warp-uniform), to which the
 // unrolled code adds immediates.  With one unrolled copy per (stage, buffer) each copy came around once in three to six
 // steps and its first MMA waited for the instruction fetch.
-// D[128 x N] (TMEM column d_tmem) = A[128 x 64*NCH] (resident, K-major) * B[N x 64*NCH]^T (streamed, K-major), N in idesc
-template <int NCH>
-__device__ __forceinline__ void mma_res_stg(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
+// D[128 x N] (TMEM column d_tmem) = A[128 x 64*NCH] (resident, K-major) * B[N x 64*NCH]^T (streamed, K-major), N in idesc;
+// landed(c) waits for chunk c of B
+template <int NCH, class Landed>
+__device__ __forceinline__ bool mma_res_stg(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, Landed landed) {
 #pragma unroll
-  for (int c = 0; c < NCH; ++c)
+  for (int c = 0; c < NCH; ++c) {
+    if (!landed(c)) return false;
 #pragma unroll
     for (int s = 0; s < 4; ++s)
       tc::mma_ss(d_tmem, tc::desc_advance(desc_a, c * dbt::kChunk + s * 32), tc::desc_advance(desc_b, c * dbt::kChunk + s * 32), idesc,
                  (c | s) ? 1u : 0u);
+  }
+  return true;
 }
 // D[128 x N] += A[128 x 16*ks] (bf16 in TMEM, 8 columns per 16-row step) * B[16*ks x N] (streamed tile read MN-major)
 __device__ __forceinline__ void mma_tmem_stg(uint32_t d_tmem, uint32_t a_tmem, uint64_t desc_b, uint32_t idesc, bool first, int ks) {
-  if (ks == 8) {
+  if (__builtin_expect(ks == 8, 1)) {
 #pragma unroll
     for (int s = 0; s < 8; ++s) tc::mma_ts(d_tmem, a_tmem + s * 8, tc::desc_advance(desc_b, s * 2048), idesc, (first && s == 0) ? 0u : 1u);
   } else {
@@ -147,6 +158,24 @@ __device__ __forceinline__ void mma_tmem_stg(uint32_t d_tmem, uint32_t a_tmem, u
 __device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t (&v)[64]) {
   tc::tmem_ld32(taddr, reinterpret_cast<uint32_t (&)[32]>(v[0]));
   tc::tmem_ld32(taddr + 32, reinterpret_cast<uint32_t (&)[32]>(v[32]));
+}
+
+// P = 2^(s * scale - lse) of 32 or 64 logits in place; minus_lse(i) is -lse of elements 2i and 2i + 1.  One pair in three on the multiply-add
+// pipe: the special function unit alone takes 1 024 clk for a step, as long as the products that it has to keep up with.
+template <int N, class MinusLse>
+__device__ __forceinline__ void row_exp2(uint32_t (&sv)[N], float scale, MinusLse minus_lse) {
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    F2 x = f2_fma(F2{__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])}, f2(scale), minus_lse(i));
+    if (i % 16 % 3 == 2) {      // (alike in steps of either length)
+      x = f2_exp2_nan(x);
+    } else {
+      x.lo = exp2f(x.lo);
+      x.hi = exp2f(x.hi);
+    }
+    sv[2 * i] = __float_as_uint(x.lo);
+    sv[2 * i + 1] = __float_as_uint(x.hi);
+  }
 }
 
 // 32 fp32 columns of an accumulator row -> bf16, times `mul`, as full 32-byte sectors (zeros when nothing was computed)
@@ -178,7 +207,9 @@ __device__ __forceinline__ void store_grad_chunk(uint32_t taddr, bool have, bool
 // The element-wise warps take S and dP into registers, which frees those columns for the next step: S(j+1) and dP(j+1) run
 // beside the element-wise work of step j, dQ(j) beside that of step j+1.
 namespace dbt {
-enum BarQ { Q_RES_FULL = 0, Q_K_FULL0, Q_K_FULL1, Q_K_EMPTY0, Q_K_EMPTY1, Q_V_FULL0, Q_V_FULL1, Q_V_EMPTY0, Q_V_EMPTY1, Q_S_FULL, Q_DP_FULL, Q_DS_FREE,
+// dP of a step and the release of its V, dQ of a chunk of columns and the release of that chunk of K (the last one: and of dS), are one
+// event each, with two barriers in turn
+enum BarQ { Q_RES_FULL = 0, Q_K_FULL0, Q_DQ_DONE0 = Q_K_FULL0 + 2 * kMaxChunks, Q_V_FULL0 = Q_DQ_DONE0 + 2 * kMaxChunks, Q_V_FULL1, Q_DP_FULL0, Q_DP_FULL1, Q_S_FULL,
             Q_S_READ, Q_DP_READ, Q_DS_FULL, Q_NUM_BARS };   // Q_S_READ and later: one arrival per element-wise warp
 }
 
@@ -219,12 +250,13 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
     nblk = last_key < 0 ? 0 : min(nblk, (last_key >> 7) + 1);
   }
 
-  auto load_k = [&](int j) {
-    const uint32_t full = bar(Q_K_FULL0 + (j & 1));
+  // chunk c of the K tile of step j, and dQ of its columns: the barriers
+  auto k_full = [&](int j, int c) { return bar(Q_K_FULL0 + (j & 1) * kMaxChunks + c); };
+  auto dq_done = [&](int j, int c) { return bar(Q_DQ_DONE0 + (j & 1) * kMaxChunks + c); };
+  auto load_k = [&](int j, int c) {
     DBT_TRACE_AT(j, 0);
-    tc::mbar_arrive_expect_tx(full, L::kWide);
-#pragma unroll
-    for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(sK + (j & 1) * L::kWide + c * kChunk, &tmap_k, c * 64, head, k0 + j * 128, full);
+    tc::mbar_arrive_expect_tx(k_full(j, c), kChunk);
+    tc::tma_load_3d(sK + (j & 1) * L::kWide + c * kChunk, &tmap_k, c * 64, head, k0 + j * 128, k_full(j, c));
   };
   auto load_v = [&](int j) {
     const int st = j % L::kNarrowStages;
@@ -243,7 +275,8 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
         tc::mbar_arrive_expect_tx(bar(Q_RES_FULL), L::kWide + L::kNarrow);
 #pragma unroll
         for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(sQ + c * kChunk, &tmap_q, c * 64, head, q0 + m_base, bar(Q_RES_FULL));
-        load_k(0);
+#pragma unroll
+        for (int c = 0; c < L::NCH; ++c) load_k(0, c);
 #pragma unroll
         for (int c = 0; c < 2; ++c) tc::tma_load_3d(sDO + c * kChunk, &tmap_do, c * 64, head, q0 + m_base, bar(Q_RES_FULL));
         load_v(0);
@@ -264,67 +297,66 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
     if (tc::elect_one()) {
       bool alive = true;
       for (int j = 1; j < nblk && alive; ++j) {
-        alive = tc::mbar_wait(bar(Q_K_EMPTY0 + (j & 1)), ((j >> 1) & 1) ^ 1, status, 51);
+#pragma unroll 1
+        for (int c = 0; c < L::NCH && alive; ++c) {
+          alive = tc::mbar_wait(dq_done(j, c), ((j >> 1) & 1) ^ 1, status, 51);
+          if (alive) load_k(j, c);
+        }
         if (!alive) break;
-        load_k(j);
-        alive = tc::mbar_wait(bar(Q_V_EMPTY0 + j % L::kNarrowStages), ((j / L::kNarrowStages) & 1) ^ 1, status, 57);
+        const int before = j - L::kNarrowStages;                 // the step whose V the stage holds
+        if (before >= 0) alive = tc::mbar_wait(bar(Q_DP_FULL0 + (before & 1)), (before >> 1) & 1, status, 57);
         if (alive) load_v(j);
       }
     }
   } else if (warp > kEwWarps) {
     // ================================ MMA issuers =======================================
-    constexpr uint32_t idesc_dq = tc::idesc_bf16_f32(128, D_QK, 0, 1);
+    constexpr uint32_t idesc_dq = tc::idesc_bf16_f32(128, 64, 0, 1);
     const uint64_t desc_q = tc::smem_desc_sw128(sQ, 16, 1024);
     const uint64_t desc_do = tc::smem_desc_sw128(sDO, 16, 1024);
     const uint64_t desc_k = tc::smem_desc_sw128(sK, 16, 1024);              // K tile of stage 0, K-major (B of S)
     const uint64_t desc_v = tc::smem_desc_sw128(sV, 16, 1024);              // V tile of stage 0, K-major (B of dP)
     const uint64_t desc_kt = tc::smem_desc_sw128(sK, kChunk, 1024);         // K tile of stage 0, MN-major (B of dQ)
     bool alive = nblk > 0;
-    // Two issuing warps: the first for the first GEMMs of a step (S, dP), the other for the second one (dQ).  Each
-    // wait on an mbarrier costs the issuing warp a few hundred cycles in which the tensor pipe would
-    // otherwise idle; with two warps the waits of one overlap the instructions of the other.
-    if (warp == kEwWarps + 1) {
-      if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_RES_FULL), 0, status, 52));
-      for (int j = 0; j < nblk && alive; ++j) {
-        const int st = j & 1, stv = j % L::kNarrowStages;
-        const uint32_t idesc_sd = tc::idesc_bf16_f32(128, k_steps(lk - j * 128) * 16, 0, 0);
-        // K has landed, and the element-wise warps have read S of step j-1
-        alive = tc::mbar_wait2(bar(Q_K_FULL0 + st), (j >> 1) & 1, bar(Q_S_READ), (j & 1) ^ 1, status, 54);
-        if (!alive) break;
-        // K rows past the end of the sequence must be exact zeros for dQ += dS K
-        if (lk - j * 128 < 128) zero_tail(smem + L::WIDE_OFF + st * L::kWide, L::NCH, lk - j * 128, lane);
-        tc::tc_fence_after();
-        if (lane == 0) DBT_TRACE_AT(j, 2);
-        if (tc::elect_one()) {
-          mma_res_stg<L::NCH>(tmem + TM_S, desc_q, tc::desc_advance(desc_k, st * L::kWide), idesc_sd);
+    // Two issuing threads: the first for the first GEMMs of a step (S, dP), the other for the second one (dQ); the waits of one
+    // overlap the instructions of the other.
+    if (tc::elect_one()) {
+      if (warp == kEwWarps + 1) {
+        if (alive) alive = tc::mbar_wait(bar(Q_RES_FULL), 0, status, 52);
+        for (int j = 0; j < nblk && alive; ++j) {
+          const int st = j & 1, stv = j % L::kNarrowStages;
+          const uint32_t idesc_sd = tc::idesc_bf16_f32(128, k_steps(lk - j * 128) * 16, 0, 0);
+          alive = tc::mbar_wait(bar(Q_S_READ), (j & 1) ^ 1, status, 54);      // the element-wise warps have read S of step j-1
+          if (!alive) break;
+          DBT_TRACE_AT(j, 2);
+          alive = mma_res_stg<L::NCH>(tmem + TM_S, desc_q, tc::desc_advance(desc_k, st * L::kWide), idesc_sd, [&](int c) {
+            const bool ok = tc::mbar_wait(k_full(j, c), (j >> 1) & 1, status, 54);
+            tc::tc_fence_after();
+            return ok;
+          });
+          if (!alive) break;
           tc::tc_commit(bar(Q_S_FULL));
+          alive = tc::mbar_wait(bar(Q_V_FULL0 + stv), (j / L::kNarrowStages) & 1, status, 58);
+          if (alive) alive = tc::mbar_wait(bar(Q_DP_READ), (j & 1) ^ 1, status, 58);
+          if (!alive) break;
+          tc::tc_fence_after();
+          DBT_TRACE_AT(j, 3);
+          mma_res_stg<2>(tmem + TM_DP, desc_do, tc::desc_advance(desc_v, stv * L::kNarrow), idesc_sd, [](int) { return true; });
+          tc::tc_commit(bar(Q_DP_FULL0 + (j & 1)));
         }
-        __syncwarp();
-        alive = tc::mbar_wait2(bar(Q_V_FULL0 + stv), (j / L::kNarrowStages) & 1, bar(Q_DP_READ), (j & 1) ^ 1, status, 58);
-        if (!alive) break;
-        tc::tc_fence_after();
-        if (lane == 0) DBT_TRACE_AT(j, 3);
-        if (tc::elect_one()) {
-          mma_res_stg<2>(tmem + TM_DP, desc_do, tc::desc_advance(desc_v, stv * L::kNarrow), idesc_sd);
-          tc::tc_commit(bar(Q_DP_FULL));
-          tc::tc_commit(bar(Q_V_EMPTY0 + stv));
-        }
-        __syncwarp();
-      }
-    } else {
-      for (int j = 0; j < nblk && alive; ++j) {
-        const int st = j & 1;
-        alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_DS_FULL), j & 1, status, 53));
-        if (!alive) break;
-        tc::tc_fence_after();
-        if (lane == 0) DBT_TRACE_AT(j, 4);
-        if (tc::elect_one()) {
-          mma_tmem_stg(tmem + TM_DQ, tmem + TM_DS, tc::desc_advance(desc_kt, st * L::kWide), idesc_dq, j == 0, k_steps(lk - j * 128));
-          tc::tc_commit(bar(Q_K_EMPTY0 + st));
-          tc::tc_commit(bar(Q_DS_FREE));
+      } else {
+        for (int j = 0; j < nblk && alive; ++j) {
+          const int st = j & 1;
+          alive = tc::mbar_wait(bar(Q_DS_FULL), j & 1, status, 53);
+          if (!alive) break;
+          tc::tc_fence_after();
+          DBT_TRACE_AT(j, 4);
+#pragma unroll
+          for (int c = 0; c < L::NCH; ++c) {
+            mma_tmem_stg(tmem + TM_DQ + c * 64, tmem + TM_DS, tc::desc_advance(desc_kt, st * L::kWide + c * kChunk), idesc_dq, j == 0, k_steps(lk - j * 128));
+            tc::tc_commit(dq_done(j, c));
+          }
           DBT_TRACE_AT(j, 5);
         }
-        __syncwarp();
       }
     }
   } else {
@@ -353,10 +385,9 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
       if (tid == 0) DBT_TRACE_AT(j, 7);
       const int cnt = limit - j * 128 - half * 64;             // visible keys of this half block: [0, cnt)
       const bool all_visible = __all_sync(0xffffffffu, cnt >= 64);
-#pragma unroll
-      for (int i = 0; i < 64; ++i) sv[i] = __float_as_uint(exp2f(fmaf(__uint_as_float(sv[i]), p.scale_log2, -lse2)));
+      row_exp2(sv, p.scale_log2, [&](int) { return f2(-lse2); });
       if (tid == 0) DBT_TRACE_AT(j, 8);
-      alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_DP_FULL), j & 1, status, 59));
+      alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_DP_FULL0 + (j & 1)), (j >> 1) & 1, status, 59));
       if (!alive) break;
       tc::tc_fence_after();
       tmem_ld64(tmem + lane_addr + TM_DP + half * 64, dp);
@@ -369,8 +400,9 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
       auto to_ds = [&](auto masked) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          float d0 = __uint_as_float(sv[2 * i]) * (__uint_as_float(dp[2 * i]) - dl);
-          float d1 = __uint_as_float(sv[2 * i + 1]) * (__uint_as_float(dp[2 * i + 1]) - dl);
+          const F2 d = f2_mul(F2{__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])},
+                              f2_add(F2{__uint_as_float(dp[2 * i]), __uint_as_float(dp[2 * i + 1])}, f2(-dl)));
+          float d0 = d.lo, d1 = d.hi;
           if constexpr (decltype(masked)::value) {             // a select, not a product: masked entries may hold Inf or NaN
             d0 = 2 * i < cnt ? d0 : 0.f;
             d1 = 2 * i + 1 < cnt ? d1 : 0.f;
@@ -382,8 +414,10 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
       else to_ds(std::true_type{});
       if (tid == 0) DBT_TRACE_AT(j, 10);
       // dQ of step j-1 has read dS
-      alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_DS_FREE), (j & 1) ^ 1, status, 60));
+      if (j > 0) alive = __all_sync(0xffffffffu, tc::mbar_wait(dq_done(j - 1, L::NCH - 1), ((j - 1) >> 1) & 1, status, 60));
       if (!alive) break;
+      // K rows past the end of the sequence must be exact zeros for dQ += dS K
+      if (lk - j * 128 < 128) zero_tail(smem + L::WIDE_OFF + (j & 1) * L::kWide, L::NCH, lk - j * 128, tid);
       tc::tc_fence_after();
       tc::tmem_st32(tmem + lane_addr + TM_DS + half * 32, pk);
       tc::tmem_wait_st();
@@ -394,7 +428,7 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
     }
     bool have = nblk > 0 && alive;
     if (have) {
-      have = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_DS_FREE), (nblk - 1) & 1, status, 56));    // the last dQ, hence all of them
+      have = __all_sync(0xffffffffu, tc::mbar_wait(dq_done(nblk - 1, L::NCH - 1), ((nblk - 1) >> 1) & 1, status, 56));    // the last dQ, hence all of them
       tc::tc_fence_after();
     }
     __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.dq) + (int64_t)(q0 + row) * p.dq_stride_t + head * p.dq_stride_h;
@@ -418,8 +452,10 @@ dense_bwd_dq_tc_kernel(const __grid_constant__ DenseKernelParams p, const __grid
 // The tensor pipe runs dV(j), S^T(j+1), dK(j), dP^T(j+1): while the element-wise warps form P^T(j+1) (from S^T(j+1)), it
 // works on dK(j) and dP^T(j+1); while they form dS^T(j), on dV(j) and S^T(j+1).
 namespace dbt {
-enum BarK { K_RES_FULL = 0, K_Q_FULL0, K_Q_FULL1, K_Q_EMPTY0, K_Q_EMPTY1, K_DO_FULL0, K_DO_FULL1, K_DO_EMPTY0, K_DO_EMPTY1, K_S_FULL, K_DP_FULL, K_DV_DONE,
-            K_DK_DONE, K_S_READ, K_DP_READ, K_P_FULL, K_DS_FULL, K_NUM_BARS };   // K_S_READ and later: one arrival per element-wise warp
+// dV of a step and the release of its dO, dK of a chunk of columns and the release of that chunk of Q (the last one: and of Y), are one
+// event each, with two barriers in turn
+enum BarK { K_RES_FULL = 0, K_Q_FULL0, K_DK_DONE0 = K_Q_FULL0 + 2 * kMaxChunks, K_DO_FULL0 = K_DK_DONE0 + 2 * kMaxChunks, K_DO_FULL1, K_DV_DONE0, K_DV_DONE1, K_S_FULL, K_DP_FULL,
+            K_S_READ, K_DP_READ, K_P_FULL, K_DS_FULL, K_NUM_BARS };   // K_S_READ and later: one arrival per element-wise warp
 }
 
 template <int D_QK>
@@ -454,11 +490,12 @@ dense_bwd_dkdv_tc_kernel(const __grid_constant__ DenseKernelParams p, const __gr
   const int jb_lo = p.is_causal ? min(jb_hi, max(0, n_base - (lk - lq)) >> 7) : 0;
   const int nstep = jb_hi - jb_lo;
 
-  auto load_q = [&](int j) {
-    const uint32_t full = bar(K_Q_FULL0 + (j & 1));
-    tc::mbar_arrive_expect_tx(full, L::kWide);
-#pragma unroll
-    for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(sQ + (j & 1) * L::kWide + c * kChunk, &tmap_q, c * 64, head, q0 + (jb_lo + j) * 128, full);
+  // chunk c of the Q tile of step j, and dK of its columns: the barriers
+  auto q_full = [&](int j, int c) { return bar(K_Q_FULL0 + (j & 1) * kMaxChunks + c); };
+  auto dk_done = [&](int j, int c) { return bar(K_DK_DONE0 + (j & 1) * kMaxChunks + c); };
+  auto load_q = [&](int j, int c) {
+    tc::mbar_arrive_expect_tx(q_full(j, c), kChunk);
+    tc::tma_load_3d(sQ + (j & 1) * L::kWide + c * kChunk, &tmap_q, c * 64, head, q0 + (jb_lo + j) * 128, q_full(j, c));
   };
   auto load_do = [&](int j) {
     const int st = j % L::kNarrowStages;
@@ -478,7 +515,8 @@ dense_bwd_dkdv_tc_kernel(const __grid_constant__ DenseKernelParams p, const __gr
         tc::mbar_arrive_expect_tx(bar(K_RES_FULL), L::kWide + L::kNarrow);
 #pragma unroll
         for (int c = 0; c < L::NCH; ++c) tc::tma_load_3d(sK + c * kChunk, &tmap_k, c * 64, head, k0 + n_base, bar(K_RES_FULL));
-        load_q(0);
+#pragma unroll
+        for (int c = 0; c < L::NCH; ++c) load_q(0, c);
 #pragma unroll
         for (int c = 0; c < 2; ++c) tc::tma_load_3d(sV + c * kChunk, &tmap_v, c * 64, head, k0 + n_base, bar(K_RES_FULL));
         load_do(0);
@@ -499,78 +537,74 @@ dense_bwd_dkdv_tc_kernel(const __grid_constant__ DenseKernelParams p, const __gr
     if (tc::elect_one()) {
       bool alive = true;
       for (int j = 1; j < nstep && alive; ++j) {
-        alive = tc::mbar_wait(bar(K_Q_EMPTY0 + (j & 1)), ((j >> 1) & 1) ^ 1, status, 61);
+#pragma unroll 1
+        for (int c = 0; c < L::NCH && alive; ++c) {
+          alive = tc::mbar_wait(dk_done(j, c), ((j >> 1) & 1) ^ 1, status, 61);
+          if (alive) load_q(j, c);
+        }
         if (!alive) break;
-        load_q(j);
-        alive = tc::mbar_wait(bar(K_DO_EMPTY0 + j % L::kNarrowStages), ((j / L::kNarrowStages) & 1) ^ 1, status, 73);
+        const int before = j - L::kNarrowStages;                 // the step whose dO the stage holds
+        if (before >= 0) alive = tc::mbar_wait(bar(K_DV_DONE0 + (before & 1)), (before >> 1) & 1, status, 73);
         if (alive) load_do(j);
       }
     }
   } else if (warp == kEwWarps + 1) {
     // ================================ MMA issuer =======================================
     constexpr uint32_t idesc_dv = tc::idesc_bf16_f32(128, 128, 0, 1);
-    constexpr uint32_t idesc_dk = tc::idesc_bf16_f32(128, D_QK, 0, 1);
+    constexpr uint32_t idesc_dk = tc::idesc_bf16_f32(128, 64, 0, 1);
     const uint64_t desc_k = tc::smem_desc_sw128(sK, 16, 1024);
     const uint64_t desc_v = tc::smem_desc_sw128(sV, 16, 1024);
     const uint64_t desc_q = tc::smem_desc_sw128(sQ, 16, 1024);              // Q tile of stage 0, K-major (B of S^T)
     const uint64_t desc_do = tc::smem_desc_sw128(sDO, 16, 1024);            // dO tile of stage 0, K-major (B of dP^T)
     const uint64_t desc_qt = tc::smem_desc_sw128(sQ, kChunk, 1024);         // Q tile, MN-major (B of dK)
     const uint64_t desc_dot = tc::smem_desc_sw128(sDO, kChunk, 1024);       // dO tile, MN-major (B of dV)
-    bool alive = nstep > 0;
-    if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(K_RES_FULL), 0, status, 62));
-    // waits (whole warp) for phase `ph` of barrier `i`
-    auto wait = [&](int i, int ph, int code) {
-      if (alive) alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(i), ph, status, code));
-      return alive;
-    };
-    auto rows_valid = [&](int j) { return lq - (jb_lo + j) * 128; };
-    // S^T of step j, once its Q tile has landed and dP^T of step j-1 has been read; dP^T of step j likewise
-    auto issue_s = [&](int j) {
-      const int st = j & 1;
-      if (!wait(K_Q_FULL0 + st, (j >> 1) & 1, 63)) return;
-      if (rows_valid(j) < 128) zero_tail(smem + L::WIDE_OFF + st * L::kWide, L::NCH, rows_valid(j), lane);
-      if (!wait(K_DP_READ, (j & 1) ^ 1, 67)) return;
-      tc::tc_fence_after();
-      if (tc::elect_one()) {
-        mma_res_stg<L::NCH>(tmem + TM_X, desc_k, tc::desc_advance(desc_q, st * L::kWide), tc::idesc_bf16_f32(128, k_steps(rows_valid(j)) * 16, 0, 0));
-        tc::tc_commit(bar(K_S_FULL));
-      }
-      __syncwarp();
-    };
-    auto issue_dp = [&](int j) {
-      const int st = j % L::kNarrowStages;
-      if (!wait(K_DO_FULL0 + st, (j / L::kNarrowStages) & 1, 74)) return;
-      if (rows_valid(j) < 128) zero_tail(smem + L::NARROW_OFF + st * L::kNarrow, 2, rows_valid(j), lane);
-      if (!wait(K_S_READ, j & 1, 64)) return;
-      tc::tc_fence_after();
-      if (tc::elect_one()) {
-        mma_res_stg<2>(tmem + TM_X, desc_v, tc::desc_advance(desc_do, st * L::kNarrow), tc::idesc_bf16_f32(128, k_steps(rows_valid(j)) * 16, 0, 0));
+    if (tc::elect_one() && nstep > 0) {
+      bool alive = tc::mbar_wait(bar(K_RES_FULL), 0, status, 62);
+      auto wait = [&](int i, int ph, int code) {
+        if (alive) alive = tc::mbar_wait(bar(i), ph, status, code);
+        return alive;
+      };
+      auto rows_valid = [&](int j) { return lq - (jb_lo + j) * 128; };
+      // S^T of step j, once its Q tile has landed and dP^T of step j-1 has been read; dP^T of step j likewise
+      auto issue_s = [&](int j) {
+        const int st = j & 1;
+        if (!wait(K_DP_READ, (j & 1) ^ 1, 67)) return;
+        alive = mma_res_stg<L::NCH>(tmem + TM_X, desc_k, tc::desc_advance(desc_q, st * L::kWide), tc::idesc_bf16_f32(128, k_steps(rows_valid(j)) * 16, 0, 0), [&](int c) {
+          const bool ok = tc::mbar_wait(q_full(j, c), (j >> 1) & 1, status, 63);
+          tc::tc_fence_after();
+          return ok;
+        });
+        if (alive) tc::tc_commit(bar(K_S_FULL));
+      };
+      auto issue_dp = [&](int j) {
+        const int st = j % L::kNarrowStages;
+        if (!wait(K_DO_FULL0 + st, (j / L::kNarrowStages) & 1, 74)) return;
+        if (!wait(K_S_READ, j & 1, 64)) return;
+        tc::tc_fence_after();
+        mma_res_stg<2>(tmem + TM_X, desc_v, tc::desc_advance(desc_do, st * L::kNarrow), tc::idesc_bf16_f32(128, k_steps(rows_valid(j)) * 16, 0, 0), [](int) { return true; });
         tc::tc_commit(bar(K_DP_FULL));
+      };
+      // step j = -1 issues the first GEMMs of step 0 (the instructions of a step exist once)
+      for (int j = -1; j < nstep && alive; ++j) {
+        const int st = j & 1, std = (j & 1) % L::kNarrowStages, ks = k_steps(rows_valid(j));
+        if (j >= 0) {
+          if (!wait(K_P_FULL, j & 1, 68)) break;
+          tc::tc_fence_after();
+          mma_tmem_stg(tmem + TM_DV, tmem + TM_Y, tc::desc_advance(desc_dot, std * L::kNarrow), idesc_dv, j == 0, ks);
+          tc::tc_commit(bar(K_DV_DONE0 + st));
+        }
+        if (j + 1 < nstep) issue_s(j + 1);
+        if (j >= 0) {
+          if (!wait(K_DS_FULL, j & 1, 69)) break;
+          tc::tc_fence_after();
+#pragma unroll
+          for (int c = 0; c < L::NCH; ++c) {
+            mma_tmem_stg(tmem + TM_DK + c * 64, tmem + TM_Y, tc::desc_advance(desc_qt, st * L::kWide + c * kChunk), idesc_dk, j == 0, ks);
+            tc::tc_commit(dk_done(j, c));              // completes after dV of this step: the tensor pipe runs in order
+          }
+        }
+        if (j + 1 < nstep) issue_dp(j + 1);
       }
-      __syncwarp();
-    };
-    if (alive) issue_s(0);
-    if (alive) issue_dp(0);
-    for (int j = 0; j < nstep && alive; ++j) {
-      const int st = j & 1, std = j % L::kNarrowStages, ks = k_steps(rows_valid(j));
-      if (!wait(K_P_FULL, j & 1, 68)) break;
-      tc::tc_fence_after();
-      if (tc::elect_one()) {
-        mma_tmem_stg(tmem + TM_DV, tmem + TM_Y, tc::desc_advance(desc_dot, std * L::kNarrow), idesc_dv, j == 0, ks);
-        tc::tc_commit(bar(K_DV_DONE));
-        tc::tc_commit(bar(K_DO_EMPTY0 + std));
-      }
-      __syncwarp();
-      if (j + 1 < nstep) issue_s(j + 1);
-      if (!wait(K_DS_FULL, j & 1, 69)) break;
-      tc::tc_fence_after();
-      if (tc::elect_one()) {
-        mma_tmem_stg(tmem + TM_DK, tmem + TM_Y, tc::desc_advance(desc_qt, st * L::kWide), idesc_dk, j == 0, ks);
-        tc::tc_commit(bar(K_DK_DONE));             // completes after dV of this step: the tensor pipe runs in order
-        tc::tc_commit(bar(K_Q_EMPTY0 + st));
-      }
-      __syncwarp();
-      if (j + 1 < nstep) issue_dp(j + 1);
     }
   } else {
     // ================================ element-wise / epilogue ==========================
@@ -579,19 +613,20 @@ dense_bwd_dkdv_tc_kernel(const __grid_constant__ DenseKernelParams p, const __gr
     const int key = n_base + rl;
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const int shift = lk - lq;                                 // query i sees keys <= i + shift
-    // per-query vectors of a step: lse * log2(e) (threads 0-127) and delta (threads 128-255); each value is loaded one
-    // step ahead, so that no step waits for global memory
+    // Per-query vectors of a step: -lse * log2(e) (threads 0-127) and -delta (threads 128-255).  Each value is loaded one step ahead and
+    // not touched before the next: a product right behind the load waited for it, some 800 clk of a step's 3 900.
+    const float* vec = tid < 128 ? p.lse + (int64_t)q0 * p.lse_stride_t + head * p.lse_stride_h : p.delta + (int64_t)head * p.total_q + q0;
+    const int64_t vec_stride = tid < 128 ? p.lse_stride_t : 1;
+    const float vec_mul = tid < 128 ? -kLog2e : -1.f;
     auto load_vec = [&](int j) {
       const int i = (jb_lo + j) * 128 + rl;
-      if (i >= lq) return 0.f;
-      return tid < 128 ? __ldg(p.lse + (int64_t)(q0 + i) * p.lse_stride_t + head * p.lse_stride_h) * kLog2e
-                       : __ldg(p.delta + (int64_t)head * p.total_q + q0 + i);
+      return i < lq ? __ldg(vec + i * vec_stride) : 0.f;
     };
     float v_next = nstep > 0 ? load_vec(0) : 0.f;
     bool alive = true;
     for (int j = 0; j < nstep && alive; ++j) {
       const int jb = jb_lo + j, vb = j & 1;
-      sVec[vb * 256 + tid] = v_next;
+      sVec[vb * 256 + tid] = v_next * vec_mul;
       if (j + 1 < nstep) v_next = load_vec(j + 1);
       if (!tc::mbar_wait(bar(K_S_FULL), j & 1, status, 65)) *sAbort = 1;
       bar_sync(1, kEwWarps * 32);                              // vectors visible; also keeps the two buffers of sVec apart
@@ -609,26 +644,30 @@ dense_bwd_dkdv_tc_kernel(const __grid_constant__ DenseKernelParams p, const __gr
       const float4* vl = reinterpret_cast<const float4*>(sVec + vb * 256 + half * 64);
       const float4* vd = reinterpret_cast<const float4*>(sVec + vb * 256 + 128 + half * 64);
       // two loops, not a test per element: the compiler makes a branch of each test (40 clk per element measured)
+      row_exp2(sv, p.scale_log2, [&](int i) {
+        const float4 l4 = vl[i >> 1];
+        return i & 1 ? F2{l4.z, l4.w} : F2{l4.x, l4.y};
+      });
       auto to_p = [&](auto masked) {
 #pragma unroll
-        for (int i4 = 0; i4 < 16; ++i4) {
-          const float4 l4 = vl[i4];
-          const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int col = i4 * 4 + e;
-            float pe = exp2f(fmaf(__uint_as_float(sv[col]), p.scale_log2, -ls[e]));
-            if constexpr (decltype(masked)::value) pe = col >= c_min && col < c_max ? pe : 0.f;      // a select: see the dQ kernel
-            sv[col] = __float_as_uint(pe);
+        for (int i = 0; i < 32; ++i) {
+          if constexpr (decltype(masked)::value) {             // a select: see the dQ kernel
+            if (!(2 * i >= c_min && 2 * i < c_max)) sv[2 * i] = 0u;
+            if (!(2 * i + 1 >= c_min && 2 * i + 1 < c_max)) sv[2 * i + 1] = 0u;
           }
-          pk[i4 * 2] = pack_bf16x2(__uint_as_float(sv[i4 * 4]), __uint_as_float(sv[i4 * 4 + 1]));
-          pk[i4 * 2 + 1] = pack_bf16x2(__uint_as_float(sv[i4 * 4 + 2]), __uint_as_float(sv[i4 * 4 + 3]));
+          pk[i] = pack_bf16x2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1]));
         }
       };
       if (all_visible) to_p(std::false_type{});
       else to_p(std::true_type{});
       // a wait that gives up here lets the step run on; the flag ends the loop at the next barrier
-      if (!tc::mbar_wait(bar(K_DK_DONE), (j & 1) ^ 1, status, 70)) *sAbort = 1;      // dK of step j-1 has read Y
+      if (j > 0 && !tc::mbar_wait(dk_done(j - 1, L::NCH - 1), ((j - 1) >> 1) & 1, status, 70)) *sAbort = 1;      // dK of step j-1 has read Y
+      if (lq - jb * 128 < 128) {      // the last step: rows past the end of the sequence must be exact zeros for dV and dK
+        const int std = j % L::kNarrowStages;
+        if (!tc::mbar_wait(bar(K_DO_FULL0 + std), (j / L::kNarrowStages) & 1, status, 74)) *sAbort = 1;
+        zero_tail(smem + L::NARROW_OFF + std * L::kNarrow, 2, lq - jb * 128, tid);
+        zero_tail(smem + L::WIDE_OFF + (j & 1) * L::kWide, L::NCH, lq - jb * 128, tid);
+      }
       tc::tc_fence_after();
       __syncwarp();
       tc::tmem_st32(tmem + lane_addr + TM_Y + half * 32, pk);
@@ -648,21 +687,23 @@ dense_bwd_dkdv_tc_kernel(const __grid_constant__ DenseKernelParams p, const __gr
 #pragma unroll
         for (int i4 = 0; i4 < 16; ++i4) {
           const float4 d4 = vd[i4];
-          const float ds[4] = {d4.x, d4.y, d4.z, d4.w};
-          float dv[4];
+          const F2 minus_d[2] = {{d4.x, d4.y}, {d4.z, d4.w}};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int col = i4 * 4 + e;
-            dv[e] = __uint_as_float(sv[col]) * (__uint_as_float(dp[col]) - ds[e]);
-            if constexpr (decltype(masked)::value) dv[e] = col >= c_min && col < c_max ? dv[e] : 0.f;
+          for (int e = 0; e < 2; ++e) {
+            const int col = i4 * 4 + e * 2;
+            F2 dv = f2_mul(F2{__uint_as_float(sv[col]), __uint_as_float(sv[col + 1])},
+                           f2_add(F2{__uint_as_float(dp[col]), __uint_as_float(dp[col + 1])}, minus_d[e]));
+            if constexpr (decltype(masked)::value) {
+              dv.lo = col >= c_min && col < c_max ? dv.lo : 0.f;
+              dv.hi = col + 1 >= c_min && col + 1 < c_max ? dv.hi : 0.f;
+            }
+            pk[i4 * 2 + e] = pack_bf16x2(dv.lo, dv.hi);
           }
-          pk[i4 * 2] = pack_bf16x2(dv[0], dv[1]);
-          pk[i4 * 2 + 1] = pack_bf16x2(dv[2], dv[3]);
         }
       };
       if (all_visible) to_ds(std::false_type{});
       else to_ds(std::true_type{});
-      if (!tc::mbar_wait(bar(K_DV_DONE), j & 1, status, 72)) *sAbort = 1;            // dV of this step has read Y
+      if (!tc::mbar_wait(bar(K_DV_DONE0 + (j & 1)), (j >> 1) & 1, status, 72)) *sAbort = 1;            // dV of this step has read Y
       tc::tc_fence_after();
       __syncwarp();
       tc::tmem_st32(tmem + lane_addr + TM_Y + half * 32, pk);
@@ -673,7 +714,7 @@ dense_bwd_dkdv_tc_kernel(const __grid_constant__ DenseKernelParams p, const __gr
     }
     bool have = nstep > 0 && alive;
     if (have) {
-      have = __all_sync(0xffffffffu, tc::mbar_wait(bar(K_DK_DONE), (nstep - 1) & 1, status, 66));   // the last dK, hence all of them
+      have = __all_sync(0xffffffffu, tc::mbar_wait(dk_done(nstep - 1, L::NCH - 1), ((nstep - 1) >> 1) & 1, status, 66));   // the last dK, hence all of them
       tc::tc_fence_after();
     }
     const bool row_ok = key < lk;

@@ -98,24 +98,6 @@ __device__ __forceinline__ void dense_pv_steps(uint32_t tmem_o, uint32_t tmem_p,
   for (int s = kFirst; s < kEnd; ++s)
     tc::mma_ts(tmem_o, tmem_p + s * 8, tc::desc_advance(desc_v, s * 2048), idesc, (first && s == 0) ? 0u : 1u);
 }
-// 2^x for x <= 2^7 on the multiply-add pipe: x = n + f with n the nearest whole number (held in the low bits of x + 1.5 * 2^23) and
-// |f| <= 1/2, and 2^f = 1 + f q(f) with the polynomial of least largest relative error (fitted with Lawson's weights; 1.6e-7 in
-// fp32 over the range, the special function unit's 2^x is specified to 2.4e-7).  Below -127 the result is 0.
-__device__ __forceinline__ F2 f2_exp2(F2 x) {
-  x.lo = fmaxf(x.lo, -127.f);
-  x.hi = fmaxf(x.hi, -127.f);
-  const F2 t = f2_add(x, f2(12582912.f));
-  const F2 n = f2_add(t, f2(-12582912.f));
-  const F2 f = f2_fma(n, f2(-1.f), x);
-  F2 r = f2_fma(f, f2(0x1.5bba14p-10f), f2(0x1.3cea88p-7f));
-  r = f2_fma(r, f, f2(0x1.c6b752p-5f));
-  r = f2_fma(r, f, f2(0x1.ebf9bcp-3f));
-  r = f2_fma(r, f, f2(0x1.62e42ap-1f));
-  r = f2_fma(r, f, f2(1.f));
-  r.lo = __uint_as_float(__float_as_uint(r.lo) + (__float_as_uint(t.lo) << 23));
-  r.hi = __uint_as_float(__float_as_uint(r.hi) + (__float_as_uint(t.hi) << 23));
-  return r;
-}
 // the largest of three; NaN if one of them is
 __device__ __forceinline__ float max3_nan(float a, float b, float c) {
   float d;

@@ -82,6 +82,38 @@ __device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
   return d;
 }
 __device__ __forceinline__ F2 f2(float x) { return F2{x, x}; }
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 d;
+  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmul.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}\n"
+      : "=f"(d.lo), "=f"(d.hi)
+      : "f"(a.lo), "f"(a.hi), "f"(b.lo), "f"(b.hi));
+  return d;
+}
+// 2^x for x <= 2^7 on the multiply-add pipe: x = n + f with n the nearest whole number (held in the low bits of x + 1.5 * 2^23) and
+// |f| <= 1/2, and 2^f = 1 + f q(f) with the polynomial of least largest relative error (fitted with Lawson's weights; 1.6e-7 in
+// fp32 over the range, the special function unit's 2^x is specified to 2.4e-7).  Below -127 the result is 0.
+__device__ __forceinline__ F2 f2_exp2(F2 x) {
+  x.lo = fmaxf(x.lo, -127.f);
+  x.hi = fmaxf(x.hi, -127.f);
+  const F2 t = f2_add(x, f2(12582912.f));
+  const F2 n = f2_add(t, f2(-12582912.f));
+  const F2 f = f2_fma(n, f2(-1.f), x);
+  F2 r = f2_fma(f, f2(0x1.5bba14p-10f), f2(0x1.3cea88p-7f));
+  r = f2_fma(r, f, f2(0x1.c6b752p-5f));
+  r = f2_fma(r, f, f2(0x1.ebf9bcp-3f));
+  r = f2_fma(r, f, f2(0x1.62e42ap-1f));
+  r = f2_fma(r, f, f2(1.f));
+  r.lo = __uint_as_float(__float_as_uint(r.lo) + (__float_as_uint(t.lo) << 23));
+  r.hi = __uint_as_float(__float_as_uint(r.hi) + (__float_as_uint(t.hi) << 23));
+  return r;
+}
+// the same with NaN for NaN
+__device__ __forceinline__ F2 f2_exp2_nan(F2 x) {
+  const F2 r = f2_exp2(x);
+  asm("max.NaN.f32 %0, %1, 0fC2FE0000;\n" : "=f"(x.lo) : "f"(x.lo));      // -127
+  asm("max.NaN.f32 %0, %1, 0fC2FE0000;\n" : "=f"(x.hi) : "f"(x.hi));
+  return f2_fma(x, f2(0.f), r);
+}
 // the largest of three (NaN only if all are)
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
