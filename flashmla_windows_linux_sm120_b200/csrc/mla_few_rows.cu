@@ -82,7 +82,7 @@ struct Layout {
   static_assert(kVSlots % 2 == 0 && kVSlots >= 16 && kVSlots <= 8 * (kPageBars - 1) + 1, "ring sizes");
 };
 enum Bar { Q_FULL = 0, Q_EMPTY, KV_FULL0, KV_EMPTY0 = KV_FULL0 + kPageBars, ROPE_EMPTY0 = KV_EMPTY0 + kPageBars, S_FULL0 = ROPE_EMPTY0 + 3, S_FULL1,
-           P_FULL0, P_FULL1, P_EMPTY0, P_EMPTY1, O_FULL, NUM_BARS };
+           P_FULL0, P_FULL1, O_FULL, NUM_BARS };
 static_assert(NUM_BARS * 8 <= 256, "barrier area too small");
 constexpr int TMEM_O = 0, TMEM_S = 256;
 constexpr float kRescaleThreshold = 8.0f;         // log2 units; below it O keeps its stale scale
@@ -433,47 +433,46 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
     }
   } else if (warp == 5) {
     // ================================ MMA issuer =======================================
-    constexpr uint32_t idesc_s = tc::idesc_bf16_f32(64, N, 0, 0, F16);
-    constexpr uint32_t idesc_o = tc::idesc_bf16_f32(128, N, 1, 0, F16);
-    const uint64_t desc_q = tc::smem_desc_sw128(sbase + L::Q_OFF, 16, 1024);        // B of S^T: K-major
-    const uint64_t desc_k = tc::smem_desc_sw128(sbase + L::V_OFF, 16, 1024);        // A of S^T: K-major (slot 0)
-    const uint64_t desc_r = tc::smem_desc_sw128(sbase + L::R_OFF, 16, 1024);        // the same, rope slot 0
-    const uint64_t desc_v = tc::smem_desc_sw128(sbase + L::V_OFF, kSlot, 1024);     // A of O^T: MN-major, 64-wide column groups 8 KB apart
-    const uint64_t desc_p = tc::smem_desc_sw128(sbase + L::P_OFF, 16, 1024);        // B of O^T: K-major
-    int g = 0, req = 0;
-    int slot_s = 0, slot_p = 0;      // first slot of the page of the next S^T / O^T (running: a division would cost more than the MMAs of a chunk)
-    auto next_page = [](int slot) { return slot + 8 >= L::kVSlots ? slot + 8 - L::kVSlots : slot + 8; };
-    auto wrap = [](int slot) { return slot >= L::kVSlots ? slot - L::kVSlots : slot; };
-    bool alive = true;
-    for (int wi = 0; wi < n_work && alive; ++wi) {
-      const Req r = request(wi);
-      const int nblk = r.blk_hi - r.blk_lo;
-      if (nblk == 0) continue;
-      alive = __all_sync(0xffffffffu, tc::mbar_wait(bar(Q_FULL), req & 1, status, 205));
-      // S^T runs one block ahead of O^T; where both could be next, whichever has its inputs first is issued, O^T first: it
-      // releases slots of the ring.  S^T(js) overwrites S^T(js - 2), and O^T(0) what the request before left: the softmax
-      // warps had read both before they arrived on a P_FULL that has been waited for here (P_FULL(js - 2), P_FULL(0)).
-      // Only what is needed is looked at: with four barriers per poll, one per lane, the warp saw P 550 clk after its last
-      // arrival, now 375 (64 heads, two query tokens, 16 x 16 000 tokens: 143 -> 140 us; 8 to 64 rows 2 % of a step).
-      int js = 0, jp = 0, idle = 0;
-      while (jp < nblk && alive) {
-        const int gs = g + js, gp = g + jp;
-        const bool want_s = js < nblk && js <= jp + 1, want_p = jp < js;
-        const uint32_t p_full = bar(P_FULL0 + gp % L::kPBufs), kv_full = bar(KV_FULL0 + gs % kPageBars);
-        const uint32_t p_ph = (gp / L::kPBufs) & 1, kv_ph = (gs / kPageBars) & 1;
-        bool go_p = false, go_s = false;
-        if (want_s && want_p) {
-          const uint32_t m = __ballot_sync(0xffffffffu, lane < 2 && tc::mbar_test_wait(lane == 0 ? p_full : kv_full, lane == 0 ? p_ph : kv_ph));
-          go_p = m & 1u;
-          go_s = m & 2u;
-        } else if (want_p) {
-          go_p = alive = __all_sync(0xffffffffu, tc::mbar_wait(p_full, p_ph, status, 207));
-        } else {
-          go_s = alive = __all_sync(0xffffffffu, tc::mbar_wait(kv_full, kv_ph, status, 212));
-        }
-        if (go_p) {
-          tc::tc_fence_after();
-          if (tc::elect_one()) {
+    // One thread.  As a warp with a vote on every wait: 16 heads, 61 x 6 000 tokens 78.6 us, 75.9 now, 60 x 300 17.6 -> 15.5, 32 heads,
+    // 32 x 500 21.8 -> 20.4, 64 heads, 8 x 3 000 22.7 -> 22.2, sparse, 64 heads, 30 x top-k 2 048 40.7 -> 39.9, 2 x 512 14.65 -> 14.8.
+    if (tc::elect_one()) {
+      constexpr uint32_t idesc_s = tc::idesc_bf16_f32(64, N, 0, 0, F16);
+      constexpr uint32_t idesc_o = tc::idesc_bf16_f32(128, N, 1, 0, F16);
+      const uint64_t desc_q = tc::smem_desc_sw128(sbase + L::Q_OFF, 16, 1024);        // B of S^T: K-major
+      const uint64_t desc_k = tc::smem_desc_sw128(sbase + L::V_OFF, 16, 1024);        // A of S^T: K-major (slot 0)
+      const uint64_t desc_r = tc::smem_desc_sw128(sbase + L::R_OFF, 16, 1024);        // the same, rope slot 0
+      const uint64_t desc_v = tc::smem_desc_sw128(sbase + L::V_OFF, kSlot, 1024);     // A of O^T: MN-major, 64-wide column groups 8 KB apart
+      const uint64_t desc_p = tc::smem_desc_sw128(sbase + L::P_OFF, 16, 1024);        // B of O^T: K-major
+      int g = 0, req = 0;
+      int slot_s = 0, slot_p = 0;      // first slot of the page of the next S^T / O^T (running: a division would cost more than the MMAs of a chunk)
+      auto next_page = [](int slot) { return slot + 8 >= L::kVSlots ? slot + 8 - L::kVSlots : slot + 8; };
+      auto wrap = [](int slot) { return slot >= L::kVSlots ? slot - L::kVSlots : slot; };
+      bool alive = true;
+      for (int wi = 0; wi < n_work && alive; ++wi) {
+        const Req r = request(wi);
+        const int nblk = r.blk_hi - r.blk_lo;
+        if (nblk == 0) continue;
+        alive = tc::mbar_wait(bar(Q_FULL), req & 1, status, 205);
+        // S^T runs one block ahead of O^T; where both could be next, whichever has its inputs first is issued, O^T first: it
+        // releases slots of the ring.  S^T(js) overwrites S^T(js - 2), and O^T(0) what the request before left: the softmax
+        // warps had read both before they arrived on a P_FULL that has been waited for here (P_FULL(js - 2), P_FULL(0)).
+        int js = 0, jp = 0, idle = 0;
+        while (jp < nblk && alive) {
+          const int gs = g + js, gp = g + jp;
+          const bool want_s = js < nblk && js <= jp + 1, want_p = jp < js;
+          const uint32_t p_full = bar(P_FULL0 + gp % L::kPBufs), kv_full = bar(KV_FULL0 + gs % kPageBars);
+          const uint32_t p_ph = (gp / L::kPBufs) & 1, kv_ph = (gs / kPageBars) & 1;
+          bool go_p = false, go_s = false;
+          if (want_s && want_p) {
+            go_p = tc::mbar_test_wait(p_full, p_ph);
+            if (!go_p) go_s = tc::mbar_test_wait(kv_full, kv_ph);
+          } else if (want_p) {
+            go_p = alive = tc::mbar_wait(p_full, p_ph, status, 207);
+          } else {
+            go_s = alive = tc::mbar_wait(kv_full, kv_ph, status, 212);
+          }
+          if (go_p) {
+            tc::tc_fence_after();
             const uint64_t dp = tc::desc_advance(desc_p, (gp % L::kPBufs) * N * 128);
 #pragma unroll
             for (int mb = 0; mb < 4; ++mb) {
@@ -483,26 +482,11 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
                 tc::mma_ss(tmem + TMEM_O + mb * N, tc::desc_advance(dv, s * 2048), tc::desc_advance(dp, s * 32), idesc_o, (jp == 0 && s == 0) ? 0u : 1u);
             }
             tc::tc_commit(bar(KV_EMPTY0 + gp % kPageBars));
-            tc::tc_commit(bar(P_EMPTY0 + gp % L::kPBufs));
-          }
-          __syncwarp();
-          slot_p = next_page(slot_p);
-          ++jp;
-          idle = 0;
-        } else if (go_s) {
-          // rows of the last page beyond the sequence may hold anything (NaN included): zeroed so that 0 * garbage
-          // cannot reach O^T
-          const int rows_valid = SPARSE ? 64 : r.seqlen - (r.blk_lo + js) * 64;
-          if (rows_valid < 64) {
-            for (int i = lane; i < (64 - rows_valid) * 64; i += 32) {
-              const int row = rows_valid + (i >> 6), c = (i >> 3) & 7, piece = i & 7;
-              *reinterpret_cast<uint4*>(smem + L::V_OFF + wrap(slot_s + c) * kSlot + row * 128 + piece * 16) = make_uint4(0, 0, 0, 0);
-            }
-            tc::fence_proxy_async_smem();
-            __syncwarp();
-          }
-          tc::tc_fence_after();
-          if (tc::elect_one()) {
+            slot_p = next_page(slot_p);
+            ++jp;
+            idle = 0;
+          } else if (go_s) {
+            tc::tc_fence_after();
             const uint32_t d = tmem + TMEM_S + (gs & 1) * N;
 #pragma unroll
             for (int c = 0; c < 9; ++c) {
@@ -515,20 +499,18 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
             tc::tc_commit(bar(S_FULL0 + (gs & 1)));
             tc::tc_commit(bar(ROPE_EMPTY0 + gs % L::kRopeSlots));
             if (js == nblk - 1) tc::tc_commit(bar(Q_EMPTY));
+            slot_s = next_page(slot_s);
+            ++js;
+            idle = 0;
+          } else if (alive && ++idle > tc::kSpinLimit) {
+            tc::report_status(status, 206);
+            alive = false;
           }
-          __syncwarp();
-          slot_s = next_page(slot_s);
-          ++js;
-          idle = 0;
-        } else if (alive && ++idle > tc::kSpinLimit) {
-          if (lane == 0) tc::report_status(status, 206);
-          alive = false;
         }
+        g += nblk;
+        if (alive) tc::tc_commit(bar(O_FULL));
+        ++req;
       }
-      g += nblk;
-      if (alive && tc::elect_one()) tc::tc_commit(bar(O_FULL));
-      __syncwarp();
-      ++req;
     }
   } else {
     // ================================ softmax / epilogue ================================
@@ -575,6 +557,13 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
               }
           }
         } else if (blk0 + 64 > r.seqlen - lag_first) {
+          // rows of the last page beyond the sequence may hold anything (NaN included): zeroed, now that S^T has read them, so that
+          // 0 * garbage cannot reach O^T
+          const int rows_valid = r.seqlen - blk0;
+          for (int i = tid; i < (64 - rows_valid) * 64; i += 128) {
+            const int row = rows_valid + (i >> 6), c = (i >> 3) & 7, piece = i & 7;
+            *reinterpret_cast<uint4*>(smem + L::V_OFF + (g * 8 + c) % L::kVSlots * kSlot + row * 128 + piece * 16) = make_uint4(0, 0, 0, 0);
+          }
 #pragma unroll
           for (int k = 0; k < K8; ++k)
 #pragma unroll
@@ -625,7 +614,7 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
           if (bar_any(1, moved)) {
             // every earlier O^T product must be complete (they complete in order)
             const int gl = g - 1;
-            if (!tc::mbar_wait(bar(P_EMPTY0 + gl % L::kPBufs), (gl / L::kPBufs) & 1, status, 209)) *sAbort = 1;
+            if (!tc::mbar_wait(bar(KV_EMPTY0 + gl % kPageBars), (gl / kPageBars) & 1, status, 209)) *sAbort = 1;
             __syncwarp();
             tc::tc_fence_after();
 #pragma unroll 1
@@ -654,7 +643,8 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
           pk[2 * k] = pack_16x2<F16>(p00, p01);
           pk[2 * k + 1] = pack_16x2<F16>(p10, p11);
         }
-        if (!tc::mbar_wait(bar(P_EMPTY0 + g % L::kPBufs), ((g / L::kPBufs) & 1) ^ 1, status, 210)) *sAbort = 1;
+        // the P buffer is free: O^T of the block that had it is complete
+        if (const int gb = g - L::kPBufs; gb >= 0 && !tc::mbar_wait(bar(KV_EMPTY0 + gb % kPageBars), (gb / kPageBars) & 1, status, 210)) *sAbort = 1;
         __syncwarp();
         // P[column][token] as the K-major 128B-swizzled B operand: 16-byte chunk (2 warp + half) ^ (column & 7) of row `column`
         const uint32_t pbase = sbase + L::P_OFF + (g % L::kPBufs) * N * 128;

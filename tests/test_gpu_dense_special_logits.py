@@ -65,3 +65,16 @@ def test_far_below_the_largest(spread, causal):
     out, lse, _ = _run(c, causal, False)
     ref, ref_lse = dense.dense_fwd_ref(c["q"], c["k"], c["v"], c["cu_q"], c["cu_k"], causal, c["scale"])
     assert check_is_allclose("out", out, ref, **TOL) and check_is_allclose("lse", lse, ref_lse, **LSE_TOL)
+
+
+@pytest.mark.parametrize("n", [100, 500])                    # steps of 64 and of 128 streamed rows
+@pytest.mark.parametrize("row", [0, 1, 2, 3, 4, 5, 30, 33, 62, 99])
+def test_a_nan_row_reaches_its_gradients(row, n):
+    """The log-sum-exp of the row is NaN, so its P is, whichever way it is formed: dQ of the row, dK and dV of every key it sees."""
+    c = _case(128, n, n, n + row)
+    c["d_out"] = torch.randn(n, 1, 128, generator=torch.Generator().manual_seed(row)).to(torch.bfloat16)
+    c["q"][row] = NAN
+    _, _, (dq, dk, dv) = _run(c, True, True)
+    assert torch.isnan(dq[row]).all() and torch.isnan(dk[:row + 1]).all() and torch.isnan(dv[:row + 1]).all()
+    rest = torch.arange(n) != row
+    assert not torch.isnan(dq[rest]).any() and not torch.isnan(dv[row + 1:]).any()      # (dK of other keys: zero times the row itself)
