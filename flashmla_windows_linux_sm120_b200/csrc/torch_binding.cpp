@@ -3,7 +3,8 @@
 // output allocation, filling the parameter block, the launches -- and the same work through Python attribute access and
 // ctypes took 38 us of host time per decode call, against 20 to 30 us of GPU work.  (Dense path: 200 tokens, 8 heads 35.5 us
 // per forward through ctypes, 18.8 here, 12.3 of GPU work; 3 sequences of 300 to 900 tokens, 16 heads, forward and backward
-// 180 to 199 -> 115 us.)  Everything that computes stays behind the C ABI (include/flashmla_b200.h); error texts are those of
+// 180 to 199 -> 115 us.  With the outputs allocated here too, instead of by torch.empty in Python: 2 sequences of 100 to 200 tokens, 8 heads
+// 18.2 -> 16.3 us of host time, with the backward 116 -> 105.)  Everything that computes stays behind the C ABI (include/flashmla_b200.h); error texts are those of
 // the extension module of the reference (csrc/pybind.cpp:383-867).
 //
 // CPython functions with vector calls instead of pybind11: an argument costs a type check and a pointer.
@@ -302,24 +303,28 @@ PyObject* sparse_prefill(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 // The arguments that both directions of the dense path have: a[0] q, a[1] k, a[2] v, a[3] cu_q, a[4] cu_k, a[5] o, a[6] lse,
 // a[7] mask mode code, a[8] softmax scale, a[9] max_seqlen_q, a[10] max_seqlen_k.
 constexpr Py_ssize_t kDenseArgs = 11;
-fmla_dense_params dense_params(PyObject* const* a) {
+// all but o and lse, whose tensors follow (`given`: the caller's, which are looked at first as the others are)
+fmla_dense_params dense_params(PyObject* const* a, bool given) {
   const char* names[] = {"q", "k", "v", "cumulative_seqlen_q", "cumulative_seqlen_kv", "o", "lse"};
-  for (int i = 0; i < 7; ++i) require_cuda(tensor(a[i], names[i]), names[i]);
+  for (int i = 0; i < (given ? 7 : 5); ++i) require_cuda(tensor(a[i], names[i]), names[i]);
   const at::Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]), &cu_q = THPVariable_Unpack(a[3]),
-                   &cu_k = THPVariable_Unpack(a[4]), &o = THPVariable_Unpack(a[5]), &lse = THPVariable_Unpack(a[6]);
-  require(q.scalar_type() == at::kBFloat16 && k.scalar_type() == at::kBFloat16 && v.scalar_type() == at::kBFloat16 && o.scalar_type() == at::kBFloat16,
+                   &cu_k = THPVariable_Unpack(a[4]);
+  const at::Tensor *o = given ? &THPVariable_Unpack(a[5]) : nullptr, *lse = given ? &THPVariable_Unpack(a[6]) : nullptr;
+  require(q.scalar_type() == at::kBFloat16 && k.scalar_type() == at::kBFloat16 && v.scalar_type() == at::kBFloat16 && (!o || o->scalar_type() == at::kBFloat16),
           "q, k, v, o must be bfloat16");
-  require(lse.scalar_type() == at::kFloat, "lse must be float32");
+  require(!lse || lse->scalar_type() == at::kFloat, "lse must be float32");
   require(cu_q.scalar_type() == at::kInt && cu_k.scalar_type() == at::kInt, "cumulative seqlens must be int32");
-  require(q.dim() == 3 && k.dim() == 3 && v.dim() == 3 && o.dim() == 3 && lse.dim() == 2, "bad ranks");
-  require(q.stride(2) == 1 && k.stride(2) == 1 && v.stride(2) == 1 && o.stride(2) == 1, "last dimensions must be contiguous");
+  require(q.dim() == 3 && k.dim() == 3 && v.dim() == 3 && (!o || (o->dim() == 3 && lse->dim() == 2)), "bad ranks");
+  require(q.stride(2) == 1 && k.stride(2) == 1 && v.stride(2) == 1 && (!o || o->stride(2) == 1), "last dimensions must be contiguous");
   require(cu_q.is_contiguous() && cu_k.is_contiguous(), "cumulative seqlens must be contiguous");
   fmla_dense_params p = {};
   p.batch = static_cast<int32_t>(cu_q.size(0) - 1);
   require(cu_k.numel() >= cu_q.size(0), "cumulative_seqlen_kv is shorter than cumulative_seqlen_q");      // the kernels read as many of both
   require(k.size(0) == v.size(0) && k.size(1) == v.size(1) && k.size(2) == q.size(2), "k shape mismatch");
-  require(o.size(0) == q.size(0) && o.size(1) == q.size(1) && o.size(2) == v.size(2), "o shape mismatch");
-  require(lse.size(0) == q.size(0) && lse.size(1) == q.size(1), "lse must be [total_q, h_q]");
+  if (given) {
+    require(o->size(0) == q.size(0) && o->size(1) == q.size(1) && o->size(2) == v.size(2), "o shape mismatch");
+    require(lse->size(0) == q.size(0) && lse->size(1) == q.size(1), "lse must be [total_q, h_q]");
+  }
   p.total_q = static_cast<int32_t>(q.size(0)); p.h_q = static_cast<int32_t>(q.size(1)); p.d_qk = static_cast<int32_t>(q.size(2));
   p.total_k = static_cast<int32_t>(v.size(0)); p.h_k = static_cast<int32_t>(v.size(1)); p.d_v = static_cast<int32_t>(v.size(2));
   p.max_seqlen_q = as_int(a[9]); p.max_seqlen_k = as_int(a[10]);
@@ -334,60 +339,91 @@ fmla_dense_params dense_params(PyObject* const* a) {
   p.v = v.const_data_ptr(); p.v_stride_t = v.stride(0); p.v_stride_h = v.stride(1);
   p.cu_seqlens_q = static_cast<const int32_t*>(cu_q.const_data_ptr());
   p.cu_seqlens_k = static_cast<const int32_t*>(cu_k.const_data_ptr());
-  p.o_stride_t = o.stride(0); p.o_stride_h = o.stride(1);
-  p.lse_stride_t = lse.stride(0); p.lse_stride_h = lse.stride(1);
   return p;
 }
+void dense_output_strides(fmla_dense_params& p, const at::Tensor& o, const at::Tensor& lse) {
+  p.o_stride_t = o.stride(0); p.o_stride_h = o.stride(1);
+  p.lse_stride_t = lse.stride(0); p.lse_stride_h = lse.stride(1);
+}
 
-// the arguments above; writes o and lse
+// the arguments above; writes o and lse, or returns new ones ([total_q, h_q, d_v], and [total_q, h_q] contiguous along tokens) where both
+// are None
 PyObject* dense_fwd(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   return guarded(nargs, kDenseArgs, [&]() -> PyObject* {
-    fmla_dense_params p = dense_params(a);
-    const at::Tensor &q = THPVariable_Unpack(a[0]), &o = THPVariable_Unpack(a[5]), &lse = THPVariable_Unpack(a[6]);
-    p.o = o.mutable_data_ptr();
-    p.lse = static_cast<float*>(lse.mutable_data_ptr());
+    const bool given = a[5] != Py_None || a[6] != Py_None;
+    fmla_dense_params p = dense_params(a, given);
+    const at::Tensor& q = THPVariable_Unpack(a[0]);
+    at::Tensor o, lse;
+    if (given) {
+      o = THPVariable_Unpack(a[5]);
+      lse = THPVariable_Unpack(a[6]);
+    }
     {
       const NoGil nogil;
       const c10::cuda::CUDAGuard guard(q.device());
+      if (!given) {
+        o = new_tensor({p.total_q, p.h_q, p.d_v}, q, at::kBFloat16);
+        lse = new_tensor({p.h_q, p.total_q}, q, at::kFloat).t();
+      }
+      p.o = o.mutable_data_ptr();
+      p.lse = static_cast<float*>(lse.mutable_data_ptr());
+      dense_output_strides(p, o, lse);
       check(fmla_dense_prefill_fwd(&p, stream_of(q)));
     }
-    Py_RETURN_NONE;
+    if (given) Py_RETURN_NONE;
+    return pair(std::move(o), std::move(lse));
   });
 }
 
-// the arguments above, then d_o, dq, dk, dv, workspace; writes dq, dk, dv
+// the arguments above, then d_o, dq, dk, dv, workspace; writes dq, dk, dv, or returns new ones where all four are None
 PyObject* dense_bwd(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   return guarded(nargs, kDenseArgs + 5, [&]() -> PyObject* {
-    fmla_dense_params p = dense_params(a);
+    fmla_dense_params p = dense_params(a, true);
     const char* names[] = {"d_o", "dq", "dk", "dv", "workspace_buffer"};
-    for (int i = 0; i < 5; ++i) {
+    const bool given = a[12] != Py_None || a[13] != Py_None || a[14] != Py_None || a[15] != Py_None;
+    for (int i = 0; i < (given ? 5 : 1); ++i) {
       const at::Tensor& t = tensor(a[kDenseArgs + i], names[i]);
       require_cuda(t, names[i]);
       if (t.stride(-1) != 1) throw std::runtime_error(std::string(names[i]) + " must have contiguous last dimension");
     }
     const at::Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]), &o = THPVariable_Unpack(a[5]),
-                     &lse = THPVariable_Unpack(a[6]), &d_o = THPVariable_Unpack(a[11]), &dq = THPVariable_Unpack(a[12]),
-                     &dk = THPVariable_Unpack(a[13]), &dv = THPVariable_Unpack(a[14]), &work = THPVariable_Unpack(a[15]);
-    require(d_o.scalar_type() == at::kBFloat16 && dq.scalar_type() == at::kBFloat16 && dk.scalar_type() == at::kBFloat16 &&
-                dv.scalar_type() == at::kBFloat16,
+                     &lse = THPVariable_Unpack(a[6]), &d_o = THPVariable_Unpack(a[11]);
+    at::Tensor dq, dk, dv, work;
+    if (given) {
+      dq = THPVariable_Unpack(a[12]); dk = THPVariable_Unpack(a[13]); dv = THPVariable_Unpack(a[14]); work = THPVariable_Unpack(a[15]);
+    }
+    require(d_o.scalar_type() == at::kBFloat16 && (!given || (dq.scalar_type() == at::kBFloat16 && dk.scalar_type() == at::kBFloat16 &&
+                                                              dv.scalar_type() == at::kBFloat16)),
             "d_o, dq, dk, dv must be bfloat16");
-    require(d_o.sizes() == o.sizes() && dq.sizes() == q.sizes() && dk.sizes() == k.sizes() && dv.sizes() == v.sizes(), "gradient shape mismatch");
+    require(d_o.sizes() == o.sizes() && (!given || (dq.sizes() == q.sizes() && dk.sizes() == k.sizes() && dv.sizes() == v.sizes())), "gradient shape mismatch");
     p.o = const_cast<void*>(o.const_data_ptr());               // o and lse are read by this direction
     p.lse = const_cast<float*>(static_cast<const float*>(lse.const_data_ptr()));
+    dense_output_strides(p, o, lse);
     p.d_o = d_o.const_data_ptr(); p.do_stride_t = d_o.stride(0); p.do_stride_h = d_o.stride(1);
-    p.dq = dq.mutable_data_ptr(); p.dq_stride_t = dq.stride(0); p.dq_stride_h = dq.stride(1);
-    p.dk = dk.mutable_data_ptr(); p.dk_stride_t = dk.stride(0); p.dk_stride_h = dk.stride(1);
-    p.dv = dv.mutable_data_ptr(); p.dv_stride_t = dv.stride(0); p.dv_stride_h = dv.stride(1);
-    const size_t need = fmla_dense_bwd_workspace_bytes(p.total_q, p.h_q, p.d_qk), have = work.numel() * work.element_size();
-    if (have < need) throw std::runtime_error("workspace_buffer too small: need " + std::to_string(need) + " bytes");
-    p.workspace = work.mutable_data_ptr();
-    p.workspace_bytes = have;
+    const size_t need = fmla_dense_bwd_workspace_bytes(p.total_q, p.h_q, p.d_qk);
     {
       const NoGil nogil;
       const c10::cuda::CUDAGuard guard(q.device());
+      if (!given) {
+        dq = new_tensor(q.sizes(), q, at::kBFloat16);
+        dk = new_tensor(k.sizes(), q, at::kBFloat16);
+        dv = new_tensor(v.sizes(), q, at::kBFloat16);
+        work = new_tensor({static_cast<int64_t>(need)}, q, at::kByte);
+      }
+      p.dq = dq.mutable_data_ptr(); p.dq_stride_t = dq.stride(0); p.dq_stride_h = dq.stride(1);
+      p.dk = dk.mutable_data_ptr(); p.dk_stride_t = dk.stride(0); p.dk_stride_h = dk.stride(1);
+      p.dv = dv.mutable_data_ptr(); p.dv_stride_t = dv.stride(0); p.dv_stride_h = dv.stride(1);
+      p.workspace_bytes = work.numel() * work.element_size();
+      if (p.workspace_bytes < need) throw std::runtime_error("workspace_buffer too small: need " + std::to_string(need) + " bytes");
+      p.workspace = work.mutable_data_ptr();
       check(fmla_dense_prefill_bwd(&p, stream_of(q)));
     }
-    Py_RETURN_NONE;
+    if (given) Py_RETURN_NONE;
+    PyObject* list = pair(std::move(dq), std::move(dk));
+    PyObject* third = THPVariable_Wrap(std::move(dv));
+    PyList_Append(list, third);
+    Py_DECREF(third);
+    return list;
   });
 }
 

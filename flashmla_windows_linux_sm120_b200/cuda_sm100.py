@@ -105,12 +105,26 @@ def dense_prefill_fwd(workspace_buffer, q, k, v, cumulative_seqlen_q, cumulative
                       max_seqlen_q, max_seqlen_kv)
 
 
+def dense_prefill_fwd_new(q, k, v, cumulative_seqlen_q, cumulative_seqlen_kv, mask_mode_code: int, softmax_scale: float,
+                          max_seqlen_q: int, max_seqlen_kv: int) -> List[torch.Tensor]:
+    """dense_prefill_fwd into new tensors: [o [total_q, h_q, d_v], lse [total_q, h_q] contiguous along tokens]."""
+    return _native.dense_fwd(q, k, v, cumulative_seqlen_q, cumulative_seqlen_kv, None, None, mask_mode_code, softmax_scale,
+                             max_seqlen_q, max_seqlen_kv)
+
+
 def dense_prefill_bwd(workspace_buffer, d_o, q, k, v, o, lse, cumulative_seqlen_q, cumulative_seqlen_kv,
                       dq, dk, dv, mask_mode_code: int, softmax_scale: float, max_seqlen_q: int,
                       max_seqlen_kv: int, is_varlen: bool = True) -> None:
     """csrc/pybind.cpp:841-867.  Writes dq, dk, dv in place."""
     _native.dense_bwd(q, k, v, cumulative_seqlen_q, cumulative_seqlen_kv, o, lse, mask_mode_code, softmax_scale,
                       max_seqlen_q, max_seqlen_kv, d_o, dq, dk, dv, workspace_buffer)
+
+
+def dense_prefill_bwd_new(d_o, q, k, v, o, lse, cumulative_seqlen_q, cumulative_seqlen_kv, mask_mode_code: int,
+                          softmax_scale: float, max_seqlen_q: int, max_seqlen_kv: int) -> List[torch.Tensor]:
+    """dense_prefill_bwd into new tensors, with a workspace of its own: [dq, dk, dv]."""
+    return _native.dense_bwd(q, k, v, cumulative_seqlen_q, cumulative_seqlen_kv, o, lse, mask_mode_code, softmax_scale,
+                             max_seqlen_q, max_seqlen_kv, d_o, None, None, None, None)
 
 
 def combine_partials(lse_accum: torch.Tensor, o_accum: torch.Tensor):

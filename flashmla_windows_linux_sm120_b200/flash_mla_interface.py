@@ -87,6 +87,9 @@ def _flash_attn_varlen_forward(q, k, v, cu_seqlens_qo, cu_seqlens_kv, max_seqlen
     _, _, d_vo = v.shape
     if softmax_scale is None:
         softmax_scale = d_qk ** (-0.5)
+    if out is None and lse is None:
+        return tuple(flash_mla_cuda.dense_prefill_fwd_new(q, k, v, cu_seqlens_qo, cu_seqlens_kv, 1 if causal else 0, softmax_scale,
+                                                          max_seqlen_qo, max_seqlen_kv))
     if out is None:
         out = torch.empty(total_q, h_q, d_vo, device=q.device, dtype=q.dtype)
     if lse is None:
@@ -105,6 +108,11 @@ def _flash_attn_varlen_backward(do, q, k, v, out, lse, cu_seqlens_qo, cu_seqlens
         raise ValueError(f"SM100 bwd doesn't support GQA now. num_qo_heads: {h_q}, num_kv_heads: {h_k}.")
     if softmax_scale is None:
         softmax_scale = d_qk ** (-0.5)
+    if do.stride(-1) != 1:
+        do = do.contiguous()
+    if dq is None and dk is None and dv is None:
+        return tuple(flash_mla_cuda.dense_prefill_bwd_new(do, q, k, v, out, lse, cu_seqlens_qo, cu_seqlens_kv, 1 if causal else 0,
+                                                          softmax_scale, max_seqlen_qo, max_seqlen_kv))
     if dq is None:
         dq = torch.empty(total_q, h_q, d_qk, device=q.device, dtype=q.dtype)
     if dk is None:
@@ -113,8 +121,6 @@ def _flash_attn_varlen_backward(do, q, k, v, out, lse, cu_seqlens_qo, cu_seqlens
         dv = torch.empty(total_k, h_k, d_vo, device=q.device, dtype=q.dtype)
     ws_bytes = flash_mla_cuda.lib.fmla_dense_bwd_workspace_bytes(total_q, h_q, d_qk)
     workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-    if do.stride(-1) != 1:
-        do = do.contiguous()
     flash_mla_cuda.dense_prefill_bwd(workspace, do, q, k, v, out, lse, cu_seqlens_qo, cu_seqlens_kv, dq, dk, dv,
                                      1 if causal else 0, softmax_scale, max_seqlen_qo, max_seqlen_kv, is_varlen)
     return dq, dk, dv
