@@ -20,61 +20,60 @@ constexpr int kCombineWarps = 8;
 
 // Weights 2^(lse_i - lse) of the parts of a row -> s_w (whole warp); returns the base-2 LSE of the row.  A NaN among the parts gives NaN
 // outputs and, for requests that the schedule splits, +inf.  keep_nan: what one CTA gives for the whole row, NaN; for rows that the
-// schedule, or the caller, knows as whole.
+// schedule, or the caller, knows as whole.  Each part's LSE is read once by rows of up to 32 parts: the lane keeps it.
 template <class LseAt>
 __device__ __forceinline__ float combine_weights(int nparts, LseAt lse_at, float* s_w, bool keep_nan = false) {
   const int lane = threadIdx.x & 31;
-  float mx = neg_inf();
+  const float own = lane < nparts ? lse_at(lane) : neg_inf();
+  float mx = own;
 #pragma unroll 1
-  for (int i = lane; i < nparts; i += 32) mx = fmaxf(mx, lse_at(i));
+  for (int i = lane + 32; i < nparts; i += 32) mx = fmaxf(mx, lse_at(i));
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
   if (mx == neg_inf()) mx = 0.f;
-  float sum = 0.f;
+  float sum = lane < nparts ? exp2f(own - mx) : 0.f;
 #pragma unroll 1
-  for (int i = lane; i < nparts; i += 32) sum += exp2f(lse_at(i) - mx);
+  for (int i = lane + 32; i < nparts; i += 32) sum += exp2f(lse_at(i) - mx);
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
   const float glse = (sum == 0.f || (sum != sum && !keep_nan)) ? pos_inf() : log2f(sum) + mx;
+  if (lane < nparts) s_w[lane] = exp2f(own - glse);
 #pragma unroll 1
-  for (int i = lane; i < nparts; i += 32) s_w[i] = exp2f(lse_at(i) - glse);
+  for (int i = lane + 32; i < nparts; i += 32) s_w[i] = exp2f(lse_at(i) - glse);
   __syncwarp();
   return glse;
 }
 
 // Weighted sum of the parts share, share + SHARES, .. over column groups [first, first + NG) of 128 columns (lane = 4 columns of a
 // group), in the order of the parts; with several shares each has the CTA's warps 4 share .. 4 share + 3, and those of share 0 add up
-// what the others leave in s_acc.  A part with weight 0 is not read: 0 * (Inf or NaN) must not reach the sum.
-// The loads of 4 / NG parts are in flight at a time: four 16-byte loads per lane.  With four parts of four groups each the merge
-// needed 98 registers, too many to wait beside an attention CTA, and 1024 of its CTAs (64 requests x 128 heads) took three
-// and a half waves.
+// what the others leave in s_acc.  weights() fills s_w; the first loads are in flight meanwhile.  A part with weight 0 is left out of
+// the sum (0 * (Inf or NaN) must not reach it) and, past the first loads, not read.
+// What bounds a merge of few rows is its chain of round trips to L2 (about 0.6 us each): the schedule, the LSEs, then PARTS parts at
+// a time.  With the schedule read ahead of the wait, the first parts asked for together with the LSEs and these read once, a decode
+// with a merge takes 0.7 to 2 us less: 64 heads, 4 x 400 tokens 18.9 -> 17.7 us, 128 heads, 4 x 500 17.2 -> 15.7.
+// PARTS is what keeps four 16-byte loads per lane in flight, and more where that leaves all CTAs resident (launch_decode_combine).  With
+// four parts of four groups each the merge needed 98 registers, too many to wait beside an attention CTA, and 1024 of its CTAs
+// (64 requests x 128 heads) took three and a half waves.
 // COHERENT: the partial outputs may have been written by another GPU while this kernel was already resident (peer
 // merge), so they are read with ld.global.cv.  Otherwise plain loads: the merge of a decode call is resident, waiting in
 // pdl_wait(), while the attention kernel writes the partials, and the non-coherent path (__ldg) is undefined for memory
 // modified during the kernel's lifetime.
-template <int NG, bool COHERENT, int SHARES = 1, class OAt>
-__device__ __forceinline__ void combine_columns(int nparts, OAt o_at, const float* s_w, __nv_bfloat16* out_row, int first, bool f16, int share = 0,
-                                                float4 (*s_acc)[4][32] = nullptr) {
-  constexpr int kPartsInFlight = 4 / NG;
+template <int NG, bool COHERENT, int SHARES = 1, int PARTS = 4 / NG, class OAt, class Weights>
+__device__ __forceinline__ void combine_columns(int nparts, OAt o_at, const float* s_w, Weights weights, __nv_bfloat16* out_row, int first, bool f16,
+                                                int share = 0, float4 (*s_acc)[4][32] = nullptr) {
   const int lane = threadIdx.x & 31;
-  float4 acc[NG];
+  float4 acc[NG], v[PARTS][NG];
+  float w[PARTS];
 #pragma unroll
   for (int j = 0; j < NG; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-  for (int i0 = share; i0 < nparts; i0 += kPartsInFlight * SHARES) {
-    float4 v[kPartsInFlight][NG];
-    float w[kPartsInFlight];
+  const auto load = [&](int i, float4 (&to)[NG]) {
+    const float4* src = reinterpret_cast<const float4*>(o_at(i)) + first * 32 + lane;
 #pragma unroll
-    for (int u = 0; u < kPartsInFlight; ++u) {
-      const int i = i0 + u * SHARES;
-      w[u] = i < nparts ? s_w[i] : 0.f;
-      if (w[u] == 0.f) continue;
-      const float4* src = reinterpret_cast<const float4*>(o_at(i)) + first * 32 + lane;
+    for (int j = 0; j < NG; ++j) to[j] = COHERENT ? __ldcv(src + j * 32) : src[j * 32];
+  };
+  const auto add = [&] {
 #pragma unroll
-      for (int j = 0; j < NG; ++j) v[u][j] = COHERENT ? __ldcv(src + j * 32) : src[j * 32];
-    }
-#pragma unroll
-    for (int u = 0; u < kPartsInFlight; ++u) {
+    for (int u = 0; u < PARTS; ++u) {
       if (w[u] == 0.f) continue;
 #pragma unroll
       for (int j = 0; j < NG; ++j) {
@@ -84,6 +83,23 @@ __device__ __forceinline__ void combine_columns(int nparts, OAt o_at, const floa
         acc[j].w += w[u] * v[u][j].w;
       }
     }
+  };
+#pragma unroll
+  for (int u = 0; u < PARTS; ++u)
+    if (share + u * SHARES < nparts) load(share + u * SHARES, v[u]);
+  weights();
+#pragma unroll
+  for (int u = 0; u < PARTS; ++u) w[u] = share + u * SHARES < nparts ? s_w[share + u * SHARES] : 0.f;
+  add();
+#pragma unroll 1
+  for (int i0 = share + PARTS * SHARES; i0 < nparts; i0 += PARTS * SHARES) {
+#pragma unroll
+    for (int u = 0; u < PARTS; ++u) {
+      const int i = i0 + u * SHARES;
+      w[u] = i < nparts ? s_w[i] : 0.f;
+      if (w[u] != 0.f) load(i, v[u]);
+    }
+    add();
   }
   if constexpr (SHARES > 1) {
     static_assert(NG == 1, "one column group per warp");
@@ -111,9 +127,11 @@ __device__ __forceinline__ void combine_columns(int nparts, OAt o_at, const floa
 template <bool COHERENT = false, class LseAt, class OAt>
 __device__ __forceinline__ void combine_row(int nparts, LseAt lse_at, OAt o_at, float* s_w, __nv_bfloat16* out_row,
                                             float* lse_out) {
-  const float glse = combine_weights(nparts, lse_at, s_w);
-  if ((threadIdx.x & 31) == 0) *lse_out = glse * kLn2;
-  combine_columns<4, COHERENT>(nparts, o_at, s_w, out_row, 0, false);
+  const auto weights = [&] {
+    const float glse = combine_weights(nparts, lse_at, s_w);
+    if ((threadIdx.x & 31) == 0) *lse_out = glse * kLn2;
+  };
+  combine_columns<4, COHERENT>(nparts, o_at, s_w, weights, out_row, 0, false);
 }
 
 // grid (b, ceil(h_k*q_seq_per_hk / rows per CTA)); requests with a single part were written
@@ -121,10 +139,12 @@ __device__ __forceinline__ void combine_row(int nparts, LseAt lse_at, OAt o_at, 
 // WPR warps per row, each for 4 / WPR of the row's four 128-column groups; with more than four, a CTA takes one row and every four
 // warps a share of its parts.
 constexpr int combine_warps(int wpr) { return wpr > kCombineWarps ? wpr : kCombineWarps; }
-template <int WPR, bool SHARED>
+// PARTS: parts in flight per warp where a row has several shares.
+template <int WPR, bool SHARED, int PARTS>
 __global__ void __launch_bounds__(combine_warps(WPR) * 32) decode_combine_kernel(const __grid_constant__ DecodeKernelParams p) {
   extern __shared__ float s_weights[];  // [8][num_sm_parts]
-  pdl_wait();                           // launched as a programmatic dependent of the attention kernel: plain loads from here on
+  // The schedule is read before the wait for the attention kernel: each of its CTAs waits for the kernels in front of it before it
+  // lets this one start, so whoever writes the schedule has completed.  Plain loads all the same (mla_work.cuh).
   const int batch = blockIdx.x;
   int lo = p.num_splits[batch], hi = p.num_splits[batch + 1];
   const bool whole = hi - lo == 1;      // in the schedule
@@ -149,10 +169,13 @@ __global__ void __launch_bounds__(combine_warps(WPR) * 32) decode_combine_kernel
   const float* o_base = p.o_accum + ((int64_t)lo * rows + r) * 512;
   const int64_t part_stride = rows;
   float* w = s_weights + warp * p.num_sm_parts;
-  const float glse = combine_weights(nparts, [&](int i) { return lse_base[i * part_stride]; }, w, SHARED && whole);
-  if (sub == 0 && (threadIdx.x & 31) == 0) p.softmax_lse[((int64_t)batch * p.h_q + head) * p.s_q + sq] = glse * kLn2;
-  combine_columns<4 / kGroups, false, kShares>(
-      nparts, [&](int i) { return o_base + i * part_stride * 512; }, w,
+  const auto weights = [&] {
+    const float glse = combine_weights(nparts, [&](int i) { return lse_base[i * part_stride]; }, w, SHARED && whole);
+    if (sub == 0 && (threadIdx.x & 31) == 0) p.softmax_lse[((int64_t)batch * p.h_q + head) * p.s_q + sq] = glse * kLn2;
+  };
+  pdl_wait();                           // launched as a programmatic dependent of the attention kernel: plain loads of what it leaves
+  combine_columns<4 / kGroups, false, kShares, PARTS>(
+      nparts, [&](int i) { return o_base + i * part_stride * 512; }, w, weights,
       reinterpret_cast<__nv_bfloat16*>(p.out) + batch * p.o_stride_b + sq * p.o_stride_s + head * p.o_stride_h, sub % kGroups * (4 / kGroups),
       p.is_f16 != 0, sub / kGroups, s_acc);
 }
@@ -167,19 +190,21 @@ __global__ void __launch_bounds__(kCombineWarps * 32) sparse_prefill_combine_ker
   const int64_t first = (int64_t)blockIdx.x * p.per * p.h_q + head;
   pdl_wait();                           // launched as a programmatic dependent of the attention kernel: plain loads from here on
   float* w = s_weights + warp * p.per;
-  const float glse = combine_weights(p.per, [&](int i) { return p.lse_accum[first + (int64_t)i * p.h_q]; }, w, true);
   const int64_t out_row = (int64_t)(p.whole + blockIdx.x) * p.h_q + head;
-  if (sub == 0) {
-    float mx = neg_inf();
-    for (int i = lane; i < p.per; i += 32) mx = fmaxf(mx, p.max_accum[first + (int64_t)i * p.h_q]);
+  const auto weights = [&] {
+    const float glse = combine_weights(p.per, [&](int i) { return p.lse_accum[first + (int64_t)i * p.h_q]; }, w, true);
+    if (sub == 0) {
+      float mx = neg_inf();
+      for (int i = lane; i < p.per; i += 32) mx = fmaxf(mx, p.max_accum[first + (int64_t)i * p.h_q]);
 #pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    if (lane == 0) {
-      p.max_logits[out_row] = mx;
-      p.lse[out_row] = glse == pos_inf() ? neg_inf() : glse;
+      for (int off = 16; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      if (lane == 0) {
+        p.max_logits[out_row] = mx;
+        p.lse[out_row] = glse == pos_inf() ? neg_inf() : glse;
+      }
     }
-  }
-  combine_columns<4 / WPR, false>(p.per, [&](int i) { return p.o_accum + (first + (int64_t)i * p.h_q) * 512; }, w,
+  };
+  combine_columns<4 / WPR, false>(p.per, [&](int i) { return p.o_accum + (first + (int64_t)i * p.h_q) * 512; }, w, weights,
                                   reinterpret_cast<__nv_bfloat16*>(p.out) + out_row * 512, sub * (4 / WPR), false);
 }
 
@@ -346,12 +371,12 @@ cudaError_t read_merge_status(int* host_status, bool reset) {
   return e;
 }
 
-template <int WPR, bool SHARED>
+template <int WPR, bool SHARED, int PARTS = WPR < 4 ? 1 : 4>
 static cudaError_t launch_decode_combine_wpr(const DecodeKernelParams& p, int rows, cudaStream_t stream) {
   constexpr int kWarps = combine_warps(WPR), kRows = kWarps / WPR;
   const size_t smem = sizeof(float) * kWarps * p.num_sm_parts;
-  if (cudaError_t e = allow_dynamic_smem(decode_combine_kernel<WPR, SHARED>, smem); e != cudaSuccess) return e;
-  return launch_dependent(decode_combine_kernel<WPR, SHARED>, dim3(p.b, (rows + kRows - 1) / kRows), kWarps * 32, smem, stream, p);
+  if (cudaError_t e = allow_dynamic_smem(decode_combine_kernel<WPR, SHARED, PARTS>, smem); e != cudaSuccess) return e;
+  return launch_dependent(decode_combine_kernel<WPR, SHARED, PARTS>, dim3(p.b, (rows + kRows - 1) / kRows), kWarps * 32, smem, stream, p);
 }
 
 cudaError_t launch_decode_combine(const DecodeKernelParams& p, cudaStream_t stream) {
@@ -371,8 +396,15 @@ cudaError_t launch_decode_combine(const DecodeKernelParams& p, cudaStream_t stre
   const int64_t all = (int64_t)p.b * rows, room = (int64_t)sms * 64;
   if (!p.sub_split) return all * 4 <= room ? launch_decode_combine_wpr<4, false>(p, rows, stream) : launch_decode_combine_wpr<1, false>(p, rows, stream);
   const bool many = p.num_sm_parts >= 8 * p.b;
-  if (many && all * 32 <= room) return launch_decode_combine_wpr<16, true>(p, rows, stream);
-  if (many && all * 8 <= room) return launch_decode_combine_wpr<8, true>(p, rows, stream);
+  // Parts in flight: the most with which all CTAs are resident, by their registers: eight with one CTA of 16 warps (88 registers) or three of
+  // eight (80) per SM, six with four of eight (62), or four.  Four / six / eight: 64 heads, 1 x 8 000 19.2 / 19.4 / 18.3 us; 16 heads,
+  // 16 x 1 000 (256 CTAs of 16 warps) 12.1 / 12.5 / 14.0; 32 heads, 10 x 800 (320 of eight) 13.6 / 13.6 / 12.7; 64 heads, 9 x 900 (576)
+  // 16.2 / 15.8 / 17.4; sparse, 5 requests of two tokens (640) 15.6 / 16.3 / 17.0.
+  if (many && all * 32 <= room) return all <= sms ? launch_decode_combine_wpr<16, true, 8>(p, rows, stream) : launch_decode_combine_wpr<16, true>(p, rows, stream);
+  if (many && all * 8 <= room) {
+    if (all <= 3 * sms) return launch_decode_combine_wpr<8, true, 8>(p, rows, stream);
+    return all <= 4 * sms ? launch_decode_combine_wpr<8, true, 6>(p, rows, stream) : launch_decode_combine_wpr<8, true>(p, rows, stream);
+  }
   return all * 4 <= room ? launch_decode_combine_wpr<4, true>(p, rows, stream) : launch_decode_combine_wpr<1, true>(p, rows, stream);
 }
 

@@ -288,6 +288,8 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
       for (int wi = 0; wi < n_work && alive; ++wi) {
         const Req r = request(wi);
         if (r.blk_hi == r.blk_lo) continue;
+        const int* bt = SPARSE ? nullptr : p.block_table + (int64_t)r.batch * p.block_table_stride_b;
+        int page_next = SPARSE ? 0 : bt[r.blk_lo];      // on the way while the queries are asked for
         alive = tc::mbar_wait(bar(Q_EMPTY), (req & 1) ^ 1, status, 201);
         if (!alive) break;
         // the box of the map covers all rows of one token (rows past the tensor read as zero); 64-column chunks
@@ -299,8 +301,6 @@ mla_few_rows_kernel(const __grid_constant__ FewParams P, const __grid_constant__
             tc::tma_load_4d(sbase + L::Q_OFF + c * L::kQChunk + t * hq * 128, &tmap_q, c * 64, head0, sq0 + t, r.batch, bar(Q_FULL));
         ++req;
         if constexpr (SPARSE) continue;
-        const int* bt = p.block_table + (int64_t)r.batch * p.block_table_stride_b;
-        int page_next = bt[r.blk_lo];
         const bool ahead = r.blk_hi - r.blk_lo >= kPrefetchBlocks && p.k_stride_row == 576;
         const char* kv_head = reinterpret_cast<const char*>(p.kcache) + kh * p.k_stride_head * 2;
         for (int blk = r.blk_lo; blk < r.blk_hi && alive; ++blk, ++g) {
