@@ -394,7 +394,7 @@ mla_tile64_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CU
     const int r_row = tid & 63, th = tid >> 6;           // TMEM lane tid: row tid%64, token/column half tid/64
     const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
     int g = 0, req = 0;
-    Ring at = {0, 0u}, before = {0, 0u}, before2 = {0, 0u};      // first stage of this block; second stages of the two before
+    Ring at = {0, 0u}, before = {0, 0u};      // first stage of this block; second stage of the one before
     bool aborted = false;        // uniform over the 128 softmax threads: only read right after a bar_sync
     for (int wi = 0; wi < tile.n_work; ++wi) {
       const Work r = get_work<MODE>(P, tile, wi);
@@ -501,8 +501,8 @@ mla_tile64_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CU
         sum[0] = f2_add(sum[0], sum[1]);
         l_part += sum[0].lo + sum[0].hi;
         if (stop) { aborted = true; break; }
-        // P has two buffers: P V of the block before the last one is complete
-        if (g >= 2 && !tc::mbar_wait(bar(EMPTY0 + before2.st), before2.ph, status, 9)) *sAbort = 1;
+        // P has two buffers.  P V of block g - 2 was issued before the last products of S of block g, whose commit tells of both: it is
+        // complete.  (Its stages do not tell: where a request has one block, Q of the next but one has passed through them since.)
         if (tid == 0) FMLA_TRACE_AT(g, 9);
         // P[row][th*32 .. +32) -> K-major 128B-swizzled A operand: 16-byte chunk (th*4 + q) ^ (row & 7)
 #pragma unroll
@@ -514,7 +514,6 @@ mla_tile64_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CU
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(bar(P_FULL0 + st));
         if (tid == 0) FMLA_TRACE_AT(g, 11);
-        before2 = before;
         before = at;
         before.step(1);
         at.step(2);
