@@ -69,6 +69,10 @@ cudaError_t launch_decode_sparse_tc(const DecodeKernelParams& p, cudaStream_t st
 // over (four parts of two blocks, taken) 37.0 -> 34.5; 38, 44, 50, 62 and 74 (three and two parts, refused) 37.0 -> 36.8, 36.8 -> 37.0, 36.8 ->
 // 36.9, 37.0 -> 36.9, 37.4 -> 37.7; two rounds in front 37: 53.7 -> 53.2, 50: 53.3 -> 54.9.  Top-k 1024, 38 to 74 (taken) 65.8 -> 56.4 to 59.6.  128 heads, top-k
 // 1024, 74 in front, 18 (refused) 50.7 -> 47.1, 25: 50.9 -> 50.8, 31: 51.0 -> 51.2.
+// With the kernels as they are now a block takes a CTA 1.39 and the merge and its partials some 2 to 3; over 100 shapes of up to one round in
+// front the constants still choose within 0.8 us of the better side, but for pairs with one round in front, where less is lost than
+// assumed (refused: 92 tokens, top-k 1024 47.1 -> 43.5, 111, top-k 1536 64.6 -> 60.4; two rounds 1 to 6 us of it, three all of it).  They stay
+// because they also say which calls need scratch, and a caller of the C entry may bring none where none was needed.
 void plan_sparse_prefill(SparsePrefillKernelParams& sp, int sms, bool can_split) {
   const int cap = std::max(1, sms / (sp.h_q / 64)), nblk = sp.topk / 64;      // pairs for 128 heads, CTAs per 64-head tile otherwise
   sp.units = std::min(sp.s_q, cap);
