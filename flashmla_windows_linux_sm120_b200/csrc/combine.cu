@@ -144,7 +144,9 @@ template <int WPR, bool SHARED, int PARTS>
 __global__ void __launch_bounds__(combine_warps(WPR) * 32) decode_combine_kernel(const __grid_constant__ DecodeKernelParams p) {
   extern __shared__ float s_weights[];  // [8][num_sm_parts]
   // The schedule is read before the wait for the attention kernel: each of its CTAs waits for the kernels in front of it before it
-  // lets this one start, so whoever writes the schedule has completed.  Plain loads all the same (mla_work.cuh).
+  // lets this one start, so whoever writes the schedule has completed.  That its writes are visible here by then is not written
+  // down for a kernel two places behind; it holds because the wait of the attention kernel completes them to L2 and this grid starts later, with
+  // nothing of the schedule in its SMs' L1.  Plain loads all the same (mla_work.cuh).
   const int batch = blockIdx.x;
   int lo = p.num_splits[batch], hi = p.num_splits[batch + 1];
   const bool whole = hi - lo == 1;      // in the schedule
@@ -154,7 +156,6 @@ __global__ void __launch_bounds__(combine_warps(WPR) * 32) decode_combine_kernel
     hi *= k;
   }
   const int nparts = hi - lo;
-  if (nparts <= 1) return;
   const int q_seq_per_hk = p.s_q * p.hq_per_hk;
   const int rows = p.h_k * q_seq_per_hk;
   constexpr int kShares = WPR > 4 ? WPR / 4 : 1, kGroups = WPR > 4 ? 4 : WPR;
@@ -162,7 +163,6 @@ __global__ void __launch_bounds__(combine_warps(WPR) * 32) decode_combine_kernel
   __shared__ float4 s_acc[kShares > 1 ? kShares - 1 : 1][4][32];
   const int warp = threadIdx.x >> 5, sub = warp % WPR;
   const int r = blockIdx.y * (combine_warps(WPR) / WPR) + warp / WPR;
-  if (r >= rows) return;
   const int kh = r / q_seq_per_hk, row = r % q_seq_per_hk;
   const int sq = row / p.hq_per_hk, head = kh * p.hq_per_hk + row % p.hq_per_hk;
   const float* lse_base = p.lse_accum + (int64_t)lo * rows + r;
@@ -173,7 +173,11 @@ __global__ void __launch_bounds__(combine_warps(WPR) * 32) decode_combine_kernel
     const float glse = combine_weights(nparts, [&](int i) { return lse_base[i * part_stride]; }, w, SHARED && whole);
     if (sub == 0 && (threadIdx.x & 31) == 0) p.softmax_lse[((int64_t)batch * p.h_q + head) * p.s_q + sq] = glse * kLn2;
   };
-  pdl_wait();                           // launched as a programmatic dependent of the attention kernel: plain loads of what it leaves
+  // Launched as a programmatic dependent of the attention kernel: plain loads of what it leaves.  Warps without a part to merge wait
+  // too: what follows in the stream, or in a graph, is ordered behind this kernel alone, which must not end before that one, and
+  // where no request is split all of it is without parts.
+  pdl_wait();
+  if (nparts <= 1 || r >= rows) return;
   combine_columns<4 / kGroups, false, kShares, PARTS>(
       nparts, [&](int i) { return o_base + i * part_stride * 512; }, w, weights,
       reinterpret_cast<__nv_bfloat16*>(p.out) + batch * p.o_stride_b + sq * p.o_stride_s + head * p.o_stride_h, sub % kGroups * (4 / kGroups),
