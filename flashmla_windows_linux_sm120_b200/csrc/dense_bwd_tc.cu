@@ -168,7 +168,7 @@ __device__ __forceinline__ void row_exp2(uint32_t (&sv)[N], float scale, MinusLs
   for (int i = 0; i < N / 2; ++i) {
     F2 x = f2_fma(F2{__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])}, f2(scale), minus_lse(i));
     if (i % 16 % 3 == 2) {      // (alike in steps of either length)
-      x = f2_exp2_nan(x);
+      x = f2_exp2(x);
     } else {
       x.lo = exp2f(x.lo);
       x.hi = exp2f(x.hi);

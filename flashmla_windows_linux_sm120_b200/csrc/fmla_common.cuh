@@ -89,12 +89,11 @@ __device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
       : "f"(a.lo), "f"(a.hi), "f"(b.lo), "f"(b.hi));
   return d;
 }
-// 2^x for x <= 2^7 on the multiply-add pipe: x = n + f with n the nearest whole number (held in the low bits of x + 1.5 * 2^23) and
-// |f| <= 1/2, and 2^f = 1 + f q(f) with the polynomial of least largest relative error (fitted with Lawson's weights; 1.6e-7 in
-// fp32 over the range, the special function unit's 2^x is specified to 2.4e-7).  Below -127 the result is 0.
-__device__ __forceinline__ F2 f2_exp2(F2 x) {
-  x.lo = fmaxf(x.lo, -127.f);
-  x.hi = fmaxf(x.hi, -127.f);
+// 2^x for -127 <= x <= 128 on the multiply-add pipe: x = n + f with n the nearest whole number (held in the low bits of x + 1.5 * 2^23)
+// and |f| <= 1/2, and 2^f = 1 + f q(f) with the polynomial of least largest relative error (fitted with Lawson's weights: 1.1e-7, in
+// fp32 1.7e-7 over the range; the special function unit's 2^x is specified to 2.4e-7).  At the ends exactly 0 and infinity; beyond
+// them the sum of the exponents would wrap into the sign.  tests/test_gpu_exp2.py
+__device__ __forceinline__ F2 f2_exp2_inside(F2 x) {
   const F2 t = f2_add(x, f2(12582912.f));
   const F2 n = f2_add(t, f2(-12582912.f));
   const F2 f = f2_fma(n, f2(-1.f), x);
@@ -107,12 +106,21 @@ __device__ __forceinline__ F2 f2_exp2(F2 x) {
   r.hi = __uint_as_float(__float_as_uint(r.hi) + (__float_as_uint(t.hi) << 23));
   return r;
 }
-// the same with NaN for NaN
-__device__ __forceinline__ F2 f2_exp2_nan(F2 x) {
-  const F2 r = f2_exp2(x);
-  asm("max.NaN.f32 %0, %1, 0fC2FE0000;\n" : "=f"(x.lo) : "f"(x.lo));      // -127
-  asm("max.NaN.f32 %0, %1, 0fC2FE0000;\n" : "=f"(x.hi) : "f"(x.hi));
-  return f2_fma(x, f2(0.f), r);
+// 2^x for x <= 128, 0 for NaN
+__device__ __forceinline__ F2 f2_exp2_to_128(F2 x) {
+  x.lo = fmaxf(x.lo, -127.f);
+  x.hi = fmaxf(x.hi, -127.f);
+  return f2_exp2_inside(x);
+}
+// 2^x for every x, NaN for NaN
+__device__ __forceinline__ F2 f2_exp2(F2 x) {
+  const auto inside = [](float v) {
+    asm("{\n.reg .f32 t;\nmax.NaN.f32 t, %0, 0fC2FE0000;\nmin.NaN.f32 %0, t, 0f43000000;\n}\n" : "+f"(v));      // -127, 128
+    return v;
+  };
+  x.lo = inside(x.lo);
+  x.hi = inside(x.hi);
+  return f2_fma(x, f2(0.f), f2_exp2_inside(x));
 }
 // the largest of three (NaN only if all are)
 __device__ __forceinline__ float max3(float a, float b, float c) {
