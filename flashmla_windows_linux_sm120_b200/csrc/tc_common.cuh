@@ -135,11 +135,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* tmap, int 
                "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
                : "memory");
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, int c0, int c1, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
-               "l"(tmap), "r"(c0), "r"(c1), "r"(bar)
-               : "memory");
-}
 
 // ---- tcgen05 ----------------------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_result_addr, uint32_t ncols) {
@@ -216,7 +211,8 @@ __device__ __forceinline__ void mma_ws_ss(uint32_t tmem_d, uint64_t da, uint64_t
 // One thread of the leader CTA (cluster rank 0) issues MMAs that run on the tensor cores of both SMs: M = 128
 // means 64 accumulator rows per CTA, the A operand comes from each CTA's own shared memory and the B operand
 // is split along N (first half from the leader's shared memory, second half from its peer's), at the same
-// shared-memory offsets in both CTAs.  Every commit or copy names one barrier of one CTA (nothing is broadcast to several CTAs).
+// shared-memory offsets in both CTAs.  A load fills the shared memory of one CTA and completes on a barrier there; a commit arrives in
+// both CTAs.
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
@@ -238,19 +234,7 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_bar) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t cluster_bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], %1;\n" ::"r"(cluster_bar), "r"(bytes) : "memory");
-}
 // wait on a barrier of this CTA whose arrivals come from both CTAs
-__device__ __forceinline__ bool mbar_test_wait_cluster(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -269,14 +253,6 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
   }
   return ok;
 }
-// 4-D tile load into this CTA's shared memory whose completion is counted on a barrier that may live in the
-// other CTA of the pair (given as a shared::cluster address)
-__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const void* tmap, int c0, int c1, int c2, int c3, uint32_t cluster_bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(dst),
-      "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(cluster_bar)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_result_addr, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_result_addr), "r"(ncols) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
@@ -284,11 +260,7 @@ __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_result_addr, uint3
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// arrive on ONE barrier (shared::cluster address: this CTA's or the peer's) once every MMA issued so far has completed
-__device__ __forceinline__ void tc_commit_pair(uint32_t cluster_bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(cluster_bar) : "memory");
-}
-// the same for one barrier of both CTAs, at the same shared-memory offset
+// arrive on the barrier at this shared-memory offset in both CTAs once every MMA issued so far has completed
 __device__ __forceinline__ void tc_commit_pair_both(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(bar),
                "h"(static_cast<uint16_t>(3))
