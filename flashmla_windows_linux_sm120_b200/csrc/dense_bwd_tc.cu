@@ -26,8 +26,9 @@
 // The GEMMs are issued by single threads (waits, votes and branches of whole warps left the tensor pipe idle), the element-wise
 // warps clear what lies past the end of a sequence, and the second GEMM on the wide tile goes chunk by chunk of its columns, each
 // followed by the load of that chunk for the step after next: with one release for the whole tile the next loads came 500 clk late at
-// 192/128.  A step of dK/dV at 192/128 took 3 900 clk and takes 3 480; the element-wise warps (1 300 clk for P, 650 for dS) now set the
-// pace.  Sixteen of them, with half the columns each, were no faster.  4 x 1 000 tokens, 8 heads, 192/128, causal (steps of 64) 72.0 ->
+// 192/128.  A step of dK/dV took 4 130 clk at 192/128 and 3 810 at 128/128 and takes 3 220 and 2 935, one of dQ 3 240 and 2 900, now 2 715 and 2 420
+// (two sequences of 4 096, 32 heads, no mask, one time stamp per step); the element-wise warps (with trace points 1 300 clk for P, 650 for dS)
+// now set the pace of dK/dV.  Sixteen of them, with half the columns each, were no faster.  4 x 1 000 tokens, 8 heads, 192/128, causal (steps of 64) 72.0 ->
 // 64.2 us, 6 x 1 000, 8 heads, 128/128, no mask 121.8 -> 109.4, 2 x 4 096, 32 heads, no mask 1 916 -> 1 863.
 // Every mbarrier wait is bounded (tc_common.cuh); a pipeline fault sets a status word and lets the
 // CTA drain and free its tensor memory.
@@ -793,9 +794,11 @@ static cudaError_t launch_bwd_tc(const DenseKernelParams& p, cudaStream_t stream
 cudaError_t launch_dense_bwd_tc(const DenseKernelParams& p, cudaStream_t stream) {
   // Steps of 64 rows for short sequences: the last step of 128 works for up to 127 rows in vain, and with a causal mask tiles walk half of
   // a sequence.  By the mean length, which is what the host has; steps of 64 -> steps of 128, at this length and a multiple of a step or
-  // half of one beyond it.  Causal, 16 heads, 192/128: 64 tokens 50.9 -> 62.1 us, 320 50.4 -> 57.8, 704 62.2 -> 69.1, 1088 79.7 -> 84.1, 1344 60.2 ->
-  // 61.5, 1500 71.8 -> 70.6, 2000 112.7 -> 106.6; 64 heads, 128/128: 320 170 -> 185, 704 204 -> 211, 1088 258 -> 255, 1500 222 -> 209.  Without a mask, 64
-  // heads, 128/128: 64 tokens 186 -> 214, 320 209 -> 213, 384 207 -> 193, 512 216 -> 195; 192/128: 320 233 -> 241, 384 233 -> 219, 512 240 -> 220.
+  // half of one beyond it, some 2 400 tokens in all.  Causal, 16 heads, 192/128: 64 tokens 49.4 -> 59.7 us, 320 47.7 -> 51.6, 512 47.8 -> 46.8, 704
+  // 57.8 -> 60.1, 1088 72.7 -> 73.1, 1216 48.4 -> 46.4, 1500 63.9 -> 61.5, 2000 99.1 -> 92.0; 64 heads, 128/128: 320 163 -> 172, 512 157 -> 150, 704 190 -> 193,
+  // 1088 240 -> 236, 1500 201 -> 193.  Without a mask, 64 heads, 128/128: 64 tokens 179 -> 207, 320 185 -> 195, 384 185 -> 180, 448 215 -> 222, 512 193 -> 183;
+  // 192/128: 320 212 -> 226, 384 216 -> 208, 448 255 -> 256, 512 226 -> 219.  Up to the lines steps of 64 win more on the odd halves of a step than
+  // they lose on whole ones.
   const int64_t mean = (static_cast<int64_t>(p.total_q) + p.total_k) / (2 * static_cast<int64_t>(p.batch));
   const bool short_sequences = mean <= (p.is_causal ? 1088 : 352);
   if (p.d_qk == 192) return short_sequences ? launch_bwd_tc<192, true>(p, stream) : launch_bwd_tc<192, false>(p, stream);

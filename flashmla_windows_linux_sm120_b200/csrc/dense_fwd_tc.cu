@@ -15,9 +15,10 @@
 //   warp 10    in large grids: takes over CTAs that have not been started (clusterlaunchcontrol), one after the other
 // What bounds it: a tile's chain S -> softmax -> P V -> S (P lies over S, and tensor memory has no room for a second S), of
 // which the tensor pipe can hide the part that is as long as the other tile's two GEMMs (1280 clk at 192/128, 1024 at
-// 128/128), and in long runs the power limit.  A block of a CTA (two tiles) took 3 980 clk at 192/128 and 3 760 at 128/128 with two
-// threads per row, single V stages at 192/128 (700 clk waiting for V) and issue and waits by a whole warp; it takes some 3 300 and 2 900
-// now, at a clock that the power limit lowers from 1.66 to 1.52 GHz.  What shortened it: one ring for K and V; the maximum first,
+// 128/128), and in long runs the power limit.  A block of a CTA (two tiles) took 4 240 clk at 192/128 and 3 850 at 128/128 with two
+// threads per row, single V stages at 192/128 (700 clk waiting for V) and issue and waits by a whole warp; it takes 3 295 and 3 220
+// now (two sequences of 4 096, no mask, one time stamp per block; 3 890 -> 3 235 and 3 560 -> 3 055 with 2 000), at a clock that falls from 1.84 to
+// 1.65 GHz at 128/128 in a burst of four calls and from 1.60 to 1.44 in a loop.  What shortened it: one ring for K and V; the maximum first,
 // so that a warp decides alone whether the scale moves and P can be handed over in halves; part of the exponentials off the special
 // function unit; and little code: the warps of both tiles and the issuing thread share an instruction cache, and the block's body
 // rolled up to 64 logits, with masked blocks rewritten in place first, is 6 % faster than unrolled to 128.
@@ -591,9 +592,9 @@ static cudaError_t launch_fwd_tc(DenseKernelParams p, const CUtensorMap& tq, con
   // longest leave CTAs without rows, which count for nothing here: no more than (total_q / 256 + batch) per head have some.  Device
   // time in a graph, plain -> taking over: 80 CTAs (4 sequences of 500 tokens, 10 heads, 192/128) 13.5 -> 13.9 us, 144 (18 heads) 14.3 -> 14.6, 160
   // (4 of 200, 40 heads) 18.5 -> 16.5, 256 (32 heads) 24.3 -> 21.0, 512 (8 of 512, 32 heads, 128/128) 47.6 -> 37.6, 2048 (64 of 64) 81.6 -> 47.7;
-  // 480 of which 208 have rows (1500, 700, 300, 100 and 20 tokens, 16 heads, 192/128) 28.8 -> 29.4.  The line lies at 1.9 CTAs per SM, where it
-  // lay when the plain form's blocks took longer and taking over fewer cost up to 8 % (tests/test_gpu_dense_form.py holds it there).
-  // At 192/128 the same holds for tiles of more than 2048 keys: they cost 2 to 3 % once, and would gain 1 to 5 % now (4 of 8192 tokens, 16 heads,
+  // 480 of which 208 have rows (1500, 700, 300, 100 and 20 tokens, 16 heads, 192/128) 28.8 -> 29.4.  So the line, 1.9 CTAs per SM, lies too high
+  // for the present kernel: it was drawn for one that lost up to 8 % below it, and has not been moved since.
+  // Neither has that of 2048 keys at 192/128: longer tiles lost 2 to 3 % once, and would gain 1 to 7 % now (4 of 8192 tokens, 16 heads,
   // causal 1268 -> 1217 us, 8 of 4096 696 -> 648, no mask 1196 -> 1165).
   int dev = 0, sms = 0;
   if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;

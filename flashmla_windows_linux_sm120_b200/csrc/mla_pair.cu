@@ -246,7 +246,7 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
     // The CTA's 32 token rows of a block (32 x 1152 bytes) are gathered with 16-byte cp.async copies by four warps (4, 8 .. 10), eight
     // rows each, three copies a row.  What bounds a gather is the instructions in front of each copy: a deal of the 72 warp
     // instructions of a block over three warps, piece by piece, cost some 30 instructions a copy (a division, a shuffle and a 64-bit
-    // product) and 1 980 clk a block; by rows the addresses follow from one product a row (74 tokens, top-k 512, 18.1 -> 16.7 us, 4096 of
+    // product); by rows the addresses follow from one product a row (74 tokens, top-k 512, 18.1 -> 16.7 us, 4096 of
     // top-k 2048, which run at the power limit, 2 575 -> 2 558).  The TMA engine (tile::gather4, 4 rows x 64
     // columns per copy) gathers no faster than ~11 bytes per clock and SM (cp.async alone: up to 67), and mixing the two paths was slower
     // than either, because the gathers queue behind the forwarding copies in the TMA engine.  Each lane's copies arrive on the
@@ -676,12 +676,13 @@ mla_pair_kernel(const __grid_constant__ TcParams P, const __grid_constant__ CUte
   } else if (warp == 5) {
     // ================================ MMA issuer (leader only) =========================
     // One thread, in a fixed order: S of a block, P V of the block before.  A warp that polled the five barriers of interest, and
-    // issued what was ready first, was the longest link of the chain: from the end of one issue to the next some 850 clk, twice a block, with
-    // everything there (votes, taken branches and eight commits a block, now three that go to both CTAs), 2 460 clk a block of the
-    // dense decode with two tokens against 1 700, 2 900 against 2 050 of the sparse prefill, 3 150 against 2 350 of the sparse decode.
-    // Where the power limit holds (long dense decodes, long prefills) the clock takes most of it back: 128 x 4000 tokens 175.7 ->
-    // 174.1 us, two tokens 313.0 -> 309.2, prefill of 4096 tokens 2 648 -> 2 575; elsewhere it shows: 16 x 2000 tokens 27.5 -> 26.2,
-    // 20 prefill tokens 24.5 -> 23.3, sparse decode of 30 x 512 28.7 -> 27.8.
+    // issued what was ready first, was the longest link of the chain (votes, taken branches and eight commits a block, now three that go to
+    // both CTAs).  Clocks a block, with one time stamp per block (a build with all trace points holds the polling warp up: 2 555 against
+    // 1 770 on 128 x 4000): dense decode of 128 x 4000 tokens 1 730 -> 1 595, two tokens 1 770 -> 1 620, prefill of 4096 tokens 2 330 -> 2 195,
+    // sparse decode of 64 x 2048 2 320 -> 2 200.  In dense decodes the clock takes most of it back: inside the kernel (clock64
+    // over globaltimer) it goes from 1.54 to 1.45 GHz in a burst of 26 calls and from 1.27 to 1.21 in a loop, with 1.96 before and after.
+    // 128 x 4000 tokens 175.7 -> 174.1 us, two tokens 313.0 -> 309.2 (within the spread over boxes), prefill of 4096 tokens 2 648 -> 2 575, 16 x 2000
+    // tokens 27.5 -> 26.2, 20 prefill tokens 24.5 -> 23.3, sparse decode of 30 x 512 28.7 -> 27.8.
     if (tc::elect_one()) {
       constexpr uint32_t idesc_s = tc::idesc_bf16_f32(128, 64, 0, 0, F16);
       constexpr uint32_t idesc_o = tc::idesc_bf16_f32(128, 256, 0, 1, F16);

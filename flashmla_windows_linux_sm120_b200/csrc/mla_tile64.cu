@@ -18,9 +18,9 @@
 // of their own.  That there is room for two and a half blocks beside the P buffers is due to Q: its chunks 0..5 live in the 192
 // columns of tensor memory that O and S leave idle, and pass through two stages on their way there.  S starts on the first half while
 // the second is gathered, and P V releases half by half.
-// What bounds it: the chain of a block (gather 1 500 to 2 000 clk, of which 1 150 are the 64 bytes a clock that an SM takes from L2; S
-// 1 050; softmax 1 500; P V 650) over two and a half blocks in flight: some 2 900 clk a block, against 1 700 of tensor pipe.  With two whole
-// pages as stages it was 3 300 (3 600 with a polling issuer).  333 tokens, top-k 512 51.3 -> 45.3 us, 4096, top-k 2048 1 765 -> 1 456; dense,
+// What bounds it: the chain of a block (with trace points: gather 1 500 to 2 000 clk, of which 1 150 are the 64 bytes a clock that an SM
+// takes from L2; S 1 050; softmax 1 500; P V 650) over two and a half blocks in flight: 2 560 clk a block (148 tokens, top-k 2048, one time
+// stamp per block), against 1 700 of tensor pipe.  With two whole pages as stages and a polling issuer it was 3 300.  333 tokens, top-k 512 51.3 -> 45.3 us, 4096, top-k 2048 1 765 -> 1 456; dense,
 // 64 heads x 3 tokens, 16 x 3 000 53.8 -> 45.4; a call of one or two blocks is up to 0.4 us slower than with whole pages (one token, top-k
 // 128, 8.9 -> 9.3), for the copy of Q.
 // The transposed products of mla_few_rows.cu were measured slower in the prefill (333 query tokens, top-k 512: 105 us against 64 us then).
@@ -620,10 +620,11 @@ static cudaError_t launch_dense_tile64(const TcParams& P, const CUtensorMap& tq,
   return launch_dependent(kern, grid, dtc::threads(kDense), dtc::SMEM_BYTES, stream, P, tq, tkv);
 }
 
-// Several 64-row tiles read the same pages (and the pair does not apply, mla_dispatch.cu).  Against mla_few_rows.cu, device time with
-// the whole-page stages of before: 64 heads x 3 tokens, 16 requests of 16 000 tokens 188 -> 158 us, 64 of 4 000 179 -> 153, 128 of 1 000 115 -> 102, 16 of 1 000
-// 34.6 -> 35.5, one of 1 000 21.6 -> 23.3; 96 and 192 heads, one and two tokens, alike.  The lengths are on the device, so the
-// line is drawn for the larger calls.
+// Several 64-row tiles read the same pages (and the pair does not apply, mla_dispatch.cu).  Device time, mla_few_rows.cu -> this kernel:
+// 64 heads x 3 tokens, 16 requests of 16 000 tokens 163 -> 135 us, 64 of 4 000 160 -> 138, 128 of 1 000 103 -> 90, 16 of 1 000 31.3 -> 30.7, 4 of 500
+// 22.0 -> 21.3; 96 heads, 16 of 3 000 38.9 -> 35.2, two tokens 50.6 -> 45.0; 192 heads, 16 of 3 000 51.6 -> 44.3.  The other way where that
+// kernel shares the rows of the schedule (one request of 1 000 14.3 -> 19.6, 96 heads, 4 of 500 14.6 -> 18.9).  The lengths are on the
+// device, so the line is drawn for the larger calls.
 bool decode_dense_tile64_applies(const DecodeKernelParams& p) { return p.hq_per_hk >= 64 && p.s_q * ((p.hq_per_hk + 63) / 64) > 1; }
 
 cudaError_t launch_decode_dense_tile64(const DecodeKernelParams& p, cudaStream_t stream) {
